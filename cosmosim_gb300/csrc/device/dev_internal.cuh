@@ -38,7 +38,7 @@ struct __align__(16) NodeW32 {
     int next;
     int body;
     float s;                // 2 * half_size
-    float pad;
+    int first;              // first sorted position below it (imported leaves: the body's, or -1)
 };
 
 // FP32 neighbour-search record: the cell cube, and for a leaf its body

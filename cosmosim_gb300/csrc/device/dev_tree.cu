@@ -614,7 +614,7 @@ __device__ __forceinline__ void write_cell(csgd_t dd, DevScalars *sc, double hs0
     *(int2 *)&w.next = make_int2(next, body);
     NodeW32 &v = dd.w32[id];
     v.s2 = (float)s2;
-    *(int4 *)&v.next = make_int4(next, body, __float_as_int((float)s), 0);
+    *(int4 *)&v.next = make_int4(next, body, __float_as_int((float)s), first);
     dd.link[id] = NodeLink{parent, L, first, count};
     int4 *c = (int4 *)(dd.child + 8 * (size_t)id);
     c[0] = make_int4(-1, -1, -1, -1);
@@ -1189,9 +1189,20 @@ __global__ void k_imp_sizes(csgd_t dd, DevScalars *sc, int nn, const int *__rest
     }
 }
 
+// Sorted position of every alive body (-1 for the others).
+__global__ void k_imp_pos(const DevScalars *sc, int n, const int *__restrict__ perm,
+                          const double *__restrict__ m, int *__restrict__ pos_of)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < n && m[p] <= 0.0)
+        pos_of[p] = -1;
+    if (p < sc->n_alive)
+        pos_of[perm[p]] = p;
+}
+
 __global__ void k_imp_write(csgd_t dd, DevScalars *sc, int nn, int root,
                             const int *__restrict__ par, const int *__restrict__ slot,
-                            const int *__restrict__ size)
+                            const int *__restrict__ size, const int *__restrict__ pos_of)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nn || sc->err != 0)
@@ -1244,11 +1255,16 @@ __global__ void k_imp_write(csgd_t dd, DevScalars *sc, int nn, int root,
     v.body = w.body;
     v.s2 = (float)w.s2;
     v.s = (float)s;
-    v.pad = 0.0f;
+    v.first = (w.body >= 0 && w.body < dd.n) ? pos_of[w.body] : -1;
     dd.w32[id] = v;
     dd.geo[id] = make_double4_32a(o.center_x, o.center_y, o.center_z, o.half_size);
     write_s32(dd, id, o.center_x, o.center_y, o.center_z, o.half_size, w.body, w.next);
     dd.link[id] = NodeLink{-1, depth, -1, 0};
+    for (int q = 0, c = id + 1; q < 8; q++) { // the walks' child table
+        const int oc = o.children[q];
+        dd.child[8 * (size_t)id + q] = oc >= 0 ? c : -1;
+        c += oc >= 0 ? size[oc] : 0;
+    }
 }
 
 } // namespace
@@ -1472,7 +1488,10 @@ extern "C" int csgd_import_pool(csgd_t *d, const OctreeNode *pool, int n_nodes, 
     const int g = csgd_grid(n_nodes, B);
     { k_imp_links<<<g, B, 0, s>>>(*d, sc, n_nodes, root, par, slot); d->launches++; }
     { k_imp_sizes<<<g, B, 0, s>>>(*d, sc, n_nodes, par, size); d->launches++; }
-    { k_imp_write<<<g, B, 0, s>>>(*d, sc, n_nodes, root, par, slot, size); d->launches++; }
+    // d->cnt: tree scratch, free until the next build
+    if (d->n > 0)
+        { k_imp_pos<<<csgd_grid(d->n, B), B, 0, s>>>(sc, d->n, d->perm, d->m, d->cnt); d->launches++; }
+    { k_imp_write<<<g, B, 0, s>>>(*d, sc, n_nodes, root, par, slot, size, d->cnt); d->launches++; }
     { k_tasks<<<1, 256, 0, s>>>(sc, d->roots, 1, d->base, d->tasks, d->task_cap, 1); d->launches++; }
     d->geometry_valid = 1;
     d->imported = 1;
