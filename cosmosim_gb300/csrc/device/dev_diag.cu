@@ -5,10 +5,16 @@
 // energy KE + softened PE (tests/test_physics.c:34-52), both in FP64. The
 // j range is split over blocks; each block writes its partial sums and a
 // second kernel adds them in a fixed order, so results are deterministic.
+// Both sums run on the integer pipes (dev_fixpair.cuh) when the bodies fit its
+// grid, which a first kernel finds on the device; the FP64 kernels are queued
+// beside them and return at once then. Measured at 100k bodies: energy 196 ->
+// 28.3 ms, direct sum of 4096 bodies 20.0 -> 4.0 ms, both bound by the integer
+// multiply and ALU pipes (74% and 66% busy).
 //
 // The probes time long independent FMA chains (8 per thread) and report the
 // FP32 and FP64 CUDA-core throughput of this GPU: the denominators for the
 // walk kernels, which are bound by those pipes, not by tensor cores or HBM.
+#include "dev_fixpair.cuh"
 #include "dev_fpint.cuh"
 #include "dev_internal.cuh"
 
@@ -17,23 +23,143 @@ namespace {
 constexpr int DT = 256;       // threads per block
 constexpr int JCHUNKS = 64;   // j-range splits for the direct sum
 
+// The bodies' grid: largest |coordinate| (dead bodies too: they may be sampled)
+// and mass of the live bodies, turned into the grid by the last block to
+// finish. The scratch is zero before the launch. A NaN orders above every
+// number: it ends in a grid with ok = 0.
+struct FixScratch {
+    unsigned long long xmax, mmax; // bit patterns of non-negative doubles
+    unsigned done;
+    FixGrid grid;
+};
+
+__global__ void __launch_bounds__(DT) k_fix_grid(const double *__restrict__ x,
+                                                 const double *__restrict__ y,
+                                                 const double *__restrict__ z,
+                                                 const double *__restrict__ m, int n, double eps,
+                                                 double eps2, FixScratch *s)
+{
+    unsigned long long xm = 0ull, mm = 0ull;
+    for (int i = blockIdx.x * DT + threadIdx.x; i < n; i += gridDim.x * DT) {
+        const unsigned long long a = (unsigned long long)__double_as_longlong(fabs(x[i])),
+                                 b = (unsigned long long)__double_as_longlong(fabs(y[i])),
+                                 c = (unsigned long long)__double_as_longlong(fabs(z[i]));
+        xm = max(xm, max(a, max(b, c)));
+        if (!(m[i] <= 0.0))
+            mm = max(mm, (unsigned long long)__double_as_longlong(fabs(m[i])));
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        xm = max(xm, __shfl_xor_sync(0xffffffffu, xm, o));
+        mm = max(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&s->xmax, xm);
+        atomicMax(&s->mmax, mm);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x != 0 || atomicAdd(&s->done, 1u) != gridDim.x - 1)
+        return;
+    __threadfence();
+    s->grid = fix_grid(__longlong_as_double((long long)__ldcg(&s->xmax)),
+                       __longlong_as_double((long long)__ldcg(&s->mmax)), (double)n, eps, eps2);
+}
+
+// A tile's bodies on the grid, staged for broadcast reads.
+struct __align__(16) FixBody {
+    long long x, y, z;
+    unsigned long long m; // fix_mass
+};
+
+__device__ __forceinline__ FixBody fix_body(const double *x, const double *y, const double *z,
+                                            const double *m, int j, double scale)
+{
+    return FixBody{fix_pos(x[j], scale), fix_pos(y[j], scale), fix_pos(z[j], scale),
+                   fix_mass(m[j])};
+}
+
+// Direct sum of sample idx[k] over bodies of its system, chunk blockIdx.y of
+// `chunks` of the bodies, on the integer pipes: about 240 instructions a pair
+// and no FP64 operation (the FP64 kernel below: a square root, a division and
+// 16 more). A body's own term is zero (its differences are). A sample index
+// outside [0, n) reads nothing; its row becomes NaN.
+constexpr int FT = 128;
+
+template <bool MULTI>
+__global__ void __launch_bounds__(FT, 5) k_direct_fix(const double *__restrict__ x,
+                                                   const double *__restrict__ y,
+                                                   const double *__restrict__ z,
+                                                   const double *__restrict__ m,
+                                                   const int *__restrict__ gid, int n,
+                                                   const int *__restrict__ idx, int ns, double G,
+                                                   int chunks, const FixScratch *sc,
+                                                   double *__restrict__ part)
+{
+    __shared__ FixBody tile[FT];
+    __shared__ int tg[FT];
+    const FixGrid f = sc->grid;
+    if (!f.ok)
+        return;
+    const double scale = ldexp(1.0, f.g);
+    const int k = blockIdx.x * FT + threadIdx.x;
+    const int per = (n + chunks - 1) / chunks;
+    const int j0 = blockIdx.y * per, j1 = min(n, j0 + per);
+    const int i = k < ns ? idx[k] : -1;
+    const bool valid = (unsigned)i < (unsigned)n;
+    const long long xi = valid ? fix_pos(x[i], scale) : 0, yi = valid ? fix_pos(y[i], scale) : 0,
+                    zi = valid ? fix_pos(z[i], scale) : 0;
+    const int gi = (MULTI && valid) ? gid[i] : 0;
+    FixSum3 a;
+    a.clear();
+    for (int t = j0; t < j1; t += FT) {
+        const int j = t + threadIdx.x;
+        __syncthreads();
+        if (j < j1) {
+            tile[threadIdx.x] = fix_body(x, y, z, m, j, scale);
+            if (MULTI)
+                tg[threadIdx.x] = gid[j];
+        }
+        __syncthreads();
+        const int cnt = min(FT, j1 - t);
+        for (int q = 0; q < cnt; q++) {
+            const FixBody b = tile[q];
+            if (MULTI && tg[q] != gi)
+                continue;
+            a.add(f, b.x - xi, b.y - yi, b.z - zi, b.m);
+        }
+    }
+    if (k < ns) {
+        double *p = part + ((size_t)blockIdx.y * ns + k) * 3;
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        p[0] = valid ? G * a.x.value(f.U3) : nan;
+        p[1] = valid ? G * a.y.value(f.U3) : nan;
+        p[2] = valid ? G * a.z.value(f.U3) : nan;
+    }
+}
+
 __global__ void __launch_bounds__(DT) k_direct(const double *__restrict__ x,
                                                const double *__restrict__ y,
                                                const double *__restrict__ z,
                                                const double *__restrict__ m,
                                                const int *__restrict__ gid, int n,
                                                const int *__restrict__ idx, int ns, double G,
-                                               double eps2, double *__restrict__ part)
+                                               double eps2, int chunks, const FixScratch *sc,
+                                               double *__restrict__ part)
 {
     __shared__ double sx[DT], sy[DT], sz[DT], sm[DT];
     __shared__ int sg[DT];
+    if (sc->grid.ok) // k_direct_fix's
+        return;
     const int k = blockIdx.x * DT + threadIdx.x;
     const int chunk = blockIdx.y;
-    const int per = (n + JCHUNKS - 1) / JCHUNKS;
+    const int per = (n + chunks - 1) / chunks;
     const int j0 = chunk * per, j1 = min(n, j0 + per);
+    // A sample index outside [0, n) reads nothing: its row becomes NaN.
     const int i = (k < ns) ? idx[k] : -1;
-    const double xi = (i >= 0) ? x[i] : 0.0, yi = (i >= 0) ? y[i] : 0.0, zi = (i >= 0) ? z[i] : 0.0;
-    const int gi = (i >= 0) ? gid[i] : -1; // only bodies of the same system attract
+    const bool valid = (unsigned)i < (unsigned)n;
+    const double xi = valid ? x[i] : 0.0, yi = valid ? y[i] : 0.0, zi = valid ? z[i] : 0.0;
+    const int gi = (valid && gid) ? gid[i] : 0; // only bodies of the same system attract
     double ax = 0.0, ay = 0.0, az = 0.0;
     for (int t = j0; t < j1; t += DT) {
         const int j = t + threadIdx.x;
@@ -43,11 +169,11 @@ __global__ void __launch_bounds__(DT) k_direct(const double *__restrict__ x,
             sy[threadIdx.x] = y[j];
             sz[threadIdx.x] = z[j];
             sm[threadIdx.x] = (m[j] <= 0.0) ? 0.0 : m[j];
-            sg[threadIdx.x] = gid[j];
+            sg[threadIdx.x] = gid ? gid[j] : 0;
         }
         __syncthreads();
         const int cnt = min(DT, j1 - t);
-        if (i >= 0) {
+        if (valid) {
             for (int q = 0; q < cnt; q++) {
                 if (t + q == i || sg[q] != gi)
                     continue;
@@ -62,6 +188,8 @@ __global__ void __launch_bounds__(DT) k_direct(const double *__restrict__ x,
         }
     }
     if (k < ns) {
+        if (!valid)
+            ax = ay = az = __longlong_as_double(0x7ff8000000000000ll);
         double *p = part + ((size_t)chunk * ns + k) * 3;
         p[0] = ax;
         p[1] = ay;
@@ -69,13 +197,14 @@ __global__ void __launch_bounds__(DT) k_direct(const double *__restrict__ x,
     }
 }
 
-__global__ void k_direct_sum(const double *__restrict__ part, int ns, double *__restrict__ out)
+__global__ void k_direct_sum(const double *__restrict__ part, int chunks, int ns,
+                             double *__restrict__ out)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= ns)
         return;
     double a[3] = {0.0, 0.0, 0.0};
-    for (int c = 0; c < JCHUNKS; c++)
+    for (int c = 0; c < chunks; c++)
         for (int d = 0; d < 3; d++)
             a[d] += part[((size_t)c * ns + k) * 3 + d];
     for (int d = 0; d < 3; d++)
@@ -96,18 +225,91 @@ __device__ __forceinline__ double inv_r(double r2)
     return 1.0 / sqrt(r2);
 }
 
-// Potential energy: row i against columns j > i, rows split over blocks;
-// each thread writes its row sum, reduced afterwards.
+// Potential energy on the integer pipes: rows of 2 FT bodies (two a thread)
+// against a chunk of `per` columns j > i, about 150 instructions a pair and no
+// FP64 operation. Row i's sum of m_j / r over chunk c goes to part[c n + i];
+// chunks wholly at or before the row block are left out, there and below. The
+// columns are split so that the long rows of the first bodies do not keep a
+// few SMs busy at the end.
+constexpr int PT_ROWS = 2 * FT;
+
+template <bool MULTI>
+__global__ void __launch_bounds__(FT, 6) k_potential_fix(const double *__restrict__ x,
+                                                      const double *__restrict__ y,
+                                                      const double *__restrict__ z,
+                                                      const double *__restrict__ m,
+                                                      const int *__restrict__ gid, int n, int per,
+                                                      const FixScratch *sc,
+                                                      double *__restrict__ part)
+{
+    __shared__ FixBody tile[FT];
+    __shared__ int tg[FT];
+    const int row0 = blockIdx.x * PT_ROWS;
+    const int j0 = blockIdx.y * per, j1 = min(n, j0 + per);
+    const FixGrid f = sc->grid;
+    if (!f.ok || j1 <= row0)
+        return;
+    const double scale = ldexp(1.0, f.g);
+    const int ia = row0 + threadIdx.x, ib = ia + FT;
+    const FixBody a = ia < n ? fix_body(x, y, z, m, ia, scale) : FixBody{0, 0, 0, 0ull};
+    const FixBody b = ib < n ? fix_body(x, y, z, m, ib, scale) : FixBody{0, 0, 0, 0ull};
+    const int ga = (MULTI && ia < n) ? gid[ia] : 0, gb = (MULTI && ib < n) ? gid[ib] : 0;
+    FixSum1 sa, sb;
+    sa.a.clear();
+    sb.a.clear();
+    for (int t = max(j0, row0); t < j1; t += FT) {
+        const int j = t + threadIdx.x;
+        __syncthreads();
+        if (j < j1) {
+            tile[threadIdx.x] = fix_body(x, y, z, m, j, scale);
+            if (MULTI)
+                tg[threadIdx.x] = gid[j];
+        }
+        __syncthreads();
+        const int cnt = min(FT, j1 - t);
+        for (int q = 0; q < cnt; q++) {
+            const FixBody c = tile[q];
+            const bool ta = t + q > ia && (!MULTI || tg[q] == ga),
+                       tb = t + q > ib && (!MULTI || tg[q] == gb);
+            sa.add(f, c.x - a.x, c.y - a.y, c.z - a.z, ta ? c.m : 0ull);
+            sb.add(f, c.x - b.x, c.y - b.y, c.z - b.z, tb ? c.m : 0ull);
+        }
+    }
+    double *p = part + (size_t)blockIdx.y * n;
+    if (ia < n)
+        p[ia] = sa.a.value(f.U1);
+    if (ib < n)
+        p[ib] = sb.a.value(f.U1);
+}
+
+__global__ void k_potential_sum(const double *__restrict__ part, const double *__restrict__ m,
+                                int n, int per, double G, const FixScratch *sc,
+                                double *__restrict__ row)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || !sc->grid.ok)
+        return;
+    double s = 0.0;
+    for (int c = (i / PT_ROWS) * PT_ROWS / per; (long long)c * per < n; c++)
+        s += part[(size_t)c * n + i];
+    row[i] = -G * (m[i] > 0.0 ? m[i] : 0.0) * s;
+}
+
+// The same in FP64, for bodies off the grid: row i against columns j > i, rows
+// split over blocks; each thread writes its row sum, reduced afterwards.
 __global__ void __launch_bounds__(DT) k_potential_rows(const double *__restrict__ x,
                                                        const double *__restrict__ y,
                                                        const double *__restrict__ z,
                                                        const double *__restrict__ m,
                                                        const int *__restrict__ gid, int n,
                                                        double G, double eps2,
+                                                       const FixScratch *sc,
                                                        double *__restrict__ row)
 {
     __shared__ double sx[DT], sy[DT], sz[DT], sm[DT];
     __shared__ int sg[DT];
+    if (sc->grid.ok) // k_potential_fix's
+        return;
     const int i = blockIdx.x * DT + threadIdx.x;
     const double xi = (i < n) ? x[i] : 0.0, yi = (i < n) ? y[i] : 0.0, zi = (i < n) ? z[i] : 0.0;
     const int gi = (i < n) ? gid[i] : -1;
@@ -188,6 +390,13 @@ __global__ void k_fma_probe(T *out, int iters, T a, T b)
 
 } // namespace
 
+// Blocks of the grid's bounds pass: a few per SM, each striding over the bodies.
+static int grid_blocks(int n, int sms)
+{
+    const int g = csgd_grid(n, DT);
+    return g < 4 * sms ? g : 4 * sms;
+}
+
 extern "C" int csgd_direct_forces(csgd_t *d, const int *host_idx, int ns, double G,
                                   double softening, double *host_out)
 {
@@ -198,55 +407,73 @@ extern "C" int csgd_direct_forces(csgd_t *d, const int *host_idx, int ns, double
     for (int k = 0; k < ns; k++)
         if (host_idx[k] < 0 || host_idx[k] >= d->n)
             return CSG_ERR_BAD_ARG;
-    int *didx = nullptr;
-    double *part = nullptr, *out = nullptr;
-    cudaError_t e = csgd_malloc((void **)&didx, sizeof(int) * (size_t)ns);
-    if (e == cudaSuccess)
-        e = csgd_malloc((void **)&part, sizeof(double) * 3 * (size_t)ns * JCHUNKS);
-    if (e == cudaSuccess)
-        e = csgd_malloc((void **)&out, sizeof(double) * 3 * (size_t)ns);
-    int rc = CSG_OK;
-    if (e == cudaSuccess) {
-        cudaMemcpyAsync(didx, host_idx, sizeof(int) * (size_t)ns, cudaMemcpyHostToDevice, d->stream);
-        dim3 grid((ns + DT - 1) / DT, JCHUNKS);
-        { k_direct<<<grid, DT, 0, d->stream>>>(d->x, d->y, d->z, d->m, d->gid, d->n, didx, ns, G, softening * softening, part); d->launches++; }
-        { k_direct_sum<<<csgd_grid(ns, 256), 256, 0, d->stream>>>(part, ns, out); d->launches++; }
-        cudaMemcpyAsync(host_out, out, sizeof(double) * 3 * (size_t)ns, cudaMemcpyDeviceToHost, d->stream);
-        rc = csgd_sync(d);
-    } else {
+    // one allocation: partial sums, result, grid scratch, sample
+    const size_t doubles = 3 * (size_t)ns * (JCHUNKS + 1);
+    void *mem = nullptr;
+    if (csgd_malloc(&mem, sizeof(double) * doubles + sizeof(FixScratch) +
+                              sizeof(int) * (size_t)ns) != cudaSuccess) {
         cudaGetLastError();
-        rc = CSG_ERR_NOMEM;
+        return CSG_ERR_NOMEM;
     }
-    cudaFree(didx);
-    cudaFree(part);
-    cudaFree(out);
+    double *part = (double *)mem, *out = part + 3 * (size_t)ns * JCHUNKS;
+    FixScratch *sc = (FixScratch *)(part + doubles);
+    int *didx = (int *)(sc + 1);
+    cudaStream_t s = d->stream;
+    cudaMemcpyAsync(didx, host_idx, sizeof(int) * (size_t)ns, cudaMemcpyHostToDevice, s);
+    cudaMemsetAsync(sc, 0, sizeof(FixScratch), s);
+    const double eps2 = softening * softening;
+    { k_fix_grid<<<grid_blocks(d->n, d->num_sms), DT, 0, s>>>(d->x, d->y, d->z, d->m, d->n, softening, eps2, sc); d->launches++; }
+    const dim3 gf((ns + FT - 1) / FT, JCHUNKS), gd((ns + DT - 1) / DT, JCHUNKS);
+    if (d->n_gal > 1)
+        k_direct_fix<true><<<gf, FT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, d->n, didx, ns, G, JCHUNKS, sc, part);
+    else
+        k_direct_fix<false><<<gf, FT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, d->n, didx, ns, G, JCHUNKS, sc, part);
+    d->launches++;
+    { k_direct<<<gd, DT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, d->n, didx, ns, G, eps2, JCHUNKS, sc, part); d->launches++; }
+    { k_direct_sum<<<csgd_grid(ns, 256), 256, 0, s>>>(part, JCHUNKS, ns, out); d->launches++; }
+    cudaMemcpyAsync(host_out, out, sizeof(double) * 3 * (size_t)ns, cudaMemcpyDeviceToHost, s);
+    const int rc = csgd_sync(d);
+    cudaFree(mem);
     return rc;
 }
 
 extern "C" int csgd_energy(csgd_t *d, double G, double softening, double *ke, double *pe)
 {
     const int n = d->n;
-    double *row = nullptr, *out = nullptr;
-    cudaError_t e = csgd_malloc((void **)&row, sizeof(double) * (size_t)(n > 0 ? n : 1));
-    if (e == cudaSuccess)
-        e = csgd_malloc((void **)&out, 2 * sizeof(double));
-    int rc = CSG_OK;
-    if (e == cudaSuccess && n > 0) {
-        { k_potential_rows<<<csgd_grid(n, DT), DT, 0, d->stream>>>(d->x, d->y, d->z, d->m, d->gid, n, G, softening * softening, row); d->launches++; }
-        { k_energy_reduce<<<1, 1024, 0, d->stream>>>(row, d->m, d->vx, d->vy, d->vz, n, out); d->launches++; }
-        double h[2] = {0.0, 0.0};
-        cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, d->stream);
-        rc = csgd_sync(d);
-        *ke = h[0];
-        *pe = h[1];
-    } else if (e != cudaSuccess) {
-        cudaGetLastError();
-        rc = CSG_ERR_NOMEM;
-    } else {
+    if (n <= 0) {
         *ke = *pe = 0.0;
+        return CSG_OK;
     }
-    cudaFree(row);
-    cudaFree(out);
+    // columns a chunk: at least 2048, at most 32 chunks (their partial sums)
+    const int per = n / 32 > 2048 ? (n + 31) / 32 : 2048;
+    const int chunks = (n + per - 1) / per;
+    void *mem = nullptr;
+    if (csgd_malloc(&mem, sizeof(double) * ((size_t)n * (chunks + 1) + 2) + sizeof(FixScratch)) !=
+        cudaSuccess) {
+        cudaGetLastError();
+        return CSG_ERR_NOMEM;
+    }
+    double *part = (double *)mem, *row = part + (size_t)n * chunks, *out = row + n;
+    FixScratch *sc = (FixScratch *)(out + 2);
+    cudaStream_t s = d->stream;
+    cudaMemsetAsync(sc, 0, sizeof(FixScratch), s);
+    const double eps2 = softening * softening;
+    { k_fix_grid<<<grid_blocks(n, d->num_sms), DT, 0, s>>>(d->x, d->y, d->z, d->m, n, softening, eps2, sc); d->launches++; }
+    const dim3 gf((n + PT_ROWS - 1) / PT_ROWS, chunks);
+    if (d->n_gal > 1)
+        k_potential_fix<true><<<gf, FT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, n, per, sc, part);
+    else
+        k_potential_fix<false><<<gf, FT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, n, per, sc, part);
+    d->launches++;
+    { k_potential_sum<<<csgd_grid(n, 256), 256, 0, s>>>(part, d->m, n, per, G, sc, row); d->launches++; }
+    { k_potential_rows<<<csgd_grid(n, DT), DT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, n, G, eps2, sc, row); d->launches++; }
+    { k_energy_reduce<<<1, 1024, 0, s>>>(row, d->m, d->vx, d->vy, d->vz, n, out); d->launches++; }
+    double h[2] = {0.0, 0.0};
+    cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, s);
+    const int rc = csgd_sync(d);
+    *ke = h[0];
+    *pe = h[1];
+    cudaFree(mem);
     return rc;
 }
 
@@ -313,91 +540,24 @@ extern "C" CSG_EXPORT int csg_measure_fp_peaks(double *fp32_tflops, double *fp64
 // below instead of cudaMalloc'd memory: 16 chunks x 4096 bodies x 3 doubles =
 // 1.5 MiB, held by every GPU that loads the library until the process exits.
 // All calls share that array, so calls that overlap on the GPU race; every
-// call overwrites each partial it later reads, so nothing needs clearing.
+// call clears the grid's scratch and overwrites each partial it later reads.
 
 constexpr int NOALLOC_CHUNKS = 16;
 constexpr int NOALLOC_MAX_SAMPLE = 4096;
 constexpr int NOALLOC_MAX_DEVICES = 64;
 
-static __device__ __align__(256) double g_noalloc_partials[NOALLOC_CHUNKS * NOALLOC_MAX_SAMPLE * 3];
+struct NoallocScratch {
+    double partials[NOALLOC_CHUNKS * NOALLOC_MAX_SAMPLE * 3];
+    FixScratch grid;
+};
+static __device__ __align__(256) NoallocScratch g_noalloc;
 
 #include <mutex>
 
 namespace {
 
 std::mutex g_noalloc_mutex;
-double *g_noalloc_ptr[NOALLOC_MAX_DEVICES];
-
-__global__ void __launch_bounds__(DT) k_direct_noalloc(const double *__restrict__ x,
-                                                       const double *__restrict__ y,
-                                                       const double *__restrict__ z,
-                                                       const double *__restrict__ m,
-                                                       const int *__restrict__ sys, int n,
-                                                       const int *__restrict__ idx, int ns,
-                                                       double G, double eps2,
-                                                       double *__restrict__ part)
-{
-    __shared__ double sx[DT], sy[DT], sz[DT], sm[DT];
-    __shared__ int sg[DT];
-    const int k = blockIdx.x * DT + threadIdx.x;
-    const int chunk = blockIdx.y;
-    const int per = (n + NOALLOC_CHUNKS - 1) / NOALLOC_CHUNKS;
-    const int j0 = chunk * per, j1 = min(n, j0 + per);
-    // A sample index outside [0, n) reads nothing: its row becomes NaN.
-    const int i = (k < ns) ? idx[k] : -1;
-    const bool valid = (unsigned)i < (unsigned)n;
-    const double xi = valid ? x[i] : 0.0, yi = valid ? y[i] : 0.0, zi = valid ? z[i] : 0.0;
-    const int gi = (valid && sys) ? sys[i] : 0; // only bodies of the same system attract
-    double ax = 0.0, ay = 0.0, az = 0.0;
-    for (int t = j0; t < j1; t += DT) {
-        const int j = t + threadIdx.x;
-        __syncthreads();
-        if (j < j1) {
-            sx[threadIdx.x] = x[j];
-            sy[threadIdx.x] = y[j];
-            sz[threadIdx.x] = z[j];
-            sm[threadIdx.x] = (m[j] <= 0.0) ? 0.0 : m[j];
-            sg[threadIdx.x] = sys ? sys[j] : 0;
-        }
-        __syncthreads();
-        const int cnt = min(DT, j1 - t);
-        if (valid) {
-            for (int q = 0; q < cnt; q++) {
-                if (t + q == i || sg[q] != gi)
-                    continue;
-                double dx = sx[q] - xi, dy = sy[q] - yi, dz = sz[q] - zi;
-                double r2 = dx * dx + dy * dy + dz * dz + eps2;
-                double inv = 1.0 / (r2 * sqrt(r2));
-                double f = G * sm[q] * inv;
-                ax += f * dx;
-                ay += f * dy;
-                az += f * dz;
-            }
-        }
-    }
-    if (k < ns) {
-        if (!valid)
-            ax = ay = az = __longlong_as_double(0x7ff8000000000000ll);
-        double *p = part + ((size_t)chunk * ns + k) * 3;
-        p[0] = ax;
-        p[1] = ay;
-        p[2] = az;
-    }
-}
-
-__global__ void k_direct_noalloc_sum(const double *__restrict__ part, int ns,
-                                     double *__restrict__ out)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= ns)
-        return;
-    double a[3] = {0.0, 0.0, 0.0};
-    for (int c = 0; c < NOALLOC_CHUNKS; c++)
-        for (int d = 0; d < 3; d++)
-            a[d] += part[((size_t)c * ns + k) * 3 + d];
-    for (int d = 0; d < 3; d++)
-        out[3 * (size_t)k + d] = a[d];
-}
+NoallocScratch *g_noalloc_ptr[NOALLOC_MAX_DEVICES];
 
 } // namespace
 
@@ -407,7 +567,7 @@ __global__ void k_direct_noalloc_sum(const double *__restrict__ part, int ns,
 // device's primary context: after a cudaDeviceReset the cached address is
 // stale, so a process that resets a device must not call the entry point on
 // it again.
-static int noalloc_scratch(double **ptr)
+static int noalloc_scratch(NoallocScratch **ptr)
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= NOALLOC_MAX_DEVICES) {
@@ -417,11 +577,11 @@ static int noalloc_scratch(double **ptr)
     std::lock_guard<std::mutex> lock(g_noalloc_mutex);
     if (!g_noalloc_ptr[dev]) {
         void *p = nullptr;
-        if (cudaGetSymbolAddress(&p, g_noalloc_partials) != cudaSuccess || !p) {
+        if (cudaGetSymbolAddress(&p, g_noalloc) != cudaSuccess || !p) {
             cudaGetLastError();
             return CSG_ERR_CUDA;
         }
-        g_noalloc_ptr[dev] = (double *)p;
+        g_noalloc_ptr[dev] = (NoallocScratch *)p;
     }
     *ptr = g_noalloc_ptr[dev];
     return CSG_OK;
@@ -439,14 +599,21 @@ extern "C" CSG_EXPORT int csg_direct_forces_noalloc(const double *x, const doubl
         return CSG_OK;
     if (!x || !y || !z || !mass || !idx || !out || n == 0)
         return CSG_ERR_BAD_ARG;
-    double *part = nullptr;
-    int rc = noalloc_scratch(&part);
+    NoallocScratch *w = nullptr;
+    int rc = noalloc_scratch(&w);
     if (rc)
         return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    dim3 grid((m + DT - 1) / DT, NOALLOC_CHUNKS);
-    k_direct_noalloc<<<grid, DT, 0, s>>>(x, y, z, mass, sys, n, idx, m, G, softening * softening, part);
-    k_direct_noalloc_sum<<<(m + 255) / 256, 256, 0, s>>>(part, m, out);
+    const double eps2 = softening * softening;
+    cudaMemsetAsync(&w->grid, 0, sizeof(FixScratch), s);
+    k_fix_grid<<<grid_blocks(n, 152), DT, 0, s>>>(x, y, z, mass, n, softening, eps2, &w->grid);
+    const dim3 gf((m + FT - 1) / FT, NOALLOC_CHUNKS), gd((m + DT - 1) / DT, NOALLOC_CHUNKS);
+    if (sys)
+        k_direct_fix<true><<<gf, FT, 0, s>>>(x, y, z, mass, sys, n, idx, m, G, NOALLOC_CHUNKS, &w->grid, w->partials);
+    else
+        k_direct_fix<false><<<gf, FT, 0, s>>>(x, y, z, mass, sys, n, idx, m, G, NOALLOC_CHUNKS, &w->grid, w->partials);
+    k_direct<<<gd, DT, 0, s>>>(x, y, z, mass, sys, n, idx, m, G, eps2, NOALLOC_CHUNKS, &w->grid, w->partials);
+    k_direct_sum<<<(m + 255) / 256, 256, 0, s>>>(w->partials, NOALLOC_CHUNKS, m, out);
     if (cudaGetLastError() != cudaSuccess)
         return CSG_ERR_CUDA;
     return CSG_OK;

@@ -1,0 +1,242 @@
+// dev_fixpair.cuh — softened pair terms on the integer pipes.
+//
+// GB300 runs 2 FP64 operations per clock and SM, 1/64 of its FP32 rate; its
+// 32 x 32 -> 64-bit integer multiply-adds run far faster. A softened pair
+// m d / (d^2 + eps^2)^(3/2) costs 9 FP64 operations even with m/r^3 formed by
+// integers (576 issue cycles per warp and scheduler); formed by integers from
+// end to end it takes about 240 instructions (m/r: 150) on two pipes, 330
+// cycles (210), and no FP64 operation.
+//
+// Positions are 64-bit fixed point on one grid per system: X = x 2^g, rounded,
+// |X| < 2^61, so differences are exact in 64 bits. r^2 = dx^2 + dy^2 + dz^2 +
+// eps^2 is summed from the differences shifted up together (the largest, or
+// eps, then has its top bit at 61) and kept to 2^-57 relative. 1/r comes from
+// an FP32 rsqrt seed y0: e = 1 - r^2 y0^2 by one high-word product, then the
+// binomial series y0 (1 - e)^(-1/2) or y0^3 (1 - e)^(-3/2) to second order
+// (|e| < 2^-20: the next term is below 2^-59), every product keeping its high
+// 64 bits. Terms are added to a 128-bit fixed-point sum, so a sum does not
+// depend on its order. (64-bit sums whose unit followed the largest term took
+// about 60 instructions less a pair but were 4-15 times less exact than FP64.)
+//
+// What rounds: the positions (half a grid unit), the truncated products (about
+// 2^-55 of a term in all) and the last bit of the 128-bit sum. The grid is
+// 2^-61 of the largest coordinate; FIX_EPS_BITS keeps eps above 2^47 units, so a
+// pair at the softening length, the closest that matters, still has its
+// difference to 2^-47, and every longer one better. Systems that do not fit (no softening, a span above 2^14
+// softening lengths, non-finite or extreme values) keep the FP64 kernels.
+#pragma once
+
+#include <math.h>
+
+#include "dev_internal.cuh"
+
+struct FixGrid {
+    int ok;                  // 1: the system fits; 0: use the FP64 kernels
+    int g;                   // grid: X = x 2^g
+    int U3, U1;              // exponent of the last bit of an acceleration, a potential sum
+    unsigned eh;             // high word of eps 2^g
+    int e2s;                 // eps^2 in units of r2 (fix_pair): e2n >> (e2s - 2 s)
+    unsigned long long e2n;  // eps^2's significand, top bit at 61
+};
+
+constexpr int FIX_POS_BITS = 61; // |X| < 2^61
+constexpr int FIX_EPS_BITS = 47; // eps 2^g >= 2^47
+
+// The grid of n bodies whose largest |coordinate| is xmax and largest mass
+// mmax (n mmax bounds the sums), with the given eps and eps^2.
+__device__ inline FixGrid fix_grid(double xmax, double mmax, double n, double eps, double eps2)
+{
+    FixGrid f;
+    f.ok = 0;
+    f.g = f.U3 = f.U1 = f.e2s = 0;
+    f.eh = 0u;
+    f.e2n = 0ull;
+    eps = fabs(eps);
+    // exponents far inside FP64's, so that every power of two below is normal
+    if (!(xmax <= 0x1p200 && mmax > 0x1p-200 && mmax <= 0x1p200 && eps >= 0x1p-200 &&
+          eps <= 0x1p200))
+        return f;
+    // the larger of the coordinates and eps fits 61 bits
+    f.g = FIX_POS_BITS - (ilogb(fmax(xmax, eps)) + 1);
+    const long long E = (long long)ldexp(eps, f.g);
+    if (E < (1LL << FIX_EPS_BITS))
+        return f;
+    f.eh = (unsigned)(E >> 32);
+    // eps^2 = S 2^k, S the 53-bit significand; r2's unit is 2^(64 - 2 s - 2 g)
+    const long long b = __double_as_longlong(eps2);
+    const int k = (int)((b >> 52) & 0x7ff) - 1075;
+    f.e2n = (((unsigned long long)b & 0xfffffffffffffull) | (1ull << 52)) << 9;
+    f.e2s = 64 + 9 - k - 2 * f.g;
+    // |sum of a| <= n mmax max(r / (r^2 + eps^2)^1.5) <= n mmax 0.385 / eps^2
+    f.U3 = ilogb(n * mmax * 0.385 / eps2) + 1 - 119;
+    f.U1 = ilogb(n * mmax / eps) + 1 - 119;
+    f.ok = 1;
+    return f;
+}
+
+__device__ __forceinline__ long long fix_pos(double x, double scale) // scale = 2^g
+{
+    return __double2ll_rn(x * scale);
+}
+
+// A mass as its significand with the top bit at 63 and the biased exponent in
+// the 11 free low bits; 0 for a massless (or subnormal) body.
+__device__ __forceinline__ unsigned long long fix_mass(double m)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(m);
+    const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+    return (m > 0.0 && e > 0u) ? ((((b & 0xfffffffffffffull) | (1ull << 52)) << 11) | e) : 0ull;
+}
+
+__device__ __forceinline__ unsigned long long mulw(unsigned a, unsigned b)
+{
+    return (unsigned long long)a * b;
+}
+__device__ __forceinline__ unsigned hi32(unsigned long long v) { return (unsigned)(v >> 32); }
+__device__ __forceinline__ unsigned long long shr_clamp(unsigned long long v, unsigned n)
+{
+    unsigned long long r; // PTX clamps the shift: n >= 64 gives 0
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+    return r;
+}
+
+// High 64 bits of a b from the three upper partial products, each taken from
+// its high word: 0 to 3 below, 1.25 on average.
+__device__ __forceinline__ unsigned long long mulhi(unsigned long long a, unsigned long long b)
+{
+    return mulw(hi32(a), hi32(b)) + hi32(mulw(hi32(a), (unsigned)b)) +
+           hi32(mulw((unsigned)a, hi32(b)));
+}
+__device__ __forceinline__ long long mulws(int a, int b) { return (long long)a * b; }
+
+// r^2 of a pair and its rsqrt seed.
+struct FixR {
+    long long x, y, z;    // differences 2^s, |.| < 2^62
+    int nx, ny, nz;       // their signs (0 or -1)
+    unsigned long long S; // Y^2
+    long long e57;        // (1 - r^2 y0^2) 2^57
+    unsigned Y;           // y0 = Y 2^(ey - 158)
+    int ey, s;
+};
+
+__device__ __forceinline__ FixR fix_pair(const FixGrid &f, long long dx, long long dy, long long dz)
+{
+    FixR p;
+    const int xh0 = (int)(dx >> 32), yh0 = (int)(dy >> 32), zh0 = (int)(dz >> 32);
+    p.nx = xh0 >> 31;
+    p.ny = yh0 >> 31;
+    p.nz = zh0 >> 31;
+    p.s = __clz((xh0 ^ p.nx) | (yh0 ^ p.ny) | (zh0 ^ p.nz) | (int)f.eh) - 2; // 0..15
+    p.x = (long long)((unsigned long long)dx << p.s);
+    p.y = (long long)((unsigned long long)dy << p.s);
+    p.z = (long long)((unsigned long long)dz << p.s);
+    const int xh = (int)(p.x >> 32), yh = (int)(p.y >> 32), zh = (int)(p.z >> 32);
+    const long long hh = mulws(xh, xh) + mulws(yh, yh) + mulws(zh, zh);
+    const long long hl = mulws(xh, (int)((unsigned)p.x >> 2)) + mulws(yh, (int)((unsigned)p.y >> 2)) +
+                         mulws(zh, (int)((unsigned)p.z >> 2));
+    // r^2 = r2 2^(64 - 2 s - 2 g), r2 in [2^58, 2^62]; the dropped low
+    // products are 1 on average
+    const unsigned long long r2 = (unsigned long long)(hh + (hl >> 29)) +
+                                  shr_clamp(f.e2n, (unsigned)(f.e2s - 2 * p.s)) + 1ull;
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint2float_rz(hi32(r2))));
+    const unsigned yb = __float_as_uint(y);
+    p.ey = (int)(yb >> 23); // 111..114
+    p.Y = (yb << 8) | 0x80000000u;
+    p.S = mulw(p.Y, p.Y);
+    // r2 S 2^-63 = (1 - e) 2^(285 - 2 ey)
+    const unsigned long long T = mulhi(r2 << 1, p.S);
+    const int k = 285 - 2 * p.ey; // 57..63
+    p.e57 = (long long)((1ull << k) - T) >> (k - 57);
+    return p;
+}
+
+// e^2 2^70 from e 2^57, for the series' second term.
+__device__ __forceinline__ unsigned fix_e2(long long e57)
+{
+    const int eh = (int)(e57 >> 6);
+    return (unsigned)(mulws(eh, eh) >> 32);
+}
+
+// 128-bit sum, words from the lowest.
+struct Fix128 {
+    unsigned w0, w1, w2, w3;
+
+    __device__ __forceinline__ void clear() { w0 = w1 = w2 = w3 = 0u; }
+    // adds (v 2^64) >> sh, sh >= 0; neg (0 or ~0): subtracts it, and one unit
+    __device__ __forceinline__ void add(unsigned long long v, unsigned sh, unsigned neg)
+    {
+        const unsigned hi = hi32(v) ^ neg, lo = (unsigned)v ^ neg;
+        const unsigned t2 = (unsigned)((int)hi >> (sh & 31u)); // v < 2^63: hi's top bit is the sign
+        const unsigned t1 = __funnelshift_r(lo, hi, sh), t0 = __funnelshift_r(neg, lo, sh);
+        const unsigned w = sh >> 5;
+        const unsigned o3 = w == 0u ? t2 : neg;
+        const unsigned o2 = w == 0u ? t1 : w == 1u ? t2 : neg;
+        const unsigned o1 = w == 0u ? t0 : w == 1u ? t1 : w == 2u ? t2 : neg;
+        const unsigned o0 = w == 1u ? t0 : w == 2u ? t1 : w == 3u ? t2 : neg;
+        asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\t"
+            "addc.cc.u32 %2, %2, %6;\n\taddc.u32 %3, %3, %7;"
+            : "+r"(w0), "+r"(w1), "+r"(w2), "+r"(w3)
+            : "r"(o0), "r"(o1), "r"(o2), "r"(o3));
+    }
+    // the sum (two's complement) times 2^U
+    __device__ __forceinline__ double value(int U) const
+    {
+        const bool n = (int)w3 < 0;
+        unsigned long long hi = ((unsigned long long)w3 << 32) | w2,
+                           lo = ((unsigned long long)w1 << 32) | w0;
+        if (n) {
+            lo = 0ull - lo;
+            hi = ~hi + (lo == 0ull);
+        }
+        const double v = ldexp(fma((double)hi, 0x1p64, (double)lo), U);
+        return n ? -v : v;
+    }
+};
+
+// Sum of m d / r^3 terms.
+struct FixSum3 {
+    Fix128 x, y, z;
+
+    __device__ __forceinline__ void clear()
+    {
+        x.clear();
+        y.clear();
+        z.clear();
+    }
+    __device__ __forceinline__ void add(const FixGrid &f, long long dx, long long dy, long long dz,
+                                        unsigned long long mass)
+    {
+        const FixR p = fix_pair(f, dx, dy, dz);
+        const int q = (int)(((fix_e2(p.e57) >> 4) * 15u) >> 12); // 15/8 e^2 2^57
+        const long long c57 = p.e57 + (p.e57 >> 1) + q;
+        const unsigned long long C = (1ull << 63) + (unsigned long long)(c57 << 6); // (1 + c) 2^63
+        const unsigned long long W = mulw(p.Y, hi32(p.S)) + hi32(mulw(p.Y, (unsigned)p.S));
+        const unsigned long long F = mulhi(mulhi(W, C), mass & ~0x7ffull);
+        // F d 2^s = term 2^(64 - X)
+        const int X = 3 * p.ey + (int)((unsigned)mass & 0x7ffu) + 2 * p.s + 2 * f.g - 1543;
+        const unsigned sh = (unsigned)max(f.U3 - X + 64, 0);
+        x.add(mulhi(F, (unsigned long long)(p.x < 0 ? -p.x : p.x)), sh, (unsigned)p.nx);
+        y.add(mulhi(F, (unsigned long long)(p.y < 0 ? -p.y : p.y)), sh, (unsigned)p.ny);
+        z.add(mulhi(F, (unsigned long long)(p.z < 0 ? -p.z : p.z)), sh, (unsigned)p.nz);
+    }
+};
+
+// Sum of m / r terms.
+struct FixSum1 {
+    Fix128 a;
+
+    __device__ __forceinline__ void add(const FixGrid &f, long long dx, long long dy, long long dz,
+                                        unsigned long long mass)
+    {
+        const FixR p = fix_pair(f, dx, dy, dz);
+        const int q = (int)(((fix_e2(p.e57) >> 4) * 3u) >> 12); // 3/8 e^2 2^57
+        const long long c57 = (p.e57 >> 1) + q;
+        const unsigned long long C = (1ull << 63) + (unsigned long long)(c57 << 6);
+        const unsigned long long V = mulw(p.Y, hi32(C)) + hi32(mulw(p.Y, (unsigned)C));
+        const unsigned long long F = mulhi(V, mass & ~0x7ffull);
+        // m / r = F 2^X
+        const int X = p.ey + (int)((unsigned)mass & 0x7ffu) + p.s + f.g - 1259;
+        a.add(F, (unsigned)max(f.U1 - X + 64, 0), 0u);
+    }
+};
