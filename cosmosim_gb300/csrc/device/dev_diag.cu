@@ -66,12 +66,6 @@ __global__ void __launch_bounds__(DT) k_fix_grid(const double *__restrict__ x,
                        __longlong_as_double((long long)__ldcg(&s->mmax)), (double)n, eps, eps2);
 }
 
-// A tile's bodies on the grid, staged for broadcast reads.
-struct __align__(16) FixBody {
-    long long x, y, z;
-    unsigned long long m; // fix_mass
-};
-
 __device__ __forceinline__ FixBody fix_body(const double *x, const double *y, const double *z,
                                             const double *m, int j, double scale)
 {
@@ -110,8 +104,10 @@ __global__ void __launch_bounds__(FT, 5) k_direct_fix(const double *__restrict__
     const long long xi = valid ? fix_pos(x[i], scale) : 0, yi = valid ? fix_pos(y[i], scale) : 0,
                     zi = valid ? fix_pos(z[i], scale) : 0;
     const int gi = (MULTI && valid) ? gid[i] : 0;
-    FixSum3 a;
-    a.clear();
+    Fix128 ax, ay, az;
+    ax.clear();
+    ay.clear();
+    az.clear();
     for (int t = j0; t < j1; t += FT) {
         const int j = t + threadIdx.x;
         __syncthreads();
@@ -126,15 +122,15 @@ __global__ void __launch_bounds__(FT, 5) k_direct_fix(const double *__restrict__
             const FixBody b = tile[q];
             if (MULTI && tg[q] != gi)
                 continue;
-            a.add(f, b.x - xi, b.y - yi, b.z - zi, b.m);
+            fix_add3(f, b.x - xi, b.y - yi, b.z - zi, b.m, ax, ay, az);
         }
     }
     if (k < ns) {
         double *p = part + ((size_t)blockIdx.y * ns + k) * 3;
         const double nan = __longlong_as_double(0x7ff8000000000000ll);
-        p[0] = valid ? G * a.x.value(f.U3) : nan;
-        p[1] = valid ? G * a.y.value(f.U3) : nan;
-        p[2] = valid ? G * a.z.value(f.U3) : nan;
+        p[0] = valid ? G * ax.value(f.U3) : nan;
+        p[1] = valid ? G * ay.value(f.U3) : nan;
+        p[2] = valid ? G * az.value(f.U3) : nan;
     }
 }
 

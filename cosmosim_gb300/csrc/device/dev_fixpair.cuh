@@ -14,15 +14,16 @@
 // an FP32 rsqrt seed y0: e = 1 - r^2 y0^2 by one high-word product, then the
 // binomial series y0 (1 - e)^(-1/2) or y0^3 (1 - e)^(-3/2) to second order
 // (|e| < 2^-20: the next term is below 2^-59), every product keeping its high
-// 64 bits. Terms are added to a 128-bit fixed-point sum, so a sum does not
-// depend on its order. (64-bit sums whose unit followed the largest term took
+// 64 bits. Terms are added to a 128-bit fixed-point sum (the walk's, of
+// fewer terms and a tighter bound, to 96 bits), so a sum does not depend on its
+// order. (64-bit sums whose unit followed the largest term took
 // about 60 instructions less a pair but were 4-15 times less exact than FP64.)
 //
 // What rounds: the positions (half a grid unit), the truncated products (about
 // 2^-55 of a term in all) and the last bit of the 128-bit sum. The grid is
-// 2^-61 of the largest coordinate; FIX_EPS_BITS keeps eps above 2^47 units, so a
+// 2^-61 of the largest coordinate; FIX_EPS_BITS keeps eps above 2^48 units, so a
 // pair at the softening length, the closest that matters, still has its
-// difference to 2^-47, and every longer one better. Systems that do not fit (no softening, a span above 2^14
+// difference to 2^-48, and every longer one better. Systems that do not fit (no softening, a span above 2^13
 // softening lengths, non-finite or extreme values) keep the FP64 kernels.
 #pragma once
 
@@ -30,17 +31,8 @@
 
 #include "dev_internal.cuh"
 
-struct FixGrid {
-    int ok;                  // 1: the system fits; 0: use the FP64 kernels
-    int g;                   // grid: X = x 2^g
-    int U3, U1;              // exponent of the last bit of an acceleration, a potential sum
-    unsigned eh;             // high word of eps 2^g
-    int e2s;                 // eps^2 in units of r2 (fix_pair): e2n >> (e2s - 2 s)
-    unsigned long long e2n;  // eps^2's significand, top bit at 61
-};
-
 constexpr int FIX_POS_BITS = 61; // |X| < 2^61
-constexpr int FIX_EPS_BITS = 47; // eps 2^g >= 2^47
+constexpr int FIX_EPS_BITS = 48; // eps 2^g >= 2^48
 
 // The grid of n bodies whose largest |coordinate| is xmax and largest mass
 // mmax (n mmax bounds the sums), with the given eps and eps^2.
@@ -72,6 +64,12 @@ __device__ inline FixGrid fix_grid(double xmax, double mmax, double n, double ep
     f.U1 = ilogb(n * mmax / eps) + 1 - 119;
     f.ok = 1;
     return f;
+}
+
+// 2^e as a double, -1000 <= e <= 1000.
+__device__ __forceinline__ double fix_pow2(int e)
+{
+    return __longlong_as_double((long long)(e + 1023) << 52);
 }
 
 __device__ __forceinline__ long long fix_pos(double x, double scale) // scale = 2^g
@@ -108,6 +106,13 @@ __device__ __forceinline__ unsigned long long mulhi(unsigned long long a, unsign
            hi32(mulw((unsigned)a, hi32(b)));
 }
 __device__ __forceinline__ long long mulws(int a, int b) { return (long long)a * b; }
+
+__device__ __forceinline__ unsigned long long sar_clamp(unsigned long long v, unsigned n)
+{
+    long long r; // PTX clamps the shift: n >= 64 gives the sign
+    asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"((long long)v), "r"(n));
+    return (unsigned long long)r;
+}
 
 // r^2 of a pair and its rsqrt seed.
 struct FixR {
@@ -174,6 +179,11 @@ struct Fix128 {
         const unsigned o2 = w == 0u ? t1 : w == 1u ? t2 : neg;
         const unsigned o1 = w == 0u ? t0 : w == 1u ? t1 : w == 2u ? t2 : neg;
         const unsigned o0 = w == 1u ? t0 : w == 2u ? t1 : w == 3u ? t2 : neg;
+        sum(o0, o1, o2, o3);
+    }
+    // adds another sum
+    __device__ __forceinline__ void sum(unsigned o0, unsigned o1, unsigned o2, unsigned o3)
+    {
         asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\t"
             "addc.cc.u32 %2, %2, %6;\n\taddc.u32 %3, %3, %7;"
             : "+r"(w0), "+r"(w1), "+r"(w2), "+r"(w3)
@@ -194,33 +204,55 @@ struct Fix128 {
     }
 };
 
-// Sum of m d / r^3 terms.
-struct FixSum3 {
-    Fix128 x, y, z;
+// 96-bit sum without the 128-bit sum's lowest word. Terms are cut downwards,
+// half a unit on average: value() puts back half of their count (a sum of
+// nothing, or of terms that are all zero, stays zero).
+struct Fix96 {
+    unsigned w0, w1, w2;
 
-    __device__ __forceinline__ void clear()
+    __device__ __forceinline__ void clear() { w0 = w1 = w2 = 0u; }
+    __device__ __forceinline__ void add(unsigned long long v, unsigned sh, unsigned neg)
     {
-        x.clear();
-        y.clear();
-        z.clear();
+        const unsigned hi = hi32(v) ^ neg, lo = (unsigned)v ^ neg;
+        const unsigned long long x = ((unsigned long long)hi << 32) | lo; // top bit: the sign
+        const unsigned long long top = sar_clamp(x, sh);
+        const unsigned low = sh < 32u ? lo << ((32u - sh) & 31u) : (unsigned)sar_clamp(x, sh - 32u);
+        sum(low, (unsigned)top, hi32(top));
     }
-    __device__ __forceinline__ void add(const FixGrid &f, long long dx, long long dy, long long dz,
-                                        unsigned long long mass)
+    __device__ __forceinline__ void sum(unsigned o0, unsigned o1, unsigned o2)
     {
-        const FixR p = fix_pair(f, dx, dy, dz);
-        const int q = (int)(((fix_e2(p.e57) >> 4) * 15u) >> 12); // 15/8 e^2 2^57
-        const long long c57 = p.e57 + (p.e57 >> 1) + q;
-        const unsigned long long C = (1ull << 63) + (unsigned long long)(c57 << 6); // (1 + c) 2^63
-        const unsigned long long W = mulw(p.Y, hi32(p.S)) + hi32(mulw(p.Y, (unsigned)p.S));
-        const unsigned long long F = mulhi(mulhi(W, C), mass & ~0x7ffull);
-        // F d 2^s = term 2^(64 - X)
-        const int X = 3 * p.ey + (int)((unsigned)mass & 0x7ffu) + 2 * p.s + 2 * f.g - 1543;
-        const unsigned sh = (unsigned)max(f.U3 - X + 64, 0);
-        x.add(mulhi(F, (unsigned long long)(p.x < 0 ? -p.x : p.x)), sh, (unsigned)p.nx);
-        y.add(mulhi(F, (unsigned long long)(p.y < 0 ? -p.y : p.y)), sh, (unsigned)p.ny);
-        z.add(mulhi(F, (unsigned long long)(p.z < 0 ? -p.z : p.z)), sh, (unsigned)p.nz);
+        asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+            : "+r"(w0), "+r"(w1), "+r"(w2)
+            : "r"(o0), "r"(o1), "r"(o2));
+    }
+    __device__ __forceinline__ double value(int U, int cnt) const
+    {
+        const long long hi = (long long)(((unsigned long long)w2 << 32) | w1);
+        if ((hi == 0 && w0 == 0u) || (hi == -1 && (unsigned)cnt >= 0u - w0))
+            return 0.0;
+        return ldexp(fma((double)hi, 0x1p32, (double)w0 + 0.5 * (double)cnt), U + 32);
     }
 };
+
+// Adds one term m d / r^3 to three sums.
+template <class Acc>
+__device__ __forceinline__ void fix_add3(const FixGrid &f, long long dx, long long dy, long long dz,
+                                         unsigned long long mass, Acc &x, Acc &y, Acc &z)
+{
+    const FixR p = fix_pair(f, dx, dy, dz);
+    const int q = (int)(((fix_e2(p.e57) >> 4) * 15u) >> 12); // 15/8 e^2 2^57
+    const long long c57 = p.e57 + (p.e57 >> 1) + q;
+    const unsigned long long C = (1ull << 63) + (unsigned long long)(c57 << 6); // (1 + c) 2^63
+    const unsigned long long W = mulw(p.Y, hi32(p.S)) + hi32(mulw(p.Y, (unsigned)p.S));
+    const unsigned long long F = mulhi(mulhi(W, C), mass & ~0x7ffull);
+    // F d 2^s = term 2^(64 - X)
+    const int X = 3 * p.ey + (int)((unsigned)mass & 0x7ffu) + 2 * p.s + 2 * f.g - 1543;
+    const unsigned sh = (unsigned)max(f.U3 - X + 64, 1);
+    const int any = (int)hi32(mass) >> 31; // a massless term is zero, of either sign
+    x.add(mulhi(F, (unsigned long long)(p.x < 0 ? -p.x : p.x)), sh, (unsigned)(p.nx & any));
+    y.add(mulhi(F, (unsigned long long)(p.y < 0 ? -p.y : p.y)), sh, (unsigned)(p.ny & any));
+    z.add(mulhi(F, (unsigned long long)(p.z < 0 ? -p.z : p.z)), sh, (unsigned)(p.nz & any));
+}
 
 // Sum of m / r terms.
 struct FixSum1 {

@@ -366,6 +366,10 @@ __global__ void k_root(DevScalars *sc, DevRoot *roots, int n_gal)
         if (failed)
             roots[g].n_alive = 0;
         root_cube(&roots[g]);
+        const DevRoot &r = roots[g];
+        const double far = fmax(fabs(r.c0[0]), fmax(fabs(r.c0[1]), fabs(r.c0[2]))) + r.hs0;
+        roots[g].fix_e = ilogb(far) + 1;
+        roots[g].fix_off = 0;
     }
     __syncthreads();
     if (threadIdx.x == 0) {

@@ -9,9 +9,9 @@
 //
 // FP64 walk: the drop-in precision (k_walk64ws). Openings decided as in the
 //   FP32 walk (equal to the reference's FP64 rounding); interactions queued
-//   and evaluated densely in FP64 by a second warp per task, with 1/r^3 from
-//   an FP32 rsqrt seed by integer arithmetic (one rounding), summed per child
-//   subtree of the root as the FP32 walk does; small systems split the same
+//   and evaluated densely by two further warps per task, on the integer pipes
+//   (dev_fixpair.cuh; in FP64 for systems that do not fit their grid), summed
+//   per child subtree of the root as the FP32 walk does; small systems split the same
 //   way (k_walk64ws_units), with the same bits. k_walk64_exact instead
 //   uses the reference's own operation sequence per step (1/(r2*sqrt(r2)),
 //   no fused multiply-add) — bit-identical results on the reference's own
@@ -25,6 +25,7 @@
 //   so the interaction set equals the FP64 walk's. Small systems with few
 //   tasks for the GPU are walked by eight warps per task, one per root child
 //   (k_walk32_units), with the same bits as one warp per task (k_walk32).
+#include "dev_fixpair.cuh"
 #include "dev_internal.cuh"
 
 namespace {
@@ -35,6 +36,7 @@ struct WalkArgs {
     const NodeW64 *w64;
     const NodeW32 *w32;
     const int *child; // 8 ids per cell
+    const FixBody *wfix; // cells on their systems' grids, or nullptr: FP64 pair terms
     const WalkTask *tasks;
     const DevRoot *roots;
     DevScalars *sc;
@@ -287,7 +289,7 @@ struct __align__(16) RoundShared {
     float4 box[2];                  // centre and half extents (rounded up) of the 32 bodies
     float rec[RND_PAIRS * RND_REC]; // staged cells, two per record: word 2 k + half of field k
     uint2 stk[RND_STACK];           // cell, lanes
-    unsigned open[CSG_WARP];        // lanes that opened undecided cell e
+    uint2 open[CSG_WARP];           // lanes that opened, and that take, undecided cell e
 };
 
 // Packed FP32 pairs (two lanes of one 64-bit register): each half rounds as
@@ -408,14 +410,6 @@ __device__ __forceinline__ void stage_none(float *rec, int e)
     rec[(e >> 1) * RND_REC + (e & 1) + 16] = 0.0f;
 }
 
-__device__ __forceinline__ unsigned staged_mask(const float *rec, int e)
-{
-    return __float_as_uint(rec[(e >> 1) * RND_REC + (e & 1) + 16]);
-}
-__device__ __forceinline__ int staged_cell(const float *rec, int e)
-{
-    return __float_as_int(rec[(e >> 1) * RND_REC + (e & 1) + 18]);
-}
 
 // What every sink knows of its lane: the body, its lane bit and minus its
 // position in FP32 parts, duplicated for packed use.
@@ -432,11 +426,15 @@ struct LanePos {
     }
 };
 
-// The sink's view of a round:
-//   accept(rec, n)  n accepted cells staged from rec, with the lanes that take
-//                   each (the lanes that reached it, less a leaf's own body)
-//   terms(...)      two undecided cells: differences, d^2, masses, whether
-//                   this lane takes each, and their ids
+// The sink's view of a round, by its kind:
+//   pair terms (BLOCKS false)
+//     accept(rec, n)  n accepted cells staged from rec, with the lanes that take
+//                     each (the lanes that reached it, less a leaf's own body)
+//     terms(...)      two undecided cells: differences, d^2, masses, whether
+//                     this lane takes each
+//   interaction lists (BLOCKS true)
+//     block(cell, w)  the round's cells, one per lane, and the lane's own takes:
+//                     bit j for lane j's cell
 //
 // A cell tested by every lane for itself, outside a round (the root; cells of
 // a subtree walked stackless). Sets take/open for the lane.
@@ -464,8 +462,26 @@ __device__ __forceinline__ void lane_test(const WalkArgs &a, const LaneBody &L, 
             take = decide64(a, cell, L.me);
         open = !take;
     }
-    sink.terms(pack2(dx, dx), pack2(dy, dy), pack2(dz, dz), pack2(d2, d2), pack2(A.w, A.w), take,
-               false, cell, cell);
+    if constexpr (Sink::BLOCKS)
+        sink.block(cell, take ? 1u : 0u);
+    else
+        sink.terms(pack2(dx, dx), pack2(dy, dy), pack2(dz, dz), pack2(d2, d2), pack2(A.w, A.w),
+                   take, false);
+}
+
+// 32 x 32 bit transpose across the warp: bit l of lane j's x becomes bit j of
+// lane l's result.
+__device__ __forceinline__ unsigned warp_transpose(unsigned x)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned m = 0x0000ffffu; // bits whose index has no 'k'
+#pragma unroll
+    for (int k = 16; k; k >>= 1) {
+        const unsigned y = __shfl_xor_sync(0xffffffffu, x, k);
+        x = (lane & k) ? (x & ~m) | ((y & ~m) >> k) : (x & m) | ((y & m) << k);
+        m ^= m << (k >> 1);
+    }
+    return x;
 }
 
 // The subtree of `top` for the lanes of `mask`, one cell per step in preorder
@@ -563,21 +579,21 @@ __device__ __forceinline__ void walk_rounds(const WalkArgs &a, RoundShared &sh, 
             c47 = __ldg(cp + 1);
         }
         const int na = __popc(bacc), nu = __popc(bund);
-        const int ub = (na + 1) & ~1; // place of the first undecided cell
+        // place of the first undecided cell (a list needs no accepted cell staged)
+        const int ub = Sink::BLOCKS ? 0 : (na + 1) & ~1;
         const int place = acc ? __popc(bacc & lt) : ub + __popc(bund & lt);
         unsigned tm = c.mask; // lanes that take an accepted cell: a leaf's own body does not
         if (c.body >= 0 && (unsigned)(c.first - L.pos0) < CSG_WARP)
             tm &= ~(1u << (c.first - L.pos0));
-        if (acc || und)
+        if ((acc && !Sink::BLOCKS) || und)
             stage_cell(sh.rec, place, c.A, c.B, tm, c.cell);
-        if (lane == 0 && (na & 1))
+        if (!Sink::BLOCKS && lane == 0 && (na & 1))
             stage_none(sh.rec, na);
         if (lane == 1 && (nu & 1))
             stage_none(sh.rec, ub + nu);
         __syncwarp();
-        if (STATS)
-            for (int e = 0; e < na; e++)
-                st.hits += (staged_mask(sh.rec, e) & L.bit) != 0u;
+        if (STATS && acc)
+            st.hits += __popc(tm);
         const u64 acck = pack2(a.acc_k, a.acc_k), opnk = pack2(a.opn_k, a.opn_k);
         for (int e = 0; e < nu; e += 2) {
             const ulonglong2 *r = (const ulonglong2 *)(sh.rec + ((ub + e) >> 1) * RND_REC);
@@ -601,14 +617,25 @@ __device__ __forceinline__ void walk_rounds(const WalkArgs &a, RoundShared &sh, 
             const bool take0 = act0 && acc0, take1 = act1 && acc1;
             const unsigned o0 = __ballot_sync(0xffffffffu, act0 && !acc0);
             const unsigned o1 = __ballot_sync(0xffffffffu, act1 && !acc1);
-            if (lane == 0)
-                *(uint2 *)&sh.open[e] = make_uint2(o0, o1);
+            if constexpr (Sink::BLOCKS) {
+                const unsigned t0 = __ballot_sync(0xffffffffu, take0);
+                const unsigned t1 = __ballot_sync(0xffffffffu, take1);
+                if (lane == 0)
+                    *(uint4 *)&sh.open[e] = make_uint4(o0, t0, o1, t1);
+            } else {
+                if (lane == 0) {
+                    sh.open[e].x = o0;
+                    sh.open[e + 1].x = o1;
+                }
+                sink.terms(ux, uy, uz, d2, q1.y, take0, take1);
+            }
             if (STATS)
                 st.hits += take0 + take1;
-            sink.terms(ux, uy, uz, d2, q1.y, take0, take1, t.z, t.w);
         }
         __syncwarp();
-        const unsigned om = opn ? c.mask : und ? sh.open[place - ub] : 0u;
+        const unsigned om = opn ? c.mask : und ? sh.open[place - ub].x : 0u;
+        if constexpr (Sink::BLOCKS)
+            sink.block(c.cell, warp_transpose(acc ? tm : und ? sh.open[place].y : 0u));
         const int ch[8] = {c03.x, c03.y, c03.z, c03.w, c47.x, c47.y, c47.z, c47.w};
         int cnt = 0;
         if (om) {
@@ -653,7 +680,8 @@ __device__ __forceinline__ void walk_rounds(const WalkArgs &a, RoundShared &sh, 
         }
         sp += total;
         __syncwarp();
-        sink.accept(sh.rec, na);
+        if constexpr (!Sink::BLOCKS)
+            sink.accept(sh.rec, na);
         __syncwarp(); // records read before they are staged again
     }
 }
@@ -707,6 +735,7 @@ __device__ __forceinline__ void kahan_add2(u64 &s, u64 &c, u64 v)
 constexpr int WSEGS = 8;
 
 struct Sum32 : LanePos {
+    static constexpr bool BLOCKS = false;
     u64 eps2;
     u64 bx, by, bz;             // current block
     u64 sx, sy, sz, cx, cy, cz; // compensated sums
@@ -757,8 +786,7 @@ struct Sum32 : LanePos {
         }
         fold();
     }
-    __device__ __forceinline__ void terms(u64 dx, u64 dy, u64 dz, u64 d2, u64 m, bool t0, bool t1,
-                                          int, int)
+    __device__ __forceinline__ void terms(u64 dx, u64 dy, u64 dz, u64 d2, u64 m, bool t0, bool t1)
     {
         pair(dx, dy, dz, add2(d2, eps2), m, t0, t1);
     }
@@ -953,38 +981,137 @@ __global__ void __launch_bounds__(WARPS * CSG_WARP, WALK32_RES / WARPS) k_walk32
 // useful work on (almost) every lane instead of once per traversal step for
 // the few lanes that interact at that step.
 
-// Loads queued entry s of the lane (its cell's centre of mass and mass), or
-// zeros when s >= count (no queue read, no cell read). With MARK a negative
-// entry is a segment marker (mk; nothing loaded).
-template <int Q64, bool MARK>
-__device__ __forceinline__ void q64_load(const WalkArgs &a, const int *q, int lane, int head, int s,
-                                         int count, double2 &p01, double2 &p23, bool &mk)
-{
-    p01 = make_double2(0.0, 0.0);
-    p23 = p01;
-    mk = false;
-    if (s < count) {
-        const int c = q[((head + s) & (Q64 - 1)) * CSG_WARP + lane];
-        if (MARK)
-            mk = c < 0;
-        if (!MARK || !mk) {
-            p01 = __ldg((const double2 *)&a.w64[c]);     // cx, cy
-            p23 = __ldg((const double2 *)&a.w64[c] + 1); // cz, m
+// Pair terms of the lane's body with queued cells: the cell's record, the
+// term added to the lane's sum, and the sum as doubles (without G) with the
+// next sum started.
+//
+// FP64, with m/r^3 by integers. The cells of even and of odd blocks (counted
+// from a segment's first) are summed apart and the two sums added: by one
+// consumer or two, with the same bits.
+template <int CONS>
+struct EvalF64 {
+    struct Rec {
+        double2 xy, zm;
+    };
+    const NodeW64 *cells;
+    double eps2, px, py, pz;
+    double s[3 - CONS][3]; // one consumer: both sums; two: its own
+
+    __device__ __forceinline__ EvalF64(const WalkArgs &a, const FixGrid &, int me)
+        : cells(a.w64), eps2(a.eps2), px(me >= 0 ? a.x[me] : 0.0), py(me >= 0 ? a.y[me] : 0.0),
+          pz(me >= 0 ? a.z[me] : 0.0)
+    {
+        clear();
+    }
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int k = 0; k < 3 - CONS; k++)
+            s[k][0] = s[k][1] = s[k][2] = 0.0;
+    }
+    __device__ __forceinline__ Rec load(int c) const
+    {
+        const double2 *w = (const double2 *)&cells[c];
+        return Rec{__ldg(w), __ldg(w + 1)};
+    }
+    __device__ __forceinline__ void term(const Rec &r, int odd)
+    {
+        const double dx = r.xy.x - px, dy = r.xy.y - py, dz = r.zm.x - pz;
+        const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
+        const double f = r.zm.y == 0.0 ? 0.0 : m_inv_r3_q(r.zm.y, r2);
+        double *t = s[0];
+        if (CONS == 1 && odd)
+            t = s[2 - CONS];
+        t[0] = fma(f, dx, t[0]);
+        t[1] = fma(f, dy, t[1]);
+        t[2] = fma(f, dz, t[2]);
+    }
+    static __device__ __forceinline__ void drop(Rec &r) { r.zm.y = 0.0; }
+    // another warp's sums of the same body (6 words a lane)
+    __device__ __forceinline__ void save(unsigned *o) const
+    {
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const u64 v = (u64)__double_as_longlong(s[0][d]);
+            o[(2 * d) * CSG_WARP] = (unsigned)v;
+            o[(2 * d + 1) * CSG_WARP] = (unsigned)(v >> 32);
         }
     }
-}
+    __device__ __forceinline__ void join(const unsigned *o)
+    {
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            s[0][d] += __longlong_as_double((long long)(((u64)o[(2 * d + 1) * CSG_WARP] << 32) |
+                                                        o[(2 * d) * CSG_WARP]));
+    }
+    __device__ __forceinline__ void close(double &x, double &y, double &z)
+    {
+        x = CONS == 1 ? s[0][0] + s[2 - CONS][0] : s[0][0];
+        y = CONS == 1 ? s[0][1] + s[2 - CONS][1] : s[0][1];
+        z = CONS == 1 ? s[0][2] + s[2 - CONS][2] : s[0][2];
+        clear();
+    }
+};
 
-__device__ __forceinline__ void q64_term(const WalkArgs &a, const double2 &p01, const double2 &p23,
-                                         double px, double py, double pz, double &sx, double &sy,
-                                         double &sz)
-{
-    const double dx = p01.x - px, dy = p01.y - py, dz = p23.x - pz;
-    const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, a.eps2)));
-    const double f = m_inv_r3_q(p23.y, r2);
-    sx = fma(f, dx, sx);
-    sy = fma(f, dy, sy);
-    sz = fma(f, dz, sz);
-}
+struct EvalFix { // integers from end to end, for systems on the grid
+    typedef FixBody Rec;
+    const FixBody *cells;
+    const FixGrid f;
+    long long px, py, pz;
+    Fix96 x, y, z;
+    int cnt; // terms in them
+
+    __device__ __forceinline__ EvalFix(const WalkArgs &a, const FixGrid &g, int me)
+        : cells(a.wfix), f(g)
+    {
+        const double scale = fix_pow2(f.g);
+        px = me >= 0 ? fix_pos(a.x[me], scale) : 0;
+        py = me >= 0 ? fix_pos(a.y[me], scale) : 0;
+        pz = me >= 0 ? fix_pos(a.z[me], scale) : 0;
+        clear();
+    }
+    __device__ __forceinline__ void clear()
+    {
+        x.clear();
+        y.clear();
+        z.clear();
+        cnt = 0;
+    }
+    __device__ __forceinline__ Rec load(int c) const
+    {
+        const longlong2 *w = (const longlong2 *)&cells[c];
+        const longlong2 xy = __ldg(w), zm = __ldg(w + 1);
+        return Rec{xy.x, xy.y, zm.x, (unsigned long long)zm.y};
+    }
+    __device__ __forceinline__ void term(const Rec &r, int)
+    {
+        fix_add3(f, r.x - px, r.y - py, r.z - pz, r.m, x, y, z);
+        cnt -= (int)hi32(r.m) >> 31; // massless ones do not count
+    }
+    static __device__ __forceinline__ void drop(Rec &r) { r.m = 0ull; }
+    // another warp's sums of the same body (10 words a lane)
+    __device__ __forceinline__ void save(unsigned *o) const
+    {
+        const unsigned w[10] = {x.w0, x.w1, x.w2, y.w0, y.w1, y.w2, z.w0, z.w1, z.w2, (unsigned)cnt};
+#pragma unroll
+        for (int k = 0; k < 10; k++)
+            o[k * CSG_WARP] = w[k];
+    }
+    __device__ __forceinline__ void join(const unsigned *o)
+    {
+        x.sum(o[0], o[CSG_WARP], o[2 * CSG_WARP]);
+        y.sum(o[3 * CSG_WARP], o[4 * CSG_WARP], o[5 * CSG_WARP]);
+        z.sum(o[6 * CSG_WARP], o[7 * CSG_WARP], o[8 * CSG_WARP]);
+        cnt += (int)o[9 * CSG_WARP];
+    }
+    __device__ __forceinline__ void close(double &ox, double &oy, double &oz)
+    {
+        ox = x.value(f.U3, cnt);
+        oy = y.value(f.U3, cnt);
+        oz = z.value(f.U3, cnt);
+        clear();
+    }
+};
 
 // A unit's segment partials: part[(3 * k + d) * pstride + body].
 __device__ __forceinline__ void put_partial(const WalkArgs &a, int k, int me, double sx, double sy,
@@ -995,114 +1122,78 @@ __device__ __forceinline__ void put_partial(const WalkArgs &a, int k, int me, do
     a.part[(3 * k + 2) * a.pstride + me] = sz;
 }
 
-// Evaluates the lane's next `count` queued entries (count >= 0; lanes without
-// a body pass 0 and never read their queue), two at a time in queue order.
-// The next two cells' loads are in flight while the current two are
-// evaluated (few consumer warps per SM at small N, each waiting on its
-// loads). MARK: a marker closes segment kc (its partial written, the sum
-// restarted).
-template <int Q64, bool MARK>
-__device__ __forceinline__ void q64_eval(const WalkArgs &a, const int *q, int lane, int &head,
-                                         int count, double px, double py, double pz,
-                                         double &sx, double &sy, double &sz, int me, int &kc)
-{
-    count = max(count, 0);
-    const int kmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)count);
-    double2 a01, a23, b01, b23;
-    bool ma, mb;
-    q64_load<Q64, MARK>(a, q, lane, head, 0, count, a01, a23, ma);
-    q64_load<Q64, MARK>(a, q, lane, head, 1, count, b01, b23, mb);
-    for (int s = 0; s < kmax; s += 2) {
-        double2 c01, c23, d01, d23;
-        bool mc, md;
-        q64_load<Q64, MARK>(a, q, lane, head, s + 2, count, c01, c23, mc);
-        q64_load<Q64, MARK>(a, q, lane, head, s + 3, count, d01, d23, md);
-        if (s < count) {
-            if (MARK && ma) { // rare
-                put_partial(a, kc++, me, sx, sy, sz);
-                sx = sy = sz = 0.0;
-            } else {
-                q64_term(a, a01, a23, px, py, pz, sx, sy, sz);
-            }
-        }
-        if (s + 1 < count) {
-            if (MARK && mb) {
-                put_partial(a, kc++, me, sx, sy, sz);
-                sx = sy = sz = 0.0;
-            } else {
-                q64_term(a, b01, b23, px, py, pz, sx, sy, sz);
-            }
-        }
-        a01 = c01;
-        a23 = c23;
-        b01 = d01;
-        b23 = d23;
-        ma = mc;
-        mb = md;
-    }
-    head += count;
-}
-
-// FP64 walk, producer/consumer form. Each task has two warps: the producer
-// walks the tree (in rounds, the FP32 decisions) and appends each lane's
-// accepted cells to that lane's ring in shared memory; the consumer evaluates
-// the rings in FP64, in the order the cells were accepted. The traversal
-// (FP32/ALU pipes) and the evaluation (FP64 pipe) then overlap on every SM
-// instead of alternating in one warp. The warps hand over through per-lane
-// head and tail counters in shared memory; every wait polls with a sleep and
-// gives up after a.wait_polls polls (recording CSG_ERR_DEVICE_WAIT, then both
-// warps leave the task). A pair of the split form (G > 0) walks G segments
-// of a task: the root step, then the subtrees of the root's children k0 ..
-// k0 + G - 1, with a marker (-1) queued on every lane between two segments.
-constexpr int WS_RING = 128;   // ring slots per lane (power of two)
-constexpr int WS_BATCH = 8;    // dense batch the consumer waits for; fewer entries a lane once
-                               // some lane's ring is half full (at 3/4: 1% slower at 1M; the
-                               // producer needs room for a round, 32 entries, on every lane)
+// FP64 walk, producer/consumer form. A task's producer warp walks the tree (in
+// rounds, the FP32 decisions) and queues every round's cells as a block in
+// shared memory, 32 cell ids and, per lane, the word of the cells that lane
+// takes; its consumer warps evaluate every lane's cells, each lane reading on
+// in the blocks at its own pace. The warps hand over through head and tail
+// block counters in shared memory; every wait polls with a sleep and gives up
+// after a.wait_polls polls (recording CSG_ERR_DEVICE_WAIT, then all warps leave
+// the task). A unit of the split form (G > 0) is G segments of a task: the root
+// step, then the subtrees of the root's children k0 .. k0 + G - 1; the first
+// block of a later segment is marked.
+//
+// Bound: the integer multiply and ALU pipes (65% and 62% busy at 1M, issue
+// 70%); the walk in FP64 was bound by the FP64 pipe (9 operations a pair).
+// Measured, walk inside the substep, FP64 pairs with a ring of ids per lane and
+// one consumer -> integer pairs -> blocks and two consumers: 1M 39.0 -> 33.0 ->
+// 24.8 ms, 100k merger 2.23 -> 1.97 -> 1.35 ms, 20k disk 0.496 -> 0.448 ->
+// 0.36 ms. Off the grid (FP64 pairs, same queue): 20k 0.48, 100k 2.0, 1M 41 ms.
+//
+// Blocks rather than a ring of ids per lane: an id costs 4 bytes a block, not
+// 4 bytes a lane that takes it, so the same memory holds several times the
+// lead, and lanes that take fewer of the current cells run dry less often. The
+// takes of a round reach the lanes by one bit transpose instead of a store per
+// cell and lane.
+constexpr int WS_BLOCKS = 32; // queue length (power of two; 16: 4% slower at 1M)
+constexpr int WS_RES = 21;    // resident warps per SM that the registers are sized for (18 and
+                              // 24: 2-5% slower at 1M)
+constexpr int WS_LOW = 2;     // blocks the slowest reader wants ahead before a step
 
 struct WsShared {
-    int ring[WS_RING * CSG_WARP]; // slot-major: ring[slot * 32 + lane]
-    int tail[CSG_WARP];           // published by the producer
-    int head[CSG_WARP];           // published by the consumer
-    int done;                     // producer finished (tails final)
-    int broken;                   // a wait gave up: both warps leave
+    int ids[WS_BLOCKS * CSG_WARP];
+    unsigned take[WS_BLOCKS * CSG_WARP];
+    int mark[WS_BLOCKS]; // 2 x segments closed before this block, + 1 for an odd block of its own
+    int tail;            // blocks published by the producer
+    int head[2];         // each consumer's first block that some lane still reads
+    int done;            // producer finished (tail final)
+    int half;            // the second consumer's sums are in `other`
+    int broken;          // a wait gave up: all warps leave
+    unsigned other[10 * CSG_WARP];
 };
 
 __device__ __forceinline__ int ws_load(const volatile int *p) { return *p; }
 
-// The producer's sink: every taken cell goes to the lane's ring.
-struct PushQueue : LanePos {
+// The producer's sink.
+struct BlockQueue : LanePos {
+    static constexpr bool BLOCKS = true;
     WsShared &sh;
     DevScalars *sc;
     int wait_polls;
-    int tail, head_seen, pairs;
+    int tail, head_seen, marks, parity, cons;
     bool mute, broken;
 
-    __device__ __forceinline__ PushQueue(const WalkArgs &a, const LaneBody &L, WsShared &s)
-        : LanePos(L), sh(s), sc(a.sc), wait_polls(a.wait_polls), tail(0), head_seen(0), pairs(0),
-          mute(false), broken(false)
+    __device__ __forceinline__ BlockQueue(const WalkArgs &a, const LaneBody &L, WsShared &s, int c)
+        : LanePos(L), sh(s), sc(a.sc), wait_polls(a.wait_polls), tail(0), head_seen(0), marks(0),
+          parity(0), cons(c), mute(false), broken(false)
     {
     }
-    __device__ __forceinline__ void publish()
+    // waits until a block is free
+    __device__ __forceinline__ void room()
     {
-        __threadfence_block(); // ring entries before the tail
-        ((volatile int *)sh.tail)[threadIdx.x & 31] = tail;
-    }
-    // waits (warp-uniform) until every lane's ring has room for n entries
-    __device__ __forceinline__ void room(int n)
-    {
-        bool full = tail - head_seen + n > WS_RING;
-        if (!__any_sync(0xffffffffu, full) || broken)
+        if (tail - head_seen < WS_BLOCKS || broken)
             return;
-        publish();
         for (int i = 0; i < wait_polls; i++) {
-            head_seen = ws_load(&sh.head[threadIdx.x & 31]);
-            full = tail - head_seen + n > WS_RING;
-            if (!__any_sync(0xffffffffu, full) || ws_load(&sh.broken))
+            head_seen = ws_load(&sh.head[0]);
+            if (cons == 2)
+                head_seen = min(head_seen, ws_load(&sh.head[1]));
+            if (tail - head_seen < WS_BLOCKS || ws_load(&sh.broken))
                 break;
             __nanosleep(64);
         }
-        __threadfence_block(); // heads read before slots are overwritten
-        if (__any_sync(0xffffffffu, full)) { // gave up (or the consumer did)
+        head_seen = __shfl_sync(0xffffffffu, head_seen, 0);
+        __threadfence_block(); // the head read before its blocks are overwritten
+        if (tail - head_seen >= WS_BLOCKS) { // gave up (or the consumer did)
             if ((threadIdx.x & 31) == 0) {
                 dev_fail(sc, CSG_ERR_DEVICE_WAIT);
                 ((volatile int *)&sh.broken)[0] = 1;
@@ -1110,37 +1201,34 @@ struct PushQueue : LanePos {
             broken = true;
         }
     }
-    __device__ __forceinline__ void put(bool want, int value) // after room()
+    __device__ __forceinline__ void block(int cell, unsigned take)
     {
-        if (want && !broken) {
-            sh.ring[(tail & (WS_RING - 1)) * CSG_WARP + (threadIdx.x & 31)] = value;
-            tail++;
-        }
-    }
-    __device__ __forceinline__ void accept(const float *rec, int n)
-    {
-        room(n);
-        for (int e = 0; e < n; e++) {
-            put(staged_mask(rec, e) & bit, staged_cell(rec, e));
-        }
-        publish();
-    }
-    __device__ __forceinline__ void terms(u64, u64, u64, u64, u64, bool t0, bool t1, int c0, int c1)
-    {
-        room(2);
-        put(t0 && !mute, c0);
-        put(t1 && !mute, c1);
-        if ((++pairs & 3) == 0)
-            publish();
+        if (mute || !__any_sync(0xffffffffu, take != 0u))
+            return;
+        room();
+        if (broken)
+            return;
+        const int lane = threadIdx.x & 31, b = tail & (WS_BLOCKS - 1);
+        sh.ids[b * CSG_WARP + lane] = cell;
+        sh.take[b * CSG_WARP + lane] = take;
+        if (lane == 0)
+            sh.mark[b] = 2 * marks + parity;
+        marks = 0;
+        parity ^= 1;
+        tail++;
+        __threadfence_block(); // the block before the tail
+        __syncwarp();
+        if (lane == 0)
+            ((volatile int *)&sh.tail)[0] = tail;
     }
 };
 
 template <bool STATS, int G>
 __device__ __forceinline__ void ws_produce(const WalkArgs &a, RoundShared &rs, WsShared &sh,
-                                           const TaskRange &tr, int k0, WalkStats &st)
+                                           const TaskRange &tr, int k0, int cons, WalkStats &st)
 {
     const LaneBody L = lane_body(a, rs, tr);
-    PushQueue q(a, L, sh);
+    BlockQueue q(a, L, sh, cons);
     q.mute = G > 0 && k0 != 0; // the root's terms are segment 0's
     const unsigned open = walk_root<STATS>(a, L, tr, q, st, !q.mute);
     q.mute = false;
@@ -1150,55 +1238,137 @@ __device__ __forceinline__ void ws_produce(const WalkArgs &a, RoundShared &rs, W
         if (c <= tr.root)
             continue;
         if (G == 0 || (k >= k0 && k < k0 + G)) {
-            if (G > 0 && k > k0) { // a segment marker
-                q.room(1);
-                q.put(L.valid, -1);
+            if (G > 0 && k > k0) {
+                q.marks++;
+                q.parity = 0;
             }
             walk_subtree<STATS>(a, rs, L, c, open, q, st);
         }
         k++;
     }
-    q.publish();
+    __threadfence_block();
     __syncwarp();
     if ((threadIdx.x & 31) == 0)
-        ((volatile int *)&sh.done)[0] = 1; // after every lane's final tail (fenced above)
+        ((volatile int *)&sh.done)[0] = 1; // after the final tail
 }
 
-template <int G>
-__device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, const TaskRange &tr,
-                                           int k0)
+// A lane's place in the queue: the cells left of its current block, and the
+// next block.
+struct WsReader {
+    unsigned left;
+    int cur, next, odd;
+};
+
+// The lane's next cell, or -1 (none published, or the next block has none for
+// it); marks gets the segments closed before it.
+template <int CONS>
+__device__ __forceinline__ int ws_next(const WsShared &sh, WsReader &r, int tail, int lane,
+                                       int &marks)
 {
+    if (r.left == 0u && r.next < tail) {
+        r.cur = r.next & (WS_BLOCKS - 1);
+        r.left = sh.take[r.cur * CSG_WARP + lane];
+        marks += sh.mark[r.cur] >> 1;
+        r.odd = sh.mark[r.cur] & 1;
+        r.next += CONS;
+    }
+    if (r.left == 0u)
+        return -1;
+    const int j = __ffs((int)r.left) - 1;
+    r.left &= r.left - 1u;
+    return sh.ids[r.cur * CSG_WARP + j];
+}
+
+// A segment's end: its partial written, the sum restarted.
+template <class Eval>
+__device__ __forceinline__ void ws_close(const WalkArgs &a, Eval &ev, int me, int &kc, int n)
+{
+    for (; n > 0; n--) {
+        double x, y, z;
+        ev.close(x, y, z);
+        if (me >= 0)
+            put_partial(a, kc, me, x, y, z);
+        kc++;
+    }
+}
+
+// Cells a lane evaluates between two looks at the counters: whole tasks (16:
+// 2-5% faster from 100k bodies on), a split task's units (8: 5% faster at 20k).
+constexpr int WS_STEP_TASK = 16, WS_STEP_UNIT = 8;
+
+// Consumer `which` of CONS: the blocks which, which + CONS, ...
+template <int G, int CONS, class Eval>
+__device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, const TaskRange &tr,
+                                           const FixGrid &grid, int k0, int which)
+{
+    static_assert(CONS == 1 || G <= 1, "a segment end inside a unit is one consumer's");
     const int lane = threadIdx.x & 31;
     const bool valid = lane < tr.count;
     const int me = valid ? a.perm[tr.pos0 + lane] : -1;
-    const double px = valid ? a.x[me] : 0.0, py = valid ? a.y[me] : 0.0,
-                 pz = valid ? a.z[me] : 0.0;
-    double sx = 0.0, sy = 0.0, sz = 0.0;
-    int head = 0, polls = 0, kc = k0; // kc: the segment being summed (split form)
+    Eval ev(a, grid, me);
+    WsReader rd{0u, 0, which, 0};
+    int polls = 0, head = which, kc = k0; // kc: the segment being summed (split form)
+    // two cells are always on their way: their loads run during the terms of
+    // the two before them (massless ones at first)
+    typename Eval::Rec ra = ev.load(0), rb = ra;
+    ev.drop(ra);
+    ev.drop(rb);
+    int ma = 0, mb = 0; // 2 x segments closed before each, + 1 for an odd block's
+    auto terms = [&]() {
+        if (G > 1 && ma > 1) // rare
+            ws_close(a, ev, me, kc, ma >> 1);
+        ev.term(ra, ma & 1);
+        if (G > 1 && mb > 1)
+            ws_close(a, ev, me, kc, mb >> 1);
+        ev.term(rb, mb & 1);
+    };
     while (true) {
-        const bool done = ws_load(&sh.done) != 0; // read before the tails: they are final then
+        // read before the tail: it is final then
+        const bool done = __shfl_sync(0xffffffffu, ws_load(&sh.done), 0) != 0;
         __threadfence_block();
-        const int tail = ws_load(&sh.tail[lane]);
-        __threadfence_block(); // the tail before the entries it covers
-        const int avail = valid ? tail - head : 0;
-        const int amin = (int)__reduce_min_sync(0xffffffffu, (unsigned)(valid ? avail : INT_MAX));
-        const int amax = (int)__reduce_max_sync(0xffffffffu, (unsigned)avail);
-        int take = 0;
-        if (amin >= WS_BATCH)
-            take = amin; // dense: every lane has work
-        else if (done || amax >= WS_RING / 2)
-            take = -1; // the rest (done), or relief for a lane without room for a round's entries
-        if (take != 0) {
-            const int n = take > 0 ? (valid ? take : 0) : min(avail, done ? avail : WS_BATCH);
-            q64_eval<WS_RING, (G > 1)>(a, sh.ring, lane, head, n, px, py, pz, sx, sy, sz, me, kc);
-            __threadfence_block(); // entries read before the head is published
-            ((volatile int *)sh.head)[lane] = head;
+        const int tail = __shfl_sync(0xffffffffu, ws_load(&sh.tail), 0);
+        __threadfence_block(); // the tail before the blocks it covers
+        __syncwarp();
+        // blocks that the furthest lane still has ahead
+        const int ahead =
+            tail - (int)__reduce_max_sync(0xffffffffu, (unsigned)(valid ? rd.next : 0));
+        if (ahead >= WS_LOW || tail - head >= WS_BLOCKS || (done && head < tail)) {
+            auto fetch = [&](typename Eval::Rec &r, int &mk) {
+                int m = 0;
+                const int c = ws_next<CONS>(sh, rd, tail, lane, m);
+                r = ev.load(max(c, 0));
+                if (c < 0) // any cell was read: a massless term
+                    ev.drop(r);
+                mk = CONS == 1 ? 2 * m + rd.odd : 0;
+            };
+#pragma unroll 1
+            for (int s = 0; s < (G == 0 ? WS_STEP_TASK : WS_STEP_UNIT); s += 2) {
+                typename Eval::Rec rc, rq;
+                int mc, md;
+                fetch(rc, mc);
+                fetch(rq, md);
+                terms();
+                ra = rc;
+                rb = rq;
+                ma = mc;
+                mb = md;
+            }
+            // blocks that every lane is through with
+            const int h = (int)__reduce_min_sync(
+                0xffffffffu, (unsigned)(!valid ? tail + CONS : rd.left ? rd.next - CONS : rd.next));
+            __threadfence_block(); // blocks read before the head is published
+            __syncwarp();
+            if (h != head && lane == 0)
+                ((volatile int *)sh.head)[which] = h;
+            head = h;
             polls = 0;
-            if (done && __all_sync(0xffffffffu, !valid || head == tail))
-                break;
             continue;
         }
-        if (ws_load(&sh.broken))
+        if (done) { // head == tail: every block read
+            terms();
+            break;
+        }
+        if (__any_sync(0xffffffffu, ws_load(&sh.broken)))
             return;
         if (++polls >= a.wait_polls) {
             if (lane == 0) {
@@ -1209,99 +1379,169 @@ __device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, cons
         }
         __nanosleep(64);
     }
-    if (valid && G > 0) { // the last segment's partial (segment 0's with the root's term),
-        put_partial(a, kc, me, sx, sy, sz); // zeros for segments the walk did not reach
-        for (int kk = kc + 1; kk < k0 + G; kk++)
-            put_partial(a, kk, me, 0.0, 0.0, 0.0);
-    } else if (valid) {
-        a.ax[me] = a.G * sx;
-        a.ay[me] = a.G * sy;
-        a.az[me] = a.G * sz;
+    if constexpr (CONS == 2) { // the sums joined (integers: exact)
+        if (which == 1) {
+            ev.save(sh.other + lane);
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0)
+                ((volatile int *)&sh.half)[0] = 1;
+            return;
+        }
+        for (int i = 0; !__any_sync(0xffffffffu, ws_load(&sh.half)); i++) {
+            if (i >= a.wait_polls || __any_sync(0xffffffffu, ws_load(&sh.broken))) {
+                if (lane == 0) {
+                    dev_fail(a.sc, CSG_ERR_DEVICE_WAIT);
+                    ((volatile int *)&sh.broken)[0] = 1;
+                }
+                return;
+            }
+            __nanosleep(64);
+        }
+        __threadfence_block();
+        __syncwarp();
+        ev.join(sh.other + lane);
+    }
+    if (G > 0) { // the last segment's partial (segment 0's with the root's term),
+        ws_close(a, ev, me, kc, k0 + G - kc); // zeros for segments the walk did not reach
+    } else {
+        double sx, sy, sz;
+        ev.close(sx, sy, sz);
+        if (valid) {
+            a.ax[me] = a.G * sx;
+            a.ay[me] = a.G * sy;
+            a.az[me] = a.G * sz;
+        }
     }
 }
 
-// PAIRS producer/consumer pairs per block (task t of the grid is pair
-// t % PAIRS of block t / PAIRS), 10 pairs per SM either way (shared memory): one pair for
-// launches of few tasks (finer blocks balance better over the SMs), two
-// otherwise (measured faster from ~100k bodies on).
-// One producer/consumer pair per task (G == 0) or per unit of G segments,
-// u = (8 / G) * task + k0 / G (partials into a.part).
-template <bool STATS, int PAIRS, int G>
+// One task per block (G == 0), or one unit of G segments of a task,
+// u = (8 / G) * task + k0 / G (partials into a.part): the producer warp, then
+// CONS consumers. Two consumers where the split does not mark segment ends
+// inside a unit: the producer needs about a fifth of a consumer's time, and
+// the sums of two join to the same bits.
+template <bool STATS, int G, int CONS>
 __device__ __forceinline__ void walk64ws_body(const WalkArgs &a)
 {
-    __shared__ WsShared sh_all[PAIRS];
-    __shared__ RoundShared rs_all[PAIRS];
-    const int warp = threadIdx.x >> 5, pair = warp >> 1, lane = threadIdx.x & 31;
-    WsShared &sh = sh_all[pair];
+    __shared__ WsShared sh;
+    __shared__ RoundShared rs;
+    const int warp = threadIdx.x >> 5;
     const int nn = a.sc->n_nodes;
     if (nn > a.node_cap || nn < 1)
         return;
-    const int u = blockIdx.x * PAIRS + pair;
+    const int u = blockIdx.x;
     const int t = G > 0 ? u / (8 / G) : u, k0 = G > 0 ? (u % (8 / G)) * G : 0;
-    TaskRange tr{0, 0, 0, 0, false};
-    bool ok = t < a.sc->n_tasks;
-    if (ok) {
-        const WalkTask w = a.tasks[t];
-        const DevRoot &r = a.roots[w.gal];
-        tr = TaskRange{w.pos0, w.count, r.root, r.end, small_system(a, w.gal)};
-        if (G > 0 ? !tr.small : (tr.small && a.skip_small)) {
-            ok = false; // the other form walks this system
-        } else if (tr.root < 0 || tr.end > nn || tr.root >= tr.end) {
-            if ((warp & 1) == 0 && lane == 0)
-                dev_fail(a.sc, CSG_ERR_WALK_LIMIT);
-            ok = false;
-        }
+    if (t >= a.sc->n_tasks)
+        return;
+    const WalkTask w = a.tasks[t];
+    const DevRoot &r = a.roots[w.gal];
+    const TaskRange tr{w.pos0, w.count, r.root, r.end, small_system(a, w.gal)};
+    if (G > 0 ? !tr.small : (tr.small && a.skip_small))
+        return; // the other form walks this system
+    if (tr.root < 0 || tr.end > nn || tr.root >= tr.end) {
+        if (threadIdx.x == 0)
+            dev_fail(a.sc, CSG_ERR_WALK_LIMIT);
+        return;
     }
-    if (ok && (warp & 1) == 0) {
-        sh.tail[lane] = 0;
-        sh.head[lane] = 0;
-        if (lane == 0) {
-            sh.done = 0;
-            sh.broken = 0;
-        }
+    const bool fix = a.wfix && r.fix.ok && !r.fix_off;
+    if (threadIdx.x == 0) {
+        sh.tail = 0;
+        sh.head[0] = 0;
+        sh.head[1] = 1;
+        sh.done = 0;
+        sh.half = 0;
+        sh.broken = 0;
     }
-    __syncthreads(); // every thread: counters set before either warp of any pair starts
-    if (!ok)
-        return; // both warps of the pair
-    WalkStats st;
-    if ((warp & 1) == 0)
-        ws_produce<STATS, G>(a, rs_all[pair], sh, tr, k0, st);
-    else
-        ws_consume<G>(a, sh, tr, k0);
-    if (STATS && (warp & 1) == 0)
-        add_hits(a, st);
+    __syncthreads(); // counters set before any warp starts (the returns above are the block's)
+    if (warp == 0) {
+        WalkStats st;
+        ws_produce<STATS, G>(a, rs, sh, tr, k0, CONS, st);
+        if (STATS)
+            add_hits(a, st);
+    } else if (fix) {
+        ws_consume<G, CONS, EvalFix>(a, sh, tr, r.fix, k0, warp - 1);
+    } else {
+        ws_consume<G, CONS, EvalF64<CONS>>(a, sh, tr, r.fix, k0, warp - 1);
+    }
 }
 
-template <bool STATS, int PAIRS>
-__global__ void __launch_bounds__(2 * PAIRS * CSG_WARP, 20 / (2 * PAIRS)) k_walk64ws(WalkArgs a)
+template <bool STATS>
+__global__ void __launch_bounds__(3 * CSG_WARP, WS_RES / 3) k_walk64ws(WalkArgs a)
 {
-    walk64ws_body<STATS, PAIRS, 0>(a);
+    walk64ws_body<STATS, 0, 2>(a);
 }
 
-// The FP64 walk split by the root's children (trees built here, few tasks
-// for the GPU): partials into a.part, summed by k_walk_sum; the same bits as
-// k_walk64ws.
-template <bool STATS, int PAIRS, int G>
-__global__ void __launch_bounds__(2 * PAIRS * CSG_WARP, 20 / (2 * PAIRS)) k_walk64ws_units(WalkArgs a)
+// The FP64 walk split by the root's children (few tasks for the GPU): partials
+// into a.part, summed by k_walk_sum; the same bits for every G.
+template <bool STATS, int G>
+__global__ void __launch_bounds__((G == 1 ? 3 : 2) * CSG_WARP, WS_RES / (G == 1 ? 3 : 2))
+    k_walk64ws_units(WalkArgs a)
 {
-    walk64ws_body<STATS, PAIRS, G>(a);
+    walk64ws_body<STATS, G, (G == 1 ? 2 : 1)>(a);
 }
 
-// Dead bodies get a = 0 (src/octree.c:226-230); alive ones are overwritten by
-// the walk.
-// Also rewinds the task counter of the persistent walks.
-__global__ void k_zero_acc(const double *__restrict__ m, double *ax, double *ay, double *az, int n,
-                           DevScalars *sc)
+// Before a walk: dead bodies get a = 0 (src/octree.c:226-230; alive ones are
+// overwritten by the walk), the task counter of the persistent walks is
+// rewound, and for an FP64 walk (FIX) every system's grid is set up and its
+// cells put on it (ee: |eps| < 2^ee).
+template <bool FIX>
+__global__ void k_walk_prep(const double *__restrict__ m, double *ax, double *ay, double *az, int n,
+                            DevScalars *sc, DevRoot *roots, int n_gal,
+                            const NodeW64 *__restrict__ w64, const NodeLink *__restrict__ link,
+                            const int *__restrict__ sgid, const int *__restrict__ child,
+                            FixBody *__restrict__ wfix, int node_cap, double eps, double eps2,
+                            int ee, bool imported)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     if (i == 0)
         sc->task_next = 0;
-    if (i >= n)
+    for (int k = i; k < n; k += stride) {
+        if (m[k] <= 0.0) {
+            ax[k] = 0.0;
+            ay[k] = 0.0;
+            az[k] = 0.0;
+        }
+    }
+    if (!FIX)
         return;
-    if (m[i] <= 0.0) {
-        ax[i] = 0.0;
-        ay[i] = 0.0;
-        az[i] = 0.0;
+    const int nn = sc->n_nodes;
+    if (nn > node_cap)
+        return; // no walk
+    for (int g = i; g < n_gal; g += stride) {
+        DevRoot &r = roots[g];
+        if (r.n_alive > 0) {
+            const double far = fmax(fabs(r.c0[0]), fmax(fabs(r.c0[1]), fabs(r.c0[2]))) + r.hs0;
+            r.fix = fix_grid(far, w64[r.root].m, 1.0, eps, eps2);
+        }
+    }
+    for (int id = i; id < nn; id += stride) {
+        const int e = max(roots[n_gal > 1 ? sgid[link[id].first] : 0].fix_e, ee);
+        const double scale = fix_pow2(min(max(FIX_POS_BITS - e, -1000), 1000));
+        const double2 *w = (const double2 *)&w64[id];
+        const double2 xy = w[0], zm = w[1];
+        longlong2 *o = (longlong2 *)&wfix[id];
+        o[0] = make_longlong2(fix_pos(xy.x, scale), fix_pos(xy.y, scale));
+        o[1] = make_longlong2(fix_pos(zm.x, scale), (long long)fix_mass(zm.y));
+        if (!imported)
+            continue;
+        // a caller's cell may lie anywhere and weigh anything: off the grid, or
+        // not the sum of its children (which bounds the sums), and the whole
+        // system keeps the FP64 pair terms
+        const double lim = ldexp(1.0, e);
+        bool good = fabs(xy.x) < lim && fabs(xy.y) < lim && fabs(zm.x) < lim &&
+                    (zm.y == 0.0 || (zm.y >= 0x1p-1000 && zm.y <= 0x1p200));
+        double sum = 0.0;
+        bool any = false;
+        for (int q = 0; q < 8; q++) {
+            const int c = child[8 * (size_t)id + q];
+            if (c > id) {
+                sum += w64[c].m;
+                any = true;
+            }
+        }
+        good = good && (!any || fabs(sum - zm.y) <= 1e-6 * zm.y);
+        if (!good)
+            roots[0].fix_off = 1;
     }
 }
 
@@ -1311,28 +1551,24 @@ __global__ void k_zero_acc(const double *__restrict__ m, double *ax, double *ay,
 // writes (offs from an exclusive scan of the counts).
 template <bool FILL>
 struct ListSink : LanePos {
+    static constexpr bool BLOCKS = true;
     int *ids;
     int k, lim;
 
     __device__ __forceinline__ ListSink(const LaneBody &L) : LanePos(L), ids(nullptr), k(0), lim(0) {}
-    __device__ __forceinline__ void put(bool want, int cell)
+    __device__ __forceinline__ void block(int cell, unsigned take)
     {
-        if (want) {
-            if (FILL && k < lim)
-                ids[k] = cell;
-            k++;
+        if (!FILL) {
+            k += __popc(take);
+            return;
         }
-    }
-    __device__ __forceinline__ void accept(const float *rec, int n)
-    {
-        for (int e = 0; e < n; e++) {
-            put(staged_mask(rec, e) & bit, staged_cell(rec, e));
+        while (__any_sync(0xffffffffu, take != 0u)) { // each lane its own cells, one a step
+            const int c = __shfl_sync(0xffffffffu, cell, __ffs((int)take) - 1);
+            if (take != 0u && k < lim)
+                ids[k] = c;
+            k += take != 0u;
+            take &= take - 1u;
         }
-    }
-    __device__ __forceinline__ void terms(u64, u64, u64, u64, u64, bool t0, bool t1, int c0, int c1)
-    {
-        put(t0, c0);
-        put(t1, c1);
     }
 };
 
@@ -1373,6 +1609,7 @@ WalkArgs walk_args(csgd_t *d, const csgd_force_params *p)
     a.w64 = d->w64;
     a.w32 = d->w32;
     a.child = d->child;
+    a.wfix = nullptr;
     a.tasks = d->tasks;
     a.roots = d->roots;
     a.sc = d->sc;
@@ -1472,31 +1709,26 @@ void launch_walk(csgd_t *d, const WalkArgs &a, int precision, int exact)
             int g = 1;
             while (g < WSEGS && tasks * (WSEGS / g) > 4LL * 12 * d->num_sms)
                 g *= 2;
-            const long long nu = tasks * (WSEGS / g);
-            const int pairs = nu > 8LL * d->num_sms ? 2 : 1;
-            const int gw = (int)((nu + pairs - 1) / pairs);
+            const int gw = (int)(tasks * (WSEGS / g));
             b.part = d->wpart;
             b.pstride = d->wpart_cap;
-#define CSG_U(ST, P, GG) k_walk64ws_units<ST, P, GG><<<gw, 2 * P * CSG_WARP, 0, s>>>(b)
-#define CSG_UG(ST, P)                                                                              \
+#define CSG_U(ST, GG)                                                                              \
+    k_walk64ws_units<ST, GG><<<gw, (GG == 1 ? 3 : 2) * CSG_WARP, 0, s>>>(b)
+#define CSG_UG(ST)                                                                                 \
     do {                                                                                          \
         if (g == 1)                                                                               \
-            CSG_U(ST, P, 1);                                                                      \
+            CSG_U(ST, 1);                                                                         \
         else if (g == 2)                                                                          \
-            CSG_U(ST, P, 2);                                                                      \
+            CSG_U(ST, 2);                                                                         \
         else if (g == 4)                                                                          \
-            CSG_U(ST, P, 4);                                                                      \
+            CSG_U(ST, 4);                                                                         \
         else                                                                                      \
-            CSG_U(ST, P, 8);                                                                      \
+            CSG_U(ST, 8);                                                                         \
     } while (0)
-            if (pairs == 2 && stats)
-                CSG_UG(true, 2);
-            else if (pairs == 2)
-                CSG_UG(false, 2);
-            else if (stats)
-                CSG_UG(true, 1);
+            if (stats)
+                CSG_UG(true);
             else
-                CSG_UG(false, 1);
+                CSG_UG(false);
 #undef CSG_UG
 #undef CSG_U
             k_walk_sum<<<csgd_grid(d->n, 256), 256, 0, s>>>(d->wpart, (long long)d->wpart_cap,
@@ -1507,17 +1739,10 @@ void launch_walk(csgd_t *d, const WalkArgs &a, int precision, int exact)
                 return; // every system is small
         }
         const long long tasks = (long long)d->n / CSG_WARP + d->n_gal + 1; // >= n_tasks
-        const int pairs = tasks > 8LL * d->num_sms ? 2 : 1;
-        const int gw = (int)((tasks + pairs - 1) / pairs);
-        const int threads = 2 * pairs * CSG_WARP;
-        if (pairs == 2 && stats)
-            k_walk64ws<true, 2><<<gw, threads, 0, s>>>(b);
-        else if (pairs == 2)
-            k_walk64ws<false, 2><<<gw, threads, 0, s>>>(b);
-        else if (stats)
-            k_walk64ws<true, 1><<<gw, threads, 0, s>>>(b);
+        if (stats)
+            k_walk64ws<true><<<(int)tasks, 3 * CSG_WARP, 0, s>>>(b);
         else
-            k_walk64ws<false, 1><<<gw, threads, 0, s>>>(b);
+            k_walk64ws<false><<<(int)tasks, 3 * CSG_WARP, 0, s>>>(b);
     }
     d->launches++;
 }
@@ -1539,7 +1764,17 @@ extern "C" int csgd_gravity_ex(csgd_t *d, const csgd_force_params *p, int exact)
         if (rc)
             return rc;
     }
-    { k_zero_acc<<<csgd_grid(n, 256), 256, 0, s>>>(d->m, d->ax, d->ay, d->az, n, d->sc); d->launches++; }
+    const bool fix = p->precision == CSG_PREC_FP64 && !exact && d->wfix &&
+                     d->wfix_cap >= d->node_cap;
+    a.wfix = fix ? d->wfix : nullptr;
+    if (fix) {
+        const double e = fabs(p->softening);
+        const int ee = e > 0.0 && isfinite(e) ? ilogb(e) + 1 : -2000;
+        k_walk_prep<true><<<csgd_grid(2LL * n + 64, 256), 256, 0, s>>>(d->m, d->ax, d->ay, d->az, n, d->sc, d->roots, d->n_gal, d->w64, d->link, d->sgid, d->child, d->wfix, d->node_cap, p->softening, a.eps2, ee, d->imported != 0);
+    } else {
+        k_walk_prep<false><<<csgd_grid(n, 256), 256, 0, s>>>(d->m, d->ax, d->ay, d->az, n, d->sc, d->roots, d->n_gal, d->w64, d->link, d->sgid, d->child, nullptr, d->node_cap, 0.0, 0.0, 0, false);
+    }
+    d->launches++;
     if (exact) {
         const int saved = d->walk_warps;
         d->walk_warps = 8;

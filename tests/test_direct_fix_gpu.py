@@ -1,6 +1,6 @@
 """The direct sum and the energy on the integer pipes where their tiles, rows
 and grid can go wrong: sizes around 128 and 256, uneven masses, and bodies off
-the grid (no softening, a span of more than 2^14 softening lengths), which keep
+the grid (no softening, a span of more than 2^13 softening lengths), which keep
 the FP64 kernels. Against the oracle; 1e-12 as in test_diagnostics_gpu.py, for
 accelerations relative to the largest one (terms round relative to themselves)."""
 import numpy as np

@@ -34,7 +34,7 @@ def grid(xmax, eps):
     ex = math.frexp(max(xmax, eps))[1]
     g = 61 - ex
     E = int(math.ldexp(eps, g))
-    assert E >= 1 << 47
+    assert E >= 1 << 48
     mant, e = math.frexp(eps * eps)
     S, k = int(mant * 2**53), e - 53
     return dict(g=g, eh=E >> 32, e2n=S << 9, e2s=64 + 9 - k - 2 * g)
@@ -120,7 +120,7 @@ def test_pair_terms_against_rationals():
     rng = random.Random(11)
     for trial in range(4000):
         xmax = 2.0 ** rng.uniform(-20, 30)
-        eps = xmax * 2.0 ** rng.uniform(-12.9, 1)
+        eps = xmax * 2.0 ** rng.uniform(-11.9, 1)
         mmax = 2.0 ** rng.uniform(-40, 40)
         f = grid(xmax, eps)
         lim = min(int(math.ldexp(xmax, f["g"])), (1 << 61) - 1)
@@ -162,3 +162,19 @@ def test_sum_places_terms():
             if neg:
                 want = (-want - 1) % (1 << 128)
             assert got == want, (sh, neg)
+
+
+def test_short_sum_places_terms():
+    """Fix96::add: the 128-bit sum's term without its lowest word, cut downwards."""
+    rng = random.Random(6)
+    for sh in list(range(1, 100)) + [160, 500]:
+        for neg in (0, M32):
+            v = rng.randrange(1 << 63)
+            x = ((v >> 32) ^ neg) << 32 | ((v & M32) ^ neg)
+            sx = x - (1 << 64) if x >> 63 else x
+            top = (sx >> min(sh, 63)) & M64
+            low = ((x & M32) << (32 - sh)) & M32 if sh < 32 else (sx >> min(sh - 32, 63)) & M32
+            got = top << 32 | low
+            want = ((v << 32) >> sh) if not neg else ((-v - 1) << 32) >> sh
+            slack = 0 if not neg or sh >= 32 else (1 << (32 - sh)) - 1
+            assert 0 <= (got - want) % (1 << 96) <= slack, (sh, neg)

@@ -58,17 +58,50 @@ def test_small_and_ragged_systems(lib, orc, n, theta):
     check(lib, orc, lib.generate_ics(0, n, 40 + n), theta)
 
 
+@pytest.mark.parametrize("n", [33, 2049, 70001])
+@pytest.mark.parametrize("eps", [1e-5, 40.0])
+def test_softenings_off_and_far_inside_the_grid(lib, orc, n, eps):
+    """The FP64 walk's pair terms run on integers while the span is at most
+    2^13 softening lengths, else in FP64 (the first of the two)."""
+    check(lib, orc, lib.generate_ics(0, n, 60), 0.5, eps)
+
+
 @pytest.mark.parametrize("k", [16, 32])
 def test_full_octree_with_every_cell_opened(lib, orc, k):
     check(lib, orc, lattice(k, 7), 0.0)
 
 
+@pytest.mark.parametrize("eps", [0.01, 1e-5])
+def test_ensemble_systems_equal_themselves_alone(lib, eps):
+    """FP64: 72,000 bodies in systems of 9,000 take several child subtrees of the
+    root per unit, one system alone one: the same bits, on the grid and off."""
+    from cosmosim_gb300.lib import Sim
+
+    parts = [lib.generate_ics(3, 9000, 80 + g) for g in range(8)]
+    out = np.zeros(72000, dtype=BODY_DTYPE)
+    for g, p in enumerate(parts):
+        out[9000 * g:9000 * (g + 1)] = p
+    ens = Sim.ensemble(out, [9000] * 8, softening=eps)
+    got = fields(ens.bodies())
+    ens.close()
+    for g in (0, 5):
+        one = Sim.from_bodies(parts[g], softening=eps)
+        np.testing.assert_array_equal(got[9000 * g:9000 * (g + 1)], fields(one.bodies()))
+        one.close()
+
+
 @pytest.mark.parametrize("theta", [0.0, 0.5])
-def test_caller_pool_walks(lib, orc, theta):
+@pytest.mark.parametrize("spoil", ["no", "far", "heavy"])
+def test_caller_pool_walks(lib, orc, theta, spoil):
     """octree_compute_forces on a pool that the oracle built (its child table is
-    made by the import)."""
+    made by the import), also with a cell far outside the bodies' box or heavier
+    than its children."""
     b = lattice(8, 3)
     pool, _ = orc.octree_build(b)
+    if spoil == "far":
+        pool["cx"][70] = 1e4
+    elif spoil == "heavy":
+        pool["total_mass"][9] = 1e9
     want = b.copy()
     orc.octree_compute_forces(pool, want, 1.0, 0.02, theta)
     lib.octree_compute_forces(pool, b, 1.0, 0.02, theta)
