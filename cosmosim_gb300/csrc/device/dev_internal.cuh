@@ -240,6 +240,7 @@ struct csgd {
     int *nb_count;
     double *pr2, *cs; // SPH per-body force terms
     double *sph_term; // SPH pair terms, 3 x 128 x cap (slot-major)
+    float4 *sph_sorted; // sorted body records, then their boxes (k_sph_sort)
     int *sph_relist;  // per gas slot: 1 when the density pass changed h
     int nb_cap;
 
@@ -277,6 +278,7 @@ struct csgd {
     int graph_export_cap;
     int use_graphs;
     int imported;  // the tree came from a caller pool (no sorted order)
+    int gas_zero;  // sc->n_gas is 0 when the work queued so far is done
     int gas_valid; // d->gas / n_gas match the current tree
 };
 

@@ -4,8 +4,8 @@
 //
 // Neighbour order matters: the reference keeps the first 128 bodies within
 // the radius in depth-first octant order (src/octree.c:260-277, sph.h:9), and
-// the cap binds often. Walking the preorder tree with per-lane subtree skips
-// (as in dev_walk.cu) meets the leaves in exactly that order. Each pass runs in
+// the cap binds often. The sorted order of a tree built here is that order; in
+// a caller's pool the preorder cells meet the leaves in it. Each pass runs in
 // two kernels: the walk records every gas body's capped list, then a pair
 // kernel sums over the lists in that order — the FP64 pair arithmetic then
 // runs densely, one lane per gas body, instead of once per walk step for
@@ -68,6 +68,10 @@ struct SphArgs {
     const double4_32a *geo;
     const NodeS32 *s32;
     const NodeW64 *w64;
+    const NodeLink *link;
+    const int *child;
+    const DevRoot *root;
+    const float4 *sp, *box, *sbox; // sorted records, their boxes by 32 and by 1024 (k_sph_sort)
     DevScalars *sc;
     int *nb;       // neighbour lists, slot-major
     int *nb_count; // neighbours per gas body
@@ -164,6 +168,230 @@ __device__ __forceinline__ int warp_excl_max(int v)
 // (nb[slot * stride + k]) for coalesced reads in the pair kernels. The density
 // pass uses h before its update (src/sph.c:53-63), the force pass after it
 // (src/sph.c:112-126): each pass builds its list from the h it sees.
+//
+// On a tree built here the bodies' sorted order is the depth-first order of
+// their leaves, so a list needs no tree: the sorted positions are kept as
+// float4 records with the box of every 32 (a chunk) and of every 1024 (a
+// super-chunk), made by k_sph_sort, and a warp tests super-chunk boxes, then
+// the chunk boxes of those the query sphere meets, then the bodies of those
+// chunks, 32 at a time and always in sorted order. Per query this reads about
+// 25 chunks where the walk over preorder cells below read over a hundred
+// windows of 48-byte records: 105 -> 34 us a pass for the 100k merger's 10,000
+// gas bodies. A caller's pool (no sorted order) keeps that walk.
+//
+// A body whose FP32 distance is too close to the radius to call is decided by
+// the reference's expressions: its own distance, and the box test of every cell
+// on its path (which could reject it only within rounding).
+
+// Sorted records, chunk boxes and the gas bodies' list (in sorted order up to
+// the order in which warps count themselves in; nothing depends on it).
+constexpr int SORT_THREADS = 1024; // one super-chunk per block
+
+__global__ void __launch_bounds__(SORT_THREADS) k_sph_sort(
+    DevScalars *sc, const int *__restrict__ perm, const double *__restrict__ x,
+    const double *__restrict__ y, const double *__restrict__ z, const int *__restrict__ type,
+    const signed char *__restrict__ lcp, float4 *__restrict__ sp, float4 *__restrict__ box,
+    float4 *__restrict__ sbox, int *__restrict__ gas)
+{
+    __shared__ float4 s_lo[CSG_WARP], s_hi[CSG_WARP];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int p = blockIdx.x * SORT_THREADS + threadIdx.x, na = sc->n_alive;
+    if (blockIdx.x * SORT_THREADS >= na)
+        return; // the whole block
+    const float inf = __int_as_float(0x7f800000);
+    float4 lo = make_float4(inf, inf, inf, 0.0f), hi = make_float4(-inf, -inf, -inf, 0.0f);
+    bool is_gas = false;
+    int b = -1;
+    if (p < na) {
+        b = perm[p];
+        const float fx = (float)x[b], fy = (float)y[b], fz = (float)z[b];
+        // bodies equal to depth 64 after the first share its leaf, which names
+        // the first only
+        const bool own = p == 0 || lcp[p - 1] < CSG_MAX_LEVEL;
+        sp[p] = make_float4(fx, fy, fz, __int_as_float(own ? b : -1));
+        lo = make_float4(fx, fy, fz, fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))));
+        hi = make_float4(fx, fy, fz, 0.0f);
+        is_gas = type[b] == BODY_GAS;
+    }
+    const unsigned g = __ballot_sync(0xffffffffu, is_gas);
+    int k = 0;
+    if (lane == 0 && g)
+        k = atomicAdd(&sc->n_gas, __popc(g));
+    k = __shfl_sync(0xffffffffu, k, 0);
+    if (is_gas)
+        gas[k + __popc(g & ((1u << lane) - 1u))] = b;
+    auto join = [](float4 &l, float4 &h) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            l.x = fminf(l.x, __shfl_xor_sync(0xffffffffu, l.x, o));
+            l.y = fminf(l.y, __shfl_xor_sync(0xffffffffu, l.y, o));
+            l.z = fminf(l.z, __shfl_xor_sync(0xffffffffu, l.z, o));
+            l.w = fmaxf(l.w, __shfl_xor_sync(0xffffffffu, l.w, o));
+            h.x = fmaxf(h.x, __shfl_xor_sync(0xffffffffu, h.x, o));
+            h.y = fmaxf(h.y, __shfl_xor_sync(0xffffffffu, h.y, o));
+            h.z = fmaxf(h.z, __shfl_xor_sync(0xffffffffu, h.z, o));
+        }
+    };
+    join(lo, hi);
+    if (lane == 0) {
+        const int c = blockIdx.x * CSG_WARP + wid;
+        box[2 * c] = lo;
+        box[2 * c + 1] = hi;
+        s_lo[wid] = lo;
+        s_hi[wid] = hi;
+    }
+    __syncthreads();
+    if (wid == 0) {
+        lo = s_lo[lane];
+        hi = s_hi[lane];
+        join(lo, hi);
+        if (lane == 0) {
+            sbox[2 * blockIdx.x] = lo;
+            sbox[2 * blockIdx.x + 1] = hi;
+        }
+    }
+}
+
+struct Query {
+    double px, py, pz, r2;
+    float qx, qy, qz, mq, r2f;
+};
+
+// Whether a box of sorted bodies may hold one within the radius: never false
+// for one that does.
+__device__ __forceinline__ bool chunk_meets(const float4 *box, int c, const Query &q)
+{
+    const float4 lo = __ldg(&box[2 * c]), hi = __ldg(&box[2 * c + 1]);
+    const float e = (q.mq + lo.w) * FP32_EPS_POS;
+    const float dx = fmaxf(0.0f, fmaxf(lo.x - q.qx, q.qx - hi.x) - e);
+    const float dy = fmaxf(0.0f, fmaxf(lo.y - q.qy, q.qy - hi.y) - e);
+    const float dz = fmaxf(0.0f, fmaxf(lo.z - q.qz, q.qz - hi.z) - e);
+    return dx * dx + dy * dy + dz * dz <= q.r2f * (1.0f + FP32_EPS_SUM);
+}
+
+// The reference's own tests of the body at sorted position p (src/octree.c:
+// 250-272): every cell on its path, then its distance.
+__device__ __noinline__ bool exact_within(const SphArgs &a, int p, int j, double px, double py,
+                                          double pz, double r2)
+{
+    double bx = a.x[j] - px;
+    double by = a.y[j] - py;
+    double bz = a.z[j] - pz;
+    const double d2 = bx * bx + by * by + bz * bz;
+    if (!(d2 <= r2))
+        return false;
+    // a cell on the path lies no further than the body, but for the rounding of
+    // its centre and of the differences (a few ulp of the root's extent)
+    const DevRoot &root = *a.root;
+    const double R = fabs(root.c0[0]) + fabs(root.c0[1]) + fabs(root.c0[2]) + root.hs0 + fabs(px) +
+                     fabs(py) + fabs(pz);
+    const double slack = 1e-14 * R;
+    if (d2 + slack * (slack + 4.0 * sqrt(r2)) < r2 * (1.0 - 1e-14))
+        return true;
+    const int nn = a.sc->n_nodes;
+    for (int cell = 0, level = 0; level <= CSG_MAX_LEVEL; level++) {
+        const double4_32a g = a.geo[cell];
+        double gx = fmax(0.0, fabs(px - g.x) - g.w);
+        double gy = fmax(0.0, fabs(py - g.y) - g.w);
+        double gz = fmax(0.0, fabs(pz - g.z) - g.w);
+        if (gx * gx + gy * gy + gz * gz > r2)
+            return false;
+        int next = -1;
+        for (int o = 0; o < 8; o++) { // the child whose bodies include position p
+            const int c = a.child[8 * (size_t)cell + o];
+            if (c > cell && c < nn && a.link[c].first <= p && p < a.link[c].first + a.link[c].count)
+                next = c;
+        }
+        if (next < 0)
+            return true; // the leaf
+        cell = next;
+    }
+    return true;
+}
+
+__device__ __forceinline__ bool body_within(const SphArgs &a, const Query &q, const float4 &v, int p)
+{
+    const int j = __float_as_int(v.w);
+    if (j < 0)
+        return false;
+    const float mb = fmaxf(fabsf(v.x), fmaxf(fabsf(v.y), fabsf(v.z)));
+    const float e = (q.mq + mb) * FP32_EPS_POS;
+    const float dx = fabsf(v.x - q.qx), dy = fabsf(v.y - q.qy), dz = fabsf(v.z - q.qz);
+    const float hx = dx + e, hy = dy + e, hz = dz + e;
+    if (hx * hx + hy * hy + hz * hz < q.r2f * (1.0f - FP32_EPS_SUM))
+        return true;
+    const float lx = fmaxf(0.0f, dx - e), ly = fmaxf(0.0f, dy - e), lz = fmaxf(0.0f, dz - e);
+    if (lx * lx + ly * ly + lz * lz > q.r2f * (1.0f + FP32_EPS_SUM))
+        return false;
+    return exact_within(a, p, j, q.px, q.py, q.pz, q.r2);
+}
+
+__device__ __forceinline__ void list_sorted(const SphArgs &a, int k, int lane)
+{
+    const int na = (a.sc->n_nodes > a.node_cap) ? 0 : a.sc->n_alive;
+    const int chunks = (na + CSG_WARP - 1) / CSG_WARP, supers = (chunks + CSG_WARP - 1) / CSG_WARP;
+    const int i = a.gas[k];
+    const double h = a.h[i];
+    Query q;
+    q.px = a.x[i];
+    q.py = a.y[i];
+    q.pz = a.z[i];
+    q.r2 = h * h;
+    q.qx = (float)q.px;
+    q.qy = (float)q.py;
+    q.qz = (float)q.pz;
+    q.mq = fmaxf(fabsf(q.qx), fmaxf(fabsf(q.qy), fabsf(q.qz)));
+    q.r2f = (float)q.r2;
+    const unsigned lt = (1u << lane) - 1u;
+    const size_t stride = (size_t)a.stride;
+    int found = 0;
+    for (int s0 = 0; s0 < supers && found < CSG_SPH_MAX_NEIGHBORS; s0 += CSG_WARP) {
+        const int s = s0 + lane;
+        unsigned ms = __ballot_sync(0xffffffffu, s < supers && chunk_meets(a.sbox, s, q));
+        while (ms && found < CSG_SPH_MAX_NEIGHBORS) {
+            const int c0 = (s0 + __ffs((int)ms) - 1) * CSG_WARP;
+            ms &= ms - 1u;
+            unsigned mc = __ballot_sync(0xffffffffu,
+                                        c0 + lane < chunks && chunk_meets(a.box, c0 + lane, q));
+            if (!mc)
+                continue;
+            const float4 none = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
+            int p = (c0 + __ffs((int)mc) - 1) * CSG_WARP + lane;
+            mc &= mc - 1u;
+            float4 v = p < na ? __ldg(&a.sp[p]) : none;
+            for (;;) {
+                // the next chunk's bodies are on their way during this one's tests
+                const bool more = mc != 0u;
+                int pn = 0;
+                float4 vn = none;
+                if (more) {
+                    pn = (c0 + __ffs((int)mc) - 1) * CSG_WARP + lane;
+                    mc &= mc - 1u;
+                    vn = pn < na ? __ldg(&a.sp[pn]) : none;
+                }
+                const bool cand = body_within(a, q, v, p);
+                const unsigned m = __ballot_sync(0xffffffffu, cand);
+                if (cand) {
+                    const int slot = found + __popc(m & lt);
+                    if (slot < CSG_SPH_MAX_NEIGHBORS)
+                        a.nb[stride * slot + k] = __float_as_int(v.w);
+                }
+                found = min(CSG_SPH_MAX_NEIGHBORS, found + __popc(m));
+                if (!more || found == CSG_SPH_MAX_NEIGHBORS)
+                    break;
+                p = pn;
+                v = vn;
+            }
+        }
+    }
+    if (lane == 0) {
+        a.nb_count[k] = found;
+        if (a.density) // its pairs need 8/(pi h^3) of this body
+            a.pr2[i] = h < 1e-10 ? 0.0 : kernel_norm(h);
+    }
+}
+
+// The same on a caller's pool.
 __device__ __forceinline__ void list_one(const SphArgs &a, int k, int lane)
 {
     const int nnodes = (a.sc->n_nodes > a.node_cap) ? 0 : a.sc->n_nodes;
@@ -218,6 +446,7 @@ __device__ __forceinline__ void list_one(const SphArgs &a, int k, int lane)
     }
 }
 
+template <bool SORTED>
 __global__ void __launch_bounds__(SPH_THREADS) k_sph_lists(SphArgs a)
 {
     const int lane = threadIdx.x & 31;
@@ -225,8 +454,12 @@ __global__ void __launch_bounds__(SPH_THREADS) k_sph_lists(SphArgs a)
     const int nwarps = (int)((gridDim.x * (long long)SPH_THREADS) >> 5);
     for (int k = (int)(((long long)blockIdx.x * SPH_THREADS + threadIdx.x) >> 5); k < n_gas;
          k += nwarps) // warp-uniform
-        if (!a.reuse || a.relist[k])
-            list_one(a, k, lane);
+        if (!a.reuse || a.relist[k]) {
+            if (SORTED)
+                list_sorted(a, k, lane);
+            else
+                list_one(a, k, lane);
+        }
 }
 
 // Pair kernels. Each pass runs in two kernels so that the FP64 pair
@@ -424,29 +657,6 @@ __global__ void __launch_bounds__(SUM_THREADS) k_sph_force_sums(SphArgs a)
     a.az[i] += sz * 0.1;
 }
 
-__global__ void k_gas_flags(DevScalars *sc, const int *__restrict__ perm,
-                            const int *__restrict__ type, int *__restrict__ flag)
-{
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= sc->n_alive)
-        return;
-    flag[p] = (type[perm[p]] == BODY_GAS) ? 1 : 0;
-}
-
-__global__ void k_gas_scatter(DevScalars *sc, const int *__restrict__ perm,
-                              const int *__restrict__ flag, const int *__restrict__ base,
-                              int *__restrict__ gas)
-{
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const int na = sc->n_alive;
-    if (p == 0)
-        sc->n_gas = base[na];
-    if (p >= na)
-        return;
-    if (flag[p])
-        gas[base[p]] = perm[p];
-}
-
 // One query, one thread: src/octree.c:293-318.
 __global__ void k_find_one(SphArgs a, double cx, double cy, double cz, double radius, int cap,
                            int *__restrict__ buf, int *__restrict__ count)
@@ -484,6 +694,12 @@ __global__ void k_find_one(SphArgs a, double cx, double cy, double cz, double ra
     *count = c;
 }
 
+// Sorted records are held for whole super-chunks.
+size_t sorted_cap(const csgd_t *d)
+{
+    return ((size_t)(d->cap > 0 ? d->cap : 1) + SORT_THREADS - 1) / SORT_THREADS * SORT_THREADS;
+}
+
 SphArgs make_args(csgd_t *d)
 {
     SphArgs a;
@@ -506,6 +722,12 @@ SphArgs make_args(csgd_t *d)
     a.geo = d->geo;
     a.s32 = d->s32;
     a.w64 = d->w64;
+    a.link = d->link;
+    a.child = d->child;
+    a.root = d->roots;
+    a.sp = d->sph_sorted;
+    a.box = a.sp + sorted_cap(d);
+    a.sbox = a.box + 2 * (sorted_cap(d) / CSG_WARP);
     a.sc = d->sc;
     a.nb = d->nb;
     a.nb_count = d->nb_count;
@@ -548,11 +770,12 @@ int gas_list(csgd_t *d)
     const int n = d->n;
     const int g = csgd_grid(n, 256);
     if (!d->imported) {
-        { k_gas_flags<<<g, 256, 0, d->stream>>>(d->sc, d->perm, d->type, d->cnt); d->launches++; }
-        int rc = csg_scan_exclusive(d, d->cnt, d->base, n, &d->sc->n_alive);
-        if (rc)
-            return rc;
-        { k_gas_scatter<<<g, 256, 0, d->stream>>>(d->sc, d->perm, d->cnt, d->base, d->gas); d->launches++; }
+        float4 *sp = d->sph_sorted;
+        float4 *box = sp + sorted_cap(d), *sbox = box + 2 * (sorted_cap(d) / CSG_WARP);
+        if (!d->gas_zero) // the build's first kernel cleared it, unless it was counted since
+            cudaMemsetAsync(&d->sc->n_gas, 0, sizeof(int), d->stream);
+        d->gas_zero = 0;
+        { k_sph_sort<<<csgd_grid(n, SORT_THREADS), SORT_THREADS, 0, d->stream>>>(d->sc, d->perm, d->x, d->y, d->z, d->type, d->lcp, sp, box, sbox, d->gas); d->launches++; }
     } else {
         { k_gas_flags_idx<<<g, 256, 0, d->stream>>>(n, d->m, d->type, d->cnt); d->launches++; }
         int rc = csg_scan_exclusive(d, d->cnt, d->base, n, nullptr);
@@ -587,6 +810,9 @@ static int ensure_lists(csgd_t *d)
         cudaFree(d->sph_term);
     if (d->sph_relist)
         cudaFree(d->sph_relist);
+    if (d->sph_sorted)
+        cudaFree(d->sph_sorted);
+    d->sph_sorted = nullptr;
     d->nb = nullptr;
     d->nb_count = d->sph_relist = nullptr;
     d->pr2 = d->cs = d->sph_term = nullptr;
@@ -594,6 +820,10 @@ static int ensure_lists(csgd_t *d)
     if (csgd_malloc((void **)&d->nb, sizeof(int) * CSG_SPH_MAX_NEIGHBORS * c) != cudaSuccess ||
         csgd_malloc((void **)&d->nb_count, sizeof(int) * c) != cudaSuccess ||
         csgd_malloc((void **)&d->sph_relist, sizeof(int) * c) != cudaSuccess ||
+        // records, 2 words a chunk, 2 a super-chunk
+        csgd_malloc((void **)&d->sph_sorted,
+                    sizeof(float4) * (sorted_cap(d) + sorted_cap(d) / 16 + sorted_cap(d) / 512)) !=
+            cudaSuccess ||
         csgd_malloc((void **)&d->pr2, sizeof(double) * c) != cudaSuccess ||
         csgd_malloc((void **)&d->cs, sizeof(double) * c) != cudaSuccess ||
         csgd_malloc((void **)&d->sph_term, sizeof(double) * 3 * CSG_SPH_MAX_NEIGHBORS * c) !=
@@ -629,7 +859,11 @@ static int sph_pass(csgd_t *d, int forces, bool sums = true, bool reuse = false)
     int gl = csgd_grid((long long)d->n * CSG_WARP, SPH_THREADS);
     if (gl > d->num_sms * 16)
         gl = d->num_sms * 16;
-    { k_sph_lists<<<gl, SPH_THREADS, 0, d->stream>>>(a); d->launches++; }
+    if (d->imported)
+        k_sph_lists<false><<<gl, SPH_THREADS, 0, d->stream>>>(a);
+    else
+        k_sph_lists<true><<<gl, SPH_THREADS, 0, d->stream>>>(a);
+    d->launches++;
     // pair terms: a grid-stride pass over (slot, gas body), sized for 32 warps
     // per SM (the gas count is known on the device only)
     const int gp = d->num_sms * (2048 / SPH_THREADS);

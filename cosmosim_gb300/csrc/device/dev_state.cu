@@ -381,6 +381,8 @@ extern "C" void csgd_destroy(csgd_t *d)
         cudaFree(d->sph_term);
     if (d->sph_relist)
         cudaFree(d->sph_relist);
+    if (d->sph_sorted)
+        cudaFree(d->sph_sorted);
     if (d->sc)
         cudaFree(d->sc);
     if (d->roots)

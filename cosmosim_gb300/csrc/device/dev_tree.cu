@@ -1315,6 +1315,7 @@ static int order_bodies(csgd_t *d)
     const int G = d->n_gal;
     csgd_build_mark(d, 0);
     csgd_launch(d, k_reset, 1, 256, s, sc, d->roots, G);
+    d->gas_zero = 1;
     // few blocks: each warp flushes its running box with atomics on the same
     // words, so fewer warps contend less (4 blocks per SM keep HBM busy)
     int gb = min(csgd_grid(n, B), 4 * d->num_sms);
