@@ -77,24 +77,44 @@ __device__ __forceinline__ unsigned long long recip_word(unsigned long long Mb)
 
 } // namespace fpint
 
-// a / b, rounded to nearest even (bit-identical to the compiler's operator).
-__device__ __forceinline__ double div_rn(double a, double b)
+// A divisor with its reciprocal word, for several quotients.
+struct Divisor {
+    double value;
+    unsigned long long Mb, v, sign;
+    int eb; // biased exponent
+    bool normal;
+};
+
+__device__ __forceinline__ Divisor divisor(double b)
+{
+    using namespace fpint;
+    const unsigned long long bb = (unsigned long long)__double_as_longlong(b);
+    Divisor d;
+    d.value = b;
+    d.sign = bb & (1ull << 63);
+    d.eb = (int)(bb >> 52) & 0x7ff;
+    d.normal = (unsigned)(d.eb - 1) < 2046u;
+    d.Mb = (bb & MANT) | HID;
+    d.v = recip_word(d.Mb);
+    return d;
+}
+
+// a / d.value, rounded to nearest even (bit-identical to the compiler's operator).
+__device__ __forceinline__ double div_rn(double a, const Divisor &d)
 {
     using namespace fpint;
     const unsigned long long ab = (unsigned long long)__double_as_longlong(a);
-    const unsigned long long bb = (unsigned long long)__double_as_longlong(b);
-    const int ea = (int)(ab >> 52) & 0x7ff, eb = (int)(bb >> 52) & 0x7ff;
-    const int E = ea - eb + 1023; // biased exponent when Ma >= Mb
-    const unsigned long long sign = (ab ^ bb) & (1ull << 63);
-    const bool bnorm = (unsigned)(eb - 1) < 2046u;
+    const int ea = (int)(ab >> 52) & 0x7ff;
+    const int E = ea - d.eb + 1023; // biased exponent when Ma >= Mb
+    const unsigned long long sign = (ab & (1ull << 63)) ^ d.sign;
     const bool azero = (ab << 1) == 0ull;
-    if (!(bnorm && (azero || ((unsigned)(ea - 1) < 2046u && (unsigned)(E - 2) < 2044u))))
-        return a / b;
+    if (!(d.normal && (azero || ((unsigned)(ea - 1) < 2046u && (unsigned)(E - 2) < 2044u))))
+        return a / d.value;
     if (azero)
         return __longlong_as_double((long long)sign);
-    const unsigned long long Ma = (ab & MANT) | HID, Mb = (bb & MANT) | HID;
+    const unsigned long long Ma = (ab & MANT) | HID, Mb = d.Mb;
     const unsigned long long u = Ma << 1;
-    unsigned long long Q = u + __umul64hi(u, recip_word(Mb));
+    unsigned long long Q = u + __umul64hi(u, d.v);
     long long rem = (long long)((Ma << 54) - Q * Mb);
 #pragma unroll
     for (int k = 0; k < 2; k++)
@@ -115,6 +135,8 @@ __device__ __forceinline__ double div_rn(double a, double b)
     const unsigned long long M = M0 + (g & (st | ((unsigned)M0 & 1u)));
     return __longlong_as_double((long long)(sign | (((unsigned long long)(E - 2 + hi) << 52) + M)));
 }
+
+__device__ __forceinline__ double div_rn(double a, double b) { return div_rn(a, divisor(b)); }
 
 // sqrt(x), rounded to nearest even (bit-identical to the compiler's sqrt).
 __device__ __forceinline__ double sqrt_rn(double x)

@@ -239,7 +239,7 @@ struct csgd {
     int *nb;           // SPH neighbour lists, 128 slots x cap (slot-major)
     int *nb_count;
     double *pr2, *cs; // SPH per-body force terms
-    double *sph_term; // SPH pair terms, 3 x 128 x cap (slot-major)
+    double *sph_sum;  // SPH force sums of the gas bodies, 3 x cap
     float4 *sph_sorted; // sorted body records, then their boxes (k_sph_sort)
     int *sph_relist;  // per gas slot: 1 when the density pass changed h
     int nb_cap;

@@ -22,9 +22,51 @@
 namespace {
 
 constexpr int SPH_THREADS = 128;
-constexpr int SPH_WARPS = SPH_THREADS / CSG_WARP;
 constexpr double GAMMA = 5.0 / 3.0;
 constexpr double PI_D = 3.14159265358979323846;
+
+// The pair kernels are bound by the FP64 pipe, on which comparisons run too:
+// these compare (and halve and double) by the bits, with the same results.
+constexpr long long ONE_BITS = 0x3ff0000000000000ll, INF_BITS = 0x7ff0000000000000ll;
+
+// q > 1 for q that is not negative (false for NaN, as the comparison).
+__device__ __forceinline__ bool above_one(double q)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(q);
+    return b - (unsigned long long)(ONE_BITS + 1) < (unsigned long long)(INF_BITS - ONE_BITS);
+}
+// q <= 0.5 for q that is not negative (false for NaN).
+__device__ __forceinline__ bool at_most_half(double q)
+{
+    return (unsigned long long)__double_as_longlong(q) <= (unsigned long long)(ONE_BITS - (1ll << 52));
+}
+// v < 0 (false for -0 and NaN).
+__device__ __forceinline__ bool negative(double v)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    return b - ((1ull << 63) + 1ull) < (unsigned long long)INF_BITS;
+}
+// r < 1e-15 for r that is not negative.
+__device__ __forceinline__ bool tiny(double r)
+{
+    return (unsigned long long)__double_as_longlong(r) <
+           (unsigned long long)__double_as_longlong(1e-15);
+}
+// 0.5 v and 2 v: an exponent step unless a result could be subnormal or infinite.
+__device__ __forceinline__ double half_of(double v)
+{
+    const long long b = __double_as_longlong(v);
+    if ((unsigned)((int)(b >> 52) & 0x7ff) - 2u < 2045u)
+        return __longlong_as_double(b - (1ll << 52));
+    return 0.5 * v;
+}
+__device__ __forceinline__ double twice(double v)
+{
+    const long long b = __double_as_longlong(v);
+    if ((unsigned)((int)(b >> 52) & 0x7ff) - 1u < 2045u)
+        return __longlong_as_double(b + (1ll << 52));
+    return 2.0 * v;
+}
 
 // M4 cubic spline W(r, h), src/sph.c:11-25, with its normalisation 8/(pi h^3)
 // computed by the caller once per gas body (the same expression, so the same
@@ -34,29 +76,34 @@ __device__ __forceinline__ double kernel_W_norm(double r, double h, double norm)
     if (h < 1e-10)
         return 0.0;
     double q = div_rn(r, h);
-    if (q > 1.0)
+    if (above_one(q))
         return 0.0;
-    if (q <= 0.5)
-        return norm * (1.0 - 6.0 * q * q + 6.0 * q * q * q);
-    double t = 1.0 - q;
-    return norm * 2.0 * t * t * t;
+    // norm (1 - a + a q), a = 6 q q, or 2 norm t t t, t = 1 - q: three of the
+    // multiplications are shared
+    const bool in = at_most_half(q);
+    const double t = 1.0 - q, u = in ? q : t;
+    const double a = (in ? 6.0 : twice(norm)) * u * u, w = a * u;
+    return in ? norm * (1.0 - a + w) : w;
 }
 
 __device__ __forceinline__ double kernel_norm(double h) { return div_rn(8.0, PI_D * h * h * h); }
 
-// the kernel's radial derivative dW/dr(r, h), src/sph.c:27-41
+// the kernel's radial derivative dW/dr(r, h), src/sph.c:27-41; its two
+// branches, -12 q + 18 q q and -6 t t (t = 1 - q), share their operations
+// (adding -0 changes nothing)
 __device__ __forceinline__ double kernel_dWdr(double r, double h)
 {
     if (h < 1e-10)
         return 0.0;
-    double q = div_rn(r, h);
-    if (q > 1.0 || r < 1e-15)
+    const Divisor by_h = divisor(h); // one reciprocal for both quotients
+    double q = div_rn(r, by_h);
+    if (above_one(q) || tiny(r))
         return 0.0;
     double norm = div_rn(8.0, PI_D * h * h * h);
-    if (q <= 0.5)
-        return div_rn(norm * (-12.0 * q + 18.0 * q * q), h);
-    double t = 1.0 - q;
-    return div_rn(norm * (-6.0 * t * t), h);
+    const bool in = at_most_half(q);
+    const double t = 1.0 - q, u = in ? q : t;
+    const double linear = in ? -12.0 * q : -0.0;
+    return div_rn(norm * (linear + (in ? 18.0 : -6.0) * u * u), by_h);
 }
 
 struct SphArgs {
@@ -79,7 +126,7 @@ struct SphArgs {
     int reuse;     // force pass: keep the density lists of bodies with relist 0
     int density;   // density pass (the lists also store 8/(pi h^3) in pr2)
     double *pr2, *cs; // per-body force terms (k_sph_body_terms)
-    double *term;     // pair terms, 3 planes of 128 slots x stride (slot-major)
+    double *sum;      // force sums of the gas bodies, 3 x stride
     int n, node_cap, stride;
 };
 
@@ -462,199 +509,280 @@ __global__ void __launch_bounds__(SPH_THREADS) k_sph_lists(SphArgs a)
         }
 }
 
-// Pair kernels. Each pass runs in two kernels so that the FP64 pair
-// arithmetic (sqrt, divisions) keeps every SM busy even when gas bodies are
-// few: one thread per (list slot, gas body) writes the pair's term, then one
-// thread per gas body adds its terms in list order — the reference's order,
-// with the same operations, so the sums are the reference's bit for bit
-// (a skipped pair stores 0, and x - 0 == x for every x).
-__device__ __forceinline__ bool pair_slot(const SphArgs &a, long long t, int n_gas, int &s,
-                                          int &k)
-{
-    s = (int)(t / n_gas);
-    k = (int)(t - (long long)s * n_gas);
-    return s < a.nb_count[k];
-}
-
-// Density terms m_j W(r, h_i), src/sph.c:53-63.
-__global__ void __launch_bounds__(SPH_THREADS) k_sph_density_terms(SphArgs a)
-{
-    const int n_gas = a.sc->n_gas;
-    const long long total = (long long)CSG_SPH_MAX_NEIGHBORS * n_gas;
-    const size_t stride = (size_t)a.stride;
-    for (long long t = (long long)blockIdx.x * SPH_THREADS + threadIdx.x; t < total;
-         t += (long long)gridDim.x * SPH_THREADS) {
-        int s, k;
-        if (!pair_slot(a, t, n_gas, s, k))
-            continue;
-        const int i = a.gas[k];
-        const int j = a.nb[stride * s + k];
-        double dx = a.x[i] - a.x[j];
-        double dy = a.y[i] - a.y[j];
-        double dz = a.z[i] - a.z[j];
-        double r = sqrt_rn(dx * dx + dy * dy + dz * dz);
-        a.term[stride * s + k] = a.m[j] * kernel_W_norm(r, a.h[i], a.pr2[i]);
-    }
-}
-
-// The per-body sums run one thread per gas body in small blocks (the gas
-// bodies are ~10% of all: 64-thread blocks spread them over every SM) and
-// load SUM_BATCH slots ahead of the additions, which stay in list order.
+// Pair kernels. A block takes a group of up to 32 gas bodies; its pair threads
+// compute the group's (list slot, body) terms into shared memory, PAIR_TERMS at
+// a time, and its sum warps, one lane per body and one warp per component, add
+// the terms of the slots before in list order: the reference's order, with the
+// same operations, so the sums are the reference's bit for bit (a skipped pair
+// stores 0, and x - 0 == x for every x). Two buffers, one barrier per step: the
+// long dependent chains of the sums run beside the pairs. The FP64 pipe bounds
+// both kernels, and an instruction holds it for a whole warp however few lanes
+// are active: hence a lane per body in the sums, and groups of one size, so
+// that every block gets as many bodies. For the 100k merger's 10,000 gas bodies
+// density takes 69 us and forces 174 us (the pipe busy for 3/4 of both); with
+// the terms in global memory, a second kernel for the sums and every quotient
+// with its own reciprocal 93 and 232 us, the substep 802 us instead of 865.
+// Blocks of 128, 192 or 384 pair threads (6, 4, 2 per SM): within 1%.
+constexpr int PAIR_THREADS = 256;
+constexpr int PAIR_BLOCKS = 3; // per SM
+constexpr int PAIR_TERMS = 3 * PAIR_THREADS;
+constexpr int PAIR_GROUP = CSG_WARP;
+constexpr int PAIR_SLOTS = 64; // most list slots per step
+constexpr int DENSITY_THREADS = PAIR_THREADS + CSG_WARP;
+constexpr int FORCE_THREADS = PAIR_THREADS + 3 * CSG_WARP;
 constexpr int SUM_THREADS = 64;
-constexpr int SUM_BATCH = 8;
 
-// Density, adaptive h and pressure, src/sph.c:45-97.
-__global__ void __launch_bounds__(SUM_THREADS) k_sph_density_sums(SphArgs a)
+// One step: slots first .. first + slots of the group's bodies k0 .. k0 + count.
+struct PairStep {
+    int buf, k0, count, first, slots;
+    bool last;
+};
+
+// The groups of a block: fn pairs(step) on the pair threads, then fn sums(step)
+// on the sum threads, a step behind.
+template <class Pairs, class Sums>
+__device__ __forceinline__ void for_groups(int n_gas, const int *__restrict__ nb_count, Pairs pairs,
+                                           Sums sums)
 {
-    const int k = blockIdx.x * SUM_THREADS + threadIdx.x;
-    if (k >= a.sc->n_gas)
-        return;
-    const int i = a.gas[k];
-    const double h = a.h[i];
-    const int nn = a.nb_count[k];
-    const size_t stride = (size_t)a.stride;
-    const double *__restrict__ term = a.term;
-    double rho = 0.0;
-    int s = 0;
-    for (; s + SUM_BATCH <= nn; s += SUM_BATCH) {
-        double t[SUM_BATCH];
-#pragma unroll
-        for (int u = 0; u < SUM_BATCH; u++)
-            t[u] = __ldg(&term[stride * (s + u) + k]);
-#pragma unroll
-        for (int u = 0; u < SUM_BATCH; u++)
-            rho += t[u];
+    const int grid = (int)gridDim.x, lane = threadIdx.x & 31;
+    const int rounds = (n_gas + PAIR_GROUP * grid - 1) / (PAIR_GROUP * grid);
+    const int B = rounds > 0 ? (n_gas + rounds * grid - 1) / (rounds * grid) : 1;
+    const int most_slots = min(PAIR_SLOTS, PAIR_TERMS / B);
+    PairStep before;
+    before.count = 0;
+    int buf = 0;
+    for (int round = 0; round <= rounds; round++) { // the last one: sums alone
+        PairStep now;
+        now.k0 = (round * grid + (int)blockIdx.x) * B;
+        now.count = round < rounds ? max(0, min(B, n_gas - now.k0)) : 0;
+        const int most =
+            __reduce_max_sync(0xffffffffu, lane < now.count ? nb_count[now.k0 + lane] : 0);
+        now.first = 0;
+        do {
+            now.buf = buf;
+            now.slots = min(most_slots, most - now.first);
+            now.last = now.first + most_slots >= most;
+            if (threadIdx.x < PAIR_THREADS) {
+                if (now.count > 0)
+                    pairs(now);
+            } else if (before.count > 0) {
+                sums(before);
+            }
+            __syncthreads();
+            before = now;
+            buf ^= 1;
+            now.first += most_slots;
+        } while (!before.last);
     }
-    for (; s < nn; s++)
-        rho += __ldg(&term[stride * s + k]);
-    int relist = 1;
-    if (nn < 20 && h < 50.0)
-        a.h[i] = h * 1.2;
-    else if (nn > 48 && h > 0.1)
-        a.h[i] = h * 0.8;
-    else
-        relist = 0;
-    a.relist[k] = relist;
-    if (rho < 1e-15 || isnan(rho))
-        rho = 1e-15;
-    a.rho[i] = rho;
-    double u = a.u[i];
-    if (u < 1e-15)
-        u = 1e-15;
-    a.P[i] = (GAMMA - 1.0) * rho * u;
 }
 
-// Per-body terms of the force pass: P/(rho^2 + 1e-15) and the sound speed
-// sqrt(gamma P/(rho + 1e-15)) (src/sph.c:112, :153-154, :170-171). The pair
-// terms need them for both bodies of every pair; computing them once per body
-// gives the same values as the reference's per-pair evaluation.
+// fn pair(p, slot, body of the group) for the pairs of a step
+template <class Pair>
+__device__ __forceinline__ void for_pairs(const PairStep &st, const int *nn, Pair pair)
+{
+    const int B = st.count, ds = PAIR_THREADS / B, db = PAIR_THREADS - ds * B;
+    int s = threadIdx.x / B, b = threadIdx.x - s * B;
+    for (int p = threadIdx.x; s < st.slots; p += PAIR_THREADS) {
+        if (st.first + s < nn[b])
+            pair(p, st.first + s, b);
+        s += ds;
+        b += db;
+        if (b >= B) {
+            b -= B;
+            s++;
+        }
+    }
+}
+
+__device__ __forceinline__ void pair_threads_sync()
+{
+    asm volatile("bar.sync 1, %0;" ::"n"(PAIR_THREADS) : "memory");
+}
+
+// P/(rho^2 + 1e-15) and the sound speed sqrt(gamma P/(rho + 1e-15)) of one gas
+// body (src/sph.c:112, :153-154, :170-171): the force pairs need them for both
+// bodies, computed once each they are the reference's per-pair values.
+__device__ __forceinline__ void body_terms(const SphArgs &a, int j, double rho, double P)
+{
+    a.pr2[j] = div_rn(P, rho * rho + 1e-15);
+    a.cs[j] = sqrt_rn(div_rn(GAMMA * P, rho + 1e-15));
+}
+
+// Density, adaptive h and pressure, src/sph.c:45-97 (terms m_j W(r, h_i)), and
+// the body's force terms.
+__global__ void __launch_bounds__(DENSITY_THREADS, PAIR_BLOCKS) k_sph_density(SphArgs a)
+{
+    __shared__ double term[2][PAIR_TERMS];
+    __shared__ double sx[PAIR_GROUP], sy[PAIR_GROUP], sz[PAIR_GROUP], sh[PAIR_GROUP],
+        snorm[PAIR_GROUP];
+    __shared__ int snn[PAIR_GROUP];
+    const int n_gas = a.sc->n_gas;
+    const size_t stride = (size_t)a.stride;
+    double rho = 0.0;
+    for_groups(
+        n_gas, a.nb_count,
+        [&](const PairStep &st) {
+            if (st.first == 0) {
+                const int t = threadIdx.x;
+                if (t < st.count) {
+                    const int i = a.gas[st.k0 + t];
+                    sx[t] = a.x[i];
+                    sy[t] = a.y[i];
+                    sz[t] = a.z[i];
+                    sh[t] = a.h[i];
+                    snorm[t] = a.pr2[i];
+                    snn[t] = a.nb_count[st.k0 + t];
+                }
+                pair_threads_sync();
+            }
+            for_pairs(st, snn, [&](int p, int slot, int b) {
+                const int j = a.nb[stride * slot + st.k0 + b];
+                double dx = sx[b] - a.x[j];
+                double dy = sy[b] - a.y[j];
+                double dz = sz[b] - a.z[j];
+                double r = sqrt_rn(dx * dx + dy * dy + dz * dz);
+                term[st.buf][p] = a.m[j] * kernel_W_norm(r, sh[b], snorm[b]);
+            });
+        },
+        [&](const PairStep &st) {
+            const int b = threadIdx.x - PAIR_THREADS, k = st.k0 + b;
+            if (b >= st.count)
+                return;
+            if (st.first == 0)
+                rho = 0.0;
+            const int nn = a.nb_count[k], end = min(nn - st.first, st.slots);
+            for (int s = 0; s < end; s++)
+                rho += term[st.buf][s * st.count + b];
+            if (!st.last)
+                return;
+            const int i = a.gas[k];
+            const double hi = a.h[i];
+            int relist = 1;
+            if (nn < 20 && hi < 50.0)
+                a.h[i] = hi * 1.2;
+            else if (nn > 48 && hi > 0.1)
+                a.h[i] = hi * 0.8;
+            else
+                relist = 0;
+            a.relist[k] = relist;
+            if (rho < 1e-15 || isnan(rho))
+                rho = 1e-15;
+            a.rho[i] = rho;
+            double u = a.u[i];
+            if (u < 1e-15)
+                u = 1e-15;
+            const double P = (GAMMA - 1.0) * rho * u;
+            a.P[i] = P;
+            body_terms(a, i, rho, P);
+        });
+}
+
+// The body terms alone, for a force pass that no density pass preceded.
 __global__ void __launch_bounds__(SUM_THREADS) k_sph_body_terms(SphArgs a)
 {
     const int k = blockIdx.x * SUM_THREADS + threadIdx.x;
     if (k >= a.sc->n_gas)
         return;
     const int j = a.gas[k];
-    const double rho = a.rho[j], P = a.P[j];
-    a.pr2[j] = div_rn(P, rho * rho + 1e-15);
-    a.cs[j] = sqrt_rn(div_rn(GAMMA * P, rho + 1e-15));
+    body_terms(a, j, a.rho[j], a.P[j]);
 }
 
-// Pressure gradient + Monaghan viscosity terms, src/sph.c:126-186.
-__global__ void __launch_bounds__(SPH_THREADS) k_sph_force_terms(SphArgs a)
+// Pressure gradient + Monaghan viscosity, src/sph.c:126-196: the bodies' sums
+// (k_sph_force_add adds them to the accelerations).
+__global__ void __launch_bounds__(FORCE_THREADS, PAIR_BLOCKS) k_sph_force(SphArgs a)
 {
+    __shared__ double term[2][3][PAIR_TERMS];
+    __shared__ double sx[PAIR_GROUP], sy[PAIR_GROUP], sz[PAIR_GROUP], svx[PAIR_GROUP],
+        svy[PAIR_GROUP], svz[PAIR_GROUP], sh[PAIR_GROUP], srho[PAIR_GROUP], spr2[PAIR_GROUP],
+        scs[PAIR_GROUP];
+    __shared__ int snn[PAIR_GROUP], si[PAIR_GROUP];
     const int n_gas = a.sc->n_gas;
-    const long long total = (long long)CSG_SPH_MAX_NEIGHBORS * n_gas;
     const size_t stride = (size_t)a.stride;
-    const size_t plane = stride * CSG_SPH_MAX_NEIGHBORS;
-    for (long long t = (long long)blockIdx.x * SPH_THREADS + threadIdx.x; t < total;
-         t += (long long)gridDim.x * SPH_THREADS) {
-        int s, k;
-        if (!pair_slot(a, t, n_gas, s, k))
-            continue;
-        const size_t o = stride * s + k;
-        const int i = a.gas[k];
-        const int j = a.nb[o];
-        double tx = 0.0, ty = 0.0, tz = 0.0;
-        if (j != i && a.type[j] == BODY_GAS) {
-            double dx = a.x[i] - a.x[j];
-            double dy = a.y[i] - a.y[j];
-            double dz = a.z[i] - a.z[j];
-            double r = sqrt_rn(dx * dx + dy * dy + dz * dz);
-            if (!(r < 1e-15)) {
-                const double h_i = a.h[i], rho_i = a.rho[i];
-                double h_avg = 0.5 * (h_i + a.h[j]);
-                double rho_j = a.rho[j];
-                double dvx = a.vx[i] - a.vx[j];
-                double dvy = a.vy[i] - a.vy[j];
-                double dvz = a.vz[i] - a.vz[j];
-                double vr = dvx * dx + dvy * dy + dvz * dz;
-                double visc = 0.0;
-                if (vr < 0.0) {
-                    double mu = div_rn(h_avg * vr, r * r + 0.01 * h_avg * h_avg);
-                    double c_avg = 0.5 * (a.cs[i] + a.cs[j]);
-                    double rho_avg = 0.5 * (rho_i + rho_j);
-                    visc = div_rn(-1.0 * c_avg * mu + 2.0 * mu * mu, rho_avg + 1e-15);
+    double sum = 0.0;
+    for_groups(
+        n_gas, a.nb_count,
+        [&](const PairStep &st) {
+            if (st.first == 0) {
+                const int t = threadIdx.x;
+                if (t < st.count) {
+                    const int i = a.gas[st.k0 + t];
+                    si[t] = i;
+                    sx[t] = a.x[i];
+                    sy[t] = a.y[i];
+                    sz[t] = a.z[i];
+                    svx[t] = a.vx[i];
+                    svy[t] = a.vy[i];
+                    svz[t] = a.vz[i];
+                    sh[t] = a.h[i];
+                    srho[t] = a.rho[i];
+                    spr2[t] = a.pr2[i];
+                    scs[t] = a.cs[i];
+                    snn[t] = a.nb_count[st.k0 + t];
                 }
-                double g = kernel_dWdr(r, h_avg);
-                double gx = div_rn(g * dx, r);
-                double gy = div_rn(g * dy, r);
-                double gz = div_rn(g * dz, r);
-                double f = a.m[j] * (a.pr2[i] + a.pr2[j] + visc);
-                tx = f * gx;
-                ty = f * gy;
-                tz = f * gz;
+                pair_threads_sync();
             }
-        }
-        a.term[o] = tx;
-        a.term[plane + o] = ty;
-        a.term[2 * plane + o] = tz;
-    }
+            for_pairs(st, snn, [&](int p, int slot, int b) {
+                const int j = a.nb[stride * slot + st.k0 + b];
+                double tx = 0.0, ty = 0.0, tz = 0.0;
+                if (j != si[b] && a.type[j] == BODY_GAS) {
+                    double dx = sx[b] - a.x[j];
+                    double dy = sy[b] - a.y[j];
+                    double dz = sz[b] - a.z[j];
+                    double r = sqrt_rn(dx * dx + dy * dy + dz * dz);
+                    if (!tiny(r)) {
+                        double h_avg = half_of(sh[b] + a.h[j]);
+                        double rho_j = a.rho[j];
+                        double dvx = svx[b] - a.vx[j];
+                        double dvy = svy[b] - a.vy[j];
+                        double dvz = svz[b] - a.vz[j];
+                        double vr = dvx * dx + dvy * dy + dvz * dz;
+                        double visc = 0.0;
+                        if (negative(vr)) {
+                            double mu = div_rn(h_avg * vr, r * r + 0.01 * h_avg * h_avg);
+                            double c_avg = half_of(scs[b] + a.cs[j]);
+                            double rho_avg = half_of(srho[b] + rho_j);
+                            visc = div_rn(-c_avg * mu + twice(mu) * mu, rho_avg + 1e-15);
+                        }
+                        double g = kernel_dWdr(r, h_avg);
+                        const Divisor by_r = divisor(r); // one reciprocal for the three
+                        double gx = div_rn(g * dx, by_r);
+                        double gy = div_rn(g * dy, by_r);
+                        double gz = div_rn(g * dz, by_r);
+                        double f = a.m[j] * (spr2[b] + a.pr2[j] + visc);
+                        tx = f * gx;
+                        ty = f * gy;
+                        tz = f * gz;
+                    }
+                }
+                term[st.buf][0][p] = tx;
+                term[st.buf][1][p] = ty;
+                term[st.buf][2][p] = tz;
+            });
+        },
+        [&](const PairStep &st) {
+            const int t = threadIdx.x - PAIR_THREADS, b = t & 31, c = t >> 5, k = st.k0 + b;
+            if (b >= st.count)
+                return;
+            if (st.first == 0)
+                sum = 0.0;
+            const int end = min(a.nb_count[k] - st.first, st.slots);
+            for (int s = 0; s < end; s++)
+                sum -= term[st.buf][c][s * st.count + b];
+            if (st.last)
+                a.sum[stride * c + k] = isnan(sum) ? 0.0 : sum;
+        });
 }
 
-// Sums of the force terms in list order, src/sph.c:187-196.
-__global__ void __launch_bounds__(SUM_THREADS) k_sph_force_sums(SphArgs a)
+__global__ void __launch_bounds__(SUM_THREADS) k_sph_force_add(SphArgs a)
 {
     const int k = blockIdx.x * SUM_THREADS + threadIdx.x;
     if (k >= a.sc->n_gas)
         return;
     const int i = a.gas[k];
-    const int nn = a.nb_count[k];
     const size_t stride = (size_t)a.stride;
-    const size_t plane = stride * CSG_SPH_MAX_NEIGHBORS;
-    const double *__restrict__ term = a.term;
-    double sx = 0.0, sy = 0.0, sz = 0.0;
-    int s = 0;
-    for (; s + SUM_BATCH <= nn; s += SUM_BATCH) {
-        double tx[SUM_BATCH], ty[SUM_BATCH], tz[SUM_BATCH];
-#pragma unroll
-        for (int u = 0; u < SUM_BATCH; u++) {
-            const size_t o = stride * (s + u) + k;
-            tx[u] = __ldg(&term[o]);
-            ty[u] = __ldg(&term[plane + o]);
-            tz[u] = __ldg(&term[2 * plane + o]);
-        }
-#pragma unroll
-        for (int u = 0; u < SUM_BATCH; u++) {
-            sx -= tx[u];
-            sy -= ty[u];
-            sz -= tz[u];
-        }
-    }
-    for (; s < nn; s++) {
-        const size_t o = stride * s + k;
-        sx -= __ldg(&term[o]);
-        sy -= __ldg(&term[plane + o]);
-        sz -= __ldg(&term[2 * plane + o]);
-    }
-    if (isnan(sx))
-        sx = 0.0;
-    if (isnan(sy))
-        sy = 0.0;
-    if (isnan(sz))
-        sz = 0.0;
-    a.ax[i] += sx * 0.1;
-    a.ay[i] += sy * 0.1;
-    a.az[i] += sz * 0.1;
+    a.ax[i] += a.sum[k] * 0.1;
+    a.ay[i] += a.sum[stride + k] * 0.1;
+    a.az[i] += a.sum[2 * stride + k] * 0.1;
 }
 
 // One query, one thread: src/octree.c:293-318.
@@ -736,7 +864,7 @@ SphArgs make_args(csgd_t *d)
     a.density = 0;
     a.pr2 = d->pr2;
     a.cs = d->cs;
-    a.term = d->sph_term;
+    a.sum = d->sph_sum;
     a.n = d->n;
     a.node_cap = d->node_cap;
     a.stride = d->cap;
@@ -806,8 +934,8 @@ static int ensure_lists(csgd_t *d)
         cudaFree(d->pr2);
     if (d->cs)
         cudaFree(d->cs);
-    if (d->sph_term)
-        cudaFree(d->sph_term);
+    if (d->sph_sum)
+        cudaFree(d->sph_sum);
     if (d->sph_relist)
         cudaFree(d->sph_relist);
     if (d->sph_sorted)
@@ -815,7 +943,7 @@ static int ensure_lists(csgd_t *d)
     d->sph_sorted = nullptr;
     d->nb = nullptr;
     d->nb_count = d->sph_relist = nullptr;
-    d->pr2 = d->cs = d->sph_term = nullptr;
+    d->pr2 = d->cs = d->sph_sum = nullptr;
     size_t c = (size_t)(d->cap > 0 ? d->cap : 1);
     if (csgd_malloc((void **)&d->nb, sizeof(int) * CSG_SPH_MAX_NEIGHBORS * c) != cudaSuccess ||
         csgd_malloc((void **)&d->nb_count, sizeof(int) * c) != cudaSuccess ||
@@ -826,8 +954,7 @@ static int ensure_lists(csgd_t *d)
             cudaSuccess ||
         csgd_malloc((void **)&d->pr2, sizeof(double) * c) != cudaSuccess ||
         csgd_malloc((void **)&d->cs, sizeof(double) * c) != cudaSuccess ||
-        csgd_malloc((void **)&d->sph_term, sizeof(double) * 3 * CSG_SPH_MAX_NEIGHBORS * c) !=
-            cudaSuccess) {
+        csgd_malloc((void **)&d->sph_sum, sizeof(double) * 3 * c) != cudaSuccess) {
         cudaGetLastError();
         csgd_set_err(d, CSG_ERR_NOMEM);
         return CSG_ERR_NOMEM;
@@ -864,17 +991,16 @@ static int sph_pass(csgd_t *d, int forces, bool sums = true, bool reuse = false)
     else
         k_sph_lists<true><<<gl, SPH_THREADS, 0, d->stream>>>(a);
     d->launches++;
-    // pair terms: a grid-stride pass over (slot, gas body), sized for 32 warps
-    // per SM (the gas count is known on the device only)
-    const int gp = d->num_sms * (2048 / SPH_THREADS);
+    // the gas count is known on the device only: the groups stride over the grid
+    const int gp = d->num_sms * PAIR_BLOCKS;
     if (forces) {
-        { k_sph_body_terms<<<g, SUM_THREADS, 0, d->stream>>>(a); d->launches++; }
-        { k_sph_force_terms<<<gp, SPH_THREADS, 0, d->stream>>>(a); d->launches++; }
+        if (!a.reuse)
+            { k_sph_body_terms<<<g, SUM_THREADS, 0, d->stream>>>(a); d->launches++; }
+        { k_sph_force<<<gp, FORCE_THREADS, 0, d->stream>>>(a); d->launches++; }
         if (sums)
-            { k_sph_force_sums<<<g, SUM_THREADS, 0, d->stream>>>(a); d->launches++; }
+            { k_sph_force_add<<<g, SUM_THREADS, 0, d->stream>>>(a); d->launches++; }
     } else {
-        { k_sph_density_terms<<<gp, SPH_THREADS, 0, d->stream>>>(a); d->launches++; }
-        { k_sph_density_sums<<<g, SUM_THREADS, 0, d->stream>>>(a); d->launches++; }
+        { k_sph_density<<<gp, DENSITY_THREADS, 0, d->stream>>>(a); d->launches++; }
     }
     return csgd_check(d, cudaGetLastError());
 }
@@ -898,7 +1024,7 @@ extern "C" int csgd_sph_force_sums(csgd_t *d)
     if (d->n <= 0)
         return CSG_OK;
     SphArgs a = make_args(d);
-    { k_sph_force_sums<<<csgd_grid(d->n, SUM_THREADS), SUM_THREADS, 0, d->stream>>>(a); d->launches++; }
+    { k_sph_force_add<<<csgd_grid(d->n, SUM_THREADS), SUM_THREADS, 0, d->stream>>>(a); d->launches++; }
     return csgd_check(d, cudaGetLastError());
 }
 

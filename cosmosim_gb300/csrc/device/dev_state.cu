@@ -377,8 +377,8 @@ extern "C" void csgd_destroy(csgd_t *d)
         cudaFree(d->pr2);
     if (d->cs)
         cudaFree(d->cs);
-    if (d->sph_term)
-        cudaFree(d->sph_term);
+    if (d->sph_sum)
+        cudaFree(d->sph_sum);
     if (d->sph_relist)
         cudaFree(d->sph_relist);
     if (d->sph_sorted)
