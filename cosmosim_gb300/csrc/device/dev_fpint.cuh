@@ -85,7 +85,8 @@ struct Divisor {
     bool normal;
 };
 
-__device__ __forceinline__ Divisor divisor(double b)
+// b with its reciprocal word computed before (recip_word of its significand)
+__device__ __forceinline__ Divisor divisor(double b, unsigned long long v)
 {
     using namespace fpint;
     const unsigned long long bb = (unsigned long long)__double_as_longlong(b);
@@ -95,8 +96,14 @@ __device__ __forceinline__ Divisor divisor(double b)
     d.eb = (int)(bb >> 52) & 0x7ff;
     d.normal = (unsigned)(d.eb - 1) < 2046u;
     d.Mb = (bb & MANT) | HID;
-    d.v = recip_word(d.Mb);
+    d.v = v;
     return d;
+}
+
+__device__ __forceinline__ Divisor divisor(double b)
+{
+    using namespace fpint;
+    return divisor(b, recip_word(((unsigned long long)__double_as_longlong(b) & MANT) | HID));
 }
 
 // a / d.value, rounded to nearest even (bit-identical to the compiler's operator).

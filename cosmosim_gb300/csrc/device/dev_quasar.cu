@@ -19,10 +19,10 @@
 //    blocks, in-block scan) turns the bits into an ascending list and clears
 //    them.
 //  * Accretion: only candidates inside the swallow radius or the ISCO can be
-//    accreted ("inner"), so only they form a sequential chain: one thread
-//    walks them in index order (staged a block-wide chunk at a time in shared
-//    memory), updating the SMBH and recording its mass and velocity after
-//    every accretion event. Every other candidate ("outer":
+//    accreted ("inner"), so only they form a sequential chain: three warps
+//    take them in index order (accretion_chain), updating the SMBH and
+//    recording its mass and velocity after every accretion event. Every
+//    other candidate ("outer":
 //    possibly turned into gas and dragged, never accreted) runs in parallel
 //    with the SMBH state that holds at its index, found by binary search in
 //    that event table.
@@ -81,8 +81,8 @@ struct QScratch {
     XsJumpTable *jump;
 };
 
-struct Hole { // an SMBH while its victims are processed
-    double x, y, z, vx, vy, vz, m, sx, sy, sz;
+struct Hole { // an SMBH while its candidates are processed
+    double x, y, z, vx, vy, vz, m;
 };
 
 struct Draws { // the step's random stream from a given offset
@@ -203,67 +203,263 @@ __device__ void fresh_body(const Bodies &b, int i, int type)
     b.aos[i].type = (BodyType)type;
 }
 
-// Hole H takes victim v (src/quasar.c:63-101): momentum-conserving merge,
-// spin nudged toward the victim's orbital angular momentum (relative to the
-// merged velocity), victim stopped.
-__device__ void swallow(Hole &H, const Bodies &b, int v)
+// A candidate turns into gas; SPH fields seeded if unset.
+__device__ void make_gas(const Bodies &b, const QCfg &c, int i)
 {
-    const double mv = b.m[v], mt = H.m + mv;
-    H.vx = div_rn(H.m * H.vx + mv * b.vx[v], mt);
-    H.vy = div_rn(H.m * H.vy + mv * b.vy[v], mt);
-    H.vz = div_rn(H.m * H.vz + mv * b.vz[v], mt);
-    const double px = b.x[v] - H.x, py = b.y[v] - H.y, pz = b.z[v] - H.z;
-    const double qx = b.vx[v] - H.vx, qy = b.vy[v] - H.vy, qz = b.vz[v] - H.vz;
-    const double jx = py * qz - pz * qy, jy = pz * qx - px * qz, jz = px * qy - py * qx;
-    const double j = sqrt_rn(jx * jx + jy * jy + jz * jz);
-    if (j > 1e-15) {
-        const double f = div_rn(mv, mt) * 0.01;
-        H.sx += div_rn(f * jx, j);
-        H.sy += div_rn(f * jy, j);
-        H.sz += div_rn(f * jz, j);
-        const double sn = sqrt_rn(H.sx * H.sx + H.sy * H.sy + H.sz * H.sz);
-        if (sn > 1e-15) {
-            H.sx = div_rn(H.sx, sn);
-            H.sy = div_rn(H.sy, sn);
-            H.sz = div_rn(H.sz, sn);
-        }
+    b.type[i] = BODY_GAS;
+    if (b.h[i] < 1e-10)
+        b.h[i] = c.acc_r * 0.3;
+    if (b.u[i] < 1e-10) {
+        const double v2 = b.vx[i] * b.vx[i] + b.vy[i] * b.vy[i] + b.vz[i] * b.vz[i];
+        b.u[i] = 0.001 * v2 + 0.01;
     }
-    H.m = mt;
-    stop_body(b, v);
 }
 
-// A candidate at offset (dx, dy, dz), distance r from hole H that is not
-// swallowed outright (src/quasar.c:156-183): it turns into gas when the
-// circularisation radius of its orbit lies outside the ISCO (SPH fields
-// seeded if unset); gas feels the accretion disk's radial drag
-// (src/quasar.c:103-123). Returns whether the body is gas.
-__device__ bool settle(const Bodies &b, const QCfg &c, const Hole &H, int i, double dx, double dy,
+// An outer candidate at offset (dx, dy, dz), distance r from hole H
+// (src/quasar.c:156-183): it turns into gas when the circularisation radius of
+// its orbit lies outside the ISCO; gas feels the accretion disk's radial drag
+// (src/quasar.c:103-123).
+__device__ void settle(const Bodies &b, const QCfg &c, const Hole &H, int i, double dx, double dy,
                        double dz, double r)
 {
     const double qx = b.vx[i] - H.vx, qy = b.vy[i] - H.vy, qz = b.vz[i] - H.vz;
     const double jx = dy * qz - dz * qy, jy = dz * qx - dx * qz, jz = dx * qy - dy * qx;
     const double r_circ = div_rn(jx * jx + jy * jy + jz * jz, H.m * r);
-    if (r_circ > c.isco_r && b.type[i] != BODY_GAS) {
-        b.type[i] = BODY_GAS;
-        if (b.h[i] < 1e-10)
-            b.h[i] = c.acc_r * 0.3;
-        if (b.u[i] < 1e-10) {
-            const double v2 = b.vx[i] * b.vx[i] + b.vy[i] * b.vy[i] + b.vz[i] * b.vz[i];
-            b.u[i] = 0.001 * v2 + 0.01;
-        }
-    }
+    if (r_circ > c.isco_r && b.type[i] != BODY_GAS)
+        make_gas(b, c, i);
     if (b.type[i] != BODY_GAS)
-        return false;
+        return;
     const double rx = b.x[i] - H.x, ry = b.y[i] - H.y, rz = b.z[i] - H.z;
     const double rr = sqrt_rn(rx * rx + ry * ry + rz * rz);
     if (rr < 1e-15)
-        return true;
+        return;
     const double wx = b.vx[i] - H.vx, wy = b.vy[i] - H.vy, wz = b.vz[i] - H.vz;
     const double radial = div_rn(wx * rx + wy * ry + wz * rz, rr);
     b.ax[i] -= c.alpha * div_rn(radial * rx, rr);
     b.ay[i] -= c.alpha * div_rn(radial * ry, rr);
     b.az[i] -= c.alpha * div_rn(radial * rz, rr);
-    return true;
+}
+
+// The accretion chain of one SMBH: the inner candidates in index order
+// (src/quasar.c:63-101, :125-190), by the first block. A candidate within the
+// swallow radius, or a gas one, is taken; another one (inside the ISCO) is
+// taken, as new gas, if the circularisation radius of its orbit about the SMBH
+// of that moment lies outside the ISCO (:156-183; the drag that gas feels is
+// lost when the victim stops). A victim merges with the SMBH, momentum kept,
+// and nudges its spin toward the victim's orbital angular momentum (relative
+// to the merged velocity).
+//
+// Only three short recurrences are sequential: mass (a sum), velocity (a
+// product, a sum and a quotient per component) and spin (a sum, a root and a
+// quotient). Warps take them as stages of a pipeline over chunks of 32
+// candidates, one barrier a chunk: warp 0 decides, sums the masses (every
+// lane), forms the reciprocals of the sums (one a lane) and runs the velocity
+// (lanes 0 to 2); warp 1, one lane per victim, forms the nudges, stops the
+// victims and writes the event rows; warp 2 runs the spin (lanes 0 to 2). The
+// spin's latency bounds it. @CHAIN
+struct ChainChunk {
+    int idx[CSG_WARP];
+    double pos[3][CSG_WARP], vel[3][CSG_WARP]; // relative position; velocity
+    double m[CSG_WARP], before[CSG_WARP], mt[CSG_WARP];
+    unsigned long long recip[CSG_WARP]; // of mt
+    double prod[3][CSG_WARP];           // m vel
+    double hv[3][CSG_WARP];             // the SMBH's velocity after the victim
+    double nudge[3][CSG_WARP];          // the spin's
+    unsigned eaten, made_gas, nudged;   // lanes
+    int row;                            // event row of the first victim
+};
+
+struct ChainInput { // a lane's candidate
+    int i, type;
+    double x, y, z, vx, vy, vz, m;
+};
+
+__device__ __forceinline__ ChainInput chain_input(const Bodies &b, const int *list, int k, int n)
+{
+    ChainInput c{};
+    c.i = -1;
+    if (k < n) {
+        const int i = list[k];
+        c = ChainInput{i, b.type[i], b.x[i], b.y[i], b.z[i], b.vx[i], b.vy[i], b.vz[i], b.m[i]};
+    }
+    return c;
+}
+
+struct ChainState { // warp 0's; v: component min(lane, 2)
+    double m, v, swallowed;
+    int events;
+};
+
+__device__ void chain_merge(ChainChunk &ch, ChainState &st, const ChainInput &in, const QCfg &c,
+                            double hx, double hy, double hz)
+{
+    const int lane = threadIdx.x & 31, comp = min(lane, 2);
+    const unsigned valid = __ballot_sync(FULL, in.i >= 0);
+    const int cnt = __popc(valid);
+    const double dx = in.x - hx, dy = in.y - hy, dz = in.z - hz;
+    const double d2 = dx * dx + dy * dy + dz * dz;
+    const unsigned open = // decided when its turn comes
+        __ballot_sync(FULL, in.i >= 0 && !(d2 < c.swallow_r * c.swallow_r) && in.type != BODY_GAS);
+    const double r = open ? sqrt_rn(d2) : 0.0;
+    ch.idx[lane] = in.i;
+    ch.pos[0][lane] = dx;
+    ch.pos[1][lane] = dy;
+    ch.pos[2][lane] = dz;
+    ch.vel[0][lane] = in.vx;
+    ch.vel[1][lane] = in.vy;
+    ch.vel[2][lane] = in.vz;
+    ch.m[lane] = in.m;
+    ch.prod[0][lane] = in.m * in.vx;
+    ch.prod[1][lane] = in.m * in.vy;
+    ch.prod[2][lane] = in.m * in.vz;
+    unsigned eaten = 0u;
+    for (int at = 0; at < cnt;) { // a run: a candidate and the decided ones after it
+        const unsigned later = open & ~((2u << at) - 1u);
+        const int end = later ? __ffs(later) - 1 : cnt;
+        unsigned run = (end < 32 ? (1u << end) - 1u : FULL) & ~((1u << at) - 1u);
+        if (open >> at & 1u) {
+            const double qx = __shfl_sync(FULL, in.vx, at) - __shfl_sync(FULL, st.v, 0);
+            const double qy = __shfl_sync(FULL, in.vy, at) - __shfl_sync(FULL, st.v, 1);
+            const double qz = __shfl_sync(FULL, in.vz, at) - __shfl_sync(FULL, st.v, 2);
+            const double ex = __shfl_sync(FULL, dx, at), ey = __shfl_sync(FULL, dy, at),
+                         ez = __shfl_sync(FULL, dz, at);
+            const double jx = ey * qz - ez * qy, jy = ez * qx - ex * qz, jz = ex * qy - ey * qx;
+            const double r_circ =
+                div_rn(jx * jx + jy * jy + jz * jz, st.m * __shfl_sync(FULL, r, at));
+            if (!(r_circ > c.isco_r)) // the same in every lane
+                run &= ~(1u << at);
+        }
+        at = end;
+        double before = 0.0, after = 1.0;
+        for (unsigned left = run; left; left &= left - 1u) {
+            const int e = __ffs(left) - 1;
+            const double mv = __shfl_sync(FULL, in.m, e), mt = st.m + mv;
+            if (lane == e) {
+                before = st.m;
+                after = mt;
+            }
+            st.m = mt;
+            st.swallowed += mv;
+        }
+        if (run >> lane & 1u) {
+            ch.before[lane] = before;
+            ch.mt[lane] = after;
+            ch.recip[lane] = divisor(after).v;
+        }
+        __syncwarp();
+        for (unsigned left = run; left; left &= left - 1u) {
+            const int e = __ffs(left) - 1;
+            st.v = div_rn(ch.before[e] * st.v + ch.prod[comp][e], divisor(ch.mt[e], ch.recip[e]));
+            if (lane < 3)
+                ch.hv[lane][e] = st.v;
+        }
+        eaten |= run;
+    }
+    if (lane == 0) {
+        ch.eaten = eaten;
+        ch.made_gas = eaten & open;
+        ch.row = st.events + 1;
+    }
+    st.events += __popc(eaten);
+}
+
+__device__ void chain_victims(ChainChunk &ch, const Bodies &b, const QCfg &c, const QScratch &w)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned eaten = ch.eaten;
+    bool nudged = false;
+    if (eaten >> lane & 1u) {
+        const int i = ch.idx[lane];
+        const double mv = ch.m[lane], mt = ch.mt[lane];
+        const double px = ch.pos[0][lane], py = ch.pos[1][lane], pz = ch.pos[2][lane];
+        const double bx = ch.vel[0][lane], by = ch.vel[1][lane], bz = ch.vel[2][lane];
+        const double qx = bx - ch.hv[0][lane], qy = by - ch.hv[1][lane], qz = bz - ch.hv[2][lane];
+        const double jx = py * qz - pz * qy, jy = pz * qx - px * qz, jz = px * qy - py * qx;
+        const double j = sqrt_rn(jx * jx + jy * jy + jz * jz);
+        nudged = j > 1e-15;
+        if (nudged) {
+            const double f = div_rn(mv, divisor(mt, ch.recip[lane])) * 0.01;
+            const Divisor by_j = divisor(j);
+            ch.nudge[0][lane] = div_rn(f * jx, by_j);
+            ch.nudge[1][lane] = div_rn(f * jy, by_j);
+            ch.nudge[2][lane] = div_rn(f * jz, by_j);
+        }
+        const int row = ch.row + __popc(eaten & ((1u << lane) - 1u));
+        w.ev_idx[row] = i;
+        w.ev_m[row] = mt;
+        w.ev_vx[row] = ch.hv[0][lane];
+        w.ev_vy[row] = ch.hv[1][lane];
+        w.ev_vz[row] = ch.hv[2][lane];
+        if (ch.made_gas >> lane & 1u)
+            make_gas(b, c, i);
+        stop_body(b, i);
+    }
+    const unsigned m = __ballot_sync(FULL, nudged);
+    if (lane == 0)
+        ch.nudged = m;
+}
+
+// spin: component min(lane, 2)
+__device__ void chain_spin(const ChainChunk &ch, double &spin)
+{
+    const int comp = min((int)(threadIdx.x & 31), 2);
+    for (unsigned left = ch.nudged; left; left &= left - 1u) {
+        spin += ch.nudge[comp][__ffs(left) - 1];
+        const double sq = spin * spin;
+        const double n2 =
+            __shfl_sync(FULL, sq, 0) + __shfl_sync(FULL, sq, 1) + __shfl_sync(FULL, sq, 2);
+        const double sn = sqrt_rn(n2);
+        if (sn > 1e-15)
+            spin = div_rn(spin, sn);
+    }
+}
+
+__device__ void accretion_chain(const Bodies &b, const QCfg &c, const QScratch &w, QuasarState *q,
+                                int s, int n_inner)
+{
+    __shared__ ChainChunk ch[3];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double hx = b.x[s], hy = b.y[s], hz = b.z[s];
+    const double hv[3] = {b.vx[s], b.vy[s], b.vz[s]};
+    const double hs[3] = {b.aos[s].spin_x, b.aos[s].spin_y, b.aos[s].spin_z};
+    const int comp = min(lane, 2);
+    ChainState st{b.m[s], comp == 0 ? hv[0] : comp == 1 ? hv[1] : hv[2], q->swallowed, 0};
+    double spin = comp == 0 ? hs[0] : comp == 1 ? hs[1] : hs[2];
+    ChainInput next{};
+    if (wid == 0) {
+        if (lane == 0) {
+            w.ev_idx[0] = -1; // the state before any event
+            w.ev_m[0] = st.m;
+            w.ev_vx[0] = hv[0];
+            w.ev_vy[0] = hv[1];
+            w.ev_vz[0] = hv[2];
+        }
+        next = chain_input(b, w.list, lane, n_inner);
+    }
+    __syncthreads(); // the SMBH has been read
+    const int chunks = (n_inner + CSG_WARP - 1) / CSG_WARP;
+    for (int t = 0; t < chunks + 2; t++) {
+        if (wid == 0 && t < chunks) {
+            const ChainInput in = next;
+            next = chain_input(b, w.list, (t + 1) * CSG_WARP + lane, n_inner);
+            chain_merge(ch[t % 3], st, in, c, hx, hy, hz);
+        } else if (wid == 1 && t >= 1 && t <= chunks) {
+            chain_victims(ch[(t - 1) % 3], b, c, w);
+        } else if (wid == 2 && t >= 2) {
+            chain_spin(ch[(t - 2) % 3], spin);
+        }
+        __syncthreads();
+    }
+    if (wid == 0 && lane < 3) {
+        if (lane == 0) {
+            q->n_events = st.events;
+            q->swallowed = st.swallowed;
+            b.m[s] = st.m;
+        }
+        (lane == 0 ? b.vx : lane == 1 ? b.vy : b.vz)[s] = st.v;
+    }
+    if (wid == 2 && lane < 3)
+        (lane == 0 ? b.aos[s].spin_x : lane == 1 ? b.aos[s].spin_y : b.aos[s].spin_z) = spin;
 }
 
 // Row e of the event table: the largest e with ev_idx[e] < i (row 0 holds
@@ -356,93 +552,8 @@ __global__ void __launch_bounds__(QB) k_quasar_step(Bodies b, QCfg c, QuasarStat
         grid.sync();
         const int n_inner = grid_compact(grid, w.bits, nwords, w.list, w.blockcnt);
         grid.sync();
-        if (blockIdx.x == 0) {
-            // The chain of possible accretions, in index order. The whole block
-            // stages a chunk of candidates in shared memory, one thread runs
-            // the chain over it (the same arithmetic on the staged copies),
-            // the block writes the candidates back.
-            __shared__ double cf[12][QB];
-            __shared__ int ct[QB];
-            const Bodies sb{cf[0], cf[1], cf[2], cf[3], cf[4], cf[5], cf[6], cf[7], cf[8], cf[9],
-                            nullptr, nullptr, cf[10], cf[11], ct, nullptr};
-            Hole H{hx, hy, hz, b.vx[s], b.vy[s], b.vz[s], b.m[s], b.aos[s].spin_x,
-                   b.aos[s].spin_y, b.aos[s].spin_z};
-            double swallowed = q->swallowed;
-            int e = 0;
-            if (tid == 0) {
-                w.ev_idx[0] = -1;
-                w.ev_m[0] = H.m;
-                w.ev_vx[0] = H.vx;
-                w.ev_vy[0] = H.vy;
-                w.ev_vz[0] = H.vz;
-            }
-            for (int base = 0; base < n_inner; base += QB) {
-                const int cnt = min(QB, n_inner - base);
-                const int i = tid < cnt ? w.list[base + tid] : 0;
-                if (tid < cnt) {
-                    sb.x[tid] = b.x[i];
-                    sb.y[tid] = b.y[i];
-                    sb.z[tid] = b.z[i];
-                    sb.vx[tid] = b.vx[i];
-                    sb.vy[tid] = b.vy[i];
-                    sb.vz[tid] = b.vz[i];
-                    sb.ax[tid] = b.ax[i];
-                    sb.ay[tid] = b.ay[i];
-                    sb.az[tid] = b.az[i];
-                    sb.m[tid] = b.m[i];
-                    sb.u[tid] = b.u[i];
-                    sb.h[tid] = b.h[i];
-                    sb.type[tid] = b.type[i];
-                }
-                __syncthreads();
-                if (tid == 0) {
-                    for (int t = 0; t < cnt; t++) {
-                        const double dx = sb.x[t] - hx, dy = sb.y[t] - hy, dz = sb.z[t] - hz;
-                        const double d2 = dx * dx + dy * dy + dz * dz;
-                        bool eaten = d2 < r_sw_sq;
-                        if (!eaten) {
-                            const double r = sqrt_rn(d2);
-                            eaten = settle(sb, c, H, t, dx, dy, dz, r) && r < c.isco_r;
-                        }
-                        if (eaten) {
-                            swallowed += sb.m[t];
-                            swallow(H, sb, t);
-                            e++;
-                            w.ev_idx[e] = w.list[base + t];
-                            w.ev_m[e] = H.m;
-                            w.ev_vx[e] = H.vx;
-                            w.ev_vy[e] = H.vy;
-                            w.ev_vz[e] = H.vz;
-                        }
-                    }
-                }
-                __syncthreads();
-                if (tid < cnt) {
-                    b.vx[i] = sb.vx[tid];
-                    b.vy[i] = sb.vy[tid];
-                    b.vz[i] = sb.vz[tid];
-                    b.ax[i] = sb.ax[tid];
-                    b.ay[i] = sb.ay[tid];
-                    b.az[i] = sb.az[tid];
-                    b.m[i] = sb.m[tid];
-                    b.u[i] = sb.u[tid];
-                    b.h[i] = sb.h[tid];
-                    b.type[i] = sb.type[tid];
-                }
-                __syncthreads(); // the next chunk reuses the staging
-            }
-            if (tid == 0) {
-                q->n_events = e;
-                q->swallowed = swallowed;
-                b.m[s] = H.m;
-                b.vx[s] = H.vx;
-                b.vy[s] = H.vy;
-                b.vz[s] = H.vz;
-                b.aos[s].spin_x = H.sx;
-                b.aos[s].spin_y = H.sy;
-                b.aos[s].spin_z = H.sz;
-            }
-        }
+        if (blockIdx.x == 0)
+            accretion_chain(b, c, w, q, s, n_inner);
         grid.sync();
         // outer candidates, each with the SMBH state at its index
         const int n_events = q->n_events;
@@ -457,7 +568,7 @@ __global__ void __launch_bounds__(QB) k_quasar_step(Bodies b, QCfg c, QuasarStat
             if (r < c.isco_r)
                 continue; // inner: done by the chain
             const int e = state_at(w, n_events, (int)i);
-            const Hole H{hx, hy, hz, w.ev_vx[e], w.ev_vy[e], w.ev_vz[e], w.ev_m[e], 0.0, 0.0, 0.0};
+            const Hole H{hx, hy, hz, w.ev_vx[e], w.ev_vy[e], w.ev_vz[e], w.ev_m[e]};
             settle(b, c, H, (int)i, dx, dy, dz, r);
         }
         grid.sync();
