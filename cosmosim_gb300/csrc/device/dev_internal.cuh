@@ -66,6 +66,7 @@ struct __align__(16) NodeLink {
 struct FixGrid {
     int ok;                  // 1: the system fits; 0: use the FP64 pair terms
     int g;                   // grid: X = x 2^g
+    int far;                 // cells beyond 2^61 units: X = x 2^(g - far) (walks; 0: none)
     int U3, U1;              // exponent of the last bit of an acceleration, a potential sum
     unsigned eh;             // high word of eps 2^g
     int e2s;                 // eps^2 in units of r2 (fix_pair): e2n >> (e2s - 2 s)
@@ -93,6 +94,7 @@ struct DevRoot {
     int first;                           // their first sorted position
     int root;                            // preorder id of the root cell
     int end;                             // one past the system's last cell
+    int split;                           // the cell whose children are the segments (k_tasks)
     int fix_e;                           // every |coordinate| < 2^fix_e
     int fix_off;                         // a caller's cells do not fit the grid (k_walk_prep)
     FixGrid fix;                         // of the current FP64 walk (k_walk_prep)

@@ -10,9 +10,9 @@
 // FP64 walk: the drop-in precision (k_walk64ws). Openings decided as in the
 //   FP32 walk (equal to the reference's FP64 rounding); interactions queued
 //   and evaluated densely by two further warps per task, on the integer pipes
-//   (dev_fixpair.cuh; in FP64 for systems that do not fit their grid), summed
-//   per child subtree of the root as the FP32 walk does; small systems split the same
-//   way (k_walk64ws_units), with the same bits. k_walk64_exact instead
+//   (dev_fixpair.cuh; in FP64 for systems that do not fit their grid and for
+//   bodies far outside it), small systems split by child subtrees as in the
+//   FP32 walk (k_walk64ws_units), with the same bits. k_walk64_exact instead
 //   uses the reference's own operation sequence per step (1/(r2*sqrt(r2)),
 //   no fused multiply-add) — bit-identical results on the reference's own
 //   tree; used by parity tests. It alone walks cell by cell: one cursor over
@@ -20,11 +20,12 @@
 //   ancestor), the next 32 cells staged per warp in shared memory.
 // FP32-mixed walk: positions and centres as float hi/lo pairs (differences
 //   keep ~48 bits), rsqrt/products in FP32, Kahan-compensated FP32 sums per
-//   body (small systems: per child subtree of the root, added in FP64).
+//   body (small systems: per child subtree of the split cell, mostly the root,
+//   added in FP64).
 //   Openings within the FP32 error band of the threshold are decided in FP64,
 //   so the interaction set equals the FP64 walk's. Small systems with few
-//   tasks for the GPU are walked by eight warps per task, one per root child
-//   (k_walk32_units), with the same bits as one warp per task (k_walk32).
+//   tasks for the GPU are walked by eight warps per task, one per child
+//   subtree (k_walk32_units), with the same bits as one warp per task (k_walk32).
 #include "dev_fixpair.cuh"
 #include "dev_internal.cuh"
 
@@ -53,7 +54,7 @@ struct WalkArgs {
     double *part;   // split walks: segment partials, part[(3 * k + d) * pstride + body]
     long long pstride;
     // systems of at most split_max bodies (sys_n[gal] each in an ensemble,
-    // n_bodies for one system) sum by the root's children; the FP64 whole-task
+    // n_bodies for one system) sum by the split cell's children; the FP64 whole-task
     // walk leaves them out when skip_small is set
     const int *sys_n;
     int n_bodies, split_max, skip_small;
@@ -82,6 +83,7 @@ struct WalkStats {
 // Validated task: bodies [pos0, pos0+count) and the system's cells [root, end).
 struct TaskRange {
     int pos0, count, root, end;
+    int split;  // its children are the segments of a small system
     bool small; // its system has at most split_max bodies
 };
 
@@ -100,7 +102,7 @@ __device__ __forceinline__ void for_each_task(const WalkArgs &a, Fn fn)
     auto run = [&](int t) {
         const WalkTask w = a.tasks[t];
         const DevRoot &r = a.roots[w.gal];
-        const TaskRange tr{w.pos0, w.count, r.root, r.end, small_system(a, w.gal)};
+        const TaskRange tr{w.pos0, w.count, r.root, r.end, r.split, small_system(a, w.gal)};
         if (tr.root < 0 || tr.end > nn || tr.root >= tr.end)
             dev_fail(a.sc, CSG_ERR_WALK_LIMIT);
         else
@@ -724,8 +726,8 @@ __device__ __forceinline__ void kahan_add2(u64 &s, u64 &c, u64 v)
 //
 // A large system's task sums the whole tree in one go. A small system's
 // (split_max bodies or fewer) closes its sums into double partials: first the
-// root's own term, then one per child subtree of the system's root
-// ("segment" k < 8, in child order); the body's acceleration is G times the
+// terms of the root (and of what walk_top walks), then one per child subtree
+// of the system's split cell, mostly the root ("segment" k < 8, in child order); the body's acceleration is G times the
 // sum of the partials in that order. Its tasks can so be walked by one warp
 // (all segments in turn) or by eight (one segment each; unit 0 also takes the
 // root's term, and 0 + root is the root exactly; the partials added by
@@ -825,27 +827,60 @@ __device__ __forceinline__ void clear_rec(RoundShared &sh)
     __syncwarp();
 }
 
-// The root: taken or opened lane by lane; returns the lanes that open it.
+// One cell, taken or opened lane by lane; returns the lanes that open it.
 // count: this warp's takes count (one of a split task's units counts them).
 template <bool STATS, class Sink>
-__device__ __forceinline__ unsigned walk_root(const WalkArgs &a, const LaneBody &L,
-                                              const TaskRange &tr, Sink &sink, WalkStats &st,
-                                              bool count = true)
+__device__ __forceinline__ unsigned walk_cell(const WalkArgs &a, const LaneBody &L, int cell,
+                                              unsigned lanes, Sink &sink, WalkStats &st, bool count)
 {
+    const bool mine = lanes >> (threadIdx.x & 31) & 1u;
     int next;
     bool take, open;
     if (STATS) {
         st.steps++;
-        st.active += L.valid;
+        st.active += mine;
     }
-    lane_test(a, L, tr.root, L.valid, next, take, open, sink);
+    lane_test(a, L, cell, mine, next, take, open, sink);
     if (STATS)
         st.hits += count && take;
     return __ballot_sync(0xffffffffu, open);
 }
 
+// A system's cells above its segments: the root, and down to tr.split the cells
+// on the way with their other children's subtrees (`mine`: this warp's to walk;
+// else only the way is tested). Returns the lanes that open tr.split.
+template <bool STATS, class Sink>
+__device__ __forceinline__ unsigned walk_top(const WalkArgs &a, RoundShared &sh, const LaneBody &L,
+                                             const TaskRange &tr, Sink &sink, WalkStats &st,
+                                             bool mine)
+{
+    int cell = tr.root;
+    unsigned open =
+        walk_cell<STATS>(a, L, cell, __ballot_sync(0xffffffffu, L.valid), sink, st, mine);
+    while (cell != tr.split && open) {
+        int down = -1; // the child that holds tr.split (cells are in preorder)
+        for (int o = 0; o < 8; o++) {
+            const int c = __ldg(&a.child[8 * (size_t)cell + o]);
+            if (c > cell && c <= tr.split)
+                down = max(down, c);
+        }
+        if (down < 0) { // not a cell of this tree
+            dev_fail(a.sc, CSG_ERR_WALK_LIMIT);
+            return 0u;
+        }
+        for (int o = 0; o < 8 && mine; o++) {
+            const int c = __ldg(&a.child[8 * (size_t)cell + o]);
+            if (c > cell && c != down)
+                walk_subtree<STATS>(a, sh, L, c, open, sink, st);
+        }
+        open = walk_cell<STATS>(a, L, down, open, sink, st, mine);
+        cell = down; // strictly increases: the loop ends
+    }
+    return open;
+}
+
 // The whole task by one warp: a large system's tree from the root; a small
-// system's root, then each child subtree of it as a segment, every one closed
+// system's top, then each child subtree of its split cell as a segment, every one closed
 // into the double sum g.
 template <bool STATS>
 __device__ __forceinline__ void walk32_task(const WalkArgs &a, Walk32Shared &sh,
@@ -858,9 +893,9 @@ __device__ __forceinline__ void walk32_task(const WalkArgs &a, Walk32Shared &sh,
     Sum32 sum(a, L);
     double x = 0.0, y = 0.0, z = 0.0;
     unsigned go = __ballot_sync(0xffffffffu, L.valid);
-    int q = -1; // whole: one subtree, the root's; else the root's children
+    int q = -1; // whole: one subtree, the root's; else the split cell's children
     if (tr.small) {
-        go = walk_root<STATS>(a, L, tr, sum, st);
+        go = walk_top<STATS>(a, sh.r, L, tr, sum, st, true);
         sum.close(x, y, z);
         q = 0;
     }
@@ -869,8 +904,8 @@ __device__ __forceinline__ void walk32_task(const WalkArgs &a, Walk32Shared &sh,
     g[2 * CSG_WARP] = z;
     const int qend = tr.small ? (go ? 8 : 0) : 0;
     for (; q < qend; q++) {
-        const int c = q < 0 ? tr.root : __ldg(&a.child[8 * (size_t)tr.root + q]);
-        if (q >= 0 && c <= tr.root)
+        const int c = q < 0 ? tr.root : __ldg(&a.child[8 * (size_t)tr.split + q]);
+        if (q >= 0 && c <= tr.split)
             continue;
         walk_subtree<STATS>(a, sh.r, L, c, go, sum, st);
         sum.close(x, y, z);
@@ -897,14 +932,14 @@ __device__ __forceinline__ void walk32_unit(const WalkArgs &a, Walk32Shared &sh,
     clear_rec(sh.r);
     const LaneBody L = lane_body(a, sh.r, tr);
     Sum32 sum(a, L);
-    const unsigned open = walk_root<false>(a, L, tr, sum, st);
+    const unsigned open = walk_top<false>(a, sh.r, L, tr, sum, st, k == 0);
     double rx, ry, rz, x = 0.0, y = 0.0, z = 0.0;
     sum.close(rx, ry, rz);
     double *g = sh.g + (threadIdx.x & 31);
     g[0] = rx;
     g[CSG_WARP] = ry;
     g[2 * CSG_WARP] = rz;
-    const int c = nth_child(a, tr.root, k);
+    const int c = nth_child(a, tr.split, k);
     if (open && c >= 0) {
         walk_subtree<false>(a, sh.r, L, c, open, sum, st);
         sum.close(x, y, z);
@@ -957,7 +992,7 @@ __global__ void __launch_bounds__(4 * CSG_WARP, WALK32_RES / 4) k_walk32_units(W
         return;
     const WalkTask w = a.tasks[u / WSEGS];
     const DevRoot &r = a.roots[w.gal];
-    const TaskRange tr{w.pos0, w.count, r.root, r.end, small_system(a, w.gal)};
+    const TaskRange tr{w.pos0, w.count, r.root, r.end, r.split, small_system(a, w.gal)};
     if (tr.root < 0 || tr.end > nn || tr.root >= tr.end)
         dev_fail(a.sc, CSG_ERR_WALK_LIMIT);
     else
@@ -1053,7 +1088,10 @@ struct EvalF64 {
     }
 };
 
-struct EvalFix { // integers from end to end, for systems on the grid
+// Integers from end to end, for systems on the grid. WIDE: some cells are on
+// the coarser grid of far ones, marked by bit 62 of z (no |Z| has it).
+template <bool WIDE>
+struct EvalFix {
     typedef FixBody Rec;
     const FixBody *cells;
     const FixGrid f;
@@ -1085,7 +1123,13 @@ struct EvalFix { // integers from end to end, for systems on the grid
     }
     __device__ __forceinline__ void term(const Rec &r, int)
     {
-        fix_add3(f, r.x - px, r.y - py, r.z - pz, r.m, x, y, z);
+        if (WIDE) {
+            const int hz = (int)(r.z >> 32), far = (hz >> 30 ^ hz >> 31) & 1, up = far ? f.far : 0;
+            const long long rz = r.z ^ ((long long)far << 62);
+            fix_add3(f, r.x - (px >> up), r.y - (py >> up), rz - (pz >> up), r.m, x, y, z, up);
+        } else {
+            fix_add3(f, r.x - px, r.y - py, r.z - pz, r.m, x, y, z);
+        }
         cnt -= (int)hi32(r.m) >> 31; // massless ones do not count
     }
     static __device__ __forceinline__ void drop(Rec &r) { r.m = 0ull; }
@@ -1130,7 +1174,7 @@ __device__ __forceinline__ void put_partial(const WalkArgs &a, int k, int me, do
 // block counters in shared memory; every wait polls with a sleep and gives up
 // after a.wait_polls polls (recording CSG_ERR_DEVICE_WAIT, then all warps leave
 // the task). A unit of the split form (G > 0) is G segments of a task: the root
-// step, then the subtrees of the root's children k0 .. k0 + G - 1; the first
+// step, then the subtrees of the split cell's children k0 .. k0 + G - 1; the first
 // block of a later segment is marked.
 //
 // Bound: the integer multiply and ALU pipes (65% and 62% busy at 1M, issue
@@ -1139,6 +1183,9 @@ __device__ __forceinline__ void put_partial(const WalkArgs &a, int k, int me, do
 // one consumer -> integer pairs -> blocks and two consumers: 1M 39.0 -> 33.0 ->
 // 24.8 ms, 100k merger 2.23 -> 1.97 -> 1.35 ms, 20k disk 0.496 -> 0.448 ->
 // 0.36 ms. Off the grid (FP64 pairs, same queue): 20k 0.48, 100k 2.0, 1M 41 ms.
+// A quasar of 17,000 bodies with some thrown out to 2^15 softening lengths: 1.63
+// ms in FP64, 1.18 with its far cells on a coarser grid, 0.87 with the segments
+// of a deeper split cell.
 //
 // Blocks rather than a ring of ids per lane: an id costs 4 bytes a block, not
 // 4 bytes a lane that takes it, so the same memory holds several times the
@@ -1230,12 +1277,12 @@ __device__ __forceinline__ void ws_produce(const WalkArgs &a, RoundShared &rs, W
     const LaneBody L = lane_body(a, rs, tr);
     BlockQueue q(a, L, sh, cons);
     q.mute = G > 0 && k0 != 0; // the root's terms are segment 0's
-    const unsigned open = walk_root<STATS>(a, L, tr, q, st, !q.mute);
+    const unsigned open = walk_top<STATS>(a, rs, L, tr, q, st, !q.mute);
     q.mute = false;
     int k = 0; // child (segment) number
     for (int o = 0; o < 8 && open; o++) {
-        const int c = __ldg(&a.child[8 * (size_t)tr.root + o]);
-        if (c <= tr.root)
+        const int c = __ldg(&a.child[8 * (size_t)tr.split + o]);
+        if (c <= tr.split)
             continue;
         if (G == 0 || (k >= k0 && k < k0 + G)) {
             if (G > 0 && k > k0) {
@@ -1415,6 +1462,20 @@ __device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, cons
     }
 }
 
+// Whether all of the task's bodies are close enough to the origin to meet far
+// cells (within 2^60 units).
+__device__ __forceinline__ bool near_task(const WalkArgs &a, const TaskRange &tr, const FixGrid &f)
+{
+    const int lane = threadIdx.x & 31;
+    bool ok = true;
+    if (lane < tr.count) {
+        const int me = a.perm[tr.pos0 + lane];
+        const double lim = fix_pow2(FIX_POS_BITS - 1 - f.g);
+        ok = fabs(a.x[me]) < lim && fabs(a.y[me]) < lim && fabs(a.z[me]) < lim;
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+
 // One task per block (G == 0), or one unit of G segments of a task,
 // u = (8 / G) * task + k0 / G (partials into a.part): the producer warp, then
 // CONS consumers. Two consumers where the split does not mark segment ends
@@ -1435,7 +1496,7 @@ __device__ __forceinline__ void walk64ws_body(const WalkArgs &a)
         return;
     const WalkTask w = a.tasks[t];
     const DevRoot &r = a.roots[w.gal];
-    const TaskRange tr{w.pos0, w.count, r.root, r.end, small_system(a, w.gal)};
+    const TaskRange tr{w.pos0, w.count, r.root, r.end, r.split, small_system(a, w.gal)};
     if (G > 0 ? !tr.small : (tr.small && a.skip_small))
         return; // the other form walks this system
     if (tr.root < 0 || tr.end > nn || tr.root >= tr.end) {
@@ -1443,7 +1504,7 @@ __device__ __forceinline__ void walk64ws_body(const WalkArgs &a)
             dev_fail(a.sc, CSG_ERR_WALK_LIMIT);
         return;
     }
-    const bool fix = a.wfix && r.fix.ok && !r.fix_off;
+    const bool fix = a.wfix && r.fix.ok && !r.fix_off && (r.fix.far == 0 || near_task(a, tr, r.fix));
     if (threadIdx.x == 0) {
         sh.tail = 0;
         sh.head[0] = 0;
@@ -1458,8 +1519,10 @@ __device__ __forceinline__ void walk64ws_body(const WalkArgs &a)
         ws_produce<STATS, G>(a, rs, sh, tr, k0, CONS, st);
         if (STATS)
             add_hits(a, st);
+    } else if (fix && r.fix.far == 0) {
+        ws_consume<G, CONS, EvalFix<false>>(a, sh, tr, r.fix, k0, warp - 1);
     } else if (fix) {
-        ws_consume<G, CONS, EvalFix>(a, sh, tr, r.fix, k0, warp - 1);
+        ws_consume<G, CONS, EvalFix<true>>(a, sh, tr, r.fix, k0, warp - 1);
     } else {
         ws_consume<G, CONS, EvalF64<CONS>>(a, sh, tr, r.fix, k0, warp - 1);
     }
@@ -1471,7 +1534,7 @@ __global__ void __launch_bounds__(3 * CSG_WARP, WS_RES / 3) k_walk64ws(WalkArgs 
     walk64ws_body<STATS, 0, 2>(a);
 }
 
-// The FP64 walk split by the root's children (few tasks for the GPU): partials
+// The FP64 walk split by the split cell's children (few tasks for the GPU): partials
 // into a.part, summed by k_walk_sum; the same bits for every G.
 template <bool STATS, int G>
 __global__ void __launch_bounds__((G == 1 ? 3 : 2) * CSG_WARP, WS_RES / (G == 1 ? 3 : 2))
@@ -1511,17 +1574,26 @@ __global__ void k_walk_prep(const double *__restrict__ m, double *ax, double *ay
         DevRoot &r = roots[g];
         if (r.n_alive > 0) {
             const double far = fmax(fabs(r.c0[0]), fmax(fabs(r.c0[1]), fabs(r.c0[2]))) + r.hs0;
-            r.fix = fix_grid(far, w64[r.root].m, 1.0, eps, eps2);
+            r.fix = fix_grid(far, w64[r.root].m, 1.0, eps, eps2, FIX_FAR_MAX);
         }
     }
     for (int id = i; id < nn; id += stride) {
         const int e = max(roots[n_gal > 1 ? sgid[link[id].first] : 0].fix_e, ee);
-        const double scale = fix_pow2(min(max(FIX_POS_BITS - e, -1000), 1000));
         const double2 *w = (const double2 *)&w64[id];
         const double2 xy = w[0], zm = w[1];
+        int far;
+        const int g = fix_scale(e, ee, far);
+        bool out = false;
+        if (far > 0) { // |coordinate| >= 2^61 units, by the exponent
+            const int top = max(max(__double2hiint(xy.x) & 0x7fffffff, __double2hiint(xy.y) & 0x7fffffff),
+                                __double2hiint(zm.x) & 0x7fffffff);
+            out = (top >> 20) - 1023 >= FIX_POS_BITS - g;
+        }
+        const double scale = fix_pow2(min(max(out ? g - far : g, -1000), 1000));
         longlong2 *o = (longlong2 *)&wfix[id];
         o[0] = make_longlong2(fix_pos(xy.x, scale), fix_pos(xy.y, scale));
-        o[1] = make_longlong2(fix_pos(zm.x, scale), (long long)fix_mass(zm.y));
+        o[1] = make_longlong2(fix_pos(zm.x, scale) ^ ((long long)out << 62),
+                              (long long)fix_mass(zm.y));
         if (!imported)
             continue;
         // a caller's cell may lie anywhere and weigh anything: off the grid, or
