@@ -147,9 +147,11 @@ int csgd_gravity(csgd_t *d, const csgd_force_params *p);
 int csgd_gravity_ex(csgd_t *d, const csgd_force_params *p, int exact);
 
 /* Interaction lists of the current tree (built here): with fill = 0 writes
-   counts[i] (cells body i interacts with; untouched for dead bodies); with
-   fill = 1 writes the cell ids, in the reference's depth-first order, to
-   ids[offs[i] ..], at most cap entries in all. Device pointers. */
+   counts[S i + k], the cells of segment k < S = csgd_list_segments(d, n) of body i's
+   list (untouched for dead bodies); with fill = 1 writes the cell ids to
+   ids[offs[S i + k] ..], at most cap entries in all. The reference's
+   interaction set, in the order the walk meets it. Device pointers. */
+int csgd_list_segments(const csgd_t *d, int n);
 int csgd_walk_lists(csgd_t *d, const csgd_force_params *p, int *counts, const int *offs,
                     int *ids, int cap, int fill);
 

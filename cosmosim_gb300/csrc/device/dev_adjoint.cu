@@ -29,6 +29,7 @@
 // Memory: positions and velocities are kept every K substeps; a segment's
 // trees and lists are rebuilt from its checkpoint (bit-identical: every
 // forward kernel is deterministic) before it is reversed.
+#include "dev_fpint.cuh"
 #include "dev_internal.cuh"
 
 #include <stdlib.h>
@@ -76,34 +77,97 @@ __global__ void k_adj_gather(const int *__restrict__ perm, int n, const double *
 }
 
 // Centre of mass and mass of every cell from the current positions of its
-// member bodies (sorted range [first, first+count) of sb); one warp per cell,
-// the lanes' partial sums combined by a fixed butterfly (deterministic).
-__global__ void k_adj_moments(const NodeLink *__restrict__ link, int nn,
-                              const double4_32a *__restrict__ sb, double4_32a *__restrict__ xm)
+// member bodies (sorted range [first, first+count) of sb). A block takes
+// every gridDim-th cell (big cells are neighbours in preorder): those of up to MOM_THREAD bodies by one thread each, then
+// those of up to MOM_WARP by one warp each, then the others by all its threads.
+// Partial sums are combined in a fixed order (deterministic). One warp per cell
+// was bound by the FP64 pipe (an instruction holds it for a whole warp, however
+// few bodies the cell has) and by the root's warp: 75 us for 10,000 bodies, now
+// 28 us.
+constexpr int MOM_CELLS = 64, MOM_THREAD = 8, MOM_WARP = 256;
+
+__device__ __forceinline__ void put_moments(double4_32a *xm, const double s[4])
 {
-    const int w = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (w >= nn)
-        return;
-    const NodeLink l = link[w];
-    double M = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
-    for (int q = l.first + lane; q < l.first + l.count; q += CSG_WARP) {
-        const double4_32a b = sb[q];
-        M += b.w;
-        sx += b.w * b.x;
-        sy += b.w * b.y;
-        sz += b.w * b.z;
-    }
-    M = warp_sum(M);
-    sx = warp_sum(sx);
-    sy = warp_sum(sy);
-    sz = warp_sum(sz);
-    if (lane == 0)
-        xm[w] = make_double4_32a(sx / M, sy / M, sz / M, M);
+    const Divisor M = divisor(s[3]);
+    *xm = make_double4_32a(div_rn(s[0], M), div_rn(s[1], M), div_rn(s[2], M), s[3]);
 }
 
-// a_i from the body's list; one warp per body (lanes stride the list).
-__global__ void k_adj_forces(const int *__restrict__ offs, const int *__restrict__ ids,
+__device__ __forceinline__ void moment_sums(const double4_32a *__restrict__ sb, int from, int to,
+                                            int step, double s[4])
+{
+    s[0] = s[1] = s[2] = s[3] = 0.0;
+#pragma unroll 4
+    for (int q = from; q < to; q += step) {
+        const double4_32a b = sb[q];
+        s[0] = fma(b.w, b.x, s[0]);
+        s[1] = fma(b.w, b.y, s[1]);
+        s[2] = fma(b.w, b.z, s[2]);
+        s[3] += b.w;
+    }
+}
+
+__global__ void __launch_bounds__(AT) k_adj_moments(const NodeLink *__restrict__ link, int nn,
+                                                    const double4_32a *__restrict__ sb,
+                                                    double4_32a *__restrict__ xm)
+{
+    constexpr int W = AT / CSG_WARP;
+    __shared__ int2 range[MOM_CELLS]; // first, count
+    __shared__ double part[W][4];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, grid = gridDim.x;
+    const int c0 = blockIdx.x, cells = min(MOM_CELLS, (nn - c0 + grid - 1) / grid);
+    double s[4];
+    if ((int)threadIdx.x < cells) {
+        const NodeLink l = link[c0 + grid * threadIdx.x];
+        range[threadIdx.x] = make_int2(l.first, l.count);
+        if (l.count == 1) {
+            xm[c0 + grid * threadIdx.x] = sb[l.first];
+        } else if (l.count <= MOM_THREAD) {
+            moment_sums(sb, l.first, l.first + l.count, 1, s);
+            put_moments(&xm[c0 + grid * threadIdx.x], s);
+        }
+    }
+    __syncthreads();
+    int turn = 0;
+    for (int c = 0; c < cells; c++) { // uniform in the block
+        const int2 r = range[c];
+        if (r.y <= MOM_THREAD)
+            continue;
+        if (r.y <= MOM_WARP) {
+            if (turn++ % W != wid)
+                continue;
+            moment_sums(sb, r.x + lane, r.x + r.y, CSG_WARP, s);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                s[k] = warp_sum(s[k]);
+            if (lane == 0)
+                put_moments(&xm[c0 + grid * c], s);
+            continue;
+        }
+        moment_sums(sb, r.x + (int)threadIdx.x, r.x + r.y, AT, s);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            s[k] = warp_sum(s[k]);
+        __syncthreads(); // the last large cell's part has been read
+        if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                part[wid][k] = s[k];
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < W; w++)
+                for (int k = 0; k < 4; k++)
+                    s[k] += part[w][k];
+            put_moments(&xm[c0 + grid * c], s);
+        }
+    }
+}
+
+// a_i from the body's list (entries offs[segs i] to offs[segs (i + 1)]); one
+// warp per body (lanes stride the list). Bound by the FP64 pipe: 9 operations a
+// pair, m/r^3 by integers; with FP64 series 16, 161 us for 10,000 bodies, now
+// 112 us.
+__global__ void k_adj_forces(const int *__restrict__ offs, int segs, const int *__restrict__ ids,
                              const double4_32a *__restrict__ xm, const double *__restrict__ x,
                              const double *__restrict__ y, const double *__restrict__ z,
                              const double *__restrict__ m, int n, double G, double eps2,
@@ -117,30 +181,31 @@ __global__ void k_adj_forces(const int *__restrict__ offs, const int *__restrict
     double sx = 0.0, sy = 0.0, sz = 0.0;
     if (m[i] > 0.0) {
         const double px = x[i], py = y[i], pz = z[i];
-        for (int k = offs[i] + lane; k < offs[i + 1]; k += CSG_WARP) {
+        const int end = offs[(size_t)segs * (i + 1)];
+        for (int k = offs[(size_t)segs * i] + lane; k < end; k += CSG_WARP) {
             const double4_32a c = xm[ids[k]];
             const double dx = c.x - px, dy = c.y - py, dz = c.z - pz;
-            const double r2 = dx * dx + dy * dy + dz * dz + eps2;
-            double inv3, inv5;
-            inv_r3_r5(r2, inv3, inv5);
-            const double f = G * c.w * inv3;
-            sx += f * dx;
-            sy += f * dy;
-            sz += f * dz;
+            const double f = m_inv_r3_q(c.w, fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
+            sx = fma(f, dx, sx);
+            sy = fma(f, dy, sy);
+            sz = fma(f, dz, sz);
         }
     }
     sx = warp_sum(sx);
     sy = warp_sum(sy);
     sz = warp_sum(sz);
     if (lane == 0) {
-        ax[i] = sx;
-        ay[i] = sy;
-        az[i] = sz;
+        ax[i] = G * sx;
+        ay[i] = G * sy;
+        az[i] = G * sz;
     }
 }
 
-// Self term of (J^T mu)_i and the scatter of T mu_i into the cells' g.
-__global__ void k_adj_jt(const int *__restrict__ offs, const int *__restrict__ ids,
+// Self term of (J^T mu)_i and the scatter of T mu_i (without G) into the cells'
+// g. Bound by
+// the FP64 pipe: 20 operations a pair with m/r^3 and 1/r^2 by integers; with
+// FP64 series 32, 350 us for 10,000 bodies, now 296 us.
+__global__ void k_adj_jt(const int *__restrict__ offs, int segs, const int *__restrict__ ids,
                          const double4_32a *__restrict__ xm, const double *__restrict__ x,
                          const double *__restrict__ y, const double *__restrict__ z,
                          const double *__restrict__ m, const double *__restrict__ mux,
@@ -156,18 +221,19 @@ __global__ void k_adj_jt(const int *__restrict__ offs, const int *__restrict__ i
     if (m[i] > 0.0) {
         const double px = x[i], py = y[i], pz = z[i];
         const double ux = mux[i], uy = muy[i], uz = muz[i];
-        for (int k = offs[i] + lane; k < offs[i + 1]; k += CSG_WARP) {
+        const double ux3 = 3.0 * ux, uy3 = 3.0 * uy, uz3 = 3.0 * uz;
+        const int end = offs[(size_t)segs * (i + 1)];
+        for (int k = offs[(size_t)segs * i] + lane; k < end; k += CSG_WARP) {
             const int c = ids[k];
             const double4_32a q = xm[c];
             const double dx = q.x - px, dy = q.y - py, dz = q.z - pz;
-            const double r2 = dx * dx + dy * dy + dz * dz + eps2;
-            double inv3, inv5;
-            inv_r3_r5(r2, inv3, inv5);
-            const double gm = G * q.w;
-            const double dm = 3.0 * (dx * ux + dy * uy + dz * uz) * inv5;
-            const double wx = gm * (ux * inv3 - dm * dx);
-            const double wy = gm * (uy * inv3 - dm * dy);
-            const double wz = gm * (uz * inv3 - dm * dz);
+            double inv2;
+            const double f =
+                m_inv_r3_r2(q.w, fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))), inv2);
+            const double h = -(f * inv2) * fma(dx, ux3, fma(dy, uy3, dz * uz3));
+            const double wx = fma(f, ux, h * dx);
+            const double wy = fma(f, uy, h * dy);
+            const double wz = fma(f, uz, h * dz);
             sx += wx;
             sy += wy;
             sz += wz;
@@ -180,17 +246,17 @@ __global__ void k_adj_jt(const int *__restrict__ offs, const int *__restrict__ i
     sy = warp_sum(sy);
     sz = warp_sum(sz);
     if (lane == 0) {
-        jx[i] = -sx;
-        jy[i] = -sy;
-        jz[i] = -sz;
+        jx[i] = -G * sx;
+        jy[i] = -G * sy;
+        jz[i] = -G * sz;
     }
 }
 
-// (J^T mu)_j += m_j * sum over the cells containing j of g_c / M_c.
+// (J^T mu)_j += m_j * sum over the cells containing j of G g_c / M_c.
 __global__ void k_adj_push(const int *__restrict__ perm, const int *__restrict__ leaf_of,
                            const NodeLink *__restrict__ link, const double4_32a *__restrict__ xm,
-                           const double *__restrict__ g, const double *__restrict__ m, int n_alive,
-                           int nn, double *__restrict__ jx, double *__restrict__ jy,
+                           const double *__restrict__ g, const double *__restrict__ m, double G,
+                           int n_alive, int nn, double *__restrict__ jx, double *__restrict__ jy,
                            double *__restrict__ jz, DevScalars *sc)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -204,7 +270,7 @@ __global__ void k_adj_push(const int *__restrict__ perm, const int *__restrict__
             dev_fail(sc, CSG_ERR_WALK_LIMIT);
             break;
         }
-        const double inv = 1.0 / xm[c].w;
+        const double inv = G / xm[c].w;
         sx += g[3 * (size_t)c + 0] * inv;
         sy += g[3 * (size_t)c + 1] * inv;
         sz += g[3 * (size_t)c + 2] * inv;
@@ -353,7 +419,7 @@ struct Slot {
     int *perm = nullptr;                             // sorted alive bodies
     int *leaf_of = nullptr;                          // sorted position -> leaf cell
     NodeLink *link = nullptr;                        // cells
-    int *offs = nullptr;                             // n+1 list offsets (caller order)
+    int *offs = nullptr; // segs n + 1 list offsets (caller order)
     int *ids = nullptr;                              // list entries (cell ids)
     int nn = 0, n_alive = 0;
     long long total = 0, cap_ids = 0;
@@ -382,7 +448,8 @@ struct csg_adjoint {
     double *g = nullptr;        // 3 per cell
     double4_32a *xm = nullptr;      // per cell
     double4_32a *sb = nullptr;      // per sorted position: x y z m (moment pass)
-    int *counts = nullptr;      // n
+    int segs = 1;               // a body's list is this many walks' (csgd_list_segments)
+    int *counts = nullptr;      // segs n
     int *h_total = nullptr;     // pinned: list entries of the current substep
     std::vector<double> host_m, final_x, target;
     double loss = 0.0;
@@ -432,7 +499,7 @@ int ensure_slots(csg_adjoint *a, int count)
             e = alloc(&s.perm, n);
             if (e == cudaSuccess) e = alloc(&s.leaf_of, n);
             if (e == cudaSuccess) e = alloc(&s.link, ncap);
-            if (e == cudaSuccess) e = alloc(&s.offs, (size_t)n + 1);
+            if (e == cudaSuccess) e = alloc(&s.offs, (size_t)a->segs * n + 1);
         }
         if (e != cudaSuccess) {
             free_slot(s);
@@ -440,7 +507,7 @@ int ensure_slots(csg_adjoint *a, int count)
         }
         a->bytes += sizeof(double) * 3 * (size_t)n;
         if (a->mode == CSG_ADJ_TREE)
-            a->bytes += sizeof(int) * (3 * (size_t)n + 1) + sizeof(NodeLink) * (size_t)ncap;
+            a->bytes += sizeof(int) * ((2 + (size_t)a->segs) * n + 1) + sizeof(NodeLink) * (size_t)ncap;
         a->slots.push_back(s);
     }
     return CSG_OK;
@@ -460,10 +527,21 @@ int eval(csg_adjoint *a, Slot &s)
         { k_adj_direct_forces<<<csgd_grid(n, DT2), DT2, 0, st>>>(d->x, d->y, d->z, d->m, n, a->G, a->eps * a->eps, d->ax, d->ay, d->az); d->launches++; }
         return csgd_check(d, cudaGetLastError());
     }
+    const int lists = a->segs * n;
+    const csgd_force_params p = walk_params(a);
     int rc = csgd_build_tree(d, 0);
-    int nn = 0;
+    if (rc)
+        return rc;
+    cudaMemsetAsync(a->counts, 0, sizeof(int) * (size_t)lists, st);
+    rc = csgd_walk_lists(d, &p, a->counts, nullptr, nullptr, 0, 0);
     if (!rc)
+        rc = csg_scan_exclusive(d, a->counts, s.offs, lists, nullptr);
+    int total = 0, nn = 0;
+    if (!rc) {
+        cudaMemcpyAsync(a->h_total, s.offs + lists, sizeof(int), cudaMemcpyDeviceToHost, st);
         rc = csgd_node_count(d, &nn); // syncs; also reports build errors
+        total = *a->h_total;
+    }
     if (rc)
         return rc;
     s.nn = nn;
@@ -471,19 +549,6 @@ int eval(csg_adjoint *a, Slot &s)
     cudaMemcpyAsync(s.perm, d->perm, sizeof(int) * n, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(s.link, d->link, sizeof(NodeLink) * (size_t)nn, cudaMemcpyDeviceToDevice, st);
     { k_adj_leaf_of<<<csgd_grid(nn, AT), AT, 0, st>>>(d->link, d->w64, nn, s.leaf_of); d->launches++; }
-    const csgd_force_params p = walk_params(a);
-    cudaMemsetAsync(a->counts, 0, sizeof(int) * n, st);
-    rc = csgd_walk_lists(d, &p, a->counts, nullptr, nullptr, 0, 0);
-    if (!rc)
-        rc = csg_scan_exclusive(d, a->counts, s.offs, n, nullptr);
-    int total = 0;
-    if (!rc) {
-        cudaMemcpyAsync(a->h_total, s.offs + n, sizeof(int), cudaMemcpyDeviceToHost, st);
-        rc = csgd_sync(d);
-        total = *a->h_total;
-    }
-    if (rc)
-        return rc;
     if (total < 0) { // more entries than an int offset holds
         csgd_set_err(d, CSG_ERR_NODE_CAPACITY);
         return CSG_ERR_NODE_CAPACITY;
@@ -507,8 +572,8 @@ int eval(csg_adjoint *a, Slot &s)
         return rc;
     const int wb = AT / CSG_WARP;
     { k_adj_gather<<<csgd_grid(n, AT), AT, 0, st>>>(s.perm, n, d->x, d->y, d->z, d->m, a->sb); d->launches++; }
-    { k_adj_moments<<<csgd_grid(nn, wb), AT, 0, st>>>(s.link, nn, a->sb, a->xm); d->launches++; }
-    { k_adj_forces<<<csgd_grid(n, wb), AT, 0, st>>>(s.offs, s.ids, a->xm, d->x, d->y, d->z, d->m, n, a->G, a->eps * a->eps, d->ax, d->ay, d->az); d->launches++; }
+    { k_adj_moments<<<csgd_grid(nn, MOM_CELLS), AT, 0, st>>>(s.link, nn, a->sb, a->xm); d->launches++; }
+    { k_adj_forces<<<csgd_grid(n, wb), AT, 0, st>>>(s.offs, a->segs, s.ids, a->xm, d->x, d->y, d->z, d->m, n, a->G, a->eps * a->eps, d->ax, d->ay, d->az); d->launches++; }
     return csgd_check(d, cudaGetLastError());
 }
 
@@ -524,8 +589,8 @@ int eval_frozen(csg_adjoint *a, const Slot &s)
     }
     const int wb = AT / CSG_WARP;
     { k_adj_gather<<<csgd_grid(n, AT), AT, 0, st>>>(s.perm, n, d->x, d->y, d->z, d->m, a->sb); d->launches++; }
-    { k_adj_moments<<<csgd_grid(s.nn, wb), AT, 0, st>>>(s.link, s.nn, a->sb, a->xm); d->launches++; }
-    { k_adj_forces<<<csgd_grid(n, wb), AT, 0, st>>>(s.offs, s.ids, a->xm, d->x, d->y, d->z, d->m, n, a->G, a->eps * a->eps, d->ax, d->ay, d->az); d->launches++; }
+    { k_adj_moments<<<csgd_grid(s.nn, MOM_CELLS), AT, 0, st>>>(s.link, s.nn, a->sb, a->xm); d->launches++; }
+    { k_adj_forces<<<csgd_grid(n, wb), AT, 0, st>>>(s.offs, a->segs, s.ids, a->xm, d->x, d->y, d->z, d->m, n, a->G, a->eps * a->eps, d->ax, d->ay, d->az); d->launches++; }
     return csgd_check(d, cudaGetLastError());
 }
 
@@ -544,9 +609,9 @@ int jt_product(csg_adjoint *a, const Slot &s)
     const int wb = AT / CSG_WARP;
     cudaMemsetAsync(a->g, 0, sizeof(double) * 3 * (size_t)s.nn, st);
     { k_adj_gather<<<csgd_grid(n, AT), AT, 0, st>>>(s.perm, n, s.x, s.y, s.z, d->m, a->sb); d->launches++; }
-    { k_adj_moments<<<csgd_grid(s.nn, wb), AT, 0, st>>>(s.link, s.nn, a->sb, a->xm); d->launches++; }
-    { k_adj_jt<<<csgd_grid(n, wb), AT, 0, st>>>(s.offs, s.ids, a->xm, s.x, s.y, s.z, d->m, mux, muy, muz, n, a->G, a->eps * a->eps, a->g, jx, jy, jz); d->launches++; }
-    { k_adj_push<<<csgd_grid(s.n_alive, AT), AT, 0, st>>>(s.perm, s.leaf_of, s.link, a->xm, a->g, d->m, s.n_alive, s.nn, jx, jy, jz, d->sc); d->launches++; }
+    { k_adj_moments<<<csgd_grid(s.nn, MOM_CELLS), AT, 0, st>>>(s.link, s.nn, a->sb, a->xm); d->launches++; }
+    { k_adj_jt<<<csgd_grid(n, wb), AT, 0, st>>>(s.offs, a->segs, s.ids, a->xm, s.x, s.y, s.z, d->m, mux, muy, muz, n, a->G, a->eps * a->eps, a->g, jx, jy, jz); d->launches++; }
+    { k_adj_push<<<csgd_grid(s.n_alive, AT), AT, 0, st>>>(s.perm, s.leaf_of, s.link, a->xm, a->g, d->m, a->G, s.n_alive, s.nn, jx, jy, jz, d->sc); d->launches++; }
     return csgd_check(d, cudaGetLastError());
 }
 
@@ -644,6 +709,7 @@ CSG_EXPORT csg_adjoint *csg_adjoint_create(int n, const CsgSimParams *params, in
     a->dt = params->dt;
     const size_t ncap = 8 * (size_t)n + 64;
     int rc = csgd_reserve(a->d, n);
+    a->segs = csgd_list_segments(a->d, n);
     cudaError_t e = cudaSuccess;
     if (!rc) {
         e = alloc(&a->lam, 6 * (size_t)n);
@@ -652,7 +718,7 @@ CSG_EXPORT csg_adjoint *csg_adjoint_create(int n, const CsgSimParams *params, in
         if (e == cudaSuccess) e = alloc(&a->g, 3 * ncap);
         if (e == cudaSuccess) e = alloc(&a->xm, ncap);
         if (e == cudaSuccess) e = alloc(&a->sb, (size_t)n);
-        if (e == cudaSuccess) e = alloc(&a->counts, (size_t)n);
+        if (e == cudaSuccess) e = alloc(&a->counts, (size_t)a->segs * n);
         if (e == cudaSuccess) e = csgd_malloc_host((void **)&a->h_total, sizeof(int));
         rc = cuda_rc(a, e);
     }
@@ -665,7 +731,7 @@ CSG_EXPORT csg_adjoint *csg_adjoint_create(int n, const CsgSimParams *params, in
                 a->ckpt.push_back(c);
         }
         a->bytes = sizeof(double) * (6 * (size_t)n * (nck + 1) + 6 * (size_t)n + 3 * ncap) +
-                   sizeof(double4_32a) * ncap + sizeof(int) * (size_t)n;
+                   sizeof(double4_32a) * ncap + sizeof(int) * (size_t)a->segs * n;
     }
     if (rc) {
         csg_adjoint_destroy(a);

@@ -430,7 +430,8 @@ __device__ __forceinline__ void pow23_from_f32(float y, double &y2, double &y3)
 //       exponent).
 // Relative error < 1.01 x 2^-53 (one rounding; the truncated high words and
 // series add < 2^-57).
-__device__ __forceinline__ double m_r3_from_seed(long long rb, long long mb, float y0)
+__device__ __forceinline__ double m_r3_from_seed(long long rb, long long mb, float y0,
+                                                 long long *e64 = nullptr) // e 2^64
 {
     const unsigned long long MANT = 0xfffffffffffffull, HID = 1ull << 52;
     const unsigned yb = __float_as_uint(y0);
@@ -443,6 +444,8 @@ __device__ __forceinline__ double m_r3_from_seed(long long rb, long long mb, flo
     const long long Dhi = (1LL << sh) - (long long)H - (L != 0ull);
     const unsigned long long Dlo = 0ull - L;
     const long long E64 = (long long)(((unsigned long long)Dhi << (64 - sh)) | (Dlo >> sh));
+    if (e64)
+        *e64 = E64;
     const unsigned long long aE = (unsigned long long)(E64 < 0 ? -E64 : E64);
     const long long C = (1LL << 62) + ((3 * E64) >> 3) + (long long)((15ull * __umul64hi(aE, aE)) >> 5);
     const unsigned long long hi3 = __umul64hi((unsigned long long)Y << 40, S << 16);
@@ -477,23 +480,46 @@ __device__ __forceinline__ double r3_series_w(double e)
     return ee < 960 ? 0.0 : __longlong_as_double(w);
 }
 
-// r^-3 and r^-5 for r2 = r^2 without divisions: y0 = FP32 rsqrt seed (rel.
-// error < 2^-21; y0^2 and y0^3 by pow23_from_f32), e = 1 - r2 y0^2 (one
-// fused multiply-add), then r^-2 = y0^2 (1 + e + e^2) and
-// r^-3 = y0^3 (1 + 3/2 e + 15/8 e^2) (the binomial series; the first omitted
-// terms are < 2^-60). Outside 2^-99 <= r2 < 2^100 the plain expressions.
-__device__ __forceinline__ void inv_r3_r5(double r2, double &inv3, double &inv5)
+// m/r^3 for the queued FP64 walk without FP64 operations (the FP64 pipe is
+// the walk's bottleneck on this GPU): from the FP32 rsqrt seed y0 (rel.
+// error < 2^-21) by integer arithmetic (m_r3_from_seed: the series of
+// (1-e)^-3/2, e = 1 - r2 y0^2, one rounding). The seed's conversion is a bit
+// operation. Range checks on the exponents (2^-99 <= r2 < 2^100,
+// 2^-863 <= m < 2^865) keep every integer step in range; outside them (and
+// for m = 0) the plain expression.
+__device__ __forceinline__ double m_inv_r3_q(double m, double r2)
 {
     const long long bits = __double_as_longlong(r2);
-    if ((unsigned long long)((bits >> 52) - 924) <= 198ull) {
-        double y0sq, y3;
-        pow23_from_f32(rsqrtf(f32_from_f64_bits(bits)), y0sq, y3);
-        const double e = fma(-r2, y0sq, 1.0);
-        inv3 = fma(y3, r3_series_w(e), y3);
-        const double inv2 = fma(y0sq, fma(e, e, e), y0sq);
-        inv5 = inv3 * inv2;
-        return;
+    const long long mb = __double_as_longlong(m);
+    if ((unsigned long long)((bits >> 52) - 924) <= 198ull && // sign clear, exponent 924..1122
+        (unsigned long long)((mb >> 52) - 160) < 1728ull)     // sign clear, exponent 160..1887
+        return m_r3_from_seed(bits, mb, rsqrtf(f32_from_f64_bits(bits)));
+    return m / (r2 * sqrt(r2));
+}
+
+// m r^-3 and r^-2 for r2 = r^2: by integers as m_inv_r3_q where its ranges
+// hold. r^-2 = y0^2 (1 + e + e^2), |e| < 2^-20 (the next term is below 2^-60):
+// S = Y^2 times the series in 62-bit fixed point, the high 64 bits rounded to
+// 53 and packed.
+__device__ __forceinline__ double m_inv_r3_r2(double m, double r2, double &inv2)
+{
+    const long long rb = __double_as_longlong(r2), mb = __double_as_longlong(m);
+    if ((unsigned long long)((rb >> 52) - 924) <= 198ull &&
+        (unsigned long long)((mb >> 52) - 160) <= 1727ull) {
+        const float y0 = rsqrtf(f32_from_f64_bits(rb));
+        long long E64;
+        const double f = m_r3_from_seed(rb, mb, y0, &E64);
+        const unsigned yb = __float_as_uint(y0);
+        const unsigned Y = (yb & 0x7fffffu) | 0x800000u;
+        const unsigned long long aE = (unsigned long long)(E64 < 0 ? -E64 : E64);
+        const unsigned long long C = (unsigned long long)((1LL << 62) + (E64 >> 2)) + (__umul64hi(aE, aE) >> 2);
+        const unsigned long long Q = __umul64hi(((unsigned long long)Y * Y) << 16, C << 1);
+        const int lz = __clz((unsigned)(Q >> 32)); // 0..2
+        const int s = 11 - lz;
+        const unsigned long long M = (Q + (1ull << (s - 1))) >> s;
+        inv2 = __longlong_as_double(((2 * (long long)(yb >> 23) + 770 - lz) << 52) + (long long)M);
+        return f;
     }
-    inv3 = 1.0 / (r2 * sqrt(r2));
-    inv5 = inv3 / r2;
+    inv2 = 1.0 / r2;
+    return m / (r2 * sqrt(r2));
 }
