@@ -350,6 +350,10 @@ inline void csgd_launch(csgd_t *d, void (*k)(P...), int grid, int block, cudaStr
 // the launches are sized for n).
 int csg_radix_sort(csgd_t *d, unsigned long long *key, int *val, unsigned long long *key_alt,
                    int *val_alt, int n, int bits, const int *n_dev = nullptr);
+// The same order out of place by counting, faster up to RANK_MAX keys.
+constexpr int RANK_MAX = 12288;
+int csg_rank_sort(csgd_t *d, const unsigned long long *key, const int *val,
+                  unsigned long long *key_out, int *val_out, int n);
 // Exclusive scan of in[0..n) into out[0..n], out[n] = total. count_limit, when
 // non-NULL, is a device int: items at positions >= *count_limit count as 0.
 int csg_scan_exclusive(csgd_t *d, const int *in, int *out, int n, const int *count_limit);

@@ -1346,10 +1346,12 @@ static int order_bodies(csgd_t *d)
     int gb = min(csgd_grid(n, B), 4 * d->num_sms);
     csgd_launch(d, k_bbox, gb > 0 ? gb : 1, B, s, d->x, d->y, d->z, d->m, d->gid, n, d->roots, sc);
     csgd_launch(d, k_root, 1, 256, s, sc, d->roots, G);
+    const bool rank = n <= RANK_MAX;
     if (n > 0)
-        csgd_launch(d, k_keys, csgd_grid(n, B), B, s, d->x, d->y, d->z, d->m, d->gid, n, sc, d->roots, d->key, d->perm);
+        csgd_launch(d, k_keys, csgd_grid(n, B), B, s, d->x, d->y, d->z, d->m, d->gid, n, sc, d->roots, rank ? d->key_alt : d->key, rank ? d->perm_alt : d->perm);
     csgd_build_mark(d, 1);
-    int rc = csg_radix_sort(d, d->key, d->perm, d->key_alt, d->perm_alt, n, 64);
+    int rc = rank ? csg_rank_sort(d, d->key_alt, d->perm_alt, d->key, d->perm, n)
+                  : csg_radix_sort(d, d->key, d->perm, d->key_alt, d->perm_alt, n, 64);
     if (rc)
         return rc;
     if (G > 1 && n > 1) {
