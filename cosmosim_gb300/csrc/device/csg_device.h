@@ -39,8 +39,8 @@ void *csgd_stream(csgd_t *d);
 /* The device Body staging array (capacity >= the reserved body count). */
 Body *csgd_aos(csgd_t *d);
 
-/* Tree builds also record what a reference-order pool export needs (on for
-   states that export after most builds; export works either way). */
+/* Pool exports take the tree last built as it is (on for states that export
+   after most builds; else an export rebuilds it). */
 void csgd_set_export_order(csgd_t *d, int on);
 
 /* Makes room for n bodies (grow-only). */

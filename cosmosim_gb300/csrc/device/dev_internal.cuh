@@ -91,6 +91,8 @@ struct DevRoot {
     long long key_tol;                   // fast-path guard, in units of 2^-32 grid cells
     int fast_keys;                       // 1 when the fast key path is safe
     int n_alive;                         // alive bodies of this system
+    int mass_e;                          // largest biased exponent of their masses
+    int sum_e;                           // the total mass is below 2^sum_e
     int first;                           // their first sorted position
     int root;                            // preorder id of the root cell
     int end;                             // one past the system's last cell
@@ -114,7 +116,9 @@ struct DevScalars {
     int deep;                            // positions that share a 63-bit key
     int err;                             // first device error code (0 = none)
     int n_gas;
-    int pad0;
+    int mom_tiles;     // tiles that are summed (k_mom_sums)
+    int mom_light;     // a body is too light for the fixed-point cell sums
+    int mom_climb;     // the build's cell sums do not fit 128-bit fixed point
     unsigned long long interactions;     // walk statistics (when enabled)
     unsigned long long walk_steps;       // warp traversal steps
     unsigned long long walk_active;      // lane-steps of lanes still walking
@@ -222,8 +226,8 @@ struct csgd {
     // and, for the persistent form, blocks per SM
     int walk_warps, walk_group, walk_bps;
     int num_sms;
-    int export_order; // builds also keep what pool export needs (two lowest indices per cell)
-    int minidx_valid; // the current tree has them
+    int export_order; // built trees are kept for pool exports
+    int minidx_valid; // the current tree was built so (an export takes it as it is)
 
     // keys and sort
     unsigned long long *key, *key_alt;
@@ -257,7 +261,9 @@ struct csgd {
     int *child;   // 8 per node
     int *nchild;
     int *ticket;
-    int2 *minidx; // two smallest caller indices below each cell (export order)
+    ulonglong2 *mom_sum;  // 128-bit sums before a position in its tile (m x, m y, m z, m)
+    ulonglong2 *mom_tile; // the same before a tile
+    int2 *minidx; // two smallest caller indices below each cell (formed by an export)
     unsigned long long *ord_key, *ord_key_alt;
     int *ord_id, *ord_id_alt, *rank;
 

@@ -214,7 +214,7 @@ void free_bodies(csgd_t *d)
                     d->rho, d->P, d->u, d->h, d->type, d->aos, d->key, d->key_alt, d->perm,
                     d->perm_alt, d->ext, d->sort_hist, d->lcp, d->cnt, d->base, d->scan_tmp,
                     d->gas, d->w64, d->w32, d->link, d->geo, d->s32, d->child, d->nchild, d->ticket,
-                    d->minidx, d->ord_key, d->ord_key_alt, d->ord_id, d->ord_id_alt, d->rank,
+                    d->mom_sum, d->mom_tile, d->minidx, d->ord_key, d->ord_key_alt, d->ord_id, d->ord_id_alt, d->rank,
                     d->pool, d->gid, d->sgid, d->tasks};
     for (void *p : ptrs)
         if (p)
@@ -236,6 +236,7 @@ void free_bodies(csgd_t *d)
     d->s32 = nullptr;
     d->child = d->nchild = d->ticket = nullptr;
     d->minidx = nullptr;
+    d->mom_sum = d->mom_tile = nullptr;
     d->ord_key = d->ord_key_alt = nullptr;
     d->ord_id = d->ord_id_alt = d->rank = nullptr;
     d->pool = nullptr;
@@ -528,6 +529,8 @@ extern "C" int csgd_reserve(csgd_t *d, int n)
     ok &= dalloc(&d->nchild, ncap) == cudaSuccess;
     ok &= dalloc(&d->ticket, ncap) == cudaSuccess;
     ok &= dalloc(&d->minidx, ncap) == cudaSuccess;
+    ok &= dalloc(&d->mom_sum, 4 * (cap + 1)) == cudaSuccess;
+    ok &= dalloc(&d->mom_tile, 4 * (cap / 256 + 2)) == cudaSuccess;
     ok &= dalloc(&d->ord_key, ncap) == cudaSuccess;
     ok &= dalloc(&d->ord_key_alt, ncap) == cudaSuccess;
     ok &= dalloc(&d->ord_id, ncap) == cudaSuccess;

@@ -48,6 +48,9 @@ __device__ __forceinline__ double ord_dec(unsigned long long e)
 
 __device__ __forceinline__ bool is_alive(double m) { return !(m <= 0.0); }
 
+// biased exponent (masses are positive here)
+__device__ __forceinline__ int mass_exponent(double m) { return __double2hiint(m) >> 20 & 0x7ff; }
+
 // Spreads the low 21 bits of v to every third bit (bit k -> bit 3k).
 __device__ __forceinline__ unsigned long long spread3(unsigned long long v)
 {
@@ -135,9 +138,12 @@ __global__ void k_reset(DevScalars *sc, DevRoot *roots, int n_gal)
             roots[g].omax[a] = 0ull;
         }
         roots[g].n_alive = 0;
+        roots[g].mass_e = 0;
     }
     if (threadIdx.x == 0) {
         sc->n_alive = 0;
+        sc->mom_tiles = 0;
+        sc->mom_light = 0;
         sc->deep = 0;
         sc->n_gas = 0;
         sc->key_slow = 0;
@@ -171,8 +177,9 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
 // system costs one flush per warp, not one per 32 bodies. Lanes of a warp
 // that straddles a system boundary fall back to per-lane atomics.
 __device__ __forceinline__ void bbox_flush(DevRoot *roots, int g, unsigned long long lo[3],
-                                           unsigned long long hi[3], int &cnt)
+                                           unsigned long long hi[3], int &cnt, int &me)
 {
+    me = __reduce_max_sync(0xffffffffu, me);
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         lo[a] = warp_min_u64(lo[a]);
@@ -187,14 +194,16 @@ __device__ __forceinline__ void bbox_flush(DevRoot *roots, int g, unsigned long 
             if (hi[a] != 0ull)
                 atomicMax(&roots[g].omax[a], hi[a]);
         }
-        if (cnt)
+        if (cnt) {
             atomicAdd(&roots[g].n_alive, cnt);
+            atomicMax(&roots[g].mass_e, me);
+        }
     }
     for (int a = 0; a < 3; a++) {
         lo[a] = ~0ull;
         hi[a] = 0ull;
     }
-    cnt = 0;
+    cnt = me = 0;
 }
 
 __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ y,
@@ -203,7 +212,7 @@ __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ 
 {
     pdl_enter();
     unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0ull, 0ull, 0ull};
-    int cnt = 0;
+    int cnt = 0, me = 0;
     int cur_g = -1; // warp-uniform: the system the running box belongs to
     bool bad = false; // a non-finite mass, or a non-finite position of a live body
     for (long long base = (long long)blockIdx.x * blockDim.x; base < n;
@@ -226,16 +235,18 @@ __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ 
                     atomicMax(&roots[g].omax[a], ord_enc(p[a]));
                 }
                 atomicAdd(&roots[g].n_alive, 1);
+                atomicMax(&roots[g].mass_e, mass_exponent(m[i]));
             }
             continue;
         }
         if (g0 != cur_g) {
             if (cur_g >= 0)
-                bbox_flush(roots, cur_g, lo, hi, cnt);
+                bbox_flush(roots, cur_g, lo, hi, cnt, me);
             cur_g = g0;
         }
         if (g >= 0 && is_alive(m[i])) {
             cnt++;
+            me = max(me, mass_exponent(m[i]));
             const double p[3] = {x[i], y[i], z[i]};
 #pragma unroll
             for (int a = 0; a < 3; a++) {
@@ -250,7 +261,7 @@ __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ 
     // the warps' last running boxes: combined in the block first, one set of
     // atomics per system the block ends on (one per block for a single system)
     __shared__ unsigned long long s_lo[32][3], s_hi[32][3];
-    __shared__ int s_cnt[32], s_g[32];
+    __shared__ int s_cnt[32], s_g[32], s_me[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -259,7 +270,9 @@ __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ 
     }
     for (int o = 16; o > 0; o >>= 1)
         cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    me = __reduce_max_sync(0xffffffffu, me);
     if (lane == 0) {
+        s_me[warp] = me;
         s_g[warp] = cur_g;
         s_cnt[warp] = cnt;
         for (int a = 0; a < 3; a++) {
@@ -269,7 +282,7 @@ __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ 
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        int g = -1, c = 0;
+        int g = -1, c = 0, e = 0;
         unsigned long long l[3] = {~0ull, ~0ull, ~0ull}, h[3] = {0ull, 0ull, 0ull};
         const int nw = (int)(blockDim.x >> 5);
         for (int w = 0; w <= nw; w++) {
@@ -282,13 +295,15 @@ __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ 
                         if (h[a] != 0ull)
                             atomicMax(&roots[g].omax[a], h[a]);
                     }
-                    if (c)
+                    if (c) {
                         atomicAdd(&roots[g].n_alive, c);
+                        atomicMax(&roots[g].mass_e, e);
+                    }
                 }
                 if (w == nw)
                     break;
                 g = gw;
-                c = 0;
+                c = e = 0;
                 for (int a = 0; a < 3; a++) {
                     l[a] = ~0ull;
                     h[a] = 0ull;
@@ -297,6 +312,7 @@ __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ 
             if (gw < 0)
                 continue;
             c += s_cnt[w];
+            e = max(e, s_me[w]);
             for (int a = 0; a < 3; a++) {
                 l[a] = s_lo[w][a] < l[a] ? s_lo[w][a] : l[a];
                 h[a] = s_hi[w][a] > h[a] ? s_hi[w][a] : h[a];
@@ -362,6 +378,10 @@ __global__ void k_root(DevScalars *sc, DevRoot *roots, int n_gal)
     // not yet collected) the tree is built empty: no key is formed from the
     // bodies and nothing downstream walks them.
     const bool failed = sc->err != 0;
+    __shared__ int climb;
+    if (threadIdx.x == 0)
+        climb = 0;
+    __syncthreads();
     for (int g = threadIdx.x; g < n_gal; g += blockDim.x) {
         if (failed)
             roots[g].n_alive = 0;
@@ -370,9 +390,13 @@ __global__ void k_root(DevScalars *sc, DevRoot *roots, int n_gal)
         const double far = fmax(fabs(r.c0[0]), fmax(fabs(r.c0[1]), fabs(r.c0[2]))) + r.hs0;
         roots[g].fix_e = ilogb(far) + 1;
         roots[g].fix_off = 0;
+        roots[g].sum_e = r.mass_e - 1022 + 32 - __clz(max(r.n_alive, 1));
+        if (r.n_alive > 0 && (abs(roots[g].sum_e) > 300 || abs(roots[g].fix_e) > 300))
+            climb = 1;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+        sc->mom_climb = climb;
         int off = 0;
         for (int g = 0; g < n_gal; g++) {
             roots[g].first = off;
@@ -653,7 +677,6 @@ __global__ void k_nodes(csgd_t dd, DevScalars *sc, const DevRoot *__restrict__ r
             float4 *v = (float4 *)&dd.w32[0];
             v[0] = make_float4(0.f, 0.f, 0.f, 0.f);
             v[1] = make_float4(0.f, 0.f, 0.f, dd.w32[0].s2);
-            dd.minidx[0] = make_int2(INT_MAX, INT_MAX);
             return;
         }
     }
@@ -697,6 +720,490 @@ __global__ void k_nodes(csgd_t dd, DevScalars *sc, const DevRoot *__restrict__ r
     }
 }
 
+
+// Kernels over cells loop over ids (grid-stride): the cell count is known on
+// the device only, and a grid of about 2n threads covers it in one round for
+// the usual trees (cells ~1.3-2 per body) without launching for the capacity.
+__global__ void k_link(csgd_t dd, DevScalars *sc, const unsigned long long *__restrict__ key,
+                       const unsigned long long *__restrict__ ext)
+{
+    pdl_enter();
+    const int nn = sc->n_nodes;
+    if (nn > dd.node_cap)
+        return;
+    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < nn; id += gridDim.x * blockDim.x) {
+        NodeLink l = dd.link[id];
+        if (l.parent < 0 || l.parent >= dd.node_cap)
+            continue;
+        int dg = digit_at(key, ext, l.first, l.level - 1);
+        dd.child[8 * (size_t)l.parent + dg] = id;
+        atomicAdd(&dd.nchild[l.parent], 1);
+    }
+}
+
+// Moments. Only the centre of mass and mass fields of a cell are written here
+// (write_cell set the rest): from prefix sums over the sorted bodies (k_mom_sums,
+// k_moments), or, for masses that do not fit those, by climbing the tree.
+//
+// The climb: one thread per cell of at most MOM_DIRECT bodies (and per leaf);
+// above those, the last child to finish computes its parent, summing the
+// children in octant order so the result does not depend on scheduling. It
+// carries and stores raw sums (sum of m x, sum of m) in the FP64 record, so no
+// division sits on its chain of dependent levels; k_tasks then turns every
+// cell's sums into its centre of mass and writes the FP32 record.
+__device__ __forceinline__ void put_raw(const csgd_t &dd, int node, double ax, double ay,
+                                        double az, double M)
+{
+    double2 *w = (double2 *)&dd.w64[node];
+    w[0] = make_double2(ax, ay);
+    w[1] = make_double2(az, M);
+}
+
+// v as a float and the float of the rest, by integers (the conversions run on
+// the FP64 pipe): the same values as (float)v and (float)(v - (double)hi).
+__device__ __forceinline__ void split_float(double v, float &hi, float &lo)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const int e = (int)(b >> 52) & 0x7ff;
+    if ((unsigned)(e - 949) < 201u) { // both parts normal floats
+        const unsigned long long M = (b & 0xfffffffffffffull) | (1ull << 52);
+        const unsigned low = (unsigned)M & 0x1fffffffu;
+        unsigned H = (unsigned)(M >> 29);
+        H += low > 0x10000000u || (low == 0x10000000u && (H & 1u));
+        const int rest = (int)(M - ((unsigned long long)H << 29)); // |rest| <= 2^28
+        const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
+        hi = __uint_as_float(sign | ((((unsigned)(e - 897)) << 23) + H));
+        const float r = (float)rest * __uint_as_float((unsigned)(e - 948) << 23);
+        lo = __uint_as_float(__float_as_uint(r) ^ sign);
+        return;
+    }
+    hi = (float)v;
+    lo = (float)(v - (double)hi);
+}
+
+__device__ __forceinline__ void put_moments(const csgd_t &dd, int node, double sx, double sy,
+                                            double sz, double M)
+{
+    double2 *w = (double2 *)&dd.w64[node];
+    w[0] = make_double2(sx, sy);
+    w[1] = make_double2(sz, M);
+    float4 hi;
+    float lx, ly, lz, lm;
+    split_float(sx, hi.x, lx);
+    split_float(sy, hi.y, ly);
+    split_float(sz, hi.z, lz);
+    split_float(M, hi.w, lm);
+    float *v = (float *)&dd.w32[node];
+    *(float4 *)v = hi;
+    v[4] = lx;
+    v[5] = ly;
+    v[6] = lz;
+}
+
+// The climb's cells. A cell with at most MOM_DIRECT bodies, and every leaf, sums
+// its sorted bodies directly (one thread per cell, no atomics); a larger cell
+// is formed from its children's moments by the last child to finish (a ticket
+// per cell), climbing from the directly summed cells whose parent is large.
+// A single-body leaf keeps the body's position exactly (the reference's leaf
+// centre); bodies that coincide to depth 64 share one leaf, in caller index
+// order, so the two smallest caller indices of a cell are its first two.
+constexpr int MOM_DIRECT = 16;
+
+// The ticket of a cell: one gpu-scope acquire-release add. Release: this
+// thread's sums (stored above) are visible to whichever child takes the last
+// ticket; acquire: the last child sees every sibling's sums (the adds on one
+// ticket form a release sequence).
+__device__ __forceinline__ int ticket_take(int *p)
+{
+    int old;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
+    return old;
+}
+
+__device__ __forceinline__ void moments_climb(const csgd_t &dd, int node, int parent, double ax,
+                                              double ay, double az, double M)
+{
+    while (true) {
+        put_raw(dd, node, ax, ay, az, M);
+        if (parent < 0 || parent >= node)
+            break; // preorder: a parent always precedes its children
+        // the parent's children, their count and its own parent are fixed
+        // since k_link: their loads run while the sums above drain
+        const int4 *cp = (const int4 *)(dd.child + 8 * (size_t)parent);
+        const int4 c03 = __ldg(cp), c47 = __ldg(cp + 1);
+        const int nc = __ldg(&dd.nchild[parent]);
+        const int up = __ldg(&dd.link[parent].parent);
+        if (ticket_take(&dd.ticket[parent]) != nc - 1)
+            break;
+        dd.ticket[parent] = 0; // for the next climb on this tree
+        M = 0.0;
+        ax = ay = az = 0.0;
+        const int ch[8] = {c03.x, c03.y, c03.z, c03.w, c47.x, c47.y, c47.z, c47.w};
+        for (int q = 0; q < 8; q++) {
+            const int c = ch[q];
+            if (c < 0)
+                continue;
+            const double2 *cw = (const double2 *)&dd.w64[c];
+            const double2 xy = __ldcg(cw), zm = __ldcg(cw + 1);
+            M += zm.y;
+            ax += xy.x;
+            ay += xy.y;
+            az += zm.x;
+        }
+        node = parent;
+        parent = up;
+    }
+}
+
+// Bodies summed directly, four bodies' loads in flight at a time; the additions
+// keep the sorted order (M += m, then sum += m x as one fused multiply-add).
+constexpr int MOM_LOADS = 4;
+
+__device__ __forceinline__ void moments_cell(const csgd_t &dd, int id, const double *__restrict__ x,
+                                             const double *__restrict__ y,
+                                             const double *__restrict__ z,
+                                             const double *__restrict__ m,
+                                             const int *__restrict__ perm)
+{
+    const NodeLink l = dd.link[id];
+    const bool leaf = dd.nchild[id] == 0;
+    if ((!leaf && l.count > MOM_DIRECT) || l.count < 1)
+        return; // formed by the climb (or a cell without bodies)
+    // a parent of at most MOM_DIRECT bodies sums its own bodies
+    const int pcount = (l.parent >= 0) ? __ldg(&dd.link[l.parent].count) : INT_MAX;
+    double M = 0.0, ax = 0.0, ay = 0.0, az = 0.0;
+    for (int k0 = 0; k0 < l.count; k0 += MOM_LOADS) {
+        int bb[MOM_LOADS];
+        double mv[MOM_LOADS], xv[MOM_LOADS], yv[MOM_LOADS], zv[MOM_LOADS];
+#pragma unroll
+        for (int j = 0; j < MOM_LOADS; j++)
+            bb[j] = (k0 + j < l.count) ? perm[l.first + k0 + j] : -1;
+#pragma unroll
+        for (int j = 0; j < MOM_LOADS; j++) {
+            if (bb[j] >= 0) {
+                mv[j] = m[bb[j]];
+                xv[j] = x[bb[j]];
+                yv[j] = y[bb[j]];
+                zv[j] = z[bb[j]];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < MOM_LOADS; j++) {
+            if (bb[j] < 0)
+                break;
+            const double mb = mv[j];
+            M += mb;
+            ax += mb * xv[j];
+            ay += mb * yv[j];
+            az += mb * zv[j];
+        }
+    }
+    if (pcount <= MOM_DIRECT) {
+        put_raw(dd, id, ax, ay, az, M); // the parent sums its own bodies
+        return;
+    }
+    moments_climb(dd, id, l.parent, ax, ay, az, M);
+}
+
+// Raw sums to centre of mass: a single-body leaf keeps the body's position
+// exactly (the reference's leaf centre), any other cell takes
+// (sum m x) / (sum m).
+__device__ __forceinline__ void moments_norm(const csgd_t &dd, int id, const double *__restrict__ x,
+                                             const double *__restrict__ y,
+                                             const double *__restrict__ z)
+{
+    const NodeLink l = dd.link[id];
+    if (l.count < 1)
+        return;
+    const double2 *w = (const double2 *)&dd.w64[id];
+    const double2 xy = w[0], zm = w[1];
+    const int body = dd.w64[id].body;
+    if (l.count == 1 && body >= 0) {
+        put_moments(dd, id, x[body], y[body], z[body], zm.y);
+    } else {
+        const Divisor M = divisor(zm.y);
+        put_moments(dd, id, div_rn(xy.x, M), div_rn(xy.y, M), div_rn(zm.x, M), zm.y);
+    }
+}
+
+typedef unsigned __int128 u128;
+
+__device__ __forceinline__ ulonglong2 words(u128 v)
+{
+    return make_ulonglong2((unsigned long long)v, (unsigned long long)(v >> 64));
+}
+__device__ __forceinline__ u128 join(ulonglong2 w) { return (u128)w.y << 64 | w.x; }
+
+__device__ __forceinline__ u128 shfl_up128(u128 v, int o)
+{
+    const unsigned long long lo = __shfl_up_sync(0xffffffffu, (unsigned long long)v, o);
+    const unsigned long long hi = __shfl_up_sync(0xffffffffu, (unsigned long long)(v >> 64), o);
+    return (u128)hi << 64 | lo;
+}
+
+// p 2^sh, towards zero
+__device__ __forceinline__ u128 shift128(u128 p, int sh)
+{
+    return sh >= 0 ? p << min(sh, 127) : sh > -128 ? p >> -sh : (u128)0;
+}
+
+// The value of a sum (two's complement, in units of 2^u) as a double, to nearest
+// even; within the exponents that k_root allows every result is normal or zero.
+__device__ __forceinline__ double value128(u128 s, int u)
+{
+    const bool neg = (long long)(s >> 64) < 0;
+    if (neg)
+        s = (u128)0 - s;
+    const unsigned long long hi = (unsigned long long)(s >> 64), lo = (unsigned long long)s;
+    if ((hi | lo) == 0ull)
+        return 0.0;
+    const int lz = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
+    s <<= lz;
+    const unsigned long long top = (unsigned long long)(s >> 64);
+    const unsigned low = (unsigned)top & 0x7ffu;
+    unsigned long long M = top >> 11;
+    M += low > 0x400u || (low == 0x400u && ((unsigned long long)s != 0ull || (M & 1ull)));
+    const long long e = 75 - lz + u + 1074;
+    return __longlong_as_double((long long)((neg ? SIGN64 : 0ull) | (((unsigned long long)e << 52) + M)));
+}
+
+// Sums over cells as differences of prefix sums over the sorted bodies. In
+// 128-bit fixed point they are exact: a system's masses are whole units of
+// 2^(sum_e - 126), its m x are cut to units of 2^(sum_e + fix_e - 126), and no
+// sum overflows; sums over different systems (other units) wrap and are never
+// used. A body below 2^-50 of the bound of its system's mass could lose bits:
+// then (mom_climb) the cells are summed in FP64 as above.
+//
+// Every cell so costs two loads of four sums and no FP64 operation, whatever
+// its size. The climb was bound by its chain of dependent levels for few bodies
+// and by the FP64 pipe for many: with the division pass after it 33 us for 2,000
+// bodies, 70 for 100,000, 294 for 1,000,000; now 15, 27 and 180 (the sums'
+// instructions and their 64 bytes a body).
+constexpr int MOM_TILE = 256;
+
+struct MomSums {
+    u128 s[4]; // m x, m y, m z, m
+};
+
+__device__ __forceinline__ void put_sums(ulonglong2 *o, const u128 s[4])
+{
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        o[k] = words(s[k]);
+}
+
+// Exclusive prefix sums over the block's threads.
+__device__ __forceinline__ void block_prefix(MomSums &v)
+{
+    constexpr int W = MOM_TILE / CSG_WARP;
+    __shared__ ulonglong2 part[W][4];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    MomSums in = v;
+#pragma unroll
+    for (int o = 1; o < CSG_WARP; o <<= 1)
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const u128 t = shfl_up128(in.s[k], o);
+            if (lane >= o)
+                in.s[k] += t;
+        }
+    if (lane == 31)
+        put_sums(part[wid], in.s);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        v.s[k] = in.s[k] - v.s[k];
+    for (int w = 0; w < wid; w++)
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            v.s[k] += join(part[w][k]);
+    __syncthreads(); // part may be written again
+}
+
+__global__ void __launch_bounds__(MOM_TILE) k_mom_sums(csgd_t dd, DevScalars *sc,
+                                                       const DevRoot *__restrict__ roots,
+                                                       const double *__restrict__ x,
+                                                       const double *__restrict__ y,
+                                                       const double *__restrict__ z,
+                                                       const double *__restrict__ m,
+                                                       const int *__restrict__ perm,
+                                                       const int *__restrict__ sgid, int n_gal)
+{
+    pdl_enter();
+    __shared__ bool last;
+    if (sc->mom_climb) // since k_root
+        return;
+    const int na = sc->n_alive, p = blockIdx.x * MOM_TILE + threadIdx.x;
+    const int tiles = na / MOM_TILE + 1; // position na too
+    if ((int)blockIdx.x >= tiles)
+        return;
+    MomSums v, own;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        v.s[k] = 0;
+    if (p < na) {
+        const int b = perm[p];
+        const DevRoot &r = roots[n_gal > 1 ? sgid[p] : 0];
+        const long long mb = __double_as_longlong(m[b]);
+        const int em = (int)(mb >> 52); // biased
+        const int um = r.sum_e - 126;
+        if (em - 1022 < r.sum_e - 50 || em < 1)
+            sc->mom_light = 1; // every writer writes the same
+        const unsigned long long Sm = ((unsigned long long)mb & 0xfffffffffffffull) | (1ull << 52);
+        v.s[3] = shift128(Sm, em - 1075 - um);
+        const double c[3] = {x[b], y[b], z[b]};
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const unsigned long long cb = (unsigned long long)__double_as_longlong(c[k]);
+            const int ec = (int)(cb >> 52) & 0x7ff;
+            const unsigned long long Sc =
+                (cb & 0xfffffffffffffull) | (ec ? 1ull << 52 : 0ull);
+            const u128 P = shift128((u128)Sm * Sc, em + max(ec, 1) - 2150 - um - r.fix_e);
+            v.s[k] = cb >> 63 ? (u128)0 - P : P;
+        }
+    }
+    own = v;
+    block_prefix(v);
+    if (p <= na)
+        put_sums(dd.mom_sum + 4 * (size_t)p, v.s);
+    if (threadIdx.x == MOM_TILE - 1) {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            own.s[k] += v.s[k];
+        put_sums(dd.mom_tile + 4 * (size_t)blockIdx.x, own.s);
+        last = ticket_take(&sc->mom_tiles) == tiles - 1;
+    }
+    __syncthreads();
+    if (!last)
+        return;
+    // the last tile: prefix sums over the tiles, each thread a run of them
+    __threadfence();
+    const int per = (tiles + MOM_TILE - 1) / MOM_TILE;
+    const int t0 = min(tiles, (int)threadIdx.x * per), t1 = min(tiles, t0 + per);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        v.s[k] = 0;
+    for (int t = t0; t < t1; t++)
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            v.s[k] += join(__ldcg(dd.mom_tile + 4 * (size_t)t + k));
+    block_prefix(v);
+    for (int t = t0; t < t1; t++) {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            own.s[k] = join(__ldcg(dd.mom_tile + 4 * (size_t)t + k));
+        put_sums(dd.mom_tile + 4 * (size_t)t, v.s);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            v.s[k] += own.s[k];
+    }
+}
+
+__global__ void __launch_bounds__(256) k_moments(csgd_t dd, DevScalars *sc,
+                                                 const DevRoot *__restrict__ roots,
+                                                 const double *__restrict__ x,
+                                                 const double *__restrict__ y,
+                                                 const double *__restrict__ z,
+                                                 const double *__restrict__ m,
+                                                 const int *__restrict__ perm,
+                                                 const int *__restrict__ sgid, int n_gal)
+{
+    pdl_enter();
+    const int nn = sc->n_nodes;
+    if (nn > dd.node_cap || sc->n_alive == 0)
+        return;
+    const bool climb = (sc->mom_climb | sc->mom_light) != 0;
+    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < nn; id += gridDim.x * blockDim.x) {
+        if (climb) { // k_tasks divides
+            moments_cell(dd, id, x, y, z, m, perm);
+            continue;
+        }
+        const NodeLink l = dd.link[id];
+        if (l.count < 1)
+            continue;
+        const int body = dd.w64[id].body;
+        double cx, cy, cz, M;
+        if (l.count == 1 && body >= 0) { // the body's position exactly
+            cx = x[body];
+            cy = y[body];
+            cz = z[body];
+            M = m[body];
+        } else {
+            const DevRoot &r = roots[n_gal > 1 ? sgid[l.first] : 0];
+            const int um = r.sum_e - 126, from = l.first, to = l.first + l.count;
+            double v[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const u128 s = join(dd.mom_sum[4 * (size_t)to + k]) +
+                               join(dd.mom_tile[4 * (size_t)(to / MOM_TILE) + k]) -
+                               join(dd.mom_sum[4 * (size_t)from + k]) -
+                               join(dd.mom_tile[4 * (size_t)(from / MOM_TILE) + k]);
+                v[k] = value128(s, k < 3 ? um + r.fix_e : um);
+            }
+            M = v[3];
+            const Divisor by_M = divisor(M);
+            cx = div_rn(v[0], by_M);
+            cy = div_rn(v[1], by_M);
+            cz = div_rn(v[2], by_M);
+        }
+        put_moments(dd, id, cx, cy, cz, M);
+    }
+}
+
+// The two smallest caller indices below every cell (the pool export's order): a
+// cell of at most MOM_DIRECT bodies, and every leaf, from its bodies, a larger
+// one from its children's by the last child to finish.
+__global__ void __launch_bounds__(256) k_minidx(csgd_t dd, DevScalars *sc,
+                                                const int *__restrict__ perm)
+{
+    const int nn = sc->n_nodes;
+    if (nn > dd.node_cap)
+        return;
+    if (sc->n_alive == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            dd.minidx[0] = make_int2(INT_MAX, INT_MAX);
+        return;
+    }
+    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < nn; id += gridDim.x * blockDim.x) {
+        const NodeLink l = dd.link[id];
+        if ((dd.nchild[id] != 0 && l.count > MOM_DIRECT) || l.count < 1)
+            continue;
+        const int pcount = (l.parent >= 0) ? __ldg(&dd.link[l.parent].count) : INT_MAX;
+        int2 mi = make_int2(INT_MAX, INT_MAX);
+        auto take = [&](int v) {
+            if (v < mi.x) {
+                mi.y = mi.x;
+                mi.x = v;
+            } else if (v < mi.y) {
+                mi.y = v;
+            }
+        };
+        for (int k = 0; k < l.count; k++)
+            take(perm[l.first + k]);
+        dd.minidx[id] = mi;
+        int node = id, parent = pcount <= MOM_DIRECT ? -1 : l.parent;
+        while (parent >= 0 && parent < node) { // preorder: a parent precedes its children
+            const int4 *cp = (const int4 *)(dd.child + 8 * (size_t)parent);
+            const int4 c03 = __ldg(cp), c47 = __ldg(cp + 1);
+            const int up = __ldg(&dd.link[parent].parent);
+            if (ticket_take(&dd.ticket[parent]) != __ldg(&dd.nchild[parent]) - 1)
+                break;
+            dd.ticket[parent] = 0; // for the next climb on this tree
+            mi = make_int2(INT_MAX, INT_MAX);
+            const int ch[8] = {c03.x, c03.y, c03.z, c03.w, c47.x, c47.y, c47.z, c47.w};
+            for (int q = 0; q < 8; q++)
+                if (ch[q] >= 0) {
+                    const int2 c = __ldcg(&dd.minidx[ch[q]]);
+                    take(c.x);
+                    take(c.y);
+                }
+            dd.minidx[parent] = mi;
+            node = parent;
+            parent = up;
+        }
+    }
+}
+
 // Root and end cell of every system, and the walk tasks: each system's
 // sorted bodies in groups of 32 (one warp each). For a tree imported from a
 // caller pool (one system) the root is cell 0 and the end the cell count.
@@ -709,9 +1216,14 @@ __global__ void k_nodes(csgd_t dd, DevScalars *sc, const DevRoot *__restrict__ r
 __global__ void k_tasks(DevScalars *sc, DevRoot *roots, int n_gal, const int *__restrict__ base,
                         WalkTask *tasks, int task_cap, int imported,
                         const NodeLink *__restrict__ link, const int *__restrict__ child,
-                        int node_cap)
+                        int node_cap, csgd_t dd, const double *__restrict__ x,
+                        const double *__restrict__ y, const double *__restrict__ z)
 {
     pdl_enter();
+    if (!imported && (sc->mom_climb | sc->mom_light) && sc->n_nodes <= node_cap && sc->n_alive > 0)
+        for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < sc->n_nodes;
+             id += gridDim.x * blockDim.x)
+            moments_norm(dd, id, x, y, z);
     if (threadIdx.x >= blockDim.x - CSG_WARP) { // the last warp
         const int lane = threadIdx.x & 31, nn = sc->n_nodes;
         for (int g = blockIdx.x; g < n_gal; g += gridDim.x) {
@@ -752,15 +1264,16 @@ __global__ void k_tasks(DevScalars *sc, DevRoot *roots, int n_gal, const int *__
         sc->n_tasks = t;
         sc->task_next = 0;
     }
-    // every block fills the tasks of its systems (roots[].first and n_alive
-    // were final before this kernel)
-    for (int g = blockIdx.x; g < n_gal; g += gridDim.x) {
+    // every block fills the tasks of its systems, all blocks those of a single
+    // one (roots[].first and n_alive were final before this kernel)
+    const int share = n_gal == 1 ? gridDim.x : 1, part = n_gal == 1 ? blockIdx.x : 0;
+    for (int g = n_gal == 1 ? 0 : blockIdx.x; g < n_gal; g += gridDim.x) {
         int t0 = 0;
         for (int h = 0; h < g; h++) // systems are few; recompute the offset
             t0 += (roots[h].n_alive + 31) / 32;
         const int n = roots[g].n_alive;
         const int first = imported ? 0 : roots[g].first;
-        for (int j = threadIdx.x; j * 32 < n; j += blockDim.x) {
+        for (int j = part * blockDim.x + threadIdx.x; j * 32 < n; j += share * blockDim.x) {
             if (t0 + j >= task_cap)
                 break;
             WalkTask w;
@@ -771,231 +1284,6 @@ __global__ void k_tasks(DevScalars *sc, DevRoot *roots, int n_gal, const int *__
             tasks[t0 + j] = w;
         }
     }
-}
-
-// Kernels over cells loop over ids (grid-stride): the cell count is known on
-// the device only, and a grid of about 2n threads covers it in one round for
-// the usual trees (cells ~1.3-2 per body) without launching for the capacity.
-__global__ void k_link(csgd_t dd, DevScalars *sc, const unsigned long long *__restrict__ key,
-                       const unsigned long long *__restrict__ ext)
-{
-    pdl_enter();
-    const int nn = sc->n_nodes;
-    if (nn > dd.node_cap)
-        return;
-    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < nn; id += gridDim.x * blockDim.x) {
-        NodeLink l = dd.link[id];
-        if (l.parent < 0 || l.parent >= dd.node_cap)
-            continue;
-        int dg = digit_at(key, ext, l.first, l.level - 1);
-        dd.child[8 * (size_t)l.parent + dg] = id;
-        atomicAdd(&dd.nchild[l.parent], 1);
-    }
-}
-
-// Bottom-up moments: one thread per cell of at most MOM_DIRECT bodies (and
-// per leaf); above those, the last child to finish computes its parent, summing the children in
-// octant order so the result does not depend on scheduling. The climb
-// carries and stores raw sums (sum of m x, sum of m) in the FP64 record, so
-// no division sits on its chain of dependent levels; k_moments_norm then
-// turns every cell's sums into its centre of mass and writes the FP32 record.
-// Only the centre of mass and mass fields are written (write_cell set the
-// rest). EXPORT also keeps the two lowest body indices below each cell (the
-// pool export order).
-__device__ __forceinline__ void put_raw(const csgd_t &dd, int node, double ax, double ay,
-                                        double az, double M)
-{
-    double2 *w = (double2 *)&dd.w64[node];
-    w[0] = make_double2(ax, ay);
-    w[1] = make_double2(az, M);
-}
-
-__device__ __forceinline__ void put_moments(const csgd_t &dd, int node, double sx, double sy,
-                                            double sz, double M)
-{
-    double2 *w = (double2 *)&dd.w64[node];
-    w[0] = make_double2(sx, sy);
-    w[1] = make_double2(sz, M);
-    float4 hi = make_float4((float)sx, (float)sy, (float)sz, (float)M);
-    float *v = (float *)&dd.w32[node];
-    *(float4 *)v = hi;
-    v[4] = (float)(sx - (double)hi.x);
-    v[5] = (float)(sy - (double)hi.y);
-    v[6] = (float)(sz - (double)hi.z);
-}
-
-// Cell moments. A cell with at most MOM_DIRECT bodies, and every leaf, sums
-// its sorted bodies directly (one thread per cell, no atomics); a larger cell
-// is formed from its children's moments by the last child to finish (a ticket
-// per cell), climbing from the directly summed cells whose parent is large.
-// A single-body leaf keeps the body's position exactly (the reference's leaf
-// centre); bodies that coincide to depth 64 share one leaf, in caller index
-// order, so the two smallest caller indices of a cell are its first two.
-constexpr int MOM_DIRECT = 16;
-
-// The ticket of a cell: one gpu-scope acquire-release add. Release: this
-// thread's sums (stored above) are visible to whichever child takes the last
-// ticket; acquire: the last child sees every sibling's sums (the adds on one
-// ticket form a release sequence).
-__device__ __forceinline__ int ticket_take(int *p)
-{
-    int old;
-    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
-    return old;
-}
-
-template <bool EXPORT>
-__device__ __forceinline__ void moments_climb(const csgd_t &dd, int node, int parent, double ax,
-                                              double ay, double az, double M, int2 mi)
-{
-    while (true) {
-        put_raw(dd, node, ax, ay, az, M);
-        if (EXPORT)
-            dd.minidx[node] = mi;
-        if (parent < 0 || parent >= node)
-            break; // preorder: a parent always precedes its children
-        // the parent's children, their count and its own parent are fixed
-        // since k_link: their loads run while the sums above drain
-        const int4 *cp = (const int4 *)(dd.child + 8 * (size_t)parent);
-        const int4 c03 = __ldg(cp), c47 = __ldg(cp + 1);
-        const int nc = __ldg(&dd.nchild[parent]);
-        const int up = __ldg(&dd.link[parent].parent);
-        if (ticket_take(&dd.ticket[parent]) != nc - 1)
-            break;
-        M = 0.0;
-        ax = ay = az = 0.0;
-        int m1 = INT_MAX, m2 = INT_MAX;
-        const int ch[8] = {c03.x, c03.y, c03.z, c03.w, c47.x, c47.y, c47.z, c47.w};
-        for (int q = 0; q < 8; q++) {
-            const int c = ch[q];
-            if (c < 0)
-                continue;
-            const double2 *cw = (const double2 *)&dd.w64[c];
-            const double2 xy = __ldcg(cw), zm = __ldcg(cw + 1);
-            M += zm.y;
-            ax += xy.x;
-            ay += xy.y;
-            az += zm.x;
-            if (EXPORT) {
-                int2 cmi = __ldcg(&dd.minidx[c]);
-                int cand[2] = {cmi.x, cmi.y};
-                for (int j = 0; j < 2; j++) {
-                    int v2 = cand[j];
-                    if (v2 < m1) {
-                        m2 = m1;
-                        m1 = v2;
-                    } else if (v2 < m2) {
-                        m2 = v2;
-                    }
-                }
-            }
-        }
-        mi = make_int2(m1, m2);
-        node = parent;
-        parent = up;
-    }
-}
-
-// Bodies summed directly, four bodies' loads in flight at a time; the additions
-// keep the sorted order (M += m, then sum += m x as one fused multiply-add).
-constexpr int MOM_LOADS = 4;
-
-template <bool EXPORT>
-__device__ __forceinline__ void moments_cell(const csgd_t &dd, int id, const double *__restrict__ x,
-                                             const double *__restrict__ y,
-                                             const double *__restrict__ z,
-                                             const double *__restrict__ m,
-                                             const int *__restrict__ perm)
-{
-    const NodeLink l = dd.link[id];
-    const bool leaf = dd.nchild[id] == 0;
-    if ((!leaf && l.count > MOM_DIRECT) || l.count < 1)
-        return; // formed by the climb (or a cell without bodies)
-    // a parent of at most MOM_DIRECT bodies sums its own bodies
-    const int pcount = (l.parent >= 0) ? __ldg(&dd.link[l.parent].count) : INT_MAX;
-    double M = 0.0, ax = 0.0, ay = 0.0, az = 0.0;
-    int2 mi = make_int2(INT_MAX, INT_MAX);
-    for (int k0 = 0; k0 < l.count; k0 += MOM_LOADS) {
-        int bb[MOM_LOADS];
-        double mv[MOM_LOADS], xv[MOM_LOADS], yv[MOM_LOADS], zv[MOM_LOADS];
-#pragma unroll
-        for (int j = 0; j < MOM_LOADS; j++)
-            bb[j] = (k0 + j < l.count) ? perm[l.first + k0 + j] : -1;
-#pragma unroll
-        for (int j = 0; j < MOM_LOADS; j++) {
-            if (bb[j] >= 0) {
-                mv[j] = m[bb[j]];
-                xv[j] = x[bb[j]];
-                yv[j] = y[bb[j]];
-                zv[j] = z[bb[j]];
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < MOM_LOADS; j++) {
-            if (bb[j] < 0)
-                break;
-            const int b = bb[j];
-            const double mb = mv[j];
-            M += mb;
-            ax += mb * xv[j];
-            ay += mb * yv[j];
-            az += mb * zv[j];
-            if (EXPORT) {
-                if (b < mi.x) {
-                    mi.y = mi.x;
-                    mi.x = b;
-                } else if (b < mi.y) {
-                    mi.y = b;
-                }
-            }
-        }
-    }
-    if (pcount <= MOM_DIRECT) {
-        put_raw(dd, id, ax, ay, az, M); // the parent sums its own bodies
-        if (EXPORT)
-            dd.minidx[id] = mi;
-        return;
-    }
-    moments_climb<EXPORT>(dd, id, l.parent, ax, ay, az, M, mi);
-}
-
-// Raw sums to centre of mass, every cell: a single-body leaf keeps the body's
-// position exactly (the reference's leaf centre), any other cell takes
-// (sum m x) / (sum m), the reciprocal correctly rounded off the FP64 pipe.
-__global__ void k_moments_norm(csgd_t dd, DevScalars *sc, const double *__restrict__ x,
-                               const double *__restrict__ y, const double *__restrict__ z)
-{
-    pdl_enter();
-    const int nn = sc->n_nodes;
-    if (nn > dd.node_cap || sc->n_alive == 0)
-        return;
-    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < nn; id += gridDim.x * blockDim.x) {
-        const NodeLink l = dd.link[id];
-        if (l.count < 1)
-            continue;
-        const double2 *w = (const double2 *)&dd.w64[id];
-        const double2 xy = w[0], zm = w[1];
-        const int body = dd.w64[id].body;
-        if (l.count == 1 && body >= 0) {
-            put_moments(dd, id, x[body], y[body], z[body], zm.y);
-        } else {
-            const double inv = div_rn(1.0, zm.y);
-            put_moments(dd, id, xy.x * inv, xy.y * inv, zm.x * inv, zm.y);
-        }
-    }
-}
-
-template <bool EXPORT>
-__global__ void __launch_bounds__(256, 4) k_moments(csgd_t dd, DevScalars *sc, const double *__restrict__ x,
-                          const double *__restrict__ y, const double *__restrict__ z,
-                          const double *__restrict__ m, const int *__restrict__ perm)
-{
-    pdl_enter();
-    const int nn = sc->n_nodes;
-    if (nn > dd.node_cap || sc->n_alive == 0)
-        return;
-    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < nn; id += gridDim.x * blockDim.x)
-        moments_cell<EXPORT>(dd, id, x, y, z, m, perm);
 }
 
 // FP32 neighbour-search record of one cell (see NodeS32).
@@ -1406,14 +1694,11 @@ extern "C" int csgd_build_tree(csgd_t *d, int geometry)
     csgd_launch(d, k_nodes, gn, B, s, *d, sc, d->roots, d->key, d->ext, d->sgid, d->lcp, d->base, d->perm, d->cnt);
     csgd_launch(d, k_link, gn, B, s, *d, sc, d->key, d->ext);
     csgd_build_mark(d, 3);
-    if (d->export_order)
-        csgd_launch(d, k_moments<true>, gn, B, s, *d, sc, d->x, d->y, d->z, d->m, d->perm);
-    else
-        csgd_launch(d, k_moments<false>, gn, B, s, *d, sc, d->x, d->y, d->z, d->m, d->perm);
-    csgd_launch(d, k_moments_norm, gn, B, s, *d, sc, d->x, d->y, d->z);
+    csgd_launch(d, k_mom_sums, n / MOM_TILE + 1, MOM_TILE, s, *d, sc, d->roots, d->x, d->y, d->z, d->m, d->perm, d->sgid, d->n_gal);
+    csgd_launch(d, k_moments, gn, B, s, *d, sc, d->roots, d->x, d->y, d->z, d->m, d->perm, d->sgid, d->n_gal);
     d->minidx_valid = d->export_order;
     csgd_build_mark(d, 4);
-    csgd_launch(d, k_tasks, min(d->n_gal, 152), 256, s, sc, d->roots, d->n_gal, d->base, d->tasks, d->task_cap, 0, d->link, d->child, d->node_cap);
+    csgd_launch(d, k_tasks, min(d->n_gal > 1 ? d->n_gal : csgd_grid(n, 32 * 256), d->num_sms), 256, s, sc, d->roots, d->n_gal, d->base, d->tasks, d->task_cap, 0, d->link, d->child, d->node_cap, *d, d->x, d->y, d->z);
     d->geometry_valid = 0;
     d->imported = 0;
     d->gas_valid = 0;
@@ -1427,7 +1712,6 @@ extern "C" int csgd_build_tree(csgd_t *d, int geometry)
 
 // Export without a host round trip: the cell count is read on the device
 // (order keys, sort, ranks and records are sized for `capacity` cells).
-// Needs the export order (minidx) of the current tree.
 extern "C" int csgd_export_to(csgd_t *d, OctreeNode *dst, int capacity)
 {
     if (d->n_gal > 1) // one system only (see csgd_set_systems)
@@ -1447,6 +1731,7 @@ extern "C" int csgd_export_to(csgd_t *d, OctreeNode *dst, int capacity)
     const int bound = capacity < d->node_cap ? capacity : d->node_cap;
     const long long cells = cell_threads(d); // the kernels stride beyond it
     const int g = csgd_grid(cells < bound ? cells : bound, B);
+    { k_minidx<<<csgd_grid(cells, B), B, 0, s>>>(*d, sc, d->perm); d->launches++; }
     { k_order_keys<<<g, B, 0, s>>>(*d, sc); d->launches++; }
     int rc = csg_radix_sort(d, d->ord_key, d->ord_id, d->ord_key_alt, d->ord_id_alt, bound, 40,
                             &sc->n_nodes);
@@ -1471,7 +1756,7 @@ extern "C" int csgd_export_pool(csgd_t *d, OctreeNode *pool, int capacity, int *
     int erc = csgd_ensure_tree_extras(d, 1, 1);
     if (erc)
         return erc;
-    if (!d->minidx_valid) { // built without the export order: rebuild (same tree) with it
+    if (!d->minidx_valid) { // not kept for exports: rebuild (same tree)
         const int saved = d->export_order;
         d->export_order = 1;
         erc = csgd_build_tree(d, 1);
@@ -1524,10 +1809,10 @@ extern "C" int csgd_import_pool(csgd_t *d, const OctreeNode *pool, int n_nodes, 
     if (d->n > 0)
         { k_imp_pos<<<csgd_grid(d->n, B), B, 0, s>>>(sc, d->n, d->perm, d->m, d->cnt); d->launches++; }
     { k_imp_write<<<g, B, 0, s>>>(*d, sc, n_nodes, root, par, slot, size, d->cnt); d->launches++; }
-    { k_tasks<<<1, 256, 0, s>>>(sc, d->roots, 1, d->base, d->tasks, d->task_cap, 1, d->link, d->child, d->node_cap); d->launches++; }
+    { k_tasks<<<1, 256, 0, s>>>(sc, d->roots, 1, d->base, d->tasks, d->task_cap, 1, d->link, d->child, d->node_cap, *d, d->x, d->y, d->z); d->launches++; }
     d->geometry_valid = 1;
     d->imported = 1;
-    d->gas_valid = 0;
     d->minidx_valid = 0;
+    d->gas_valid = 0;
     return csgd_check(d, cudaGetLastError());
 }
