@@ -170,6 +170,9 @@ int csgd_sph_cooling(csgd_t *d, double dt);
 
 /* Leapfrog pieces: v += a*dt/2 and x += v*dt; and v += a*dt/2. */
 int csgd_kick_drift(csgd_t *d, double dt);
+/* The same for a tree build that follows at once: the pass also takes the new
+   positions' bounding boxes, and the build starts from them. */
+int csgd_kick_drift_boxed(csgd_t *d, double dt);
 int csgd_kick(csgd_t *d, double dt);
 
 /* One full KDK substep, all on the device (reference src/integrator.c:12-57). */

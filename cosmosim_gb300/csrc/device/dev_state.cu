@@ -467,8 +467,10 @@ extern "C" int csgd_reserve(csgd_t *d, int n)
     if (n != d->n && d->n_gal > 1) { // the system layout no longer fits: one system
         csgd_drop_graph(d);
         d->n_gal = 1;
-        if (d->gid)
+        if (d->gid) {
             cudaMemsetAsync(d->gid, 0, sizeof(int) * (size_t)d->cap, d->stream);
+            cudaMemsetAsync(d->sgid, 0, sizeof(int) * (size_t)d->cap, d->stream);
+        }
     }
     d->n = n;
     if (n <= d->cap && d->cap > 0)
@@ -553,6 +555,7 @@ extern "C" int csgd_reserve(csgd_t *d, int n)
     d->n = n;
     d->n_gal = 1;
     cudaMemsetAsync(d->gid, 0, sizeof(int) * cap, d->stream);
+    cudaMemsetAsync(d->sgid, 0, sizeof(int) * cap, d->stream);
     // the tree stays empty-but-valid until the first build
     cudaMemsetAsync(d->sc, 0, sizeof(DevScalars), d->stream);
     return csgd_check(d, cudaGetLastError());
@@ -646,6 +649,7 @@ extern "C" int csgd_set_systems(csgd_t *d, int n_sys, const int *host_counts)
         return csgd_check(d, cudaGetLastError());
     if (n_sys == 1) {
         cudaMemsetAsync(d->gid, 0, sizeof(int) * (size_t)d->n, d->stream);
+        cudaMemsetAsync(d->sgid, 0, sizeof(int) * (size_t)d->cap, d->stream);
         return csgd_check(d, cudaGetLastError());
     }
     int *h = (int *)malloc(sizeof(int) * (size_t)d->n);
@@ -815,10 +819,11 @@ extern "C" int csgd_substep(csgd_t *d, double dt, const csgd_force_params *p, in
     if (rc)
         return rc;
     phase_mark(d, 0);
-    rc = csgd_kick_drift(d, dt);
+    rc = csgd_kick_drift_boxed(d, dt);
     phase_mark(d, 1);
     if (!rc)
         rc = csgd_build_tree(d, sph);
+    d->boxed = 0; // not left to a later build if this one did not start
     phase_mark(d, 2);
     // the pool export reads the finished tree only: it runs beside the walk
     bool exported = false;

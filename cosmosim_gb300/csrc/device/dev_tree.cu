@@ -206,9 +206,26 @@ __device__ __forceinline__ void bbox_flush(DevRoot *roots, int g, unsigned long 
     cnt = me = 0;
 }
 
+//
+// DRIFT: the bodies are kicked and drifted first (src/integrator.c:27-41, the
+// reference's operations, unfused), their new positions still in registers: a
+// launch and a pass over the positions less than two kernels.
+struct Motion {
+    double dt;
+    double *x, *y, *z, *vx, *vy, *vz;
+    const double *ax, *ay, *az;
+};
+
+__device__ __forceinline__ double kicked(double v, double a, double dt)
+{
+    return __dadd_rn(v, __dmul_rn(__dmul_rn(0.5, a), dt));
+}
+
+template <bool DRIFT>
 __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ y,
                        const double *__restrict__ z, const double *__restrict__ m,
-                       const int *__restrict__ gid, int n, DevRoot *roots, DevScalars *gsc)
+                       const int *__restrict__ gid, int n, DevRoot *roots, DevScalars *gsc,
+                       Motion mo)
 {
     pdl_enter();
     unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0ull, 0ull, 0ull};
@@ -219,15 +236,38 @@ __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ 
          base += (long long)gridDim.x * blockDim.x) {
         const long long i = base + threadIdx.x;
         const int g = (i < n) ? gid[i] : -1;
-        if (g >= 0) {
-            const double mi = m[i];
+        double p[3] = {0.0, 0.0, 0.0}, mi = 0.0;
+        if (i < n) {
+            mi = m[i];
+            if (DRIFT) {
+                p[0] = mo.x[i];
+                p[1] = mo.y[i];
+                p[2] = mo.z[i];
+                if (!(mi <= 0.0)) {
+                    const double v[3] = {kicked(mo.vx[i], mo.ax[i], mo.dt),
+                                         kicked(mo.vy[i], mo.ay[i], mo.dt),
+                                         kicked(mo.vz[i], mo.az[i], mo.dt)};
+                    mo.vx[i] = v[0];
+                    mo.vy[i] = v[1];
+                    mo.vz[i] = v[2];
+#pragma unroll
+                    for (int a = 0; a < 3; a++)
+                        p[a] = __dadd_rn(p[a], __dmul_rn(v[a], mo.dt));
+                    mo.x[i] = p[0];
+                    mo.y[i] = p[1];
+                    mo.z[i] = p[2];
+                }
+            } else {
+                p[0] = x[i];
+                p[1] = y[i];
+                p[2] = z[i];
+            }
             bad |= !isfinite(mi) ||
-                   (is_alive(mi) && !(isfinite(x[i]) && isfinite(y[i]) && isfinite(z[i])));
+                   (is_alive(mi) && !(isfinite(p[0]) && isfinite(p[1]) && isfinite(p[2])));
         }
         const int g0 = __shfl_sync(0xffffffffu, g, 0);
         if (!__all_sync(0xffffffffu, g == g0 || g < 0)) { // straddles systems
-            if (g >= 0 && is_alive(m[i])) {
-                const double p[3] = {x[i], y[i], z[i]};
+            if (g >= 0 && is_alive(mi)) {
                 for (int a = 0; a < 3; a++) {
                     if (p[a] != p[a])
                         continue;
@@ -235,7 +275,7 @@ __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ 
                     atomicMax(&roots[g].omax[a], ord_enc(p[a]));
                 }
                 atomicAdd(&roots[g].n_alive, 1);
-                atomicMax(&roots[g].mass_e, mass_exponent(m[i]));
+                atomicMax(&roots[g].mass_e, mass_exponent(mi));
             }
             continue;
         }
@@ -244,10 +284,9 @@ __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ 
                 bbox_flush(roots, cur_g, lo, hi, cnt, me);
             cur_g = g0;
         }
-        if (g >= 0 && is_alive(m[i])) {
+        if (g >= 0 && is_alive(mi)) {
             cnt++;
-            me = max(me, mass_exponent(m[i]));
-            const double p[3] = {x[i], y[i], z[i]};
+            me = max(me, mass_exponent(mi));
 #pragma unroll
             for (int a = 0; a < 3; a++) {
                 if (p[a] != p[a])
@@ -476,12 +515,24 @@ __device__ __forceinline__ bool same_key(const unsigned long long *key, const in
     return key[a] == key[b] && sgid[a] == sgid[b];
 }
 
+__device__ __forceinline__ void count_cells(const unsigned long long *key,
+                                            const unsigned long long *ext, const int *sgid, int na,
+                                            int p, signed char *lcp, int *cnt)
+{
+    const int P = (p > 0) ? lcp_pos(key, ext, sgid, p - 1, p) : -1;
+    const int Q = (p + 1 < na) ? lcp_pos(key, ext, sgid, p, p + 1) : -1;
+    lcp[p] = (signed char)Q;
+    const int internal = min(Q, CSG_MAX_LEVEL - 1) - P;
+    cnt[p] = (internal > 0 ? internal : 0) + (P < CSG_MAX_LEVEL ? 1 : 0);
+}
+
 __global__ void k_deep_mark(const double *__restrict__ x, const double *__restrict__ y,
                             const double *__restrict__ z, DevScalars *sc,
                             const DevRoot *__restrict__ roots,
                             const unsigned long long *__restrict__ key,
                             const int *__restrict__ sgid, const int *__restrict__ perm,
-                            unsigned long long *__restrict__ ext)
+                            unsigned long long *__restrict__ ext, signed char *__restrict__ lcp,
+                            int *__restrict__ cnt)
 {
     pdl_enter();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -490,8 +541,10 @@ __global__ void k_deep_mark(const double *__restrict__ x, const double *__restri
         return;
     bool deep = (p > 0 && same_key(key, sgid, p - 1, p)) ||
                 (p + 1 < na && same_key(key, sgid, p, p + 1));
-    if (!deep)
+    if (!deep) {
+        count_cells(key, ext, sgid, na, p, lcp, cnt);
         return;
+    }
     const int b = perm[p];
     const DevRoot *r = &roots[sgid[p]];
     ext[3 * (size_t)p + 0] = exact_digits(x[b], y[b], z[b], r, 21, 21);
@@ -514,7 +567,8 @@ __device__ __forceinline__ bool ext_less(const unsigned long long *e, int a, int
 // stable, so equal full keys keep body index order.
 __global__ void k_deep_sort(DevScalars *sc, const unsigned long long *__restrict__ key,
                             const int *__restrict__ sgid, int *__restrict__ perm,
-                            unsigned long long *__restrict__ ext)
+                            unsigned long long *__restrict__ ext, signed char *__restrict__ lcp,
+                            int *__restrict__ cnt)
 {
     pdl_enter();
     if (sc->deep == 0)
@@ -550,25 +604,11 @@ __global__ void k_deep_sort(DevScalars *sc, const unsigned long long *__restrict
         ext[3 * (size_t)(j + 1) + 2] = t2;
         perm[j + 1] = tp;
     }
+    for (int i = p; i < e; i++)
+        count_cells(key, ext, sgid, na, i, lcp, cnt);
 }
 
 // ---- 5/6. cells ----------------------------------------------------------
-
-__global__ void k_count(DevScalars *sc, const unsigned long long *__restrict__ key,
-                        const unsigned long long *__restrict__ ext, const int *__restrict__ sgid,
-                        signed char *__restrict__ lcp, int *__restrict__ cnt)
-{
-    pdl_enter();
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const int na = sc->n_alive;
-    if (p >= na)
-        return;
-    int P = (p > 0) ? lcp_pos(key, ext, sgid, p - 1, p) : -1;
-    int Q = (p + 1 < na) ? lcp_pos(key, ext, sgid, p, p + 1) : -1;
-    lcp[p] = (signed char)Q;
-    int internal = min(Q, CSG_MAX_LEVEL - 1) - P;
-    cnt[p] = (internal > 0 ? internal : 0) + (P < CSG_MAX_LEVEL ? 1 : 0);
-}
 
 __device__ int search_hi(const unsigned long long *key, const unsigned long long *ext,
                          const int *sgid, int na, int p, int L)
@@ -1619,6 +1659,31 @@ __global__ void k_gather_sorted(const int *__restrict__ idx,
 
 // Steps 1-3: root cubes, keys, sorted order of the alive bodies (n_alive),
 // by (system, key) for a forest, and each sorted position's system.
+// The systems' bounding boxes; after a kick and drift with `mo`.
+static void boxes(csgd_t *d, const Motion *mo)
+{
+    csgd_launch(d, k_reset, 1, 256, d->stream, d->sc, d->roots, d->n_gal);
+    d->gas_zero = 1;
+    // few blocks: each warp flushes its running box with atomics on the same
+    // words, so fewer warps contend less (4 blocks per SM keep HBM busy)
+    const int B = 256, per_sm = mo ? 8 : 4;
+    const int gb = max(min(csgd_grid(d->n, B), per_sm * d->num_sms), 1);
+    if (mo)
+        csgd_launch(d, k_bbox<true>, gb, B, d->stream, d->x, d->y, d->z, d->m, d->gid, d->n, d->roots, d->sc, *mo);
+    else
+        csgd_launch(d, k_bbox<false>, gb, B, d->stream, d->x, d->y, d->z, d->m, d->gid, d->n, d->roots, d->sc, Motion{});
+}
+
+extern "C" int csgd_kick_drift_boxed(csgd_t *d, double dt)
+{
+    if (d->n <= 0)
+        return CSG_OK;
+    const Motion mo{dt, d->x, d->y, d->z, d->vx, d->vy, d->vz, d->ax, d->ay, d->az};
+    boxes(d, &mo);
+    d->boxed = 1;
+    return csgd_check(d, cudaGetLastError());
+}
+
 static int order_bodies(csgd_t *d)
 {
     const int n = d->n;
@@ -1627,12 +1692,9 @@ static int order_bodies(csgd_t *d)
     const int B = 256;
     const int G = d->n_gal;
     csgd_build_mark(d, 0);
-    csgd_launch(d, k_reset, 1, 256, s, sc, d->roots, G);
-    d->gas_zero = 1;
-    // few blocks: each warp flushes its running box with atomics on the same
-    // words, so fewer warps contend less (4 blocks per SM keep HBM busy)
-    int gb = min(csgd_grid(n, B), 4 * d->num_sms);
-    csgd_launch(d, k_bbox, gb > 0 ? gb : 1, B, s, d->x, d->y, d->z, d->m, d->gid, n, d->roots, sc);
+    if (!d->boxed)
+        boxes(d, nullptr);
+    d->boxed = 0;
     csgd_launch(d, k_root, 1, 256, s, sc, d->roots, G);
     const bool rank = n <= RANK_MAX;
     if (n > 0)
@@ -1659,7 +1721,8 @@ static int order_bodies(csgd_t *d)
                         cudaMemcpyDeviceToDevice, s);
         cudaMemcpyAsync(d->perm, d->perm_alt, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, s);
     }
-    csgd_launch(d, k_sgid, csgd_grid(n > 0 ? n : 1, B), B, s, sc, d->perm, d->gid, d->sgid, n);
+    if (G > 1) // one system's numbers stay 0 (csgd_reserve, csgd_set_systems)
+        csgd_launch(d, k_sgid, csgd_grid(n > 0 ? n : 1, B), B, s, sc, d->perm, d->gid, d->sgid, n);
     return csgd_check(d, cudaGetLastError());
 }
 
@@ -1683,9 +1746,8 @@ extern "C" int csgd_build_tree(csgd_t *d, int geometry)
         return rc;
     const int g = csgd_grid(n > 0 ? n : 1, B);
     csgd_build_mark(d, 2);
-    csgd_launch(d, k_deep_mark, g, B, s, d->x, d->y, d->z, sc, d->roots, d->key, d->sgid, d->perm, d->ext);
-    csgd_launch(d, k_deep_sort, g, B, s, sc, d->key, d->sgid, d->perm, d->ext);
-    csgd_launch(d, k_count, g, B, s, sc, d->key, d->ext, d->sgid, d->lcp, d->cnt);
+    csgd_launch(d, k_deep_mark, g, B, s, d->x, d->y, d->z, sc, d->roots, d->key, d->sgid, d->perm, d->ext, d->lcp, d->cnt);
+    csgd_launch(d, k_deep_sort, g, B, s, sc, d->key, d->sgid, d->perm, d->ext, d->lcp, d->cnt);
     rc = csg_scan_exclusive(d, d->cnt, d->base, n, &sc->n_alive);
     if (rc)
         return rc;
