@@ -1003,17 +1003,14 @@ __global__ void __launch_bounds__(WARPS * CSG_WARP, WALK32_RES / WARPS) k_walk32
 // term added to the lane's sum, and the sum as doubles (without G) with the
 // next sum started.
 //
-// FP64, with m/r^3 by integers. The cells of even and of odd blocks (counted
-// from a segment's first) are summed apart and the two sums added: by one
-// consumer or two, with the same bits.
-template <int CONS>
+// FP64, with m/r^3 by integers.
 struct EvalF64 {
     struct Rec {
         double2 xy, zm;
     };
     const NodeW64 *cells;
     double eps2, px, py, pz;
-    double s[3 - CONS][3]; // one consumer: both sums; two: its own
+    double s[3];
 
     __device__ __forceinline__ EvalF64(const WalkArgs &a, const FixGrid &, int me)
         : cells(a.w64), eps2(a.eps2), px(me >= 0 ? a.x[me] : 0.0), py(me >= 0 ? a.y[me] : 0.0),
@@ -1023,26 +1020,21 @@ struct EvalF64 {
     }
     __device__ __forceinline__ void clear()
     {
-#pragma unroll
-        for (int k = 0; k < 3 - CONS; k++)
-            s[k][0] = s[k][1] = s[k][2] = 0.0;
+        s[0] = s[1] = s[2] = 0.0;
     }
     __device__ __forceinline__ Rec load(int c) const
     {
         const double2 *w = (const double2 *)&cells[c];
         return Rec{__ldg(w), __ldg(w + 1)};
     }
-    __device__ __forceinline__ void term(const Rec &r, int odd)
+    __device__ __forceinline__ void term(const Rec &r)
     {
         const double dx = r.xy.x - px, dy = r.xy.y - py, dz = r.zm.x - pz;
         const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
         const double f = r.zm.y == 0.0 ? 0.0 : m_inv_r3_q(r.zm.y, r2);
-        double *t = s[0];
-        if (CONS == 1 && odd)
-            t = s[2 - CONS];
-        t[0] = fma(f, dx, t[0]);
-        t[1] = fma(f, dy, t[1]);
-        t[2] = fma(f, dz, t[2]);
+        s[0] = fma(f, dx, s[0]);
+        s[1] = fma(f, dy, s[1]);
+        s[2] = fma(f, dz, s[2]);
     }
     static __device__ __forceinline__ void drop(Rec &r) { r.zm.y = 0.0; }
     // another warp's sums of the same body (6 words a lane)
@@ -1050,7 +1042,7 @@ struct EvalF64 {
     {
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            const u64 v = (u64)__double_as_longlong(s[0][d]);
+            const u64 v = (u64)__double_as_longlong(s[d]);
             o[(2 * d) * CSG_WARP] = (unsigned)v;
             o[(2 * d + 1) * CSG_WARP] = (unsigned)(v >> 32);
         }
@@ -1059,15 +1051,14 @@ struct EvalF64 {
     {
 #pragma unroll
         for (int d = 0; d < 3; d++)
-            s[0][d] += __longlong_as_double((long long)(((u64)o[(2 * d + 1) * CSG_WARP] << 32) |
-                                                        o[(2 * d) * CSG_WARP]));
+            s[d] += __longlong_as_double((long long)(((u64)o[(2 * d + 1) * CSG_WARP] << 32) |
+                                                     o[(2 * d) * CSG_WARP]));
     }
-    __device__ __forceinline__ void close(double &x, double &y, double &z)
+    __device__ __forceinline__ void value(double &x, double &y, double &z) const
     {
-        x = CONS == 1 ? s[0][0] + s[2 - CONS][0] : s[0][0];
-        y = CONS == 1 ? s[0][1] + s[2 - CONS][1] : s[0][1];
-        z = CONS == 1 ? s[0][2] + s[2 - CONS][2] : s[0][2];
-        clear();
+        x = s[0];
+        y = s[1];
+        z = s[2];
     }
 };
 
@@ -1104,7 +1095,7 @@ struct EvalFix {
         const longlong2 xy = __ldg(w), zm = __ldg(w + 1);
         return Rec{xy.x, xy.y, zm.x, (unsigned long long)zm.y};
     }
-    __device__ __forceinline__ void term(const Rec &r, int)
+    __device__ __forceinline__ void term(const Rec &r)
     {
         if (WIDE) {
             const int hz = (int)(r.z >> 32), far = (hz >> 30 ^ hz >> 31) & 1, up = far ? f.far : 0;
@@ -1131,12 +1122,11 @@ struct EvalFix {
         z.sum(o[6 * CSG_WARP], o[7 * CSG_WARP], o[8 * CSG_WARP]);
         cnt += (int)o[9 * CSG_WARP];
     }
-    __device__ __forceinline__ void close(double &ox, double &oy, double &oz)
+    __device__ __forceinline__ void value(double &ox, double &oy, double &oz) const
     {
         ox = x.value(f.U3, cnt);
         oy = y.value(f.U3, cnt);
         oz = z.value(f.U3, cnt);
-        clear();
     }
 };
 
@@ -1156,9 +1146,8 @@ __device__ __forceinline__ void put_partial(const WalkArgs &a, int k, int me, do
 // in the blocks at its own pace. The warps hand over through head and tail
 // block counters in shared memory; every wait polls with a sleep and gives up
 // after a.wait_polls polls (recording CSG_ERR_DEVICE_WAIT, then all warps leave
-// the task). A unit of the split form (G > 0) is G segments of a task: the root
-// step, then the subtrees of the split cell's children k0 .. k0 + G - 1; the first
-// block of a later segment is marked.
+// the task). A unit of the split form is one segment of a task: the subtree of
+// the split cell's child k0 (segment 0: also the cells above the segments).
 //
 // Bound: the integer multiply and ALU pipes (65% and 62% busy at 1M, issue
 // 70%); the walk in FP64 was bound by the FP64 pipe (9 operations a pair).
@@ -1178,12 +1167,12 @@ __device__ __forceinline__ void put_partial(const WalkArgs &a, int k, int me, do
 constexpr int WS_BLOCKS = 32; // queue length (power of two; 16: 4% slower at 1M)
 constexpr int WS_RES = 21;    // resident warps per SM that the registers are sized for (18 and
                               // 24: 2-5% slower at 1M)
+constexpr int WS_CONS = 2;    // consumer warps
 constexpr int WS_LOW = 2;     // blocks the slowest reader wants ahead before a step
 
 struct WsShared {
     int ids[WS_BLOCKS * CSG_WARP];
     unsigned take[WS_BLOCKS * CSG_WARP];
-    int mark[WS_BLOCKS]; // 2 x segments closed before this block, + 1 for an odd block of its own
     int tail;            // blocks published by the producer
     int head[2];         // each consumer's first block that some lane still reads
     int done;            // producer finished (tail final)
@@ -1200,12 +1189,12 @@ struct BlockQueue : LanePos {
     WsShared &sh;
     DevScalars *sc;
     int wait_polls;
-    int tail, head_seen, marks, parity, cons;
+    int tail, head_seen;
     bool mute, broken;
 
-    __device__ __forceinline__ BlockQueue(const WalkArgs &a, const LaneBody &L, WsShared &s, int c)
-        : LanePos(L), sh(s), sc(a.sc), wait_polls(a.wait_polls), tail(0), head_seen(0), marks(0),
-          parity(0), cons(c), mute(false), broken(false)
+    __device__ __forceinline__ BlockQueue(const WalkArgs &a, const LaneBody &L, WsShared &s)
+        : LanePos(L), sh(s), sc(a.sc), wait_polls(a.wait_polls), tail(0), head_seen(0),
+          mute(false), broken(false)
     {
     }
     // waits until a block is free
@@ -1214,9 +1203,7 @@ struct BlockQueue : LanePos {
         if (tail - head_seen < WS_BLOCKS || broken)
             return;
         for (int i = 0; i < wait_polls; i++) {
-            head_seen = ws_load(&sh.head[0]);
-            if (cons == 2)
-                head_seen = min(head_seen, ws_load(&sh.head[1]));
+            head_seen = min(ws_load(&sh.head[0]), ws_load(&sh.head[1]));
             if (tail - head_seen < WS_BLOCKS || ws_load(&sh.broken))
                 break;
             __nanosleep(64);
@@ -1241,10 +1228,6 @@ struct BlockQueue : LanePos {
         const int lane = threadIdx.x & 31, b = tail & (WS_BLOCKS - 1);
         sh.ids[b * CSG_WARP + lane] = cell;
         sh.take[b * CSG_WARP + lane] = take;
-        if (lane == 0)
-            sh.mark[b] = 2 * marks + parity;
-        marks = 0;
-        parity ^= 1;
         tail++;
         __threadfence_block(); // the block before the tail
         __syncwarp();
@@ -1253,13 +1236,13 @@ struct BlockQueue : LanePos {
     }
 };
 
-template <bool STATS, int G>
+template <bool STATS, bool UNITS>
 __device__ __forceinline__ void ws_produce(const WalkArgs &a, RoundShared &rs, WsShared &sh,
-                                           const TaskRange &tr, int k0, int cons, WalkStats &st)
+                                           const TaskRange &tr, int k0, WalkStats &st)
 {
     const LaneBody L = lane_body(a, rs, tr);
-    BlockQueue q(a, L, sh, cons);
-    q.mute = G > 0 && k0 != 0; // the root's terms are segment 0's
+    BlockQueue q(a, L, sh);
+    q.mute = UNITS && k0 != 0; // the terms above the segments are segment 0's
     const unsigned open = walk_top<STATS>(a, rs, L, tr, q, st, !q.mute);
     q.mute = false;
     int k = 0; // child (segment) number
@@ -1267,13 +1250,8 @@ __device__ __forceinline__ void ws_produce(const WalkArgs &a, RoundShared &rs, W
         const int c = __ldg(&a.child[8 * (size_t)tr.split + o]);
         if (c <= tr.split)
             continue;
-        if (G == 0 || (k >= k0 && k < k0 + G)) {
-            if (G > 0 && k > k0) {
-                q.marks++;
-                q.parity = 0;
-            }
+        if (!UNITS || k == k0)
             walk_subtree<STATS>(a, rs, L, c, open, q, st);
-        }
         k++;
     }
     __threadfence_block();
@@ -1286,21 +1264,17 @@ __device__ __forceinline__ void ws_produce(const WalkArgs &a, RoundShared &rs, W
 // next block.
 struct WsReader {
     unsigned left;
-    int cur, next, odd;
+    int cur, next;
 };
 
 // The lane's next cell, or -1 (none published, or the next block has none for
-// it); marks gets the segments closed before it.
-template <int CONS>
-__device__ __forceinline__ int ws_next(const WsShared &sh, WsReader &r, int tail, int lane,
-                                       int &marks)
+// it).
+__device__ __forceinline__ int ws_next(const WsShared &sh, WsReader &r, int tail, int lane)
 {
     if (r.left == 0u && r.next < tail) {
         r.cur = r.next & (WS_BLOCKS - 1);
         r.left = sh.take[r.cur * CSG_WARP + lane];
-        marks += sh.mark[r.cur] >> 1;
-        r.odd = sh.mark[r.cur] & 1;
-        r.next += CONS;
+        r.next += WS_CONS;
     }
     if (r.left == 0u)
         return -1;
@@ -1309,49 +1283,26 @@ __device__ __forceinline__ int ws_next(const WsShared &sh, WsReader &r, int tail
     return sh.ids[r.cur * CSG_WARP + j];
 }
 
-// A segment's end: its partial written, the sum restarted.
-template <class Eval>
-__device__ __forceinline__ void ws_close(const WalkArgs &a, Eval &ev, int me, int &kc, int n)
-{
-    for (; n > 0; n--) {
-        double x, y, z;
-        ev.close(x, y, z);
-        if (me >= 0)
-            put_partial(a, kc, me, x, y, z);
-        kc++;
-    }
-}
-
 // Cells a lane evaluates between two looks at the counters: whole tasks (16:
 // 2-5% faster from 100k bodies on), a split task's units (8: 5% faster at 20k).
 constexpr int WS_STEP_TASK = 16, WS_STEP_UNIT = 8;
 
-// Consumer `which` of CONS: the blocks which, which + CONS, ...
-template <int G, int CONS, class Eval>
+// Consumer `which`: the blocks which, which + 2, ...
+template <bool UNITS, class Eval>
 __device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, const TaskRange &tr,
                                            const FixGrid &grid, int k0, int which)
 {
-    static_assert(CONS == 1 || G <= 1, "a segment end inside a unit is one consumer's");
     const int lane = threadIdx.x & 31;
     const bool valid = lane < tr.count;
     const int me = valid ? a.perm[tr.pos0 + lane] : -1;
     Eval ev(a, grid, me);
-    WsReader rd{0u, 0, which, 0};
-    int polls = 0, head = which, kc = k0; // kc: the segment being summed (split form)
+    WsReader rd{0u, 0, which};
+    int polls = 0, head = which;
     // two cells are always on their way: their loads run during the terms of
     // the two before them (massless ones at first)
     typename Eval::Rec ra = ev.load(0), rb = ra;
     ev.drop(ra);
     ev.drop(rb);
-    int ma = 0, mb = 0; // 2 x segments closed before each, + 1 for an odd block's
-    auto terms = [&]() {
-        if (G > 1 && ma > 1) // rare
-            ws_close(a, ev, me, kc, ma >> 1);
-        ev.term(ra, ma & 1);
-        if (G > 1 && mb > 1)
-            ws_close(a, ev, me, kc, mb >> 1);
-        ev.term(rb, mb & 1);
-    };
     while (true) {
         // read before the tail: it is final then
         const bool done = __shfl_sync(0xffffffffu, ws_load(&sh.done), 0) != 0;
@@ -1363,29 +1314,25 @@ __device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, cons
         const int ahead =
             tail - (int)__reduce_max_sync(0xffffffffu, (unsigned)(valid ? rd.next : 0));
         if (ahead >= WS_LOW || tail - head >= WS_BLOCKS || (done && head < tail)) {
-            auto fetch = [&](typename Eval::Rec &r, int &mk) {
-                int m = 0;
-                const int c = ws_next<CONS>(sh, rd, tail, lane, m);
+            auto fetch = [&](typename Eval::Rec &r) {
+                const int c = ws_next(sh, rd, tail, lane);
                 r = ev.load(max(c, 0));
                 if (c < 0) // any cell was read: a massless term
                     ev.drop(r);
-                mk = CONS == 1 ? 2 * m + rd.odd : 0;
             };
 #pragma unroll 1
-            for (int s = 0; s < (G == 0 ? WS_STEP_TASK : WS_STEP_UNIT); s += 2) {
+            for (int s = 0; s < (UNITS ? WS_STEP_UNIT : WS_STEP_TASK); s += 2) {
                 typename Eval::Rec rc, rq;
-                int mc, md;
-                fetch(rc, mc);
-                fetch(rq, md);
-                terms();
+                fetch(rc);
+                fetch(rq);
+                ev.term(ra);
+                ev.term(rb);
                 ra = rc;
                 rb = rq;
-                ma = mc;
-                mb = md;
             }
             // blocks that every lane is through with
             const int h = (int)__reduce_min_sync(
-                0xffffffffu, (unsigned)(!valid ? tail + CONS : rd.left ? rd.next - CONS : rd.next));
+                0xffffffffu, (unsigned)(!valid ? tail + WS_CONS : rd.left ? rd.next - WS_CONS : rd.next));
             __threadfence_block(); // blocks read before the head is published
             __syncwarp();
             if (h != head && lane == 0)
@@ -1395,7 +1342,8 @@ __device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, cons
             continue;
         }
         if (done) { // head == tail: every block read
-            terms();
+            ev.term(ra);
+            ev.term(rb);
             break;
         }
         if (__any_sync(0xffffffffu, ws_load(&sh.broken)))
@@ -1409,39 +1357,38 @@ __device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, cons
         }
         __nanosleep(64);
     }
-    if constexpr (CONS == 2) { // the sums joined (integers: exact)
-        if (which == 1) {
-            ev.save(sh.other + lane);
-            __threadfence_block();
-            __syncwarp();
-            if (lane == 0)
-                ((volatile int *)&sh.half)[0] = 1;
-            return;
-        }
-        for (int i = 0; !__any_sync(0xffffffffu, ws_load(&sh.half)); i++) {
-            if (i >= a.wait_polls || __any_sync(0xffffffffu, ws_load(&sh.broken))) {
-                if (lane == 0) {
-                    dev_fail(a.sc, CSG_ERR_DEVICE_WAIT);
-                    ((volatile int *)&sh.broken)[0] = 1;
-                }
-                return;
-            }
-            __nanosleep(64);
-        }
+    // the second consumer's sums joined to the first's (integers: exact)
+    if (which == 1) {
+        ev.save(sh.other + lane);
         __threadfence_block();
         __syncwarp();
-        ev.join(sh.other + lane);
+        if (lane == 0)
+            ((volatile int *)&sh.half)[0] = 1;
+        return;
     }
-    if (G > 0) { // the last segment's partial (segment 0's with the root's term),
-        ws_close(a, ev, me, kc, k0 + G - kc); // zeros for segments the walk did not reach
-    } else {
-        double sx, sy, sz;
-        ev.close(sx, sy, sz);
-        if (valid) {
-            a.ax[me] = a.G * sx;
-            a.ay[me] = a.G * sy;
-            a.az[me] = a.G * sz;
+    for (int i = 0; !__any_sync(0xffffffffu, ws_load(&sh.half)); i++) {
+        if (i >= a.wait_polls || __any_sync(0xffffffffu, ws_load(&sh.broken))) {
+            if (lane == 0) {
+                dev_fail(a.sc, CSG_ERR_DEVICE_WAIT);
+                ((volatile int *)&sh.broken)[0] = 1;
+            }
+            return;
         }
+        __nanosleep(64);
+    }
+    __threadfence_block();
+    __syncwarp();
+    ev.join(sh.other + lane);
+    if (!valid)
+        return;
+    double x, y, z;
+    ev.value(x, y, z);
+    if (UNITS) { // the segment's partial (zero for one that the walk did not reach)
+        put_partial(a, k0, me, x, y, z);
+    } else {
+        a.ax[me] = a.G * x;
+        a.ay[me] = a.G * y;
+        a.az[me] = a.G * z;
     }
 }
 
@@ -1459,12 +1406,12 @@ __device__ __forceinline__ bool near_task(const WalkArgs &a, const TaskRange &tr
     return __all_sync(0xffffffffu, ok);
 }
 
-// One task per block (G == 0), or one unit of G segments of a task,
-// u = (8 / G) * task + k0 / G (partials into a.part): the producer warp, then
-// CONS consumers. Two consumers where the split does not mark segment ends
-// inside a unit: the producer needs about a fifth of a consumer's time, and
-// the sums of two join to the same bits.
-template <bool STATS, int G, int CONS>
+// One task per block, or (UNITS) one segment of a task, u = 8 task + segment
+// (partials into a.part): the producer warp, then the consumers. The producer needs about a
+// fifth of a consumer's time. Units of several segments of a task, for fewer root steps,
+// needed the segments' ends in the queue and so had one consumer: 30,000 bodies 0.79 ms
+// against 0.51, 64 systems of 2,000 to 50,000 18.0 against 12.9.
+template <bool STATS, bool UNITS>
 __device__ __forceinline__ void walk64ws_body(const WalkArgs &a)
 {
     __shared__ WsShared sh;
@@ -1474,13 +1421,13 @@ __device__ __forceinline__ void walk64ws_body(const WalkArgs &a)
     if (nn > a.node_cap || nn < 1)
         return;
     const int u = blockIdx.x;
-    const int t = G > 0 ? u / (8 / G) : u, k0 = G > 0 ? (u % (8 / G)) * G : 0;
+    const int t = UNITS ? u / WSEGS : u, k0 = UNITS ? u % WSEGS : 0;
     if (t >= a.sc->n_tasks)
         return;
     const WalkTask w = a.tasks[t];
     const DevRoot &r = a.roots[w.gal];
     const TaskRange tr{w.pos0, w.count, r.root, r.end, r.split, small_system(a, w.gal)};
-    if (G > 0 ? !tr.small : (tr.small && a.skip_small))
+    if (UNITS ? !tr.small : (tr.small && a.skip_small))
         return; // the other form walks this system
     if (tr.root < 0 || tr.end > nn || tr.root >= tr.end) {
         if (threadIdx.x == 0)
@@ -1499,31 +1446,32 @@ __device__ __forceinline__ void walk64ws_body(const WalkArgs &a)
     __syncthreads(); // counters set before any warp starts (the returns above are the block's)
     if (warp == 0) {
         WalkStats st;
-        ws_produce<STATS, G>(a, rs, sh, tr, k0, CONS, st);
+        ws_produce<STATS, UNITS>(a, rs, sh, tr, k0, st);
         if (STATS)
             add_hits(a, st);
     } else if (fix && r.fix.far == 0) {
-        ws_consume<G, CONS, EvalFix<false>>(a, sh, tr, r.fix, k0, warp - 1);
+        ws_consume<UNITS, EvalFix<false>>(a, sh, tr, r.fix, k0, warp - 1);
     } else if (fix) {
-        ws_consume<G, CONS, EvalFix<true>>(a, sh, tr, r.fix, k0, warp - 1);
+        ws_consume<UNITS, EvalFix<true>>(a, sh, tr, r.fix, k0, warp - 1);
     } else {
-        ws_consume<G, CONS, EvalF64<CONS>>(a, sh, tr, r.fix, k0, warp - 1);
+        ws_consume<UNITS, EvalF64>(a, sh, tr, r.fix, k0, warp - 1);
     }
 }
 
 template <bool STATS>
-__global__ void __launch_bounds__(3 * CSG_WARP, WS_RES / 3) k_walk64ws(WalkArgs a)
+__global__ void __launch_bounds__((1 + WS_CONS) * CSG_WARP, WS_RES / (1 + WS_CONS))
+    k_walk64ws(WalkArgs a)
 {
-    walk64ws_body<STATS, 0, 2>(a);
+    walk64ws_body<STATS, false>(a);
 }
 
 // The FP64 walk split by the split cell's children (few tasks for the GPU): partials
-// into a.part, summed by k_walk_sum; the same bits for every G.
-template <bool STATS, int G>
-__global__ void __launch_bounds__((G == 1 ? 3 : 2) * CSG_WARP, WS_RES / (G == 1 ? 3 : 2))
+// into a.part, summed by k_walk_sum.
+template <bool STATS>
+__global__ void __launch_bounds__((1 + WS_CONS) * CSG_WARP, WS_RES / (1 + WS_CONS))
     k_walk64ws_units(WalkArgs a)
 {
-    walk64ws_body<STATS, G, (G == 1 ? 2 : 1)>(a);
+    walk64ws_body<STATS, true>(a);
 }
 
 // Before a walk: dead bodies get a = 0 (src/octree.c:226-230; alive ones are
@@ -1784,41 +1732,20 @@ void launch_walk(csgd_t *d, const WalkArgs &a, int precision, int exact)
             CSG_LAUNCH_WALK(k_walk32, 4, grid, s, b);
         else
             CSG_LAUNCH_WALK(k_walk32, 8, grid, s, b);
-    } else { // FP64: producer/consumer pairs (the task group applies to FP32 only)
-        // small systems (split_max bodies or fewer): pairs per (task, root
-        // children), partials added by k_walk_sum; the rest a pair per task
+    } else { // FP64: producer and consumer warps (the task group applies to FP32 only)
+        // small systems (split_max bodies or fewer): a block per (task,
+        // segment), partials added by k_walk_sum; the rest a block per task
         const bool units = d->wpart && d->wpart_cap >= d->n &&
                            csgd_sys_min_n(d) <= b.split_max;
         b.skip_small = units;
         if (units) {
-            // G segments per pair: one while the units fit about four waves of
-            // pairs (about 12 per SM), more (with markers between them) for larger launches
-            const long long tasks = (long long)d->n / CSG_WARP + d->n_gal + 1;
-            int g = 1;
-            while (g < WSEGS && tasks * (WSEGS / g) > 4LL * 12 * d->num_sms)
-                g *= 2;
-            const int gw = (int)(tasks * (WSEGS / g));
+            const int gw = (int)(((long long)d->n / CSG_WARP + d->n_gal + 1) * WSEGS);
             b.part = d->wpart;
             b.pstride = d->wpart_cap;
-#define CSG_U(ST, GG)                                                                              \
-    k_walk64ws_units<ST, GG><<<gw, (GG == 1 ? 3 : 2) * CSG_WARP, 0, s>>>(b)
-#define CSG_UG(ST)                                                                                 \
-    do {                                                                                          \
-        if (g == 1)                                                                               \
-            CSG_U(ST, 1);                                                                         \
-        else if (g == 2)                                                                          \
-            CSG_U(ST, 2);                                                                         \
-        else if (g == 4)                                                                          \
-            CSG_U(ST, 4);                                                                         \
-        else                                                                                      \
-            CSG_U(ST, 8);                                                                         \
-    } while (0)
             if (stats)
-                CSG_UG(true);
+                k_walk64ws_units<true><<<gw, (1 + WS_CONS) * CSG_WARP, 0, s>>>(b);
             else
-                CSG_UG(false);
-#undef CSG_UG
-#undef CSG_U
+                k_walk64ws_units<false><<<gw, (1 + WS_CONS) * CSG_WARP, 0, s>>>(b);
             k_walk_sum<<<csgd_grid(d->n, 256), 256, 0, s>>>(d->wpart, (long long)d->wpart_cap,
                                                               d->m, d->n, b.G, d->ax, d->ay, d->az,
                                                               d->gid, b.sys_n, b.split_max);
@@ -1828,9 +1755,9 @@ void launch_walk(csgd_t *d, const WalkArgs &a, int precision, int exact)
         }
         const long long tasks = (long long)d->n / CSG_WARP + d->n_gal + 1; // >= n_tasks
         if (stats)
-            k_walk64ws<true><<<(int)tasks, 3 * CSG_WARP, 0, s>>>(b);
+            k_walk64ws<true><<<(int)tasks, (1 + WS_CONS) * CSG_WARP, 0, s>>>(b);
         else
-            k_walk64ws<false><<<(int)tasks, 3 * CSG_WARP, 0, s>>>(b);
+            k_walk64ws<false><<<(int)tasks, (1 + WS_CONS) * CSG_WARP, 0, s>>>(b);
     }
     d->launches++;
 }
