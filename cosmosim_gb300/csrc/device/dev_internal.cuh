@@ -367,17 +367,25 @@ int csg_scan_exclusive(csgd_t *d, const int *in, int *out, int n, const int *cou
 
 // Polls a bounded device wait makes before it gives up (csgd::wait_polls).
 constexpr int CSG_WAIT_POLLS_DEFAULT = 1 << 22;
-// The walks split each task by the root's children when there are few tasks
-// for the GPU: up to 12 per SM (about 58k bodies on 152 SMs). Above that the
-// whole-task walk already fills the SMs and the split only adds root-level
-// work. The FP32 walk decides per launch (both forms give the same bits); the
-// FP64 walk per system, by its body count (the forms sum differently, and a
-// system must come out the same alone and in an ensemble).
+// The walks split each task by child subtrees when there are few tasks for the
+// GPU. Above that the whole-task walk already fills the SMs and the split only
+// adds root-level work. The FP32 walk decides per launch, up to 12 tasks per SM
+// (about 58k bodies on 152 SMs; both forms give the same bits); the FP64 walk
+// per system, by its body count (the forms sum differently, and a system must
+// come out the same alone and in an ensemble), up to 12 for opening angles
+// below 0.45 and 6 (29,184 bodies) from there on: small angles make long tasks,
+// of which the last wave of whole ones leaves most SMs idle. Split against whole,
+// us: 36,901 bodies at angles 0.3, 0.4, 0.5, 0.7: 1354 and 1873, 854 and 957, 634
+// and 603, 397 and 325; 58,000: 2287 and 2902, 1388 and 1416, 1000 and 919, 617
+// and 487; 25,000 at 0.5: 431 and 485.
 inline bool csgd_walk_split(const csgd_t *d)
 {
     return (long long)d->n / 32 + d->n_gal + 1 <= 12LL * d->num_sms;
 }
-inline long long csgd_split_max_bodies(const csgd_t *d) { return 12LL * 32 * d->num_sms; }
+inline long long csgd_split_max_bodies(const csgd_t *d, int precision, double theta)
+{
+    return (precision == CSG_PREC_FP64 && !(theta < 0.45) ? 6LL : 12LL) * 32 * d->num_sms;
+}
 inline int csgd_sys_min_n(const csgd_t *d) { return d->n_gal > 1 ? d->sys_min_n : d->n; }
 inline int csgd_sys_max_n(const csgd_t *d) { return d->n_gal > 1 ? d->sys_max_n : d->n; }
 // Scratch of the split walks, allocated on first use outside any capture

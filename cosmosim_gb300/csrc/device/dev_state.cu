@@ -885,7 +885,7 @@ extern "C" int csgd_substep(csgd_t *d, double dt, const csgd_force_params *p, in
 int csgd_prepare_walk(csgd_t *d, int precision)
 {
     const bool split = precision == CSG_PREC_FP32_MIXED ? csgd_walk_split(d)
-                       : precision == CSG_PREC_FP64     ? csgd_sys_min_n(d) <= csgd_split_max_bodies(d)
+                       : precision == CSG_PREC_FP64     ? csgd_sys_min_n(d) <= csgd_split_max_bodies(d, precision, 0.0)
                                                         : false;
     if (precision == CSG_PREC_FP64 && !(d->wfix && d->wfix_cap >= d->node_cap)) {
         csgd_drop_graph(d);

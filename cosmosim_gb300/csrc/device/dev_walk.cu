@@ -1673,7 +1673,7 @@ WalkArgs walk_args(csgd_t *d, const csgd_force_params *p)
     a.group = d->walk_group;
     a.sys_n = d->n_gal > 1 ? d->sys_n : nullptr;
     a.n_bodies = d->n;
-    a.split_max = (int)csgd_split_max_bodies(d);
+    a.split_max = (int)csgd_split_max_bodies(d, p->precision, p->theta);
     a.skip_small = 0;
     return a;
 }
