@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(8 * CSG_WARP) k_walk64_exact(WalkArgs a)
 // galaxies 3.40 -> 2.48 ms; 10k-body interaction lists 0.25 -> 0.13 ms. It is
 // bound by instruction issue (67% busy at 1M); 42% of the lane slots idle in
 // cells that only some lanes reach. Measured and not used: starting the next
-// round's loads before this round's evaluations (12 more live registers: 1M
+// round's loads before the same round's evaluations (12 more live registers: 1M
 // 4.28-4.5 ms), 24 resident warps per SM (more spills: 4.31 ms).
 //
 // Children come from the child table (8 ids per cell), loaded before the
