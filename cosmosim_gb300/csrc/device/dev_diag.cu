@@ -5,11 +5,9 @@
 // energy KE + softened PE (tests/test_physics.c:34-52), both in FP64. The
 // j range is split over blocks; each block writes its partial sums and a
 // second kernel adds them in a fixed order, so results are deterministic.
-// Both sums run on the integer pipes (dev_fixpair.cuh) when the bodies fit its
-// grid, which a first kernel finds on the device; the FP64 kernels are queued
-// beside them and return at once then. Measured at 100k bodies: energy 196 ->
-// 28.3 ms, direct sum of 4096 bodies 20.0 -> 4.0 ms, both bound by the integer
-// multiply and ALU pipes (74% and 66% busy).
+// The direct sum runs on the integer pipes (dev_fixpair.cuh) when the bodies fit its
+// grid, which a first kernel finds on the device; the FP64 kernel is queued
+// beside it and returns at once then (4096 of 100k bodies: 20.0 -> 4.0 ms).
 //
 // The probes time long independent FMA chains (8 per thread) and report the
 // FP32 and FP64 CUDA-core throughput of this GPU: the denominators for the
@@ -22,6 +20,7 @@ namespace {
 
 constexpr int DT = 256;       // threads per block
 constexpr int JCHUNKS = 64;   // j-range splits for the direct sum
+constexpr int FT = 128;       // threads per block of the sums on the integer pipes
 
 // The bodies' grid: largest |coordinate| (dead bodies too: they may be sampled)
 // and mass of the live bodies, turned into the grid by the last block to
@@ -78,8 +77,6 @@ __device__ __forceinline__ FixBody fix_body(const double *x, const double *y, co
 // and no FP64 operation (the FP64 kernel below: a square root, a division and
 // 16 more). A body's own term is zero (its differences are). A sample index
 // outside [0, n) reads nothing; its row becomes NaN.
-constexpr int FT = 128;
-
 template <bool MULTI>
 __global__ void __launch_bounds__(FT, 5) k_direct_fix(const double *__restrict__ x,
                                                    const double *__restrict__ y,
@@ -207,140 +204,72 @@ __global__ void k_direct_sum(const double *__restrict__ part, int chunks, int ns
         out[3 * (size_t)k + d] = a[d];
 }
 
-// 1/r in FP64 with few FP64 operations: FP32 rsqrt seed y0 (rel. error
-// < 2^-21), e = 1 - r2*y0^2 by one fused multiply-add (y0^2 exact), then
-// y0 (1 + e/2 + 3e^2/8) (the series of (1-e)^-1/2; the next term is < 2^-60).
-__device__ __forceinline__ double inv_r(double r2)
-{
-    const float r2f = (float)r2;
-    if (r2f >= 1e-30f && r2f <= 1e30f) {
-        const double y0 = (double)rsqrtf(r2f);
-        const double e = fma(-r2, y0 * y0, 1.0);
-        return fma(y0 * e, fma(0.375, e, 0.5), y0);
-    }
-    return 1.0 / sqrt(r2);
-}
-
-// Potential energy on the integer pipes: rows of 2 FT bodies (two a thread)
-// against a chunk of `per` columns j > i, about 150 instructions a pair and no
-// FP64 operation. Row i's sum of m_j / r over chunk c goes to part[c n + i];
-// chunks wholly at or before the row block are left out, there and below. The
-// columns are split so that the long rows of the first bodies do not keep a
-// few SMs busy at the end.
+// Potential energy: rows of 2 FT bodies (two a thread) against a chunk of `per`
+// columns j > i. Differences and sums in FP64, 1/r by integers (pair_inv_r): 4 FP64
+// operations a pair, 256 cycles a warp and scheduler, beside about 150 integer
+// instructions: 37.9 ms at 100k bodies. With the whole 1/r in FP64 (14 operations,
+// and rows not split) 196 ms; with positions and sums in fixed point 28.3 ms, but the
+// bits of close pairs near the origin lost to the grid. The block's sum of m_i m_j / r goes to part[c gridDim.x + b] (0 for
+// a chunk wholly at or before the rows). The columns are split so that the long
+// rows of the first bodies do not keep a few SMs busy at the end.
 constexpr int PT_ROWS = 2 * FT;
 
 template <bool MULTI>
-__global__ void __launch_bounds__(FT, 6) k_potential_fix(const double *__restrict__ x,
-                                                      const double *__restrict__ y,
-                                                      const double *__restrict__ z,
-                                                      const double *__restrict__ m,
-                                                      const int *__restrict__ gid, int n, int per,
-                                                      const FixScratch *sc,
-                                                      double *__restrict__ part)
+__global__ void __launch_bounds__(FT, 6) k_potential(const double *__restrict__ x,
+                                                  const double *__restrict__ y,
+                                                  const double *__restrict__ z,
+                                                  const double *__restrict__ m,
+                                                  const int *__restrict__ gid, int n, int per,
+                                                  PairEps eps, double *__restrict__ part)
 {
-    __shared__ FixBody tile[FT];
+    __shared__ double tx[FT], ty[FT], tz[FT], tm[FT];
     __shared__ int tg[FT];
-    const int row0 = blockIdx.x * PT_ROWS;
-    const int j0 = blockIdx.y * per, j1 = min(n, j0 + per);
-    const FixGrid f = sc->grid;
-    if (!f.ok || j1 <= row0)
-        return;
-    const double scale = ldexp(1.0, f.g);
+    const int row0 = blockIdx.x * PT_ROWS, j0 = blockIdx.y * per, j1 = min(n, j0 + per);
     const int ia = row0 + threadIdx.x, ib = ia + FT;
-    const FixBody a = ia < n ? fix_body(x, y, z, m, ia, scale) : FixBody{0, 0, 0, 0ull};
-    const FixBody b = ib < n ? fix_body(x, y, z, m, ib, scale) : FixBody{0, 0, 0, 0ull};
+    const double xa = ia < n ? x[ia] : 0.0, ya = ia < n ? y[ia] : 0.0, za = ia < n ? z[ia] : 0.0;
+    const double xb = ib < n ? x[ib] : 0.0, yb = ib < n ? y[ib] : 0.0, zb = ib < n ? z[ib] : 0.0;
     const int ga = (MULTI && ia < n) ? gid[ia] : 0, gb = (MULTI && ib < n) ? gid[ib] : 0;
-    FixSum1 sa, sb;
-    sa.a.clear();
-    sb.a.clear();
+    double sa = 0.0, sb = 0.0;
     for (int t = max(j0, row0); t < j1; t += FT) {
         const int j = t + threadIdx.x;
         __syncthreads();
         if (j < j1) {
-            tile[threadIdx.x] = fix_body(x, y, z, m, j, scale);
+            tx[threadIdx.x] = x[j];
+            ty[threadIdx.x] = y[j];
+            tz[threadIdx.x] = z[j];
+            tm[threadIdx.x] = (m[j] > 0.0) ? m[j] : 0.0;
             if (MULTI)
                 tg[threadIdx.x] = gid[j];
         }
         __syncthreads();
         const int cnt = min(FT, j1 - t);
         for (int q = 0; q < cnt; q++) {
-            const FixBody c = tile[q];
             const bool ta = t + q > ia && (!MULTI || tg[q] == ga),
                        tb = t + q > ib && (!MULTI || tg[q] == gb);
-            sa.add(f, c.x - a.x, c.y - a.y, c.z - a.z, ta ? c.m : 0ull);
-            sb.add(f, c.x - b.x, c.y - b.y, c.z - b.z, tb ? c.m : 0ull);
+            const double va = pair_inv_r(eps, tx[q] - xa, ty[q] - ya, tz[q] - za);
+            const double vb = pair_inv_r(eps, tx[q] - xb, ty[q] - yb, tz[q] - zb);
+            sa = fma(tm[q], ta ? va : 0.0, sa);
+            sb = fma(tm[q], tb ? vb : 0.0, sb);
         }
     }
-    double *p = part + (size_t)blockIdx.y * n;
-    if (ia < n)
-        p[ia] = sa.a.value(f.U1);
-    if (ib < n)
-        p[ib] = sb.a.value(f.U1);
-}
-
-__global__ void k_potential_sum(const double *__restrict__ part, const double *__restrict__ m,
-                                int n, int per, double G, const FixScratch *sc,
-                                double *__restrict__ row)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !sc->grid.ok)
-        return;
-    double s = 0.0;
-    for (int c = (i / PT_ROWS) * PT_ROWS / per; (long long)c * per < n; c++)
-        s += part[(size_t)c * n + i];
-    row[i] = -G * (m[i] > 0.0 ? m[i] : 0.0) * s;
-}
-
-// The same in FP64, for bodies off the grid: row i against columns j > i, rows
-// split over blocks; each thread writes its row sum, reduced afterwards.
-__global__ void __launch_bounds__(DT) k_potential_rows(const double *__restrict__ x,
-                                                       const double *__restrict__ y,
-                                                       const double *__restrict__ z,
-                                                       const double *__restrict__ m,
-                                                       const int *__restrict__ gid, int n,
-                                                       double G, double eps2,
-                                                       const FixScratch *sc,
-                                                       double *__restrict__ row)
-{
-    __shared__ double sx[DT], sy[DT], sz[DT], sm[DT];
-    __shared__ int sg[DT];
-    if (sc->grid.ok) // k_potential_fix's
-        return;
-    const int i = blockIdx.x * DT + threadIdx.x;
-    const double xi = (i < n) ? x[i] : 0.0, yi = (i < n) ? y[i] : 0.0, zi = (i < n) ? z[i] : 0.0;
-    const int gi = (i < n) ? gid[i] : -1;
-    const double mi = (i < n && m[i] > 0.0) ? m[i] : 0.0;
-    double pe = 0.0;
-    const int jstart = blockIdx.x * DT; // columns from the block's first row
-    for (int t = jstart; t < n; t += DT) {
-        const int j = t + threadIdx.x;
+    // the block's rows, added in a fixed order
+    __syncthreads();
+    const double ma = (ia < n && m[ia] > 0.0) ? m[ia] : 0.0, mb = (ib < n && m[ib] > 0.0) ? m[ib] : 0.0;
+    tx[threadIdx.x] = ma * sa + mb * sb;
+    __syncthreads();
+    for (int s = FT / 2; s > 0; s >>= 1) {
+        if (threadIdx.x < s)
+            tx[threadIdx.x] += tx[threadIdx.x + s];
         __syncthreads();
-        if (j < n) {
-            sx[threadIdx.x] = x[j];
-            sy[threadIdx.x] = y[j];
-            sz[threadIdx.x] = z[j];
-            sm[threadIdx.x] = (m[j] > 0.0) ? m[j] : 0.0;
-            sg[threadIdx.x] = gid[j];
-        }
-        __syncthreads();
-        const int cnt = min(DT, n - t);
-        if (i < n) {
-            for (int q = 0; q < cnt; q++) {
-                if (t + q <= i || sg[q] != gi)
-                    continue;
-                const double dx = sx[q] - xi, dy = sy[q] - yi, dz = sz[q] - zi;
-                const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-                pe = fma(-sm[q], inv_r(r2), pe);
-            }
-        }
     }
-    if (i < n)
-        row[i] = G * mi * pe;
+    if (threadIdx.x == 0)
+        part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = tx[0];
 }
 
-__global__ void k_energy_reduce(const double *__restrict__ row, const double *__restrict__ m,
-                                const double *__restrict__ vx, const double *__restrict__ vy,
-                                const double *__restrict__ vz, int n, double *__restrict__ out)
+__global__ void k_energy_reduce(const double *__restrict__ part, int parts, double G,
+                                const double *__restrict__ m, const double *__restrict__ vx,
+                                const double *__restrict__ vy, const double *__restrict__ vz, int n,
+                                double *__restrict__ out)
 {
     // one block; fixed-order tree reduction in shared memory
     __shared__ double ske[1024], spe[1024];
@@ -348,8 +277,9 @@ __global__ void k_energy_reduce(const double *__restrict__ row, const double *__
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         double mm = (m[i] > 0.0) ? m[i] : 0.0;
         ke += 0.5 * mm * (vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i]);
-        pe += row[i];
     }
+    for (int i = threadIdx.x; i < parts; i += blockDim.x)
+        pe += part[i];
     ske[threadIdx.x] = ke;
     spe[threadIdx.x] = pe;
     __syncthreads();
@@ -362,7 +292,7 @@ __global__ void k_energy_reduce(const double *__restrict__ row, const double *__
     }
     if (threadIdx.x == 0) {
         out[0] = ske[0];
-        out[1] = spe[0];
+        out[1] = -G * spe[0];
     }
 }
 
@@ -443,33 +373,28 @@ extern "C" int csgd_energy(csgd_t *d, double G, double softening, double *ke, do
     // columns a chunk: at least 2048, at most 32 chunks (their partial sums)
     const int per = n / 32 > 2048 ? (n + 31) / 32 : 2048;
     const int chunks = (n + per - 1) / per;
-    void *mem = nullptr;
-    if (csgd_malloc(&mem, sizeof(double) * ((size_t)n * (chunks + 1) + 2) + sizeof(FixScratch)) !=
-        cudaSuccess) {
+    const dim3 grid((n + PT_ROWS - 1) / PT_ROWS, chunks);
+    const int parts = (int)grid.x * chunks;
+    double *part = nullptr;
+    if (csgd_malloc((void **)&part, sizeof(double) * ((size_t)parts + 2)) != cudaSuccess) {
         cudaGetLastError();
         return CSG_ERR_NOMEM;
     }
-    double *part = (double *)mem, *row = part + (size_t)n * chunks, *out = row + n;
-    FixScratch *sc = (FixScratch *)(out + 2);
+    double *out = part + parts;
     cudaStream_t s = d->stream;
-    cudaMemsetAsync(sc, 0, sizeof(FixScratch), s);
-    const double eps2 = softening * softening;
-    { k_fix_grid<<<grid_blocks(n, d->num_sms), DT, 0, s>>>(d->x, d->y, d->z, d->m, n, softening, eps2, sc); d->launches++; }
-    const dim3 gf((n + PT_ROWS - 1) / PT_ROWS, chunks);
+    const PairEps eps = pair_eps(softening);
     if (d->n_gal > 1)
-        k_potential_fix<true><<<gf, FT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, n, per, sc, part);
+        k_potential<true><<<grid, FT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, n, per, eps, part);
     else
-        k_potential_fix<false><<<gf, FT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, n, per, sc, part);
+        k_potential<false><<<grid, FT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, n, per, eps, part);
     d->launches++;
-    { k_potential_sum<<<csgd_grid(n, 256), 256, 0, s>>>(part, d->m, n, per, G, sc, row); d->launches++; }
-    { k_potential_rows<<<csgd_grid(n, DT), DT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, n, G, eps2, sc, row); d->launches++; }
-    { k_energy_reduce<<<1, 1024, 0, s>>>(row, d->m, d->vx, d->vy, d->vz, n, out); d->launches++; }
+    { k_energy_reduce<<<1, 1024, 0, s>>>(part, parts, G, d->m, d->vx, d->vy, d->vz, n, out); d->launches++; }
     double h[2] = {0.0, 0.0};
     cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, s);
     const int rc = csgd_sync(d);
     *ke = h[0];
     *pe = h[1];
-    cudaFree(mem);
+    cudaFree(part);
     return rc;
 }
 

@@ -36,6 +36,7 @@
 #pragma once
 
 #include <math.h>
+#include <string.h>
 
 #include "dev_internal.cuh"
 
@@ -188,6 +189,131 @@ __device__ __forceinline__ unsigned fix_e2(long long e57)
 {
     const int eh = (int)(e57 >> 6);
     return (unsigned)(mulws(eh, eh) >> 32);
+}
+
+// ---- terms from FP64 differences ------------------------------------------
+//
+// 1/r and m/r^3 for FP64 differences dx, dy, dz and eps^2, with no FP64 operation:
+// r^2 is summed from the differences' significands, shifted right to the largest
+// one's exponent (or eps's), its top bit then at 61, and kept to 2^-56 relative; 1/r
+// from an FP32 rsqrt seed y0 and a series in e = 1 - r^2 y0^2 (one high-word
+// product, |e| < 2^-20: y0 (1 + e/2 + 3/8 e^2), y0^3 (1 + 3/2 e + 15/8 e^2), the next
+// term below 2^-59), every product keeping its high 64 bits; the result is rounded
+// once and packed. So a term is within 1.1 x 2^-53 of the exact function of its
+// differences, where FP64 operations round r^2 three times more. Differences and
+// sums stay FP64: a fixed-point grid for the positions or the sums would lose the
+// bits of bodies much closer to the origin, or much lighter, than the system's
+// largest.
+
+// eps^2 as the pair terms take it.
+struct PairEps {
+    unsigned long long e2n; // significand, top bit at 61 (0 for eps = 0)
+    int e2s;                // biased exponent + 1020: r2 gets e2n >> (2 er - e2s)
+    unsigned eh;            // high word of |eps|
+    double eps2;
+};
+
+// eps^2 zero while eps is not, subnormal or infinite: an exponent of 2047 takes
+// every pair to the plain expression.
+__host__ __device__ inline PairEps pair_eps(double eps)
+{
+    PairEps p;
+    p.eps2 = eps * eps;
+    unsigned long long b, c;
+    const double a = fabs(eps);
+    memcpy(&b, &p.eps2, sizeof(b));
+    memcpy(&c, &a, sizeof(c));
+    const int eb = (int)(b >> 52);
+    p.eh = (unsigned)(c >> 32);
+    p.e2n = 0ull;
+    p.e2s = 0;
+    if (eb > 0 && eb < 2047) {
+        p.e2n = ((b & 0xfffffffffffffull) | (1ull << 52)) << 9;
+        p.e2s = eb + 1020;
+    } else if (!(eps == 0.0)) {
+        p.eh = 0x7ff00000u;
+    }
+    return p;
+}
+
+// r^2 = r2 2^(2 (er - 1023) - 58), r2 in [2^58, 2^62], and its seed.
+struct PairR {
+    unsigned long long S; // Y^2
+    long long e57;        // (1 - r^2 y0^2) 2^57
+    unsigned Y;           // y0 = Y 2^(ey - 158), seed of (r2 2^-32)^(-1/2)
+    int ey, er;           // er: the largest difference's (or eps's) biased exponent
+};
+
+__device__ __forceinline__ unsigned long long pair_word(double d, int er)
+{
+    const unsigned h = (unsigned)__double2hiint(d), l = (unsigned)__double2loint(d);
+    const unsigned top = (h & 0xfffffu) | 0x100000u; // a subnormal's shifts out
+    const unsigned long long v = ((unsigned long long)__funnelshift_l(l, top, 9) << 32) | (l << 9);
+    return shr_clamp(v, (unsigned)(er - (int)(h >> 20 & 0x7ffu)));
+}
+
+__device__ __forceinline__ PairR pair_r(const PairEps &p, double dx, double dy, double dz)
+{
+    PairR r;
+    const unsigned M = 0x7fffffffu;
+    r.er = (int)(max(max((unsigned)__double2hiint(dx) & M, (unsigned)__double2hiint(dy) & M),
+                     max((unsigned)__double2hiint(dz) & M, p.eh)) >> 20);
+    const unsigned long long x = pair_word(dx, r.er), y = pair_word(dy, r.er),
+                             z = pair_word(dz, r.er);
+    // the words are below 2^62; the dropped low products are 1 on average
+    const unsigned long long hh = mulw(hi32(x), hi32(x)) + mulw(hi32(y), hi32(y)) +
+                                  mulw(hi32(z), hi32(z));
+    const unsigned long long hl = mulw(hi32(x), (unsigned)x) + mulw(hi32(y), (unsigned)y) +
+                                  mulw(hi32(z), (unsigned)z);
+    const unsigned long long r2 =
+        hh + (hl >> 31) + shr_clamp(p.e2n, (unsigned)(2 * r.er - p.e2s)) + 1ull;
+    float s;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(__uint2float_rz(hi32(r2))));
+    const unsigned sb = __float_as_uint(s);
+    r.ey = (int)(sb >> 23); // 111..114
+    r.Y = (sb << 8) | 0x80000000u;
+    r.S = mulw(r.Y, r.Y);
+    // r2 S 2^-63 = (1 - e) 2^(285 - 2 ey)
+    const unsigned long long T = mulhi(r2 << 1, r.S);
+    const int k = 285 - 2 * r.ey; // 57..63
+    r.e57 = (long long)((1ull << k) - T) >> (k - 57);
+    return r;
+}
+
+// F 2^(E - 1086) rounded to nearest, for F > 0; E is then the result's biased
+// exponent plus the leading zeros of F. Returned as bits, the exponent in E.
+__device__ __forceinline__ double pair_pack(unsigned long long F, int &E)
+{
+    const int lz = __clz((int)hi32(F)); // the callers' F are above 2^58
+    const unsigned hi = __funnelshift_l((unsigned)F, hi32(F), lz), lo = (unsigned)F << lz;
+    E -= lz;
+    const unsigned long long v =
+        ((unsigned long long)(((unsigned)(E - 1) << 20) + (hi >> 11)) << 32) |
+        __funnelshift_r(lo, hi, 11);
+    return __longlong_as_double((long long)(v + (lo >> 10 & 1u)));
+}
+
+static __device__ __noinline__ double pair_plain_1(double dx, double dy, double dz, double eps2)
+{
+    return 1.0 / sqrt(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
+}
+
+// (dx^2 + dy^2 + dz^2 + eps^2)^(-1/2); the plain expression where an exponent
+// would leave FP64's normal range.
+__device__ __forceinline__ double pair_inv_r(const PairEps &p, double dx, double dy, double dz)
+{
+    const PairR r = pair_r(p, dx, dy, dz);
+    const int q = (int)(((fix_e2(r.e57) >> 4) * 3u) >> 12); // 3/8 e^2 2^57
+    const long long c57 = (r.e57 >> 1) + q;
+    const unsigned long long C = (1ull << 63) + (unsigned long long)(c57 << 6); // (1 + c) 2^63
+    const unsigned long long V = mulw(r.Y, hi32(C)) + hi32(mulw(r.Y, (unsigned)C));
+    int E = r.ey - r.er + 1933; // V = Y (1 + c) 2^31, 1/r = V 2^(ey - er + 847)
+    const double v = pair_pack(V, E);
+    // er is 0 where all are zero, 2047 for infinities and NaN; above 64 a
+    // subnormal difference does not count
+    return (unsigned)(r.er - 65) < 1980u && (unsigned)(E - 1) < 2045u
+               ? v
+               : pair_plain_1(dx, dy, dz, p.eps2);
 }
 
 // 128-bit sum, words from the lowest.
