@@ -5,9 +5,6 @@
 // energy KE + softened PE (tests/test_physics.c:34-52), both in FP64. The
 // j range is split over blocks; each block writes its partial sums and a
 // second kernel adds them in a fixed order, so results are deterministic.
-// The direct sum runs on the integer pipes (dev_fixpair.cuh) when the bodies fit its
-// grid, which a first kernel finds on the device; the FP64 kernel is queued
-// beside it and returns at once then (4096 of 100k bodies: 20.0 -> 4.0 ms).
 //
 // The probes time long independent FMA chains (8 per thread) and report the
 // FP32 and FP64 CUDA-core throughput of this GPU: the denominators for the
@@ -20,130 +17,25 @@ namespace {
 
 constexpr int DT = 256;       // threads per block
 constexpr int JCHUNKS = 64;   // j-range splits for the direct sum
-constexpr int FT = 128;       // threads per block of the sums on the integer pipes
+constexpr int FT = 128;       // threads per block of the energy
 
-// The bodies' grid: largest |coordinate| (dead bodies too: they may be sampled)
-// and mass of the live bodies, turned into the grid by the last block to
-// finish. The scratch is zero before the launch. A NaN orders above every
-// number: it ends in a grid with ok = 0.
-struct FixScratch {
-    unsigned long long xmax, mmax; // bit patterns of non-negative doubles
-    unsigned done;
-    FixGrid grid;
-};
-
-__global__ void __launch_bounds__(DT) k_fix_grid(const double *__restrict__ x,
-                                                 const double *__restrict__ y,
-                                                 const double *__restrict__ z,
-                                                 const double *__restrict__ m, int n, double eps,
-                                                 double eps2, FixScratch *s)
-{
-    unsigned long long xm = 0ull, mm = 0ull;
-    for (int i = blockIdx.x * DT + threadIdx.x; i < n; i += gridDim.x * DT) {
-        const unsigned long long a = (unsigned long long)__double_as_longlong(fabs(x[i])),
-                                 b = (unsigned long long)__double_as_longlong(fabs(y[i])),
-                                 c = (unsigned long long)__double_as_longlong(fabs(z[i]));
-        xm = max(xm, max(a, max(b, c)));
-        if (!(m[i] <= 0.0))
-            mm = max(mm, (unsigned long long)__double_as_longlong(fabs(m[i])));
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        xm = max(xm, __shfl_xor_sync(0xffffffffu, xm, o));
-        mm = max(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(&s->xmax, xm);
-        atomicMax(&s->mmax, mm);
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x != 0 || atomicAdd(&s->done, 1u) != gridDim.x - 1)
-        return;
-    __threadfence();
-    s->grid = fix_grid(__longlong_as_double((long long)__ldcg(&s->xmax)),
-                       __longlong_as_double((long long)__ldcg(&s->mmax)), (double)n, eps, eps2);
-}
-
-__device__ __forceinline__ FixBody fix_body(const double *x, const double *y, const double *z,
-                                            const double *m, int j, double scale)
-{
-    return FixBody{fix_pos(x[j], scale), fix_pos(y[j], scale), fix_pos(z[j], scale),
-                   fix_mass(m[j])};
-}
-
-// Direct sum of sample idx[k] over bodies of its system, chunk blockIdx.y of
-// `chunks` of the bodies, on the integer pipes: about 240 instructions a pair
-// and no FP64 operation (the FP64 kernel below: a square root, a division and
-// 16 more). A body's own term is zero (its differences are). A sample index
-// outside [0, n) reads nothing; its row becomes NaN.
-template <bool MULTI>
-__global__ void __launch_bounds__(FT, 5) k_direct_fix(const double *__restrict__ x,
-                                                   const double *__restrict__ y,
-                                                   const double *__restrict__ z,
-                                                   const double *__restrict__ m,
-                                                   const int *__restrict__ gid, int n,
-                                                   const int *__restrict__ idx, int ns, double G,
-                                                   int chunks, const FixScratch *sc,
-                                                   double *__restrict__ part)
-{
-    __shared__ FixBody tile[FT];
-    __shared__ int tg[FT];
-    const FixGrid f = sc->grid;
-    if (!f.ok)
-        return;
-    const double scale = ldexp(1.0, f.g);
-    const int k = blockIdx.x * FT + threadIdx.x;
-    const int per = (n + chunks - 1) / chunks;
-    const int j0 = blockIdx.y * per, j1 = min(n, j0 + per);
-    const int i = k < ns ? idx[k] : -1;
-    const bool valid = (unsigned)i < (unsigned)n;
-    const long long xi = valid ? fix_pos(x[i], scale) : 0, yi = valid ? fix_pos(y[i], scale) : 0,
-                    zi = valid ? fix_pos(z[i], scale) : 0;
-    const int gi = (MULTI && valid) ? gid[i] : 0;
-    Fix128 ax, ay, az;
-    ax.clear();
-    ay.clear();
-    az.clear();
-    for (int t = j0; t < j1; t += FT) {
-        const int j = t + threadIdx.x;
-        __syncthreads();
-        if (j < j1) {
-            tile[threadIdx.x] = fix_body(x, y, z, m, j, scale);
-            if (MULTI)
-                tg[threadIdx.x] = gid[j];
-        }
-        __syncthreads();
-        const int cnt = min(FT, j1 - t);
-        for (int q = 0; q < cnt; q++) {
-            const FixBody b = tile[q];
-            if (MULTI && tg[q] != gi)
-                continue;
-            fix_add3(f, b.x - xi, b.y - yi, b.z - zi, b.m, ax, ay, az);
-        }
-    }
-    if (k < ns) {
-        double *p = part + ((size_t)blockIdx.y * ns + k) * 3;
-        const double nan = __longlong_as_double(0x7ff8000000000000ll);
-        p[0] = valid ? G * ax.value(f.U3) : nan;
-        p[1] = valid ? G * ay.value(f.U3) : nan;
-        p[2] = valid ? G * az.value(f.U3) : nan;
-    }
-}
-
+// Direct sum of sample idx[k] over bodies of its system, chunk blockIdx.y of `chunks`
+// of the bodies: the reference's expression in FP64 throughout, its square root and
+// its division correctly rounded on the integer pipes (dev_fpint.cuh), so with the
+// compiler's operators' bits. It shares nothing with the walks' pair terms, which it
+// checks. Bound by the FP64 pipe: 12 operations a pair (28 with the compiler's
+// operators; 4096 of 100k bodies: 9.8 ms against 20.0).
 __global__ void __launch_bounds__(DT) k_direct(const double *__restrict__ x,
                                                const double *__restrict__ y,
                                                const double *__restrict__ z,
                                                const double *__restrict__ m,
                                                const int *__restrict__ gid, int n,
                                                const int *__restrict__ idx, int ns, double G,
-                                               double eps2, int chunks, const FixScratch *sc,
+                                               double eps2, int chunks,
                                                double *__restrict__ part)
 {
-    __shared__ double sx[DT], sy[DT], sz[DT], sm[DT];
+    __shared__ double sx[DT], sy[DT], sz[DT], sgm[DT];
     __shared__ int sg[DT];
-    if (sc->grid.ok) // k_direct_fix's
-        return;
     const int k = blockIdx.x * DT + threadIdx.x;
     const int chunk = blockIdx.y;
     const int per = (n + chunks - 1) / chunks;
@@ -161,7 +53,7 @@ __global__ void __launch_bounds__(DT) k_direct(const double *__restrict__ x,
             sx[threadIdx.x] = x[j];
             sy[threadIdx.x] = y[j];
             sz[threadIdx.x] = z[j];
-            sm[threadIdx.x] = (m[j] <= 0.0) ? 0.0 : m[j];
+            sgm[threadIdx.x] = G * ((m[j] <= 0.0) ? 0.0 : m[j]);
             sg[threadIdx.x] = gid ? gid[j] : 0;
         }
         __syncthreads();
@@ -172,8 +64,8 @@ __global__ void __launch_bounds__(DT) k_direct(const double *__restrict__ x,
                     continue;
                 double dx = sx[q] - xi, dy = sy[q] - yi, dz = sz[q] - zi;
                 double r2 = dx * dx + dy * dy + dz * dz + eps2;
-                double inv = 1.0 / (r2 * sqrt(r2));
-                double f = G * sm[q] * inv;
+                double inv = div_rn(1.0, r2 * sqrt_rn(r2));
+                double f = sgm[q] * inv;
                 ax += f * dx;
                 ay += f * dy;
                 az += f * dz;
@@ -316,13 +208,6 @@ __global__ void k_fma_probe(T *out, int iters, T a, T b)
 
 } // namespace
 
-// Blocks of the grid's bounds pass: a few per SM, each striding over the bodies.
-static int grid_blocks(int n, int sms)
-{
-    const int g = csgd_grid(n, DT);
-    return g < 4 * sms ? g : 4 * sms;
-}
-
 extern "C" int csgd_direct_forces(csgd_t *d, const int *host_idx, int ns, double G,
                                   double softening, double *host_out)
 {
@@ -333,33 +218,24 @@ extern "C" int csgd_direct_forces(csgd_t *d, const int *host_idx, int ns, double
     for (int k = 0; k < ns; k++)
         if (host_idx[k] < 0 || host_idx[k] >= d->n)
             return CSG_ERR_BAD_ARG;
-    // one allocation: partial sums, result, grid scratch, sample
+    // one allocation: partial sums, result, sample
     const size_t doubles = 3 * (size_t)ns * (JCHUNKS + 1);
-    void *mem = nullptr;
-    if (csgd_malloc(&mem, sizeof(double) * doubles + sizeof(FixScratch) +
-                              sizeof(int) * (size_t)ns) != cudaSuccess) {
+    double *part = nullptr;
+    if (csgd_malloc((void **)&part, sizeof(double) * doubles + sizeof(int) * (size_t)ns) !=
+        cudaSuccess) {
         cudaGetLastError();
         return CSG_ERR_NOMEM;
     }
-    double *part = (double *)mem, *out = part + 3 * (size_t)ns * JCHUNKS;
-    FixScratch *sc = (FixScratch *)(part + doubles);
-    int *didx = (int *)(sc + 1);
+    double *out = part + 3 * (size_t)ns * JCHUNKS;
+    int *didx = (int *)(part + doubles);
     cudaStream_t s = d->stream;
     cudaMemcpyAsync(didx, host_idx, sizeof(int) * (size_t)ns, cudaMemcpyHostToDevice, s);
-    cudaMemsetAsync(sc, 0, sizeof(FixScratch), s);
-    const double eps2 = softening * softening;
-    { k_fix_grid<<<grid_blocks(d->n, d->num_sms), DT, 0, s>>>(d->x, d->y, d->z, d->m, d->n, softening, eps2, sc); d->launches++; }
-    const dim3 gf((ns + FT - 1) / FT, JCHUNKS), gd((ns + DT - 1) / DT, JCHUNKS);
-    if (d->n_gal > 1)
-        k_direct_fix<true><<<gf, FT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, d->n, didx, ns, G, JCHUNKS, sc, part);
-    else
-        k_direct_fix<false><<<gf, FT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, d->n, didx, ns, G, JCHUNKS, sc, part);
-    d->launches++;
-    { k_direct<<<gd, DT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, d->n, didx, ns, G, eps2, JCHUNKS, sc, part); d->launches++; }
+    const dim3 grid((ns + DT - 1) / DT, JCHUNKS);
+    { k_direct<<<grid, DT, 0, s>>>(d->x, d->y, d->z, d->m, d->gid, d->n, didx, ns, G, softening * softening, JCHUNKS, part); d->launches++; }
     { k_direct_sum<<<csgd_grid(ns, 256), 256, 0, s>>>(part, JCHUNKS, ns, out); d->launches++; }
     cudaMemcpyAsync(host_out, out, sizeof(double) * 3 * (size_t)ns, cudaMemcpyDeviceToHost, s);
     const int rc = csgd_sync(d);
-    cudaFree(mem);
+    cudaFree(part);
     return rc;
 }
 
@@ -461,24 +337,20 @@ extern "C" CSG_EXPORT int csg_measure_fp_peaks(double *fp32_tflops, double *fp64
 // below instead of cudaMalloc'd memory: 16 chunks x 4096 bodies x 3 doubles =
 // 1.5 MiB, held by every GPU that loads the library until the process exits.
 // All calls share that array, so calls that overlap on the GPU race; every
-// call clears the grid's scratch and overwrites each partial it later reads.
+// call overwrites each partial it later reads, so nothing needs clearing.
 
 constexpr int NOALLOC_CHUNKS = 16;
 constexpr int NOALLOC_MAX_SAMPLE = 4096;
 constexpr int NOALLOC_MAX_DEVICES = 64;
 
-struct NoallocScratch {
-    double partials[NOALLOC_CHUNKS * NOALLOC_MAX_SAMPLE * 3];
-    FixScratch grid;
-};
-static __device__ __align__(256) NoallocScratch g_noalloc;
+static __device__ __align__(256) double g_noalloc_partials[NOALLOC_CHUNKS * NOALLOC_MAX_SAMPLE * 3];
 
 #include <mutex>
 
 namespace {
 
 std::mutex g_noalloc_mutex;
-NoallocScratch *g_noalloc_ptr[NOALLOC_MAX_DEVICES];
+double *g_noalloc_ptr[NOALLOC_MAX_DEVICES];
 
 } // namespace
 
@@ -488,7 +360,7 @@ NoallocScratch *g_noalloc_ptr[NOALLOC_MAX_DEVICES];
 // device's primary context: after a cudaDeviceReset the cached address is
 // stale, so a process that resets a device must not call the entry point on
 // it again.
-static int noalloc_scratch(NoallocScratch **ptr)
+static int noalloc_scratch(double **ptr)
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= NOALLOC_MAX_DEVICES) {
@@ -498,11 +370,11 @@ static int noalloc_scratch(NoallocScratch **ptr)
     std::lock_guard<std::mutex> lock(g_noalloc_mutex);
     if (!g_noalloc_ptr[dev]) {
         void *p = nullptr;
-        if (cudaGetSymbolAddress(&p, g_noalloc) != cudaSuccess || !p) {
+        if (cudaGetSymbolAddress(&p, g_noalloc_partials) != cudaSuccess || !p) {
             cudaGetLastError();
             return CSG_ERR_CUDA;
         }
-        g_noalloc_ptr[dev] = (NoallocScratch *)p;
+        g_noalloc_ptr[dev] = (double *)p;
     }
     *ptr = g_noalloc_ptr[dev];
     return CSG_OK;
@@ -520,21 +392,14 @@ extern "C" CSG_EXPORT int csg_direct_forces_noalloc(const double *x, const doubl
         return CSG_OK;
     if (!x || !y || !z || !mass || !idx || !out || n == 0)
         return CSG_ERR_BAD_ARG;
-    NoallocScratch *w = nullptr;
-    int rc = noalloc_scratch(&w);
+    double *part = nullptr;
+    int rc = noalloc_scratch(&part);
     if (rc)
         return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    const double eps2 = softening * softening;
-    cudaMemsetAsync(&w->grid, 0, sizeof(FixScratch), s);
-    k_fix_grid<<<grid_blocks(n, 152), DT, 0, s>>>(x, y, z, mass, n, softening, eps2, &w->grid);
-    const dim3 gf((m + FT - 1) / FT, NOALLOC_CHUNKS), gd((m + DT - 1) / DT, NOALLOC_CHUNKS);
-    if (sys)
-        k_direct_fix<true><<<gf, FT, 0, s>>>(x, y, z, mass, sys, n, idx, m, G, NOALLOC_CHUNKS, &w->grid, w->partials);
-    else
-        k_direct_fix<false><<<gf, FT, 0, s>>>(x, y, z, mass, sys, n, idx, m, G, NOALLOC_CHUNKS, &w->grid, w->partials);
-    k_direct<<<gd, DT, 0, s>>>(x, y, z, mass, sys, n, idx, m, G, eps2, NOALLOC_CHUNKS, &w->grid, w->partials);
-    k_direct_sum<<<(m + 255) / 256, 256, 0, s>>>(w->partials, NOALLOC_CHUNKS, m, out);
+    const dim3 grid((m + DT - 1) / DT, NOALLOC_CHUNKS);
+    k_direct<<<grid, DT, 0, s>>>(x, y, z, mass, sys, n, idx, m, G, softening * softening, NOALLOC_CHUNKS, part);
+    k_direct_sum<<<(m + 255) / 256, 256, 0, s>>>(part, NOALLOC_CHUNKS, m, out);
     if (cudaGetLastError() != cudaSuccess)
         return CSG_ERR_CUDA;
     return CSG_OK;

@@ -1,6 +1,7 @@
-"""Accuracy of the energy where a sum or a difference held in too few bits would show:
-close pairs near the origin of a wide system, a heavy body among light ones, masses
-just below a power of two.
+"""Accuracy of directly summed accelerations, and of the energy, where a sum or a difference
+held in too few bits would show: close pairs near the origin of a wide system, a heavy
+body among light ones, systems of very different masses in one handle, masses just
+below a power of two.
 
 Against extended precision over all pairs (theta 0). Errors are relative to the sum of
 the terms' magnitudes. Bar: n pairs in FP64, each term within 4 roundings (difference,
@@ -58,12 +59,41 @@ def exact(b, eps):
     return acc, mag, pe
 
 
+def errors(got, acc, mag):
+    d = got.astype(LD) - acc
+    return np.sqrt((d * d).sum(1)) / mag
+
+
 def scenes():
     for eps, far in ((0.01, 5.0), (0.01, 40.0), (0.01, 80.0), (0.3, 80.0), (0.01, 2e4), (1e-6, 5.0)):
         for sep in (1e-2, 1e-3, 1e-4, 1e-6):
             yield eps, [near_pair(sep, far, s) for s in range(20)]
     for eps in (1e-2, 1e-3):
         yield eps, [heavy_among_light(s) for s in range(3)]
+
+
+def test_direct_sum(lib):
+    for eps, systems in scenes():
+        for b in systems:
+            s = lib.Sim.from_bodies(b, softening=eps)
+            err = errors(s.direct_forces(np.arange(len(b))), *exact(b, eps)[:2])
+            s.close()
+            assert err.max() <= (len(b) + 8) * U, (eps, float(err.max()))
+
+
+def test_direct_sum_and_energy_of_systems_of_unequal_mass(lib):
+    parts = [near_pair(0.1, 4.0, 1), near_pair(0.1, 4.0, 2), near_pair(0.1, 4.0, 3)]
+    for p, w in zip(parts, (1.0, 1e-25, 1e12)):
+        p["mass"] *= w
+    s = lib.Sim.ensemble(np.concatenate(parts).astype(BODY_DTYPE), [3, 3, 3], softening=0.01)
+    got, (_, pe) = s.direct_forces(np.arange(9)), s.energy()
+    s.close()
+    want = LD(0)
+    for g, p in enumerate(parts):
+        acc, mag, e = exact(p, 0.01)
+        assert errors(got[3 * g:3 * g + 3], acc, mag).max() <= 11 * U, g
+        want += e
+    assert abs(LD(pe) - want) <= 19 * U * abs(want)
 
 
 def test_energy(lib):
