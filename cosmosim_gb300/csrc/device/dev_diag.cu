@@ -24,7 +24,7 @@ constexpr int FT = 128;       // threads per block of the energy
 // its division correctly rounded on the integer pipes (dev_fpint.cuh), so with the
 // compiler's operators' bits. It shares nothing with the walks' pair terms, which it
 // checks. Bound by the FP64 pipe: 12 operations a pair (28 with the compiler's
-// operators; 4096 of 100k bodies: 9.8 ms against 20.0).
+// operators; 4096 of 100k bodies: 9.3 ms against 20.0, the pipe 87% busy).
 __global__ void __launch_bounds__(DT) k_direct(const double *__restrict__ x,
                                                const double *__restrict__ y,
                                                const double *__restrict__ z,
@@ -98,8 +98,8 @@ __global__ void k_direct_sum(const double *__restrict__ part, int chunks, int ns
 
 // Potential energy: rows of 2 FT bodies (two a thread) against a chunk of `per`
 // columns j > i. Differences and sums in FP64, 1/r by integers (pair_inv_r): 4 FP64
-// operations a pair, 256 cycles a warp and scheduler, beside about 150 integer
-// instructions: 37.9 ms at 100k bodies. With the whole 1/r in FP64 (14 operations,
+// operations a pair, 256 cycles a warp and scheduler, beside about 150 on
+// the other pipes: 38.3 ms at 100k bodies, the FP64 pipe 87% busy. With the whole 1/r in FP64 (14 operations,
 // and rows not split) 196 ms; with positions and sums in fixed point 28.3 ms, but the
 // bits of close pairs near the origin lost to the grid. The block's sum of m_i m_j / r goes to part[c gridDim.x + b] (0 for
 // a chunk wholly at or before the rows). The columns are split so that the long

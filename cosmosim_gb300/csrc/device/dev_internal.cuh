@@ -61,24 +61,6 @@ struct __align__(16) NodeLink {
     int count;  // number of bodies in the cell
 };
 
-// Fixed-point grid of a system's positions for the integer pair terms
-// (dev_fixpair.cuh).
-struct FixGrid {
-    int ok;                  // 1: the system fits; 0: use the FP64 pair terms
-    int g;                   // grid: X = x 2^g
-    int far;                 // cells beyond 2^61 units: X = x 2^(g - far) (walks; 0: none)
-    int U3, U1;              // exponent of the last bit of an acceleration, a potential sum
-    unsigned eh;             // high word of eps 2^g
-    int e2s;                 // eps^2 in units of r2 (fix_pair): e2n >> (e2s - 2 s)
-    unsigned long long e2n;  // eps^2's significand, top bit at 61
-};
-
-// A body or cell on the grid.
-struct __align__(16) FixBody {
-    long long x, y, z;
-    unsigned long long m; // fix_mass
-};
-
 // One system of the forest (a single simulation is a forest of one): its
 // alive-body bounding box, root cube, key parameters, where its bodies sit in
 // the sorted order and where its cells sit in the preorder node array.
@@ -98,8 +80,6 @@ struct DevRoot {
     int end;                             // one past the system's last cell
     int split;                           // the cell whose children are the segments (k_tasks)
     int fix_e;                           // every |coordinate| < 2^fix_e
-    int fix_off;                         // a caller's cells do not fit the grid (k_walk_prep)
-    FixGrid fix;                         // of the current FP64 walk (k_walk_prep)
 };
 
 // A walk task: up to 32 consecutive sorted bodies of one system (one warp).
@@ -254,8 +234,6 @@ struct csgd {
     // nodes
     NodeW64 *w64;
     NodeW32 *w32;
-    FixBody *wfix; // the cells on their system's grid (FP64 walks; allocated on first use)
-    int wfix_cap;
     NodeLink *link;
     double4_32a *geo;
     NodeS32 *s32;

@@ -398,8 +398,6 @@ extern "C" void csgd_destroy(csgd_t *d)
         cudaFree(d->qs);
     if (d->wpart)
         cudaFree(d->wpart);
-    if (d->wfix)
-        cudaFree(d->wfix);
     csgd_quasar_free(d);
     if (d->aux) {
         cudaStreamSynchronize(d->aux);
@@ -887,22 +885,6 @@ int csgd_prepare_walk(csgd_t *d, int precision)
     const bool split = precision == CSG_PREC_FP32_MIXED ? csgd_walk_split(d)
                        : precision == CSG_PREC_FP64     ? csgd_sys_min_n(d) <= csgd_split_max_bodies(d, precision, 0.0)
                                                         : false;
-    if (precision == CSG_PREC_FP64 && !(d->wfix && d->wfix_cap >= d->node_cap)) {
-        csgd_drop_graph(d);
-        if (d->wfix) {
-            cudaStreamSynchronize(d->stream);
-            cudaFree(d->wfix);
-        }
-        d->wfix = nullptr;
-        d->wfix_cap = 0;
-        const size_t cells = (size_t)(d->node_cap > 0 ? d->node_cap : 64);
-        if (csgd_malloc((void **)&d->wfix, sizeof(FixBody) * cells) != cudaSuccess) {
-            cudaGetLastError();
-            d->wfix = nullptr;
-            return CSG_ERR_NOMEM;
-        }
-        d->wfix_cap = (int)cells;
-    }
     if (!split || (d->wpart && d->wpart_cap >= d->cap))
         return CSG_OK;
     csgd_drop_graph(d); // a captured walk holds the old pointer

@@ -428,7 +428,6 @@ __global__ void k_root(DevScalars *sc, DevRoot *roots, int n_gal)
         const DevRoot &r = roots[g];
         const double far = fmax(fabs(r.c0[0]), fmax(fabs(r.c0[1]), fabs(r.c0[2]))) + r.hs0;
         roots[g].fix_e = ilogb(far) + 1;
-        roots[g].fix_off = 0;
         roots[g].sum_e = r.mass_e - 1022 + 32 - __clz(max(r.n_alive, 1));
         if (r.n_alive > 0 && (abs(roots[g].sum_e) > 300 || abs(roots[g].fix_e) > 300))
             climb = 1;

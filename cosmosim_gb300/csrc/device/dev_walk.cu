@@ -2,17 +2,17 @@
 //
 // Both walks give every body exactly the reference's interaction set: the
 // cells it accepts by the monopole test (s*s)/d^2 < theta^2 with d^2 > 0, or
-// reaches as leaves other than itself, in depth-first octant order.
+// reaches as leaves other than itself (in the order of the rounds, not the
+// reference's depth-first one).
 //
 // Traversal: one warp walks the tree for 32 bodies that are neighbours in key
 // order, up to 32 cells a round (see "traversal in rounds" below).
 //
 // FP64 walk: the drop-in precision (k_walk64ws). Openings decided as in the
 //   FP32 walk (equal to the reference's FP64 rounding); interactions queued
-//   and evaluated densely by two further warps per task, on the integer pipes
-//   (dev_fixpair.cuh; in FP64 for systems that do not fit their grid and for
-//   bodies far outside it), small systems split by child subtrees as in the
-//   FP32 walk (k_walk64ws_units), with the same bits. k_walk64_exact instead
+//   and evaluated densely by two further warps per task, differences and sums
+//   in FP64 and m/r^3 by integers (dev_fixpair.cuh), small systems split by
+//   child subtrees as in the FP32 walk (k_walk64ws_units). k_walk64_exact instead
 //   uses the reference's own operation sequence per step (1/(r2*sqrt(r2)),
 //   no fused multiply-add) — bit-identical results on the reference's own
 //   tree; used by parity tests. It alone walks cell by cell: one cursor over
@@ -37,13 +37,13 @@ struct WalkArgs {
     const NodeW64 *w64;
     const NodeW32 *w32;
     const int *child; // 8 ids per cell
-    const FixBody *wfix; // cells on their systems' grids, or nullptr: FP64 pair terms
     const WalkTask *tasks;
     const DevRoot *roots;
     DevScalars *sc;
     double *ax, *ay, *az;
     double G, eps2, theta2, t2lo, t2hi;
-    float Gf, eps2f;
+    float eps2f;
+    PairEps eps; // FP64 walk
     // FP32 opening test: accept when s^2 acc_k < d^2, open when s^2 opn_k > d^2
     // (acc_k, opn_k = (1 +- g) / theta^2); in between, |theta^2 d^2 - s^2| is
     // inside the FP32 error band g s^2 and the FP64 test decides
@@ -993,32 +993,21 @@ __global__ void __launch_bounds__(WARPS * CSG_WARP, WALK32_RES / WARPS) k_walk32
         add_hits(a, st);
 }
 
-// FP64 evaluation: accepted cells are queued per lane in shared memory and
-// evaluated in FP64 in batches where every lane has work, in the order they
-// were accepted (the reference's depth-first order). The FP64 pipe then does
-// useful work on (almost) every lane instead of once per traversal step for
-// the few lanes that interact at that step.
-
-// Pair terms of the lane's body with queued cells: the cell's record, the
-// term added to the lane's sum, and the sum as doubles (without G) with the
-// next sum started.
-//
-// FP64, with m/r^3 by integers.
+// Pair terms of the lane's body with queued cells: differences and sums in FP64, m/r^3
+// by integers (pair_m_r3). Every system takes them, whatever its extent, masses and
+// softening.
 struct EvalF64 {
     struct Rec {
         double2 xy, zm;
     };
     const NodeW64 *cells;
-    double eps2, px, py, pz;
-    double s[3];
+    const PairEps eps;
+    double px, py, pz;
+    double s[3]; // without G
 
-    __device__ __forceinline__ EvalF64(const WalkArgs &a, const FixGrid &, int me)
-        : cells(a.w64), eps2(a.eps2), px(me >= 0 ? a.x[me] : 0.0), py(me >= 0 ? a.y[me] : 0.0),
+    __device__ __forceinline__ EvalF64(const WalkArgs &a, int me)
+        : cells(a.w64), eps(a.eps), px(me >= 0 ? a.x[me] : 0.0), py(me >= 0 ? a.y[me] : 0.0),
           pz(me >= 0 ? a.z[me] : 0.0)
-    {
-        clear();
-    }
-    __device__ __forceinline__ void clear()
     {
         s[0] = s[1] = s[2] = 0.0;
     }
@@ -1030,103 +1019,24 @@ struct EvalF64 {
     __device__ __forceinline__ void term(const Rec &r)
     {
         const double dx = r.xy.x - px, dy = r.xy.y - py, dz = r.zm.x - pz;
-        const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-        const double f = r.zm.y == 0.0 ? 0.0 : m_inv_r3_q(r.zm.y, r2);
+        const double f = pair_m_r3(eps, dx, dy, dz, r.zm.y);
         s[0] = fma(f, dx, s[0]);
         s[1] = fma(f, dy, s[1]);
         s[2] = fma(f, dz, s[2]);
     }
     static __device__ __forceinline__ void drop(Rec &r) { r.zm.y = 0.0; }
-    // another warp's sums of the same body (6 words a lane)
-    __device__ __forceinline__ void save(unsigned *o) const
-    {
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            const u64 v = (u64)__double_as_longlong(s[d]);
-            o[(2 * d) * CSG_WARP] = (unsigned)v;
-            o[(2 * d + 1) * CSG_WARP] = (unsigned)(v >> 32);
-        }
-    }
-    __device__ __forceinline__ void join(const unsigned *o)
+    // the other consumer's sums of the same body (3 doubles a lane)
+    __device__ __forceinline__ void save(double *o) const
     {
 #pragma unroll
         for (int d = 0; d < 3; d++)
-            s[d] += __longlong_as_double((long long)(((u64)o[(2 * d + 1) * CSG_WARP] << 32) |
-                                                     o[(2 * d) * CSG_WARP]));
+            o[d * CSG_WARP] = s[d];
     }
-    __device__ __forceinline__ void value(double &x, double &y, double &z) const
+    __device__ __forceinline__ void join(const double *o)
     {
-        x = s[0];
-        y = s[1];
-        z = s[2];
-    }
-};
-
-// Integers from end to end, for systems on the grid. WIDE: some cells are on
-// the coarser grid of far ones, marked by bit 62 of z (no |Z| has it).
-template <bool WIDE>
-struct EvalFix {
-    typedef FixBody Rec;
-    const FixBody *cells;
-    const FixGrid f;
-    long long px, py, pz;
-    Fix96 x, y, z;
-    int cnt; // terms in them
-
-    __device__ __forceinline__ EvalFix(const WalkArgs &a, const FixGrid &g, int me)
-        : cells(a.wfix), f(g)
-    {
-        const double scale = fix_pow2(f.g);
-        px = me >= 0 ? fix_pos(a.x[me], scale) : 0;
-        py = me >= 0 ? fix_pos(a.y[me], scale) : 0;
-        pz = me >= 0 ? fix_pos(a.z[me], scale) : 0;
-        clear();
-    }
-    __device__ __forceinline__ void clear()
-    {
-        x.clear();
-        y.clear();
-        z.clear();
-        cnt = 0;
-    }
-    __device__ __forceinline__ Rec load(int c) const
-    {
-        const longlong2 *w = (const longlong2 *)&cells[c];
-        const longlong2 xy = __ldg(w), zm = __ldg(w + 1);
-        return Rec{xy.x, xy.y, zm.x, (unsigned long long)zm.y};
-    }
-    __device__ __forceinline__ void term(const Rec &r)
-    {
-        if (WIDE) {
-            const int hz = (int)(r.z >> 32), far = (hz >> 30 ^ hz >> 31) & 1, up = far ? f.far : 0;
-            const long long rz = r.z ^ ((long long)far << 62);
-            fix_add3(f, r.x - (px >> up), r.y - (py >> up), rz - (pz >> up), r.m, x, y, z, up);
-        } else {
-            fix_add3(f, r.x - px, r.y - py, r.z - pz, r.m, x, y, z);
-        }
-        cnt -= (int)hi32(r.m) >> 31; // massless ones do not count
-    }
-    static __device__ __forceinline__ void drop(Rec &r) { r.m = 0ull; }
-    // another warp's sums of the same body (10 words a lane)
-    __device__ __forceinline__ void save(unsigned *o) const
-    {
-        const unsigned w[10] = {x.w0, x.w1, x.w2, y.w0, y.w1, y.w2, z.w0, z.w1, z.w2, (unsigned)cnt};
 #pragma unroll
-        for (int k = 0; k < 10; k++)
-            o[k * CSG_WARP] = w[k];
-    }
-    __device__ __forceinline__ void join(const unsigned *o)
-    {
-        x.sum(o[0], o[CSG_WARP], o[2 * CSG_WARP]);
-        y.sum(o[3 * CSG_WARP], o[4 * CSG_WARP], o[5 * CSG_WARP]);
-        z.sum(o[6 * CSG_WARP], o[7 * CSG_WARP], o[8 * CSG_WARP]);
-        cnt += (int)o[9 * CSG_WARP];
-    }
-    __device__ __forceinline__ void value(double &ox, double &oy, double &oz) const
-    {
-        ox = x.value(f.U3, cnt);
-        oy = y.value(f.U3, cnt);
-        oz = z.value(f.U3, cnt);
+        for (int d = 0; d < 3; d++)
+            s[d] += o[d * CSG_WARP];
     }
 };
 
@@ -1149,15 +1059,14 @@ __device__ __forceinline__ void put_partial(const WalkArgs &a, int k, int me, do
 // the task). A unit of the split form is one segment of a task: the subtree of
 // the split cell's child k0 (segment 0: also the cells above the segments).
 //
-// Bound: the integer multiply and ALU pipes (65% and 62% busy at 1M, issue
-// 70%); the walk in FP64 was bound by the FP64 pipe (9 operations a pair).
-// Measured, walk inside the substep, FP64 pairs with a ring of ids per lane and
-// one consumer -> integer pairs -> blocks and two consumers: 1M 39.0 -> 33.0 ->
-// 24.8 ms, 100k merger 2.23 -> 1.97 -> 1.35 ms, 20k disk 0.496 -> 0.448 ->
-// 0.36 ms. Off the grid (FP64 pairs, same queue): 20k 0.48, 100k 2.0, 1M 41 ms.
-// A quasar of 17,000 bodies with some thrown out to 2^15 softening lengths: 1.63
-// ms in FP64, 1.18 with its far cells on a coarser grid, 0.87 with the segments
-// of a deeper split cell.
+// Bound: the FP64 pipe, 6 operations a pair (79% busy in the 100k merger, issue 55%).
+// Measured, walk inside the substep: r^2 in FP64 too (9 operations), a ring of ids
+// per lane and one consumer -> now: 1M 39.0 -> 25.7 ms, 100k merger 2.23 -> 1.41
+// ms, 20k disk 0.496 -> 0.34 ms. With blocks and two consumers but 9 operations 42, 2.0
+// and 0.49 ms. With positions and sums in fixed point, no FP64 operation at all, 24.9,
+// 1.36 and 0.36 ms; a grid of 2^-61 of a system's extent and 96-bit sums lost the
+// bits of close pairs near the origin (up to 6e-11 of the acceleration at 1e-4 softenings)
+// and of a heavy body among light ones.
 //
 // Blocks rather than a ring of ids per lane: an id costs 4 bytes a block, not
 // 4 bytes a lane that takes it, so the same memory holds several times the
@@ -1178,7 +1087,7 @@ struct WsShared {
     int done;            // producer finished (tail final)
     int half;            // the second consumer's sums are in `other`
     int broken;          // a wait gave up: all warps leave
-    unsigned other[10 * CSG_WARP];
+    double other[3 * CSG_WARP];
 };
 
 __device__ __forceinline__ int ws_load(const volatile int *p) { return *p; }
@@ -1288,19 +1197,19 @@ __device__ __forceinline__ int ws_next(const WsShared &sh, WsReader &r, int tail
 constexpr int WS_STEP_TASK = 16, WS_STEP_UNIT = 8;
 
 // Consumer `which`: the blocks which, which + 2, ...
-template <bool UNITS, class Eval>
+template <bool UNITS>
 __device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, const TaskRange &tr,
-                                           const FixGrid &grid, int k0, int which)
+                                           int k0, int which)
 {
     const int lane = threadIdx.x & 31;
     const bool valid = lane < tr.count;
     const int me = valid ? a.perm[tr.pos0 + lane] : -1;
-    Eval ev(a, grid, me);
+    EvalF64 ev(a, me);
     WsReader rd{0u, 0, which};
     int polls = 0, head = which;
     // two cells are always on their way: their loads run during the terms of
-    // the two before them (massless ones at first)
-    typename Eval::Rec ra = ev.load(0), rb = ra;
+    // the two before them (massless ones at first; no cell to read: the root)
+    EvalF64::Rec ra = ev.load(tr.root), rb = ra;
     ev.drop(ra);
     ev.drop(rb);
     while (true) {
@@ -1314,15 +1223,15 @@ __device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, cons
         const int ahead =
             tail - (int)__reduce_max_sync(0xffffffffu, (unsigned)(valid ? rd.next : 0));
         if (ahead >= WS_LOW || tail - head >= WS_BLOCKS || (done && head < tail)) {
-            auto fetch = [&](typename Eval::Rec &r) {
+            auto fetch = [&](EvalF64::Rec &r) {
                 const int c = ws_next(sh, rd, tail, lane);
-                r = ev.load(max(c, 0));
-                if (c < 0) // any cell was read: a massless term
+                r = ev.load(c < 0 ? tr.root : c);
+                if (c < 0)
                     ev.drop(r);
             };
 #pragma unroll 1
             for (int s = 0; s < (UNITS ? WS_STEP_UNIT : WS_STEP_TASK); s += 2) {
-                typename Eval::Rec rc, rq;
+                EvalF64::Rec rc, rq;
                 fetch(rc);
                 fetch(rq);
                 ev.term(ra);
@@ -1357,7 +1266,7 @@ __device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, cons
         }
         __nanosleep(64);
     }
-    // the second consumer's sums joined to the first's (integers: exact)
+    // the second consumer's sums joined to the first's
     if (which == 1) {
         ev.save(sh.other + lane);
         __threadfence_block();
@@ -1381,29 +1290,13 @@ __device__ __forceinline__ void ws_consume(const WalkArgs &a, WsShared &sh, cons
     ev.join(sh.other + lane);
     if (!valid)
         return;
-    double x, y, z;
-    ev.value(x, y, z);
     if (UNITS) { // the segment's partial (zero for one that the walk did not reach)
-        put_partial(a, k0, me, x, y, z);
+        put_partial(a, k0, me, ev.s[0], ev.s[1], ev.s[2]);
     } else {
-        a.ax[me] = a.G * x;
-        a.ay[me] = a.G * y;
-        a.az[me] = a.G * z;
+        a.ax[me] = a.G * ev.s[0];
+        a.ay[me] = a.G * ev.s[1];
+        a.az[me] = a.G * ev.s[2];
     }
-}
-
-// Whether all of the task's bodies are close enough to the origin to meet far
-// cells (within 2^60 units).
-__device__ __forceinline__ bool near_task(const WalkArgs &a, const TaskRange &tr, const FixGrid &f)
-{
-    const int lane = threadIdx.x & 31;
-    bool ok = true;
-    if (lane < tr.count) {
-        const int me = a.perm[tr.pos0 + lane];
-        const double lim = fix_pow2(FIX_POS_BITS - 1 - f.g);
-        ok = fabs(a.x[me]) < lim && fabs(a.y[me]) < lim && fabs(a.z[me]) < lim;
-    }
-    return __all_sync(0xffffffffu, ok);
 }
 
 // One task per block, or (UNITS) one segment of a task, u = 8 task + segment
@@ -1434,7 +1327,6 @@ __device__ __forceinline__ void walk64ws_body(const WalkArgs &a)
             dev_fail(a.sc, CSG_ERR_WALK_LIMIT);
         return;
     }
-    const bool fix = a.wfix && r.fix.ok && !r.fix_off && (r.fix.far == 0 || near_task(a, tr, r.fix));
     if (threadIdx.x == 0) {
         sh.tail = 0;
         sh.head[0] = 0;
@@ -1449,12 +1341,8 @@ __device__ __forceinline__ void walk64ws_body(const WalkArgs &a)
         ws_produce<STATS, UNITS>(a, rs, sh, tr, k0, st);
         if (STATS)
             add_hits(a, st);
-    } else if (fix && r.fix.far == 0) {
-        ws_consume<UNITS, EvalFix<false>>(a, sh, tr, r.fix, k0, warp - 1);
-    } else if (fix) {
-        ws_consume<UNITS, EvalFix<true>>(a, sh, tr, r.fix, k0, warp - 1);
     } else {
-        ws_consume<UNITS, EvalF64>(a, sh, tr, r.fix, k0, warp - 1);
+        ws_consume<UNITS>(a, sh, tr, k0, warp - 1);
     }
 }
 
@@ -1475,76 +1363,18 @@ __global__ void __launch_bounds__((1 + WS_CONS) * CSG_WARP, WS_RES / (1 + WS_CON
 }
 
 // Before a walk: dead bodies get a = 0 (src/octree.c:226-230; alive ones are
-// overwritten by the walk), the task counter of the persistent walks is
-// rewound, and for an FP64 walk (FIX) every system's grid is set up and its
-// cells put on it (ee: |eps| < 2^ee).
-template <bool FIX>
+// overwritten by the walk), and the task counter of the persistent walks is
+// rewound.
 __global__ void k_walk_prep(const double *__restrict__ m, double *ax, double *ay, double *az, int n,
-                            DevScalars *sc, DevRoot *roots, int n_gal,
-                            const NodeW64 *__restrict__ w64, const NodeLink *__restrict__ link,
-                            const int *__restrict__ sgid, const int *__restrict__ child,
-                            FixBody *__restrict__ wfix, int node_cap, double eps, double eps2,
-                            int ee, bool imported)
+                            DevScalars *sc)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0)
         sc->task_next = 0;
-    for (int k = i; k < n; k += stride) {
-        if (m[k] <= 0.0) {
-            ax[k] = 0.0;
-            ay[k] = 0.0;
-            az[k] = 0.0;
-        }
-    }
-    if (!FIX)
-        return;
-    const int nn = sc->n_nodes;
-    if (nn > node_cap)
-        return; // no walk
-    for (int g = i; g < n_gal; g += stride) {
-        DevRoot &r = roots[g];
-        if (r.n_alive > 0) {
-            const double far = fmax(fabs(r.c0[0]), fmax(fabs(r.c0[1]), fabs(r.c0[2]))) + r.hs0;
-            r.fix = fix_grid(far, w64[r.root].m, 1.0, eps, eps2, FIX_FAR_MAX);
-        }
-    }
-    for (int id = i; id < nn; id += stride) {
-        const int e = max(roots[n_gal > 1 ? sgid[link[id].first] : 0].fix_e, ee);
-        const double2 *w = (const double2 *)&w64[id];
-        const double2 xy = w[0], zm = w[1];
-        int far;
-        const int g = fix_scale(e, ee, far);
-        bool out = false;
-        if (far > 0) { // |coordinate| >= 2^61 units, by the exponent
-            const int top = max(max(__double2hiint(xy.x) & 0x7fffffff, __double2hiint(xy.y) & 0x7fffffff),
-                                __double2hiint(zm.x) & 0x7fffffff);
-            out = (top >> 20) - 1023 >= FIX_POS_BITS - g;
-        }
-        const double scale = fix_pow2(min(max(out ? g - far : g, -1000), 1000));
-        longlong2 *o = (longlong2 *)&wfix[id];
-        o[0] = make_longlong2(fix_pos(xy.x, scale), fix_pos(xy.y, scale));
-        o[1] = make_longlong2(fix_pos(zm.x, scale) ^ ((long long)out << 62),
-                              (long long)fix_mass(zm.y));
-        if (!imported)
-            continue;
-        // a caller's cell may lie anywhere and weigh anything: off the grid, or
-        // not the sum of its children (which bounds the sums), and the whole
-        // system keeps the FP64 pair terms
-        const double lim = ldexp(1.0, e);
-        bool good = fabs(xy.x) < lim && fabs(xy.y) < lim && fabs(zm.x) < lim &&
-                    (zm.y == 0.0 || (zm.y >= 0x1p-1000 && zm.y <= 0x1p200));
-        double sum = 0.0;
-        bool any = false;
-        for (int q = 0; q < 8; q++) {
-            const int c = child[8 * (size_t)id + q];
-            if (c > id) {
-                sum += w64[c].m;
-                any = true;
-            }
-        }
-        good = good && (!any || fabs(sum - zm.y) <= 1e-6 * zm.y);
-        if (!good)
-            roots[0].fix_off = 1;
+    if (i < n && m[i] <= 0.0) {
+        ax[i] = 0.0;
+        ay[i] = 0.0;
+        az[i] = 0.0;
     }
 }
 
@@ -1645,7 +1475,6 @@ WalkArgs walk_args(csgd_t *d, const csgd_force_params *p)
     a.w64 = d->w64;
     a.w32 = d->w32;
     a.child = d->child;
-    a.wfix = nullptr;
     a.tasks = d->tasks;
     a.roots = d->roots;
     a.sc = d->sc;
@@ -1658,7 +1487,7 @@ WalkArgs walk_args(csgd_t *d, const csgd_force_params *p)
     a.theta2 = p->theta * p->theta;
     a.t2lo = a.theta2 * (1.0 - 0x1p-50);
     a.t2hi = a.theta2 * (1.0 + 0x1p-50);
-    a.Gf = (float)p->G;
+    a.eps = pair_eps(p->softening);
     // at least the smallest normal number: no sum of squares below 2e-31
     // changes, and under that y^3 of the pair term overflows to inf either way
     a.eps2f = fmaxf((float)a.eps2, 1.17549435e-38f);
@@ -1779,16 +1608,7 @@ extern "C" int csgd_gravity_ex(csgd_t *d, const csgd_force_params *p, int exact)
         if (rc)
             return rc;
     }
-    const bool fix = p->precision == CSG_PREC_FP64 && !exact && d->wfix &&
-                     d->wfix_cap >= d->node_cap;
-    a.wfix = fix ? d->wfix : nullptr;
-    if (fix) {
-        const double e = fabs(p->softening);
-        const int ee = e > 0.0 && isfinite(e) ? ilogb(e) + 1 : -2000;
-        k_walk_prep<true><<<csgd_grid(2LL * n + 64, 256), 256, 0, s>>>(d->m, d->ax, d->ay, d->az, n, d->sc, d->roots, d->n_gal, d->w64, d->link, d->sgid, d->child, d->wfix, d->node_cap, p->softening, a.eps2, ee, d->imported != 0);
-    } else {
-        k_walk_prep<false><<<csgd_grid(n, 256), 256, 0, s>>>(d->m, d->ax, d->ay, d->az, n, d->sc, d->roots, d->n_gal, d->w64, d->link, d->sgid, d->child, nullptr, d->node_cap, 0.0, 0.0, 0, false);
-    }
+    k_walk_prep<<<csgd_grid(n, 256), 256, 0, s>>>(d->m, d->ax, d->ay, d->az, n, d->sc);
     d->launches++;
     if (exact) {
         const int saved = d->walk_warps;

@@ -1,4 +1,4 @@
-"""Accuracy of directly summed accelerations, and of the energy, where a sum or a difference
+"""Accuracy of one body's acceleration, and of the energy, where a sum or a difference
 held in too few bits would show: close pairs near the origin of a wide system, a heavy
 body among light ones, systems of very different masses in one handle, masses just
 below a power of two.
@@ -10,6 +10,7 @@ m/r^3, product), the sums in any order within one a term: (n + 8) 2^-53.
 import numpy as np
 import pytest
 
+from conftest import fields
 from cosmosim_gb300.abi import BODY_DTYPE
 
 pytestmark = pytest.mark.gpu
@@ -70,6 +71,15 @@ def scenes():
             yield eps, [near_pair(sep, far, s) for s in range(20)]
     for eps in (1e-2, 1e-3):
         yield eps, [heavy_among_light(s) for s in range(3)]
+
+
+def test_walk(lib):
+    for eps, systems in scenes():
+        for b in systems:
+            s = lib.Sim.from_bodies(b, softening=eps, theta=0.0, precision=0)
+            err = errors(fields(s.bodies()), *exact(b, eps)[:2])
+            s.close()
+            assert err.max() <= (len(b) + 8) * U, (eps, float(err.max()))
 
 
 def test_direct_sum(lib):
