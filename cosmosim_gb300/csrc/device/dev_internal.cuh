@@ -79,7 +79,8 @@ struct DevRoot {
     int root;                            // preorder id of the root cell
     int end;                             // one past the system's last cell
     int split;                           // the cell whose children are the segments (k_tasks)
-    int fix_e;                           // every |coordinate| < 2^fix_e
+    int pos_e;                           // every |coordinate| < 2^pos_e
+    int climb;                           // its cell sums are formed in FP64 (k_mom_sums)
 };
 
 // A walk task: up to 32 consecutive sorted bodies of one system (one warp).
@@ -97,8 +98,7 @@ struct DevScalars {
     int err;                             // first device error code (0 = none)
     int n_gas;
     int mom_tiles;     // tiles that are summed (k_mom_sums)
-    int mom_light;     // a body is too light for the fixed-point cell sums
-    int mom_climb;     // the build's cell sums do not fit 128-bit fixed point
+    int mom_climb;     // some system's cell sums are formed in FP64
     unsigned long long interactions;     // walk statistics (when enabled)
     unsigned long long walk_steps;       // warp traversal steps
     unsigned long long walk_active;      // lane-steps of lanes still walking

@@ -143,7 +143,6 @@ __global__ void k_reset(DevScalars *sc, DevRoot *roots, int n_gal)
     if (threadIdx.x == 0) {
         sc->n_alive = 0;
         sc->mom_tiles = 0;
-        sc->mom_light = 0;
         sc->deep = 0;
         sc->n_gas = 0;
         sc->key_slow = 0;
@@ -427,9 +426,11 @@ __global__ void k_root(DevScalars *sc, DevRoot *roots, int n_gal)
         root_cube(&roots[g]);
         const DevRoot &r = roots[g];
         const double far = fmax(fabs(r.c0[0]), fmax(fabs(r.c0[1]), fabs(r.c0[2]))) + r.hs0;
-        roots[g].fix_e = ilogb(far) + 1;
+        const bool fits = far >= 0x1p-300 && far <= 0x1p300;
+        roots[g].pos_e = fits ? ilogb(far) + 1 : 0;
         roots[g].sum_e = r.mass_e - 1022 + 32 - __clz(max(r.n_alive, 1));
-        if (r.n_alive > 0 && (abs(roots[g].sum_e) > 300 || abs(roots[g].fix_e) > 300))
+        roots[g].climb = r.n_alive > 0 && (!fits || abs(roots[g].sum_e) > 300);
+        if (roots[g].climb)
             climb = 1;
     }
     __syncthreads();
@@ -782,7 +783,9 @@ __global__ void k_link(csgd_t dd, DevScalars *sc, const unsigned long long *__re
 
 // Moments. Only the centre of mass and mass fields of a cell are written here
 // (write_cell set the rest): from prefix sums over the sorted bodies (k_mom_sums,
-// k_moments), or, for masses that do not fit those, by climbing the tree.
+// k_moments), or, for systems whose bodies do not fit those, by climbing the tree.
+// Which of the two is a system's own (DevRoot::climb): it has the same moments alone
+// and in an ensemble.
 //
 // The climb: one thread per cell of at most MOM_DIRECT bodies (and per leaf);
 // above those, the last child to finish computes its parent, summing the
@@ -1008,10 +1011,10 @@ __device__ __forceinline__ double value128(u128 s, int u)
 
 // Sums over cells as differences of prefix sums over the sorted bodies. In
 // 128-bit fixed point they are exact: a system's masses are whole units of
-// 2^(sum_e - 126), its m x are cut to units of 2^(sum_e + fix_e - 126), and no
+// 2^(sum_e - 126), its m x are cut to units of 2^(sum_e + pos_e - 126), and no
 // sum overflows; sums over different systems (other units) wrap and are never
 // used. A body below 2^-50 of the bound of its system's mass could lose bits:
-// then (mom_climb) the cells are summed in FP64 as above.
+// then (DevRoot::climb) that system's cells are summed in FP64 as above.
 //
 // Every cell so costs two loads of four sums and no FP64 operation, whatever
 // its size. The climb was bound by its chain of dependent levels for few bodies
@@ -1060,7 +1063,7 @@ __device__ __forceinline__ void block_prefix(MomSums &v)
 }
 
 __global__ void __launch_bounds__(MOM_TILE) k_mom_sums(csgd_t dd, DevScalars *sc,
-                                                       const DevRoot *__restrict__ roots,
+                                                       DevRoot *roots,
                                                        const double *__restrict__ x,
                                                        const double *__restrict__ y,
                                                        const double *__restrict__ z,
@@ -1070,8 +1073,6 @@ __global__ void __launch_bounds__(MOM_TILE) k_mom_sums(csgd_t dd, DevScalars *sc
 {
     pdl_enter();
     __shared__ bool last;
-    if (sc->mom_climb) // since k_root
-        return;
     const int na = sc->n_alive, p = blockIdx.x * MOM_TILE + threadIdx.x;
     const int tiles = na / MOM_TILE + 1; // position na too
     if ((int)blockIdx.x >= tiles)
@@ -1082,12 +1083,12 @@ __global__ void __launch_bounds__(MOM_TILE) k_mom_sums(csgd_t dd, DevScalars *sc
         v.s[k] = 0;
     if (p < na) {
         const int b = perm[p];
-        const DevRoot &r = roots[n_gal > 1 ? sgid[p] : 0];
+        DevRoot &r = roots[n_gal > 1 ? sgid[p] : 0];
         const long long mb = __double_as_longlong(m[b]);
         const int em = (int)(mb >> 52); // biased
-        const int um = r.sum_e - 126;
+        const int um = r.sum_e - 126, pos_e = r.pos_e;
         if (em - 1022 < r.sum_e - 50 || em < 1)
-            sc->mom_light = 1; // every writer writes the same
+            r.climb = sc->mom_climb = 1; // every writer writes the same
         const unsigned long long Sm = ((unsigned long long)mb & 0xfffffffffffffull) | (1ull << 52);
         v.s[3] = shift128(Sm, em - 1075 - um);
         const double c[3] = {x[b], y[b], z[b]};
@@ -1097,7 +1098,7 @@ __global__ void __launch_bounds__(MOM_TILE) k_mom_sums(csgd_t dd, DevScalars *sc
             const int ec = (int)(cb >> 52) & 0x7ff;
             const unsigned long long Sc =
                 (cb & 0xfffffffffffffull) | (ec ? 1ull << 52 : 0ull);
-            const u128 P = shift128((u128)Sm * Sc, em + max(ec, 1) - 2150 - um - r.fix_e);
+            const u128 P = shift128((u128)Sm * Sc, em + max(ec, 1) - 2150 - um - pos_e);
             v.s[k] = cb >> 63 ? (u128)0 - P : P;
         }
     }
@@ -1151,15 +1152,15 @@ __global__ void __launch_bounds__(256) k_moments(csgd_t dd, DevScalars *sc,
     const int nn = sc->n_nodes;
     if (nn > dd.node_cap || sc->n_alive == 0)
         return;
-    const bool climb = (sc->mom_climb | sc->mom_light) != 0;
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < nn; id += gridDim.x * blockDim.x) {
-        if (climb) { // k_tasks divides
-            moments_cell(dd, id, x, y, z, m, perm);
-            continue;
-        }
         const NodeLink l = dd.link[id];
         if (l.count < 1)
             continue;
+        const DevRoot &r = roots[n_gal > 1 ? sgid[l.first] : 0];
+        if (r.climb) { // k_tasks divides
+            moments_cell(dd, id, x, y, z, m, perm);
+            continue;
+        }
         const int body = dd.w64[id].body;
         double cx, cy, cz, M;
         if (l.count == 1 && body >= 0) { // the body's position exactly
@@ -1168,7 +1169,6 @@ __global__ void __launch_bounds__(256) k_moments(csgd_t dd, DevScalars *sc,
             cz = z[body];
             M = m[body];
         } else {
-            const DevRoot &r = roots[n_gal > 1 ? sgid[l.first] : 0];
             const int um = r.sum_e - 126, from = l.first, to = l.first + l.count;
             double v[4];
 #pragma unroll
@@ -1177,7 +1177,7 @@ __global__ void __launch_bounds__(256) k_moments(csgd_t dd, DevScalars *sc,
                                join(dd.mom_tile[4 * (size_t)(to / MOM_TILE) + k]) -
                                join(dd.mom_sum[4 * (size_t)from + k]) -
                                join(dd.mom_tile[4 * (size_t)(from / MOM_TILE) + k]);
-                v[k] = value128(s, k < 3 ? um + r.fix_e : um);
+                v[k] = value128(s, k < 3 ? um + r.pos_e : um);
             }
             M = v[3];
             const Divisor by_M = divisor(M);
@@ -1259,10 +1259,11 @@ __global__ void k_tasks(DevScalars *sc, DevRoot *roots, int n_gal, const int *__
                         const double *__restrict__ y, const double *__restrict__ z)
 {
     pdl_enter();
-    if (!imported && (sc->mom_climb | sc->mom_light) && sc->n_nodes <= node_cap && sc->n_alive > 0)
+    if (!imported && sc->mom_climb && sc->n_nodes <= node_cap && sc->n_alive > 0)
         for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < sc->n_nodes;
              id += gridDim.x * blockDim.x)
-            moments_norm(dd, id, x, y, z);
+            if (link[id].count > 0 && roots[n_gal > 1 ? dd.sgid[link[id].first] : 0].climb)
+                moments_norm(dd, id, x, y, z);
     if (threadIdx.x >= blockDim.x - CSG_WARP) { // the last warp
         const int lane = threadIdx.x & 31, nn = sc->n_nodes;
         for (int g = blockIdx.x; g < n_gal; g += gridDim.x) {
