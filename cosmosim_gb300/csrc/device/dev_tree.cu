@@ -1010,11 +1010,12 @@ __device__ __forceinline__ double value128(u128 s, int u)
 }
 
 // Sums over cells as differences of prefix sums over the sorted bodies. In
-// 128-bit fixed point they are exact: a system's masses are whole units of
-// 2^(sum_e - 126), its m x are cut to units of 2^(sum_e + pos_e - 126), and no
-// sum overflows; sums over different systems (other units) wrap and are never
-// used. A body below 2^-50 of the bound of its system's mass could lose bits:
-// then (DevRoot::climb) that system's cells are summed in FP64 as above.
+// 128-bit fixed point they take no rounding but the terms' own: a system's masses
+// are whole units of 2^(sum_e - 126), its m x are cut to units of 2^(sum_e + pos_e -
+// 126), and no sum overflows; sums over different systems (other units) wrap and
+// are never used. Every m x that is not 0 has at least 55 bits above its unit, more
+// than an FP64 product keeps; a system with a body too light or, for its mass, too
+// close to a coordinate's 0 for that (DevRoot::climb) is summed in FP64 as above.
 //
 // Every cell so costs two loads of four sums and no FP64 operation, whatever
 // its size. The climb was bound by its chain of dependent levels for few bodies
@@ -1087,8 +1088,8 @@ __global__ void __launch_bounds__(MOM_TILE) k_mom_sums(csgd_t dd, DevScalars *sc
         const long long mb = __double_as_longlong(m[b]);
         const int em = (int)(mb >> 52); // biased
         const int um = r.sum_e - 126, pos_e = r.pos_e;
-        if (em - 1022 < r.sum_e - 50 || em < 1)
-            r.climb = sc->mom_climb = 1; // every writer writes the same
+        // a mass below the unit, or a product with fewer than 55 bits above it
+        bool light = em < 1 || em - 1075 < um;
         const unsigned long long Sm = ((unsigned long long)mb & 0xfffffffffffffull) | (1ull << 52);
         v.s[3] = shift128(Sm, em - 1075 - um);
         const double c[3] = {x[b], y[b], z[b]};
@@ -1098,9 +1099,12 @@ __global__ void __launch_bounds__(MOM_TILE) k_mom_sums(csgd_t dd, DevScalars *sc
             const int ec = (int)(cb >> 52) & 0x7ff;
             const unsigned long long Sc =
                 (cb & 0xfffffffffffffull) | (ec ? 1ull << 52 : 0ull);
+            light |= (cb << 1) != 0ull && em + max(ec, 1) - 2046 - um - pos_e < 55;
             const u128 P = shift128((u128)Sm * Sc, em + max(ec, 1) - 2150 - um - pos_e);
             v.s[k] = cb >> 63 ? (u128)0 - P : P;
         }
+        if (light)
+            r.climb = sc->mom_climb = 1; // every writer writes the same
     }
     own = v;
     block_prefix(v);
