@@ -266,6 +266,7 @@ __global__ void __launch_bounds__(8 * CSG_WARP) k_walk64_exact(WalkArgs a)
 constexpr int RND_STACK = 384; // 1M, theta 0.5: fits all but rare rounds (256: 6% slower)
 constexpr int RND_PAIRS = 17;  // accepted cells from pair 0, undecided from the next pair on
 constexpr int RND_REC = 20;    // words per staged pair
+constexpr int SUM_BLOCK = 16;  // undecided cells a block of uncompensated terms
 constexpr unsigned RND_OPEN = 0x80000000u; // stack entry: known open, children not pushed yet
 
 typedef unsigned long long u64;
@@ -417,6 +418,7 @@ struct LanePos {
 //                     each (the lanes that reached it, less a leaf's own body)
 //     terms(...)      two undecided cells: differences, d^2, masses, whether
 //                     this lane takes each
+//     fold()          ends a block of uncompensated terms
 //   interaction lists (BLOCKS true)
 //     block(cell, w)  the round's cells, one per lane, and the lane's own takes:
 //                     bit j for lane j's cell
@@ -486,6 +488,8 @@ __device__ __forceinline__ void walk_stackless(const WalkArgs &a, const LaneBody
             st.active += active;
         }
         lane_test(a, L, cur, active, next, take, open, sink);
+        if constexpr (!Sink::BLOCKS)
+            sink.fold();
         if (STATS)
             st.hits += take;
         if (active && !open)
@@ -580,42 +584,46 @@ __device__ __forceinline__ void walk_rounds(const WalkArgs &a, RoundShared &sh, 
         if (STATS && acc)
             st.hits += __popc(tm);
         const u64 acck = pack2(a.acc_k, a.acc_k), opnk = pack2(a.opn_k, a.opn_k);
-        for (int e = 0; e < nu; e += 2) {
-            const ulonglong2 *r = (const ulonglong2 *)(sh.rec + ((ub + e) >> 1) * RND_REC);
-            const ulonglong2 q0 = r[0], q1 = r[1], q2 = r[2], q3 = r[3];
-            const int4 t = *(const int4 *)(r + 4); // masks, cells
-            const u64 ux = add2(add2(q0.x, sink.nhx), add2(q2.x, sink.nlx));
-            const u64 uy = add2(add2(q0.y, sink.nhy), add2(q2.y, sink.nly));
-            const u64 uz = add2(add2(q1.x, sink.nhz), add2(q3.x, sink.nlz));
-            const u64 d2 = fma2(ux, ux, fma2(uy, uy, mul2(uz, uz)));
-            const u64 sa = mul2(q3.y, acck), so = mul2(q3.y, opnk);
-            const bool act0 = t.x & L.bit, act1 = t.y & L.bit;
-            bool acc0 = lo2(sa) < lo2(d2), acc1 = hi2(sa) < hi2(d2); // implies d2 > 0
-            const bool amb0 = act0 && !acc0 && !(lo2(so) > lo2(d2));
-            const bool amb1 = act1 && !acc1 && !(hi2(so) > hi2(d2));
-            if (amb0 || amb1) { // inside the FP32 band: rare
-                if (amb0)
-                    acc0 = decide64(a, t.z, L.me);
-                if (amb1)
-                    acc1 = decide64(a, t.w, L.me);
-            }
-            const bool take0 = act0 && acc0, take1 = act1 && acc1;
-            const unsigned o0 = __ballot_sync(0xffffffffu, act0 && !acc0);
-            const unsigned o1 = __ballot_sync(0xffffffffu, act1 && !acc1);
-            if constexpr (Sink::BLOCKS) {
-                const unsigned t0 = __ballot_sync(0xffffffffu, take0);
-                const unsigned t1 = __ballot_sync(0xffffffffu, take1);
-                if (lane == 0)
-                    *(uint4 *)&sh.open[e] = make_uint4(o0, t0, o1, t1);
-            } else {
-                if (lane == 0) {
-                    sh.open[e].x = o0;
-                    sh.open[e + 1].x = o1;
+        for (int e = 0; e < nu;) {
+            for (const int stop = Sink::BLOCKS ? nu : min(nu, e + SUM_BLOCK); e < stop; e += 2) {
+                const ulonglong2 *r = (const ulonglong2 *)(sh.rec + ((ub + e) >> 1) * RND_REC);
+                const ulonglong2 q0 = r[0], q1 = r[1], q2 = r[2], q3 = r[3];
+                const int4 t = *(const int4 *)(r + 4); // masks, cells
+                const u64 ux = add2(add2(q0.x, sink.nhx), add2(q2.x, sink.nlx));
+                const u64 uy = add2(add2(q0.y, sink.nhy), add2(q2.y, sink.nly));
+                const u64 uz = add2(add2(q1.x, sink.nhz), add2(q3.x, sink.nlz));
+                const u64 d2 = fma2(ux, ux, fma2(uy, uy, mul2(uz, uz)));
+                const u64 sa = mul2(q3.y, acck), so = mul2(q3.y, opnk);
+                const bool act0 = t.x & L.bit, act1 = t.y & L.bit;
+                bool acc0 = lo2(sa) < lo2(d2), acc1 = hi2(sa) < hi2(d2); // implies d2 > 0
+                const bool amb0 = act0 && !acc0 && !(lo2(so) > lo2(d2));
+                const bool amb1 = act1 && !acc1 && !(hi2(so) > hi2(d2));
+                if (amb0 || amb1) { // inside the FP32 band: rare
+                    if (amb0)
+                        acc0 = decide64(a, t.z, L.me);
+                    if (amb1)
+                        acc1 = decide64(a, t.w, L.me);
                 }
-                sink.terms(ux, uy, uz, d2, q1.y, take0, take1);
+                const bool take0 = act0 && acc0, take1 = act1 && acc1;
+                const unsigned o0 = __ballot_sync(0xffffffffu, act0 && !acc0);
+                const unsigned o1 = __ballot_sync(0xffffffffu, act1 && !acc1);
+                if constexpr (Sink::BLOCKS) {
+                    const unsigned t0 = __ballot_sync(0xffffffffu, take0);
+                    const unsigned t1 = __ballot_sync(0xffffffffu, take1);
+                    if (lane == 0)
+                        *(uint4 *)&sh.open[e] = make_uint4(o0, t0, o1, t1);
+                } else {
+                    if (lane == 0) {
+                        sh.open[e].x = o0;
+                        sh.open[e + 1].x = o1;
+                    }
+                    sink.terms(ux, uy, uz, d2, q1.y, take0, take1);
+                }
+                if (STATS)
+                    st.hits += take0 + take1;
             }
-            if (STATS)
-                st.hits += take0 + take1;
+            if constexpr (!Sink::BLOCKS)
+                sink.fold();
         }
         __syncwarp();
         const unsigned om = opn ? c.mask : und ? sh.open[place - ub].x : 0u;
@@ -703,9 +711,14 @@ __device__ __forceinline__ void kahan_add2(u64 &s, u64 &c, u64 v)
 }
 
 // FP32-mixed sums: pair terms in FP32 from ~48-bit position differences, two
-// cells at a time in packed arithmetic; the terms of a round (at most 17 per
-// half, 8 on average) are added with Kahan compensation (per-body compensated
-// FP32 summation); G applied once. Lanes that do not take a cell add zero.
+// cells at a time in packed arithmetic; blocks of them are added with Kahan
+// compensation (per-body compensated FP32 summation); G applied once. Lanes
+// that do not take a cell add zero. A block is a chain of at most 8 additions per
+// half: 8 undecided pairs, or a round's accepted pairs (16 at most), two by two.
+// One block a round, its up to 17 terms one after the other, was 1-4% faster (1M
+// 4.12 ms against 4.17, 100k merger 0.342 and 0.354) and 5-9% less exact in the
+// median, 25% at 1M in the largest error; chains of 8 single terms throughout
+// cost a second or third block a round: 1M 4.42-4.59 ms.
 //
 // A large system's task sums the whole tree in one go. A small system's
 // (split_max bodies or fewer) closes its sums into double partials: first the
@@ -747,33 +760,52 @@ struct Sum32 : LanePos {
         asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r2));
         return y;
     }
-    __device__ __forceinline__ void pair(u64 dx, u64 dy, u64 dz, u64 r2, u64 m, bool t0, bool t1)
+    static __device__ __forceinline__ u64 factor(u64 r2, u64 m, bool t0, bool t1)
     {
         const u64 y = pack2(rsq(lo2(r2)), rsq(hi2(r2)));
         const u64 f0 = mul2(m, mul2(y, mul2(y, y)));
-        const u64 f = pack2(t0 ? lo2(f0) : 0.0f, t1 ? hi2(f0) : 0.0f);
-        bx = fma2(f, dx, bx);
-        by = fma2(f, dy, by);
-        bz = fma2(f, dz, bz);
+        return pack2(t0 ? lo2(f0) : 0.0f, t1 ? hi2(f0) : 0.0f);
+    }
+    struct Pair {
+        u64 dx, dy, dz, f;
+    };
+    __device__ __forceinline__ void load(const float *rec, int e, Pair &p)
+    {
+        const ulonglong2 *r = (const ulonglong2 *)(rec + (e >> 1) * RND_REC);
+        const ulonglong2 q0 = r[0], q1 = r[1], q2 = r[2], q3 = r[3];
+        const uint2 t = *(const uint2 *)(r + 4); // masks
+        p.dx = add2(add2(q0.x, nhx), add2(q2.x, nlx));
+        p.dy = add2(add2(q0.y, nhy), add2(q2.y, nly));
+        p.dz = add2(add2(q1.x, nhz), add2(q3.x, nlz));
+        p.f = factor(fma2(p.dx, p.dx, fma2(p.dy, p.dy, fma2(p.dz, p.dz, eps2))), q1.y, t.x & bit,
+                     t.y & bit);
     }
     __device__ __forceinline__ void accept(const float *rec, int n)
     {
-#pragma unroll 2
-        for (int e = 0; e < n; e += 2) {
-            const ulonglong2 *r = (const ulonglong2 *)(rec + (e >> 1) * RND_REC);
-            const ulonglong2 q0 = r[0], q1 = r[1], q2 = r[2], q3 = r[3];
-            const uint2 t = *(const uint2 *)(r + 4); // masks
-            const u64 dx = add2(add2(q0.x, nhx), add2(q2.x, nlx));
-            const u64 dy = add2(add2(q0.y, nhy), add2(q2.y, nly));
-            const u64 dz = add2(add2(q1.x, nhz), add2(q3.x, nlz));
-            const u64 r2 = fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, eps2)));
-            pair(dx, dy, dz, r2, q1.y, t.x & bit, t.y & bit);
+        int e = 0;
+        for (; e + 2 < n; e += 4) {
+            Pair p, q;
+            load(rec, e, p);
+            load(rec, e + 2, q);
+            bx = add2(bx, fma2(q.f, q.dx, mul2(p.f, p.dx)));
+            by = add2(by, fma2(q.f, q.dy, mul2(p.f, p.dy)));
+            bz = add2(bz, fma2(q.f, q.dz, mul2(p.f, p.dz)));
+        }
+        if (e < n) {
+            Pair p;
+            load(rec, e, p);
+            bx = fma2(p.f, p.dx, bx);
+            by = fma2(p.f, p.dy, by);
+            bz = fma2(p.f, p.dz, bz);
         }
         fold();
     }
     __device__ __forceinline__ void terms(u64 dx, u64 dy, u64 dz, u64 d2, u64 m, bool t0, bool t1)
     {
-        pair(dx, dy, dz, add2(d2, eps2), m, t0, t1);
+        const u64 f = factor(add2(d2, eps2), m, t0, t1);
+        bx = fma2(f, dx, bx);
+        by = fma2(f, dy, by);
+        bz = fma2(f, dz, bz);
     }
     // one component's halves as a double: the FP32 sum of the two, its
     // rounding error (two-sum) joining the compensations
