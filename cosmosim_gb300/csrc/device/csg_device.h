@@ -39,10 +39,6 @@ void *csgd_stream(csgd_t *d);
 /* The device Body staging array (capacity >= the reserved body count). */
 Body *csgd_aos(csgd_t *d);
 
-/* Pool exports take the tree last built as it is (on for states that export
-   after most builds; else an export rebuilds it). */
-void csgd_set_export_order(csgd_t *d, int on);
-
 /* Makes room for n bodies (grow-only). */
 int csgd_reserve(csgd_t *d, int n);
 
@@ -188,7 +184,7 @@ void csgd_enable_graphs(csgd_t *d, int on);
    first SPH pass, which must not happen inside a stream capture). */
 int csgd_prepare_sph(csgd_t *d);
 
-/* The tree as a reference-layout pool, in the reference's allocation order.
+/* The tree last built as a reference-layout pool, in the reference's allocation order.
    Blocks until done. pool must hold *pool_size_out <= capacity nodes; a
    mapped (pinned) host pool is written by the export kernel directly. */
 int csgd_export_pool(csgd_t *d, OctreeNode *pool, int capacity, int *pool_size_out);
@@ -197,7 +193,7 @@ int csgd_export_pool(csgd_t *d, OctreeNode *pool, int capacity, int *pool_size_o
    dst is device-accessible (device memory or the device view of a mapped
    host array) with room for capacity cells; a larger tree records
    CSG_ERR_NODE_CAPACITY for the next csgd_sync and writes nothing. Needs a
-   tree built with the export order (csgd_set_export_order). */
+   tree built here (not an imported one). */
 int csgd_export_to(csgd_t *d, OctreeNode *dst, int capacity);
 
 /* Device view of a mapped (pinned) host pointer, or NULL for any other
@@ -206,8 +202,8 @@ void *csgd_host_view(const void *p);
 
 /* While set (dst != NULL), every substep also exports the tree it builds to
    dst (as csgd_export_to), on a third stream beside the walk. Returns 1 when
-   set, 0 when this state cannot (no third stream, no export order, several
-   systems): the caller then exports after the substep. */
+   set, 0 when this state cannot (no third stream, several systems): the caller
+   then exports after the substep. */
 int csgd_set_substep_export(csgd_t *d, OctreeNode *dst, int capacity);
 
 /* Replaces the device tree by the caller's pool (nodes reachable from root;

@@ -206,9 +206,7 @@ struct csgd {
     // and, for the persistent form, blocks per SM
     int walk_warps, walk_group, walk_bps;
     int num_sms;
-    int export_order; // built trees are kept for pool exports
     int boxed;        // the next build's boxes are there (csgd_kick_drift_boxed)
-    int minidx_valid; // the current tree was built so (an export takes it as it is)
 
     // keys and sort
     unsigned long long *key, *key_alt;

@@ -425,8 +425,6 @@ extern "C" void csgd_destroy(csgd_t *d)
     free(d);
 }
 
-extern "C" void csgd_set_export_order(csgd_t *d, int on) { d->export_order = on ? 1 : 0; }
-
 extern "C" void csgd_set_stream(csgd_t *d, void *stream)
 {
     d->stream = stream ? (cudaStream_t)stream : d->own_stream;
@@ -1004,7 +1002,7 @@ extern "C" int csgd_set_substep_export(csgd_t *d, OctreeNode *dst, int capacity)
 {
     // the export stages its records in the pool buffer (allocated here, never
     // inside a capture)
-    const bool ok = dst && d->aux2 && d->export_order && d->n_gal == 1 &&
+    const bool ok = dst && d->aux2 && d->n_gal == 1 &&
                     csgd_ensure_tree_extras(d, 1, 1) == CSG_OK;
     d->export_dst = ok ? dst : nullptr;
     d->export_cap = d->export_dst ? capacity : 0;

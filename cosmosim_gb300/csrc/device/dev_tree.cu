@@ -1762,7 +1762,6 @@ extern "C" int csgd_build_tree(csgd_t *d, int geometry)
     csgd_build_mark(d, 3);
     csgd_launch(d, k_mom_sums, n / MOM_TILE + 1, MOM_TILE, s, *d, sc, d->roots, d->x, d->y, d->z, d->m, d->perm, d->sgid, d->n_gal);
     csgd_launch(d, k_moments, gn, B, s, *d, sc, d->roots, d->x, d->y, d->z, d->m, d->perm, d->sgid, d->n_gal);
-    d->minidx_valid = d->export_order;
     csgd_build_mark(d, 4);
     csgd_launch(d, k_tasks, min(d->n_gal > 1 ? d->n_gal : csgd_grid(n, 32 * 256), d->num_sms), 256, s, sc, d->roots, d->n_gal, d->base, d->tasks, d->task_cap, 0, d->link, d->child, d->node_cap, *d, d->x, d->y, d->z);
     d->geometry_valid = 0;
@@ -1782,7 +1781,7 @@ extern "C" int csgd_export_to(csgd_t *d, OctreeNode *dst, int capacity)
 {
     if (d->n_gal > 1) // one system only (see csgd_set_systems)
         return CSG_ERR_UNSUPPORTED;
-    if (!d->minidx_valid || !dst || capacity < 1)
+    if (d->imported || !dst || capacity < 1)
         return CSG_ERR_BAD_ARG;
     cudaStream_t s = d->stream;
     DevScalars *sc = d->sc;
@@ -1822,14 +1821,6 @@ extern "C" int csgd_export_pool(csgd_t *d, OctreeNode *pool, int capacity, int *
     int erc = csgd_ensure_tree_extras(d, 1, 1);
     if (erc)
         return erc;
-    if (!d->minidx_valid) { // not kept for exports: rebuild (same tree)
-        const int saved = d->export_order;
-        d->export_order = 1;
-        erc = csgd_build_tree(d, 1);
-        d->export_order = saved;
-        if (erc)
-            return erc;
-    }
     // a caller's mapped (pinned) host array takes the records directly
     OctreeNode *mapped = (OctreeNode *)csgd_host_view(pool);
     const int cap = mapped ? capacity : (capacity < d->node_cap ? capacity : d->node_cap);
@@ -1878,7 +1869,6 @@ extern "C" int csgd_import_pool(csgd_t *d, const OctreeNode *pool, int n_nodes, 
     { k_tasks<<<1, 256, 0, s>>>(sc, d->roots, 1, d->base, d->tasks, d->task_cap, 1, d->link, d->child, d->node_cap, *d, d->x, d->y, d->z); d->launches++; }
     d->geometry_valid = 1;
     d->imported = 1;
-    d->minidx_valid = 0;
     d->gas_valid = 0;
     return csgd_check(d, cudaGetLastError());
 }
