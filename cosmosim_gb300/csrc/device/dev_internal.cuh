@@ -385,29 +385,6 @@ __device__ __forceinline__ float f32_from_f64_bits(long long b)
     return __int_as_float((int)((b >> 29) - (896LL << 23)));
 }
 
-// y^2 (exact: 48 significant bits) and y^3 (rounded to nearest, < 2^-53
-// relative error) as doubles, for a positive normal float 2^-60 < y < 2^60,
-// by integer multiplies of y's 24-bit significand Y (y = Y 2^(ey-150)):
-// no FP64 operations. Y^2 lies in [2^46, 2^48): shifted so its leading bit
-// sits at bit 52, added to (biased exponent - 1) << 52 (the leading bit
-// supplies the missing 1). Y^3 / 2^8 (the high word of (Y 2^40)(Y^2 2^16))
-// lies in [2^61, 2^64): rounded to 53 bits the same way (a carry out of the
-// significand moves into the exponent, as it should).
-__device__ __forceinline__ void pow23_from_f32(float y, double &y2, double &y3)
-{
-    const unsigned yb = __float_as_uint(y);
-    const unsigned Y = (yb & 0x7fffffu) | 0x800000u;
-    const long long ey = (long long)(yb >> 23);
-    const unsigned long long S = (unsigned long long)Y * Y;
-    const unsigned t = (unsigned)(S >> 47); // 1: leading bit at 47
-    y2 = __longlong_as_double(((2 * ey + 768 + t) << 52) + (long long)(S << (6 - t)));
-    const unsigned long long hi = __umul64hi((unsigned long long)Y << 40, S << 16);
-    const int lz = __clz((unsigned)(hi >> 32)); // 0..2
-    const int sh = 11 - lz;
-    const unsigned long long M = (hi + (1ull << (sh - 1))) >> sh;
-    y3 = __longlong_as_double(((3 * ey + 643 - lz) << 52) + (long long)M);
-}
-
 // m r^-3 by integer arithmetic only, for r2 = r^2 in [2^-99, 2^100) and m a
 // positive normal double with biased exponent in [160, 1887] (then every
 // step below stays in range and the result is a normal double), from the
@@ -452,31 +429,8 @@ __device__ __forceinline__ double m_r3_from_seed(long long rb, long long mb, flo
     return __longlong_as_double((((mb >> 52) + 3 * ey - 378 - lz) << 52) + (long long)M);
 }
 
-// w = 3/2 e + 15/8 e^2 = e c, c = 3/2 + 15/8 e, the series term of
-// (1-e)^-3/2 - 1, for |e| < 2^-7 (the seeds give |e| < 2^-20), by integer
-// arithmetic: c in 62-bit fixed point (C in [2^62, 2^63)), times e's 53-bit
-// significand by one 64 x 64 -> high-64 multiply, rounded to 53 bits (w
-// within 2^-53 relative, plus < 2^-60 from truncations). For |e| < 2^-63,
-// w = 0 (then w < 2^-62: below the result's rounding). Keeps the series off
-// the FP64 pipe.
-__device__ __forceinline__ double r3_series_w(double e)
-{
-    const long long eb = __double_as_longlong(e);
-    const long long ee = (eb >> 52) & 0x7ff;
-    const unsigned long long Em = ((unsigned long long)eb & 0xfffffffffffffull) | (1ull << 52);
-    const int s = (int)min(max(1016 - ee, 0LL), 63LL);
-    const unsigned long long T = (15ull * Em) >> s; // 15/8 |e| 2^62, < 2^57
-    const unsigned long long C = eb < 0 ? (3ull << 61) - T : (3ull << 61) + T;
-    const unsigned long long R = __umul64hi(Em << 11, C << 1); // [2^62, 2^64)
-    const int lz = __clz((unsigned)(R >> 32));                 // 0 or 1
-    const int sh = 11 - lz;
-    const unsigned long long M = (R + (1ull << (sh - 1))) >> sh;
-    const long long w = (eb & (1LL << 63)) | (((ee - lz) << 52) + (long long)M);
-    return ee < 960 ? 0.0 : __longlong_as_double(w);
-}
-
-// m/r^3 for the queued FP64 walk without FP64 operations (the FP64 pipe is
-// the walk's bottleneck on this GPU): from the FP32 rsqrt seed y0 (rel.
+// m/r^3 for the adjoint's pairs without FP64 operations (the FP64 pipe is
+// their bottleneck on this GPU): from the FP32 rsqrt seed y0 (rel.
 // error < 2^-21) by integer arithmetic (m_r3_from_seed: the series of
 // (1-e)^-3/2, e = 1 - r2 y0^2, one rounding). The seed's conversion is a bit
 // operation. Range checks on the exponents (2^-99 <= r2 < 2^100,
