@@ -238,6 +238,8 @@ struct csgd {
     int *child;   // 8 per node
     int *nchild;
     int *ticket;
+    // during a build, in the export order's buffers: a build waits for the export
+    // of the last tree, and an export starts after the build
     ulonglong2 *mom_sum;  // 128-bit sums before a position in its tile (m x, m y, m z, m)
     ulonglong2 *mom_tile; // the same before a tile
     int2 *minidx; // two smallest caller indices below each cell (formed by an export)

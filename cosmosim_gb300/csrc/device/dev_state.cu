@@ -214,7 +214,7 @@ void free_bodies(csgd_t *d)
                     d->rho, d->P, d->u, d->h, d->type, d->aos, d->key, d->key_alt, d->perm,
                     d->perm_alt, d->ext, d->sort_hist, d->lcp, d->cnt, d->base, d->scan_tmp,
                     d->gas, d->w64, d->w32, d->link, d->geo, d->s32, d->child, d->nchild, d->ticket,
-                    d->mom_sum, d->mom_tile, d->minidx, d->ord_key, d->ord_key_alt, d->ord_id, d->ord_id_alt, d->rank,
+                    d->minidx, d->ord_key, d->ord_key_alt, d->ord_id, d->ord_id_alt, d->rank,
                     d->pool, d->gid, d->sgid, d->tasks};
     for (void *p : ptrs)
         if (p)
@@ -527,10 +527,12 @@ extern "C" int csgd_reserve(csgd_t *d, int n)
     ok &= dalloc(&d->nchild, ncap) == cudaSuccess;
     ok &= dalloc(&d->ticket, ncap) == cudaSuccess;
     ok &= dalloc(&d->minidx, ncap) == cudaSuccess;
-    ok &= dalloc(&d->mom_sum, 4 * (cap + 1)) == cudaSuccess;
-    ok &= dalloc(&d->mom_tile, 4 * (cap / 256 + 2)) == cudaSuccess;
+    // 8 words a body and 64: also the moments' sums, 8 words a body and 8 (mom_sum),
+    // and a tile's, 8 words for every 256 bodies and 16 (mom_tile)
     ok &= dalloc(&d->ord_key, ncap) == cudaSuccess;
     ok &= dalloc(&d->ord_key_alt, ncap) == cudaSuccess;
+    d->mom_sum = (ulonglong2 *)d->ord_key_alt;
+    d->mom_tile = (ulonglong2 *)d->ord_key;
     ok &= dalloc(&d->ord_id, ncap) == cudaSuccess;
     ok &= dalloc(&d->ord_id_alt, ncap) == cudaSuccess;
     ok &= dalloc(&d->rank, ncap) == cudaSuccess;
