@@ -1720,10 +1720,11 @@ extern "C" int csgd_autotune_walk(csgd_t *d, const csgd_force_params *p, int rep
     if (reps < 1 || reps > 64) {
         return CSG_ERR_BAD_ARG;
     }
-    // persistent candidates: 8, 16 or 24 resident warps per SM (24 is what
-    // their register allocation allows), task groups of 1, 2 or 4
+    // persistent candidates: 8, 16 or as many resident warps per SM as their
+    // registers are sized for (in whole blocks: 16 with eight warps a block), task
+    // groups of 1, 2 or 4
     static const int groups[] = {1, 2, 4};
-    static const int resident[] = {8, 16, 24};
+    static const int resident[] = {8, 16, WALK32_RES};
     CsgWalkShape cand[2 * (1 + 9)];
     int nc = 0;
     for (int w = 4; w <= 8; w += 4) {

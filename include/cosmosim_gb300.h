@@ -51,9 +51,9 @@ extern "C" {
      blocks_per_sm    persistent launch only: blocks per SM (1..32)
      ms               filled by the autotuner: median walk time, ms
    The shape applies to the FP32-mixed walk; the FP64 walk always runs a
-   producer warp and its consumer warps per task (or, for systems of up to
-   12 x 32 bodies per SM, per child subtrees). Results do not depend on the
-   shape; only the time does. */
+   producer warp and two consumer warps per task (or, for systems of up to
+   6 x 32 bodies per SM, 12 x 32 for opening angles below 0.45, per child
+   subtree). Results do not depend on the shape; only the time does. */
 typedef struct {
     int warps_per_block;
     int task_group;
@@ -210,8 +210,8 @@ CSG_EXPORT int cosmosim_gravity_async(SimHandle handle);
    substep total is the elapsed time of the whole substep. Enabling resets
    the sums; disabling keeps them for reading and returns to graph replays. */
 typedef struct {
-    double kick_drift_ms; /* first half kick + drift */
-    double build_ms;      /* bounding box, keys, sort, cells, moments */
+    double kick_drift_ms; /* first half kick + drift, the moved bodies' bounding boxes */
+    double build_ms;      /* root cube, keys, sort, cells, moments */
     double gravity_ms;    /* the Barnes-Hut walk */
     double sph_ms;        /* neighbour lists, density, pressure and viscosity forces */
     double kick_ms;       /* second half kick */
@@ -219,11 +219,12 @@ typedef struct {
     double substep_ms;    /* whole substeps */
     long long substeps;   /* substeps timed */
     /* the build's parts (sum to build_ms): */
-    double build_keys_ms;    /* bounding box, root cube, keys */
-    double build_sort_ms;    /* radix sort of the keys */
+    double build_keys_ms;    /* root cube, keys */
+    double build_sort_ms;    /* sort of the keys */
     double build_cells_ms;   /* shared keys, cell counts and scan, cells, links */
     double build_moments_ms; /* masses and centres of mass */
-    double build_rest_ms;    /* walk tasks; SPH cell geometry */
+    double build_rest_ms;    /* walk tasks (and the centres of mass of systems too unequal
+                                for the moments' fixed point); SPH cell geometry */
 } CsgPhaseTimes;
 CSG_EXPORT int cosmosim_enable_phase_timing(SimHandle handle, int on);
 CSG_EXPORT int cosmosim_phase_times(SimHandle handle, CsgPhaseTimes *out);
