@@ -347,25 +347,40 @@ int csg_scan_exclusive(csgd_t *d, const int *in, int *out, int n, const int *cou
 constexpr int CSG_WAIT_POLLS_DEFAULT = 1 << 22;
 // The walks split each task by child subtrees when there are few tasks for the
 // GPU. Above that the whole-task walk already fills the SMs and the split only
-// adds root-level work. The FP32 walk decides per launch, up to 12 tasks per SM
-// (about 58k bodies on 152 SMs; both forms give the same bits); the FP64 walk
-// per system, by its body count (the forms sum differently, and a system must
-// come out the same alone and in an ensemble), up to 12 for opening angles
-// below 0.45 and 6 (29,184 bodies) from there on: small angles make long tasks,
-// of which the last wave of whole ones leaves most SMs idle. Split against whole,
-// us: 36,901 bodies at angles 0.3, 0.4, 0.5, 0.7: 1354 and 1873, 854 and 957, 634
-// and 603, 397 and 325; 58,000: 2287 and 2902, 1388 and 1416, 1000 and 919, 617
-// and 487; 25,000 at 0.5: 431 and 485.
-inline bool csgd_walk_split(const csgd_t *d)
+// adds root-level work. A system's sums follow its own size (the forms sum
+// differently, and a system must come out the same alone and in an ensemble). The lines are where the two cross, and twice as
+// high below an opening angle of 0.45: small angles make long tasks, of which the
+// last wave of whole ones leaves most SMs idle. Split against whole, us, disk:
+//   FP64, 12 and 6 tasks per SM (58,368 and 29,184 bodies on 152 SMs)
+//     angle    0.3            0.4            0.5          0.7
+//     19,000    834 and 1132   504 and  606  360 and 385  228 and 211
+//     29,184   1219 and 1570   730 and  832  508 and 521  310 and 265
+//     45,000   1903 and 1948  1083 and 1068  742 and 655  440 and 370
+//     58,000   2481 and 2618  1370 and 1405  927 and 866  552 and 448
+//   FP32-mixed, 8 and 4 tasks per SM (38,912 and 19,456)
+//     10,000    180 and  300   137 and  205  113 and 158   80 and  97
+//     19,000    291 and  395   205 and  252  170 and 189  115 and 109
+//     29,184    399 and  505   277 and  298  223 and 215  145 and 120
+//     45,000    594 and  584   393 and  349  309 and 244  197 and 132
+inline int csgd_split_tasks(int precision, double theta) // per SM
 {
-    return (long long)d->n / 32 + d->n_gal + 1 <= 12LL * d->num_sms;
+    return (theta < 0.45 ? 2 : 1) * (precision == CSG_PREC_FP64 ? 6 : 4);
 }
 inline long long csgd_split_max_bodies(const csgd_t *d, int precision, double theta)
 {
-    return (precision == CSG_PREC_FP64 && !(theta < 0.45) ? 6LL : 12LL) * 32 * d->num_sms;
+    return 32LL * csgd_split_tasks(precision, theta) * d->num_sms;
 }
 inline int csgd_sys_min_n(const csgd_t *d) { return d->n_gal > 1 ? d->sys_min_n : d->n; }
 inline int csgd_sys_max_n(const csgd_t *d) { return d->n_gal > 1 ? d->sys_max_n : d->n; }
+// FP32: whether a launch splits its tasks. Small systems only, and together up to
+// 7 tasks per SM (34,048 bodies): against one warp for a task's segments in turn,
+// at angle 0.5, us: 20,000 bodies 173 and 205, 29,184 224 and 232, 40,000 282 and
+// 248; 16 systems of 2,000 111 and 141.
+inline bool csgd_walk_split(const csgd_t *d, double theta)
+{
+    return (long long)d->n / 32 + d->n_gal + 1 <= 7LL * d->num_sms &&
+           csgd_sys_max_n(d) <= csgd_split_max_bodies(d, CSG_PREC_FP32_MIXED, theta);
+}
 // Scratch of the split walks, allocated on first use outside any capture
 // when `precision` and the size call for it; CSG_OK or CSG_ERR_NOMEM.
 int csgd_prepare_walk(csgd_t *d, int precision);

@@ -882,7 +882,7 @@ extern "C" int csgd_substep(csgd_t *d, double dt, const csgd_force_params *p, in
 
 int csgd_prepare_walk(csgd_t *d, int precision)
 {
-    const bool split = precision == CSG_PREC_FP32_MIXED ? csgd_walk_split(d)
+    const bool split = precision == CSG_PREC_FP32_MIXED ? csgd_walk_split(d, 0.0)
                        : precision == CSG_PREC_FP64     ? csgd_sys_min_n(d) <= csgd_split_max_bodies(d, precision, 0.0)
                                                         : false;
     if (!split || (d->wpart && d->wpart_cap >= d->cap))

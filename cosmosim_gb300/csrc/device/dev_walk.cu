@@ -1554,7 +1554,7 @@ WalkArgs walk_args(csgd_t *d, const csgd_force_params *p)
 
 
 // One walk launch with the state's launch shape.
-void launch_walk(csgd_t *d, const WalkArgs &a, int precision, int exact)
+void launch_walk(csgd_t *d, const WalkArgs &a, int precision, double theta, int exact)
 {
     cudaStream_t s = d->stream;
     const int W = d->walk_warps == 4 ? 4 : 8;
@@ -1577,9 +1577,9 @@ void launch_walk(csgd_t *d, const WalkArgs &a, int precision, int exact)
             k_walk64_exact<true><<<grid, 8 * CSG_WARP, 0, s>>>(b);
         else
             k_walk64_exact<false><<<grid, 8 * CSG_WARP, 0, s>>>(b);
-    } else if (precision == CSG_PREC_FP32_MIXED && !stats && csgd_walk_split(d) &&
+    } else if (precision == CSG_PREC_FP32_MIXED && !stats && csgd_walk_split(d, theta) &&
                d->wpart && d->wpart_cap >= d->n) {
-        // few tasks for the GPU: eight warps per task, one per root child,
+        // small systems, few tasks: eight warps per task, one per child subtree,
         // then the partials added in child order (the same bits as below)
         const long long units = ((long long)d->n / CSG_WARP + d->n_gal + 1) * WSEGS;
         k_walk32_units<<<(int)((units + 3) / 4), 4 * CSG_WARP, 0, s>>>(b, d->wpart,
@@ -1645,10 +1645,10 @@ extern "C" int csgd_gravity_ex(csgd_t *d, const csgd_force_params *p, int exact)
     if (exact) {
         const int saved = d->walk_warps;
         d->walk_warps = 8;
-        launch_walk(d, a, p->precision, 1);
+        launch_walk(d, a, p->precision, p->theta, 1);
         d->walk_warps = saved;
     } else {
-        launch_walk(d, a, p->precision, 0);
+        launch_walk(d, a, p->precision, p->theta, 0);
     }
     return csgd_check(d, cudaGetLastError());
 }
