@@ -62,12 +62,12 @@ ENSEMBLE = dict(n_gal=64, n_min=2000, n_max=50000, size_seed=12, theta=0.5, eps=
                 desc="64 independent exp.-disk galaxies, N log-uniform [2000, 50000], one handle")
 FLOP_PER_INTERACTION = 20  # monopole body-cell interaction: 3 sub, 3 fma d2, rsqrt, 3 mul, 3 fma acc
 # DRAM bytes per body of one k_walk32 launch, from the ncu capture of the
-# 100k merger (profiles/walks.md: 14.47 MB read, 0 written for 100,000 bodies):
+# 100k merger (under profiles/: 14.47 MB read, 0 written for 100,000 bodies):
 # the first touch of the tree and the bodies; the tree stays in L2 during the
 # walk. Other workloads scale it by the body count.
 WALK32_DRAM_BYTES_PER_BODY = 14.465792e6 / 100_000
-# issue slots busy in the same capture (k_walk32, 100k merger): 60.3%
-WALK32_ISSUE_BUSY = 0.603
+# issue slots busy in the same capture (k_walk32, 100k merger): 61.7%
+WALK32_ISSUE_BUSY = 0.617
 WALK32_NOTE = ("20 flop per reference interaction / the walk's time inside the substep (CUDA "
                "events around it, SPH running beside it); peak = FP32 FMA throughput "
                "measured live by csg_measure_fp_peaks (the walk is CUDA-core bound: no dense "
@@ -75,20 +75,19 @@ WALK32_NOTE = ("20 flop per reference interaction / the walk's time inside the s
                "traversal. traffic and issue_slots_busy_ncu are per-launch DRAM bytes and issue "
                "activity from the committed ncu capture of k_walk32 on the 100k merger "
                "(profiles/), traffic scaled by the body count")
-# The FP32 walk of a system with few 32-body tasks for the GPU (at most 12 per
-# SM) runs eight warps per task, one per child subtree
-# (k_walk32_units, then k_walk_sum adds the eight partials): the same bits.
-WALK32_SPLIT_TASKS_PER_SM = 12
+# The FP32 walk of a system with few 32-body tasks for the GPU (at most 5 per SM,
+# 7 below an opening angle of 0.45) runs eight warps per task, one per child
+# subtree (k_walk32_units, then k_walk_sum adds the eight partials).
 # the same two figures for k_walk32_units from its capture on the 20k disk
-# (profiles/walks.md: 2.95 MB read, 0 written; issue 40.6% busy)
-WALK32U_DRAM_BYTES_PER_BODY = 2.95424e6 / 20_000
-WALK32U_ISSUE_BUSY = 0.406
+# (2.96 MB read, 0 written; issue 41.6% busy)
+WALK32U_DRAM_BYTES_PER_BODY = 2.96e6 / 20_000
+WALK32U_ISSUE_BUSY = 0.416
 
 
-def walk32_kernel(torch, n_bodies, n_systems=1):
+def walk32_kernel(torch, n_bodies, theta):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    if n_bodies // 32 + n_systems + 1 <= WALK32_SPLIT_TASKS_PER_SM * sms:
-        return "k_walk32_units + k_walk_sum (gravity walk, a warp per root child)", True
+    if n_bodies <= 32 * sms * 5 or (theta < 0.45 and n_bodies // 32 + 2 <= 7 * sms):
+        return "k_walk32_units + k_walk_sum (gravity walk, a warp per child subtree)", True
     return "k_walk32 (gravity walk)", False
 
 
@@ -907,7 +906,7 @@ def main():
     e2e_value = job_rate(r["n_alive"] * r["e2e_steps"], world, te)
     achieved = FLOP_PER_INTERACTION * f32["interactions"] / f32["walk_s"] / 1e12
     achieved64 = FLOP_PER_INTERACTION * f64["interactions"] / f64["walk_s"] / 1e12
-    walk_name, walk_split = walk32_kernel(torch, cfg["n"])
+    walk_name, walk_split = walk32_kernel(torch, cfg["n"], cfg["theta"])
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": f32["steps"],
         "warmup": args.warmup, "ms_per_step": 1e3 * f32["secs"] / f32["steps"],
@@ -919,8 +918,9 @@ def main():
                        "walk_ms": 1e3 * f64["walk_s"],
                        "walk_tflops": achieved64, "fp64_peak_tflops": fp64_peak,
                        "walk_frac_of_fp64_peak": achieved64 / fp64_peak,
-                       "walk_note": "pair terms in integer arithmetic (no FP64 operation): the "
-                                    "rate may exceed the FP64 peak, which does not bound it"},
+                       "walk_note": "6 FP64 operations a pair (differences and sums; r^2 and "
+                                    "m/r^3 by integers): 20 flop an interaction may exceed "
+                                    "the FP64 peak"},
         "phases_ms": {"fp32_mixed": f32["phases"], "fp64": f64["phases"],
                       "walk_alone_fp32": 1e3 * f32["walk_alone_s"],
                       "walk_alone_fp64": 1e3 * f64["walk_alone_s"],
@@ -939,7 +939,7 @@ def main():
                      "issue_slots_busy_ncu": WALK32U_ISSUE_BUSY if walk_split else WALK32_ISSUE_BUSY,
                      "note": WALK32_NOTE + ("; this workload takes the split walk: traffic and "
                                             "issue from the capture of k_walk32_units on the 20k "
-                                            "disk (profiles/walks.md)"
+                                            "disk (profiles/)"
                                             if walk_split else "")},
         "errors": r["errors"],
         "e2e": {"value": e2e_value, "unit": UNIT, "api": "integrator_step (pinned host Body[])",

@@ -348,23 +348,27 @@ constexpr int CSG_WAIT_POLLS_DEFAULT = 1 << 22;
 // The walks split each task by child subtrees when there are few tasks for the
 // GPU. Above that the whole-task walk already fills the SMs and the split only
 // adds root-level work. A system's sums follow its own size (the forms sum
-// differently, and a system must come out the same alone and in an ensemble). The lines are where the two cross, and twice as
-// high below an opening angle of 0.45: small angles make long tasks, of which the
-// last wave of whole ones leaves most SMs idle. Split against whole, us, disk:
+// differently, and a system must come out the same alone and in an ensemble). The
+// lines are where the two cross at angles 0.3 and 0.4, and, from 0.45 on, at 0.5, the
+// most used (at 0.7 they cross at about 17,000 and 14,000 bodies): small angles make
+// long tasks, of which the last wave of whole ones leaves most SMs idle. Split
+// against whole, us, disk:
 //   FP64, 12 and 6 tasks per SM (58,368 and 29,184 bodies on 152 SMs)
 //     angle    0.3            0.4            0.5          0.7
 //     19,000    834 and 1132   504 and  606  360 and 385  228 and 211
 //     29,184   1219 and 1570   730 and  832  508 and 521  310 and 265
 //     45,000   1903 and 1948  1083 and 1068  742 and 655  440 and 370
 //     58,000   2481 and 2618  1370 and 1405  927 and 866  552 and 448
-//   FP32-mixed, 8 and 4 tasks per SM (38,912 and 19,456)
+//   FP32-mixed, 8 and 5 tasks per SM (38,912 and 24,320)
 //     10,000    180 and  300   137 and  205  113 and 158   80 and  97
 //     19,000    291 and  395   205 and  252  170 and 189  115 and 109
+//     25,000    356 and  457   249 and  281  199 and 205  131 and 114
 //     29,184    399 and  505   277 and  298  223 and 215  145 and 120
 //     45,000    594 and  584   393 and  349  309 and 244  197 and 132
 inline int csgd_split_tasks(int precision, double theta) // per SM
 {
-    return (theta < 0.45 ? 2 : 1) * (precision == CSG_PREC_FP64 ? 6 : 4);
+    const bool small_angle = theta < 0.45;
+    return precision == CSG_PREC_FP64 ? (small_angle ? 12 : 6) : (small_angle ? 8 : 5);
 }
 inline long long csgd_split_max_bodies(const csgd_t *d, int precision, double theta)
 {

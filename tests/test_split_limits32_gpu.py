@@ -1,5 +1,5 @@
 """The FP32-mixed walk on both sides of the sizes up to which a system is summed by child
-subtrees (4 tasks of 32 bodies per SM for opening angles of 0.45 or more, 8 below) and a
+subtrees (5 tasks of 32 bodies per SM for opening angles of 0.45 or more, 8 below) and a
 launch is split by them (7 tasks per SM in all).
 
 Against the FP64 walk, errors relative to the largest acceleration, 1e-5; a system in
@@ -15,7 +15,7 @@ from cosmosim_gb300.abi import BODY_DTYPE
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("per_sm", [4, 7, 8])
+@pytest.mark.parametrize("per_sm", [5, 7, 8])
 @pytest.mark.parametrize("theta", [0.44, 0.45])
 @pytest.mark.parametrize("over", [0, 1])
 def test_both_sides(lib, per_sm, theta, over):
