@@ -65,7 +65,7 @@ FLOP_PER_INTERACTION = 20  # monopole body-cell interaction: 3 sub, 3 fma d2, rs
 # 100k merger (under profiles/: 14.47 MB read, 0 written for 100,000 bodies):
 # the first touch of the tree and the bodies; the tree stays in L2 during the
 # walk. Other workloads scale it by the body count.
-WALK32_DRAM_BYTES_PER_BODY = 14.465792e6 / 100_000
+WALK32_DRAM_BYTES_PER_BODY = 14.470656e6 / 100_000
 # issue slots busy in the same capture (k_walk32, 100k merger): 61.7%
 WALK32_ISSUE_BUSY = 0.617
 WALK32_NOTE = ("20 flop per reference interaction / the walk's time inside the substep (CUDA "
@@ -80,7 +80,7 @@ WALK32_NOTE = ("20 flop per reference interaction / the walk's time inside the s
 # subtree (k_walk32_units, then k_walk_sum adds the eight partials).
 # the same two figures for k_walk32_units from its capture on the 20k disk
 # (2.96 MB read, 0 written; issue 41.6% busy)
-WALK32U_DRAM_BYTES_PER_BODY = 2.96e6 / 20_000
+WALK32U_DRAM_BYTES_PER_BODY = 2.960384e6 / 20_000
 WALK32U_ISSUE_BUSY = 0.416
 
 

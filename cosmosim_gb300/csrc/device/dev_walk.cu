@@ -250,9 +250,9 @@ __global__ void __launch_bounds__(8 * CSG_WARP) k_walk64_exact(WalkArgs a)
 // instructions a step (3574 steps per 32 bodies at 1M, theta 0.5), of which
 // the pair term was a fifth, and 32 dependent steps where a round has one.
 // Classifying 32 cells with one instruction stream and evaluating without a
-// decision per step takes about 25 a cell. FP32-mixed walk, alone, per cell step
-// before -> in rounds: 1M 8.43 -> 4.03 ms, 100k merger 0.66 -> 0.30 ms, 64
-// galaxies 3.40 -> 2.48 ms; 10k-body interaction lists 0.25 -> 0.13 ms. It is
+// decision per step takes about 25 a cell. FP32-mixed walk inside the substep, cell
+// by cell -> in rounds: 1M 8.43 -> 4.17 ms, 100k merger 0.83 -> 0.35 ms, 64
+// galaxies 3.40 -> 2.36 ms; 10k-body interaction lists 0.25 -> 0.13 ms. It is
 // bound by instruction issue (67% busy at 1M); 42% of the lane slots idle in
 // cells that only some lanes reach. Measured and not used: starting the next
 // round's loads before the same round's evaluations (12 more live registers: 1M
@@ -1105,9 +1105,9 @@ __device__ __forceinline__ void put_partial(const WalkArgs &a, int k, int me, do
 // lead, and lanes that take fewer of the current cells run dry less often. The
 // takes of a round reach the lanes by one bit transpose instead of a store per
 // cell and lane.
-constexpr int WS_BLOCKS = 32; // queue length (power of two; 16: 4% slower at 1M)
+constexpr int WS_BLOCKS = 32; // queue length (power of two; 16: 6% slower at 1M)
 constexpr int WS_RES = 21;    // resident warps per SM that the registers are sized for (18 and
-                              // 24: 2-5% slower at 1M)
+                              // 24: 2-6% slower)
 constexpr int WS_CONS = 2;    // consumer warps
 constexpr int WS_LOW = 2;     // blocks the slowest reader wants ahead before a step
 
@@ -1224,8 +1224,8 @@ __device__ __forceinline__ int ws_next(const WsShared &sh, WsReader &r, int tail
     return sh.ids[r.cur * CSG_WARP + j];
 }
 
-// Cells a lane evaluates between two looks at the counters: whole tasks (16:
-// 2-5% faster from 100k bodies on), a split task's units (8: 5% faster at 20k).
+// Cells a lane evaluates between two looks at the counters: whole tasks (16: 1-3%
+// faster than 8 from 100k bodies on), a split task's units (8: 7% faster at 20k).
 constexpr int WS_STEP_TASK = 16, WS_STEP_UNIT = 8;
 
 // Consumer `which`: the blocks which, which + 2, ...
